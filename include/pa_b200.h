@@ -865,6 +865,32 @@ int pa_streams_add_norm(const float* d_src, int src_streams, float* d_dst, int64
                         const float* d_gain, float* d_u, void* d_next, const int32_t* d_row_ids, int elem,
                         pa_stream_t stream);
 
+/* ---- prompt portions on tcgen05 (attention_tc.cu) --------------------------------------------------------------------
+ * pa_masked_attention_gated with tile_kind 4 or 5: bfloat16 softmax attention of prompt portions with the accumulators in
+ *   tensor memory, two (kind 4) or one (kind 5) tiles of 128 query rows per CTA.  d_q_tiles: runs of at most
+ *   pa_masked_attention_tc_tile_tokens(heads, kv_heads, dim, vdim, elem, q_tiles) tokens (0: these sizes are not served); a run
+ *   takes pa_masked_attention_tc_units(heads, kv_heads, q_tiles) CTAs.  PA_ERR_UNSUPPORTED where the form (sigmoid weights, key
+ *   scales, values that are the keys, a long bias table), the page size (a multiple of 16 tokens is served) or an alignment
+ *   rules it out.
+ * pa_latent_attention_expanded: latent attention of prompt portions with the keys and values of every head built beforehand.
+ *   d_k: row r holds head h's dim key columns at h * dim; d_v: its vdim value columns at h * vdim; d_latent: the rot_dim key
+ *   columns all heads share at rot_off, the last columns of a row; kv_rows rows each.  d_q: query of head h at q_off + h *
+ *   (dim + rot_dim).  d_q_tiles [n][4] = first batch row, tokens (at most pa_masked_attention_tc_tile_tokens(1, 1, 64, 64, 2,
+ *   q_tiles)), first row of the sequence in the key buffers, position.  d_out [rows][heads * vdim].
+ * pa_latent_gather: d_items [n][3] = slot, tokens (at most `longest`), first output row: the cached rows of whole sequences
+ *   from a latent pool into d_out [rows][row_bytes].
+ * pa_attention_tc_errors: how many CTAs of these kernels gave up on a wait since the library was loaded (0 unless something is
+ *   broken; their rows hold NaN).  Synchronises. */
+int pa_masked_attention_tc_tile_tokens(int heads, int kv_heads, int dim, int vdim, int elem, int q_tiles);
+int pa_masked_attention_tc_units(int heads, int kv_heads, int q_tiles);
+int pa_latent_attention_expanded(const void* d_q, int64_t q_stride, int q_off, const void* d_k, int64_t k_stride,
+                                 const void* d_latent, int64_t latent_stride, int rot_off, const void* d_v, int64_t v_stride,
+                                 int64_t kv_rows, const int32_t* d_q_tiles, int num_q_tiles, int heads, int dim, int rot_dim,
+                                 int vdim, float scale, const float* d_sink, void* d_out, int q_tiles, pa_stream_t stream);
+int pa_latent_gather(const void* d_pool, const int32_t* d_table, int num_slots, int num_tiles, int total_pages, int tile_size,
+                     int row_bytes, const int32_t* d_items, int num_items, int longest, void* d_out, pa_stream_t stream);
+int pa_attention_tc_errors(int* host_count);
+
 /* ---- token-pair embedding, block passes that add, convolved + turned + normed projections, sinks on the latent ---------
  * pa_embedding_bigram: x[r] = embed[ids[r]] * scale + bigram[b(r)] as float (tables in the activation type), b(r) =
  *   (prev_ids[r] * mul_prev + ids[r] * mul_cur) mod buckets, or row `buckets` (the table has buckets + 1 rows) where

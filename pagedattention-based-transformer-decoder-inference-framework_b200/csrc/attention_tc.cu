@@ -1,0 +1,604 @@
+// attention_tc.cu -- softmax attention of prompt portions on the 5th-generation tensor cores (tcgen05.mma kind::f16, bfloat16
+// operands, float accumulators in TMEM), for the ragged batches of the config-driven models.  Two forms of keys and values:
+//
+//   paged   one row per (token, kv head) in the page pools of masked_attention.cu, located through the page table; causal,
+//           window (with kept first positions) and chunk masks, temperature, soft cap, distance biases, sinks, turned-back and
+//           gated outputs, as described there
+//   dense   keys and values of every head in plain buffers (latent attention in its expanded form, see
+//           pa_latent_attention_expanded): a key is [kn columns of its head | rot columns all heads share]
+//
+// One CTA = NQ tiles of 128 query rows that share every staged key and value byte.  A row is a (query head, token) pair: the
+// heads of one kv head are stacked (TB tokens x hg heads = 128 NQ rows), so with grouped heads a 64-token work item already
+// fills the tensor core's 128 lanes twice and K/V are staged once for four heads; TB rows of one head are a multiple of 32, so a
+// warp's rows have one head.  Keys are consumed in tiles of 64:
+//   warps 0-3 (4-7)  softmax of query tile 0 (1), one thread per row = TMEM lane: tcgen05.ld of its 64 scores, modifiers and
+//                    mask, online softmax in registers, P back to TMEM as bfloat16 over the scores it came from
+//   next NQ warps    one elected thread each issues its tile's  S = Q K^T  (M128 N64, double buffered in TMEM, tile i + 1 under
+//                    the softmax of tile i)  and  O += P V  (A operand from TMEM, V as the MN-major B operand)
+//   last warp        producer: TMA boxes into a ring of 2 or 3 stages, SWIZZLE_128B (16-token boxes per page unit, or 64 rows)
+// O keeps a per-row reference maximum that is raised only when a tile exceeds it by more than 2^8 (P stays below 2^8, and l and
+// O share the reference, so O / l does not depend on it): rows are rescaled a few times instead of once per tile.
+//
+// What bounds it: per 64 keys and 128 rows 4096 / 16 = 512 cycles of ex2 on the MUFU against 512 (dim 128) to 640 (dim 192)
+// cycles of tensor pipe; two tiles per CTA keep both busy at once.  Measured, 4 x 2048 tokens causal: 16 query / 4 kv heads of 128
+// paged 123 us = 560 TFLOP/s (mma.sync kernel 918 us); latent attention at 16 heads of 128 + 64 / 128, five ragged portions
+// 129 us, and 38 us for gathering the rows and building keys and values (absorbed form on mma.sync 1360 us).
+//
+// Every wait is bounded: on a protocol error the CTA raises a flag (pa_attention_tc_errors), waits for its copies, frees its
+// TMEM and leaves NaN in its rows.
+#include "masked_attention.cuh"
+#include "tcgen05_utils.cuh"
+
+namespace pa {
+namespace atc {
+
+using namespace tc;
+
+constexpr int QT = 128, KT = 64;
+
+struct Args {
+    MaskAttnParams p;
+    int tb, hg, hchunks;     // tokens per head block, heads per CTA, head chunks per kv head
+    int qd;                  // columns of a query (multiple of 16); query of head h at q_off + h * qd
+    int kn;                  // dense: key columns per head (multiple of 64); the shared block starts at k2_col of its buffer
+    int k2_col;
+    int upt;                 // paged: 16-token units per page
+    int total_rows;          // rows of the pools: a box there is all zeros (out-of-bounds fill)
+};
+
+__device__ int g_errors;
+
+__host__ __device__ constexpr int q_bytes(int kb) { return kb * QT * 128; }
+__host__ __device__ constexpr int stage_bytes(int kb, int vb) { return (kb + vb) * KT * 128; }
+__host__ __device__ constexpr int stages_for(int kb, int nq) { return nq == 2 || kb == 3 ? 3 : 2; }
+__host__ __device__ constexpr int threads_for(int nq) { return (4 * nq + nq + 1) * 32; }
+__host__ __device__ constexpr int nbar_for(int kb, int nq) { return 2 * stages_for(kb, nq) + 7 * nq; }
+constexpr size_t smem_for(int kb, int vb, int nq) {
+    return (size_t)nq * q_bytes(kb) + stages_for(kb, nq) * stage_bytes(kb, vb) + nbar_for(kb, nq) * 8 + 8 + 4 + 4 * 4 + 1024;
+}
+
+// KB / VB: blocks of 64 columns of a key / a value; MOD: the score has more than a factor (soft cap or distance bias)
+template <int KB, int VB, int NQ, bool DENSE, bool MOD>
+__global__ void __launch_bounds__(threads_for(NQ), NQ == 1 && KB < 3 ? 2 : 1)
+attention_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmK2,
+                    const __grid_constant__ CUtensorMap tmV, const Args a) {
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    constexpr int ST = stages_for(KB, NQ), NBAR = nbar_for(KB, NQ), TMEM_COLS = NQ * 256, D = VB * 64;
+    constexpr int Q_BYTES = q_bytes(KB), K_BYTES = KB * KT * 128, STAGE = stage_bytes(KB, VB);
+    constexpr int W_MMA = 4 * NQ, W_PROD = 5 * NQ;
+    constexpr float kLog2e = 1.4426950408889634f;
+    const MaskAttnParams& p = a.p;
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    const uint32_t q_sm = base, kv_sm = q_sm + NQ * Q_BYTES, bar0 = kv_sm + ST * STAGE;
+    auto kv_full = [&](int s) { return bar0 + s * 8; };
+    auto kv_empty = [&](int s) { return bar0 + (ST + s) * 8; };
+    // two barriers each, tile i on barrier i & 1: with S one tile ahead, waiter and signaller are at most one phase apart
+    auto s_full = [&](int x, int b) { return bar0 + (2 * ST + 7 * x + b) * 8; };
+    auto p_full = [&](int x, int b) { return bar0 + (2 * ST + 7 * x + 2 + b) * 8; };
+    auto o_full = [&](int x, int b) { return bar0 + (2 * ST + 7 * x + 4 + b) * 8; };
+    auto q_ready = [&](int x) { return bar0 + (2 * ST + 7 * x + 6) * 8; };
+    const uint32_t tmem_slot = bar0 + NBAR * 8, fail_sm = tmem_slot + 8, meta_sm = fail_sm + 4;
+    float* bias_sm = reinterpret_cast<float*>(smem_raw + (meta_sm + 16 - smem_u32(smem_raw)));
+
+    auto failed = [&] { return tc_failed(fail_sm); };
+    auto wait = [&](uint32_t bar, uint32_t parity) { tc_wait(bar, parity, fail_sm); };
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < ST; ++s) {
+            mbar_init(kv_full(s), 1);
+            mbar_init(kv_empty(s), NQ);
+        }
+        for (int x = 0; x < NQ; ++x) {
+            for (int b = 0; b < 2; ++b) {
+                mbar_init(s_full(x, b), 1);
+                mbar_init(p_full(x, b), QT);
+                mbar_init(o_full(x, b), 1);
+            }
+            mbar_init(q_ready(x), QT);
+        }
+        asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(fail_sm), "r"(0u) : "memory");
+        mbar_fence_init();
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&tmK));
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&tmV));
+        if (DENSE) asm volatile("prefetch.tensormap [%0];" ::"l"(&tmK2));
+    }
+    if (warp == W_MMA) tmem_alloc(tmem_slot, TMEM_COLS);
+
+    // ---- this CTA's rows and the key tiles they see
+    const int units = p.num_kv_heads * a.hchunks, hpg = p.heads / p.num_kv_heads;
+    const int un = blockIdx.x % units;
+    const int* tile = p.tiles + 4 * (blockIdx.x / units);
+    const int row0 = tile[0], ntok = min(tile[1], a.tb), slot = tile[2], pos0 = tile[3];
+    const int g = un / a.hchunks, h0 = g * hpg + un % a.hchunks * a.hg, hend = min(h0 + a.hg, (g + 1) * hpg);
+    int kmaxs[NQ], nts[NQ], kmax_c = 0;
+#pragma unroll
+    for (int x = 0; x < NQ; ++x) {
+        const int tok0 = x * QT % a.tb;
+        const int last = min(ntok, tok0 + min(a.tb, QT)) - 1;
+        kmaxs[x] = tok0 < ntok && h0 + x * QT / a.tb < hend ? pos0 + last + 1 : 0;
+        kmax_c = max(kmax_c, kmaxs[x]);
+    }
+    const MaSteps steps = ma_steps(p, ma_first_key(p, pos0), kmax_c, KT);
+    int n_tiles = 0;
+#pragma unroll
+    for (int x = 0; x < NQ; ++x) {
+        nts[x] = kmaxs[x] > 0 ? steps.head + (kmaxs[x] + KT - 1) / KT - steps.body0 : 0;
+        n_tiles = max(n_tiles, nts[x]);
+    }
+    if (MOD && p.bias_kind == 2) {
+        const int nh = hend - h0;
+        for (int i = threadIdx.x; i < nh * p.bias_len; i += blockDim.x)
+            bias_sm[i] = p.bias[(int64_t)(i % p.bias_len) * p.heads + h0 + i / p.bias_len];
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    uint32_t tmem_base;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
+
+    if (warp == W_PROD) {
+        if (elect_one()) {
+            const int32_t* trow = DENSE ? nullptr : p.table + ((int64_t)slot * p.num_kv_heads + g) * p.num_tiles;
+            const bool slot_ok = DENSE || (unsigned)slot < (unsigned)p.num_slots;
+            int pgn[4];
+            auto load_pages = [&](int i) {
+                const int u0 = steps.step(i) * 4;
+#pragma unroll
+                for (int uu = 0; uu < 4; ++uu) {
+                    const int u = u0 + uu, t = u / a.upt;
+                    int page = slot_ok && u * 16 < kmax_c && t < p.num_tiles ? __ldg(trow + t) : -1;
+                    if ((unsigned)page >= (unsigned)p.total_pages) page = -1;
+                    pgn[uu] = page >= 0 ? page * p.tile_size + (u - t * a.upt) * 16 : -1;
+                }
+            };
+            if (!DENSE) load_pages(0);
+            int s = 0;
+            uint32_t ph = 1;
+            for (int i = 0; i < n_tiles; ++i) {
+                int r[4];
+                uint32_t mask = 0;
+                if (!DENSE) {
+#pragma unroll
+                    for (int uu = 0; uu < 4; ++uu) {
+                        r[uu] = pgn[uu] >= 0 ? pgn[uu] : a.total_rows;     // unmapped: zeros, and its scores are masked
+                        mask |= (pgn[uu] >= 0 ? 1u : 0u) << uu;
+                    }
+                    if (i + 1 < n_tiles) load_pages(i + 1);
+                }
+                wait(kv_empty(s), ph);
+                if (failed()) break;
+                const uint32_t st = kv_sm + s * STAGE;
+                if (!DENSE) asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(meta_sm + s * 4), "r"(mask) : "memory");
+                mbar_arrive_expect_tx(kv_full(s), STAGE);
+                if (DENSE) {
+                    const int row = slot + steps.step(i) * KT;
+#pragma unroll
+                    for (int kb = 0; kb < KB - 1; ++kb) tma_load_2d(st + kb * 8192, &tmK, h0 * a.kn + kb * 64, row, kv_full(s));
+                    tma_load_2d(st + (KB - 1) * 8192, &tmK2, a.k2_col, row, kv_full(s));
+#pragma unroll
+                    for (int vb = 0; vb < VB; ++vb) tma_load_2d(st + K_BYTES + vb * 8192, &tmV, h0 * D + vb * 64, row, kv_full(s));
+                } else {
+#pragma unroll
+                    for (int uu = 0; uu < 4; ++uu)
+#pragma unroll
+                        for (int kb = 0; kb < KB; ++kb) tma_load_2d(st + kb * 8192 + uu * 2048, &tmK, kb * 64, r[uu], kv_full(s));
+#pragma unroll
+                    for (int uu = 0; uu < 4; ++uu)
+#pragma unroll
+                        for (int vb = 0; vb < VB; ++vb) tma_load_2d(st + K_BYTES + vb * 8192 + uu * 2048, &tmV, vb * 64, r[uu], kv_full(s));
+                }
+                if (++s == ST) {
+                    s = 0;
+                    ph ^= 1u;
+                }
+            }
+            if (failed()) {     // let the copies in flight land before the CTA's shared memory goes away
+                for (int b = 0; b < ST; ++b)
+                    for (uint32_t n = 0; n < 4096 && !mbar_try_wait(kv_full(b), b < s ? ph ^ 1u : ph); ++n) __nanosleep(256);
+            }
+        }
+    } else if (warp >= W_MMA) {
+        constexpr uint32_t kIdescS = idesc_f16(QT, KT, 0, 0, 1), kIdescO = idesc_f16(QT, D, 0, 1, 1);
+        const int x = warp - W_MMA, ntx = nts[x], kmx = kmaxs[x], ksteps_q = a.qd >> 4;
+        auto issue_S = [&](int i, int stage) {
+            if (elect_one()) {
+                const uint32_t st = kv_sm + stage * STAGE, qx = q_sm + x * Q_BYTES;
+#pragma unroll
+                for (int ks = 0; ks < KB * 4; ++ks) {
+                    if (ks >= ksteps_q) break;
+                    const uint64_t da = make_desc(qx + (ks >> 2) * (QT * 128) + (ks & 3) * 32, 16, 1024);
+                    const uint64_t db = make_desc(st + (ks >> 2) * (KT * 128) + (ks & 3) * 32, 16, 1024);
+                    umma_f16(tmem_base + x * 2 * KT + (i & 1) * KT, da, db, kIdescS, ks > 0 ? 1u : 0u);
+                }
+                umma_commit(s_full(x, i & 1));
+            }
+            __syncwarp();
+        };
+        if (n_tiles > 0) {
+            wait(kv_full(0), 0);
+            if (ntx > 0) {
+                wait(q_ready(x), 0);
+                tc_fence_after();
+                issue_S(0, 0);
+            }
+        }
+        int s = 0;
+        uint32_t kv_ph = 0;
+        for (int i = 0; i < n_tiles; ++i) {
+            const int s_next = (s + 1 == ST) ? 0 : s + 1;
+            if (i + 1 < n_tiles) {      // every issuer waits for every stage: its arrival on kv_empty belongs to THIS use of it
+                wait(kv_full(s_next), (s + 1 == ST) ? (kv_ph ^ 1u) : kv_ph);
+                tc_fence_after();
+                if (i + 1 < ntx) issue_S(i + 1, s_next);
+            }
+            if (i < ntx) {
+                const uint32_t st = kv_sm + s * STAGE;
+                const int kp0 = steps.step(i) * KT, nvalid_c = min(KT, kmax_c - kp0);
+                if (nvalid_c & 15) {
+                    // value rows past the last key may hold anything (0 x NaN = NaN): zeros (both issuers write the same)
+                    const int r1 = (nvalid_c + 15) & ~15;
+                    for (int idx = lane; idx < (r1 - nvalid_c) * (D / 8); idx += 32) {
+                        const int r = nvalid_c + idx / (D / 8), c = idx % (D / 8);
+                        const uint32_t addr = st + K_BYTES + (c >> 3) * 8192 + r * 128 + (((c & 7) ^ (r & 7)) << 4);
+                        asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(addr), "r"(0u) : "memory");
+                    }
+                    fence_proxy_async();
+                    __syncwarp();
+                }
+                wait(p_full(x, i & 1), (uint32_t)((i >> 1) & 1));
+                tc_fence_after();
+                if (elect_one()) {
+                    const int ksteps = (min(KT, kmx - kp0) + 15) >> 4;  // keys past the tile's last token contribute nothing
+                    for (int ks = 0; ks < ksteps; ++ks) {
+                        const uint32_t ta = tmem_base + x * 2 * KT + (i & 1) * KT + ks * 8;
+                        const uint64_t db = make_desc(st + K_BYTES + ks * 2048, 8192, 1024);
+                        umma_f16_ts(tmem_base + NQ * 2 * KT + x * D, ta, db, kIdescO, (i > 0 || ks > 0) ? 1u : 0u);
+                    }
+                    umma_commit(o_full(x, i & 1));
+                }
+                __syncwarp();
+            }
+            if (elect_one()) umma_commit(kv_empty(s));
+            __syncwarp();
+            if (++s == ST) {
+                s = 0;
+                kv_ph ^= 1u;
+            }
+        }
+    } else {
+        // ---- softmax: one thread per query row
+        const int x = warp >> 2, qtr = warp & 3;
+        const int wrow = x * QT + qtr * 32;                 // first row of this warp; its rows have one head
+        const int head = min(h0 + wrow / a.tb, hend - 1), tokw = wrow % a.tb, tok = tokw + lane;
+        const int nw = h0 + wrow / a.tb < hend ? ntok : 0;  // a half of a tile may be past the last head: no rows
+        const int qpos = tok < nw ? pos0 + tok : -1;
+        const int nt = nts[x], kmax = kmaxs[x];
+        const uint32_t lane_base = (uint32_t)(qtr * 32) << 16;
+        if (nt > 0) {
+            // the warp's query rows into the swizzled K-major A tile
+            const bf16_t* qsrc = static_cast<const bf16_t*>(p.q) + p.q_off + (int64_t)head * a.qd;
+            const uint32_t qx = q_sm + x * Q_BYTES;
+            const int chunks = a.qd >> 3;
+#pragma unroll 4
+            for (int idx = lane; idx < 32 * chunks; idx += 32) {
+                const int r = idx / chunks, c = idx - r * chunks, rr = qtr * 32 + r;
+                uint4 v = make_uint4(0u, 0u, 0u, 0u);
+                if (tokw + r < nw) v = __ldg(reinterpret_cast<const uint4*>(qsrc + (int64_t)(row0 + tokw + r) * p.q_stride) + c);
+                const uint32_t addr = qx + (c >> 3) * (QT * 128) + rr * 128 + (((c & 7) ^ (rr & 7)) << 4);
+                asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+            }
+            fence_proxy_async();
+            mbar_arrive_cnt(q_ready(x));
+        }
+        const int rlo = qpos >= 0 ? ma_first_key(p, qpos) : 0;
+        const int keep = p.mask_kind == 1 ? p.mask_keep : 0;
+        const float fs = p.scale * (p.head_scale && nt > 0 ? p.head_scale[head] : 1.f);
+        // MOD: scores become log2-domain numbers one by one; else they stay raw and the factor (made positive: a raw score
+        // changes sign with it) enters the exponent's multiply-add
+        const bool flip = !MOD && fs < 0.f;
+        const float fe = MOD ? 1.f : fmaxf(fabsf(fs) * kLog2e, 1e-30f);
+        const float slope = MOD && p.bias_kind == 1 && nt > 0 ? p.bias[head] : 0.f;
+        const float hb = p.head_bias && nt > 0 ? p.head_bias[head] : 0.f;
+        const float inv_cap = MOD && p.softcap > 0.f ? 1.0f / p.softcap : 0.f;
+        const float* brow = bias_sm + (int64_t)(wrow / a.tb) * p.bias_len;
+        float m_ref = -INFINITY, l_run = 0.f;
+        const uint32_t s_addr = tmem_base + lane_base + x * 2 * KT;
+        const uint32_t o_addr = tmem_base + lane_base + NQ * 2 * KT + x * D;
+        int oc[2] = {0, 0};
+        auto ensure_pv = [&](int tp) {      // P.V(tp) is complete; phases are consumed in order, at most two tiles late
+            const int b = tp & 1, k = tp >> 1;
+            if (oc[b] <= k) {
+                wait(o_full(x, b), (uint32_t)(k & 1));
+                oc[b] = k + 1;
+            }
+        };
+        int st_i = 0;
+        uint32_t st_ph = 0;
+#pragma unroll 1
+        for (int i = 0; i < nt; ++i) {
+            const int sb = i & 1, kp0 = steps.step(i) * KT;
+            uint32_t mapped = 15u;
+            if (!DENSE) {
+                wait(kv_full(st_i), st_ph);     // long complete: makes the producer's note about this stage visible
+                asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(mapped) : "r"(meta_sm + st_i * 4) : "memory");
+            }
+            wait(s_full(x, sb), (uint32_t)((i >> 1) & 1));
+            tc_fence_after();
+            uint32_t sr[2][32];
+            tmem_ld32(s_addr + sb * KT, sr[0]);
+            tmem_ld32(s_addr + sb * KT + 32, sr[1]);
+            tmem_wait_ld();
+            const bool full = kp0 + KT - 1 <= qpos && (kp0 >= rlo || kp0 + KT <= keep) && mapped == 15u;
+            if (MOD) {
+#pragma unroll
+                for (int k = 0; k < KT; ++k) {
+                    float v = __uint_as_float(sr[k >> 5][k & 31]) * fs;
+                    if (p.softcap > 0.f) v = p.softcap * ma_tanh(v * inv_cap);
+                    const int dist = qpos - kp0 - k;
+                    if (p.bias_kind == 1) v -= slope * (float)dist;
+                    else if (p.bias_kind == 2) v += brow[max(0, min(dist, p.bias_len - 1))];
+                    sr[k >> 5][k & 31] = __float_as_uint((v + hb) * kLog2e);
+                }
+            } else if (flip) {
+#pragma unroll
+                for (int k = 0; k < KT; ++k) sr[k >> 5][k & 31] ^= 0x80000000u;
+            }
+            if (!full) {
+#pragma unroll
+                for (int k = 0; k < KT; ++k) {
+                    const int j = kp0 + k;
+                    const bool vis = j <= qpos && (j >= rlo || j < keep) && ((mapped >> (k >> 4)) & 1u);
+                    if (!vis) sr[k >> 5][k & 31] = 0xff800000u;
+                }
+            }
+            float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+            for (int k = 0; k < KT; ++k) mx4[k & 3] = fmaxf(mx4[k & 3], __uint_as_float(sr[k >> 5][k & 31]));
+            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * fe;
+            const bool raise = mx > m_ref + 8.f || (m_ref == -INFINITY && mx > -INFINITY);
+            const float m_new = raise ? mx : m_ref;
+            const float corr = raise && m_ref != -INFINITY ? fast_exp2(m_ref - m_new) : 1.f;
+            m_ref = m_new;
+            uint32_t w[32];
+            float ps4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int k = 0; k < 32; ++k) {
+                const int k0 = 2 * k;
+                const float e0 = fast_exp2(fmaf(__uint_as_float(sr[k0 >> 5][k0 & 31]), fe, -m_ref));
+                const float e1 = fast_exp2(fmaf(__uint_as_float(sr[k0 >> 5][(k0 & 31) + 1]), fe, -m_ref));
+                ps4[k & 3] += e0 + e1;
+                w[k] = pack_bf16x2(e0, e1);
+            }
+            const bool dead = m_ref == -INFINITY;       // nothing visible yet: the exponents above are NaN
+            if (i >= 2) ensure_pv(i - 2);
+            if (__any_sync(0xffffffffu, corr != 1.f)) {
+                if (i > 0) ensure_pv(i - 1);
+                tc_fence_after();
+#pragma unroll
+                for (int c4 = 0; c4 < D / 32; ++c4) {
+                    uint32_t orr[32];
+                    tmem_ld32(o_addr + c4 * 32, orr);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) orr[j] = __float_as_uint(__uint_as_float(orr[j]) * corr);
+                    tmem_st32(o_addr + c4 * 32, orr);
+                }
+                l_run *= corr;
+            }
+            if (dead) {
+#pragma unroll
+                for (int k = 0; k < 32; ++k) w[k] = 0u;
+            } else {
+                l_run += (ps4[0] + ps4[1]) + (ps4[2] + ps4[3]);
+            }
+            tmem_st32(s_addr + sb * KT, w);
+            tmem_wait_st();
+            tc_fence_before();
+            mbar_arrive_cnt(p_full(x, sb));
+            if (++st_i == ST) {
+                st_i = 0;
+                st_ph ^= 1u;
+            }
+        }
+        if (nt > 0) {
+            if (nt > 1) ensure_pv(nt - 2);
+            ensure_pv(nt - 1);
+            tc_fence_after();
+            float inv = 1.0f / l_run;
+            if (p.sink) {                               // the reference maximum is in the log2 domain
+                const float sk = p.sink[head] * kLog2e, mn = fmaxf(m_ref, sk);
+                const float c = fast_exp2(m_ref - mn);
+                inv = c / (l_run * c + fast_exp2(sk - mn));
+            }
+            if (failed()) inv = __int_as_float(0x7fc00000);
+            // rows leave through shared memory (this warp's part of its tile's idle query buffer), 64 columns a round, so
+            // that a store instruction writes whole 128-byte row segments
+            const uint32_t ebuf = q_sm + x * Q_BYTES + qtr * (Q_BYTES / 4);
+            const int64_t ostride = (int64_t)p.heads * D;
+            bf16_t* out = static_cast<bf16_t*>(p.out) + (int64_t)(row0 + tokw) * ostride + (int64_t)head * D;
+#pragma unroll 1
+            for (int cb = 0; cb < VB; ++cb) {
+                uint32_t o[2][32];
+                tmem_ld32(o_addr + cb * 64, o[0]);
+                tmem_ld32(o_addr + cb * 64 + 32, o[1]);
+                tmem_wait_ld();
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    float f[8];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(o[j >> 2][(j & 3) * 8 + e]) * inv;
+                    if (p.out_rot && qpos >= 0) {
+#pragma unroll
+                        for (int e = 0; e < 8; e += 2) {
+                            const int col = cb * 64 + j * 8 + e;
+                            const float u = f[e], v = f[e + 1];
+                            f[e] = ma_unturn(p, row0 + tok, col, u, v);
+                            f[e + 1] = ma_unturn(p, row0 + tok, col + 1, v, u);
+                        }
+                    }
+                    if (p.gate && qpos >= 0) {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) f[e] *= ma_gate<bf16_t>(p, row0 + tok, head * D + cb * 64 + j * 8 + e);
+                    }
+                    const uint4 v = bf16x8_pack(f);
+                    asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(ebuf + lane * 128 + ((j ^ (lane & 7)) << 4)),
+                                 "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+                }
+                __syncwarp();
+#pragma unroll
+                for (int it = 0; it < 8; ++it) {
+                    const int r = it * 4 + (lane >> 3), j = lane & 7;
+                    const uint4 v = lds_128(ebuf + r * 128 + ((j ^ (r & 7)) << 4));
+                    if (tokw + r < nw) *reinterpret_cast<uint4*>(out + r * ostride + cb * 64 + j * 8) = v;
+                }
+                __syncwarp();
+            }
+        }
+        tc_fence_before();
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == W_MMA) {
+        tc_fence_after();
+        if (failed()) {
+            __nanosleep(1000000);       // products in flight write TMEM for microseconds at most
+            if (lane == 0) atomicAdd(&g_errors, 1);
+        }
+        tmem_dealloc(tmem_base, TMEM_COLS);
+    }
+}
+
+template <int KB, int VB, int NQ, bool DENSE, bool MOD>
+static int launch(const CUtensorMap& k, const CUtensorMap& k2, const CUtensorMap& v, const Args& a, int ntiles, size_t extra,
+                  cudaStream_t st) {
+    const size_t smem = smem_for(KB, VB, NQ) + extra;
+    const int64_t ctas = (int64_t)ntiles * a.p.num_kv_heads * a.hchunks;
+    if (ctas > 0x7fffffff) return PA_ERR_INVALID_ARG;
+    auto kern = attention_tc_kernel<KB, VB, NQ, DENSE, MOD>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    kern<<<(unsigned)ctas, threads_for(NQ), smem, st>>>(k, k2, v, a);
+    PA_RETURN_LAUNCH_STATUS();
+}
+
+// Rows of a CTA: tokens per head block and heads.  Four (two) heads of a kv head over 64 tokens where there are that many, so
+// that the keys and values of a kv head are staged once for them; a head of its own takes its rows from its tokens.
+static void plan(int hpg, int q_tiles, int& tb, int& hg) {
+    if (hpg >= 3) {
+        tb = 64;
+        hg = 2 * q_tiles;
+    } else if (hpg == 2) {
+        tb = 64 * q_tiles;
+        hg = 2;
+    } else {
+        tb = QT * q_tiles;
+        hg = 1;
+    }
+}
+
+}  // namespace atc
+
+int masked_attention_tc_launch(const MaskAttnParams& p, int ntiles, int q_tiles, cudaStream_t st) {
+    using namespace atc;
+    const bool mod = p.softcap > 0.f || p.bias_kind != 0 || p.head_bias;
+    if ((p.dim != 64 && p.dim != 128) || (p.vdim != 64 && p.vdim != 128) || p.sigm || p.key_scale || p.k_pool == p.v_pool)
+        return PA_ERR_UNSUPPORTED;
+    if (p.tile_size % 16 || p.q_stride % 8 || p.q_off % 8 || (uintptr_t)p.q % 16 || (uintptr_t)p.out % 16 ||
+        (uintptr_t)p.k_pool % 16 || (uintptr_t)p.v_pool % 16)
+        return PA_ERR_UNSUPPORTED;
+    const int64_t rows = (int64_t)p.total_pages * p.tile_size;
+    if (rows >= 0x7fffff00ll) return PA_ERR_UNSUPPORTED;
+    Args a;
+    a.p = p;
+    plan(p.heads / p.num_kv_heads, q_tiles, a.tb, a.hg);
+    a.hchunks = (p.heads / p.num_kv_heads + a.hg - 1) / a.hg;
+    a.qd = p.dim;
+    a.kn = a.k2_col = 0;
+    a.upt = p.tile_size / 16;
+    a.total_rows = (int)rows;
+    const size_t extra = p.bias_kind == 2 ? (size_t)p.bias_len * a.hg * 4 : 0;
+    if (extra > 40 * 1024) return PA_ERR_UNSUPPORTED;
+    CUtensorMap k, v;
+    if (!make_bf16_map(&k, p.k_pool, rows, p.dim, p.dim, 16) || !make_bf16_map(&v, p.v_pool, rows, p.vdim, p.vdim, 16)) return PA_ERR_UNSUPPORTED;
+#define PA_ATC(KB, VB)                                                                                            \
+    if (p.dim == KB * 64 && p.vdim == VB * 64) {                                                                  \
+        if (q_tiles == 2)                                                                                         \
+            return mod ? launch<KB, VB, 2, false, true>(k, k, v, a, ntiles, extra, st) : launch<KB, VB, 2, false, false>(k, k, v, a, ntiles, extra, st); \
+        return mod ? launch<KB, VB, 1, false, true>(k, k, v, a, ntiles, extra, st) : launch<KB, VB, 1, false, false>(k, k, v, a, ntiles, extra, st); \
+    }
+    PA_ATC(1, 1) PA_ATC(1, 2) PA_ATC(2, 1) PA_ATC(2, 2)
+#undef PA_ATC
+    return PA_ERR_UNSUPPORTED;
+}
+
+}  // namespace pa
+
+using namespace pa;
+
+PA_API int pa_masked_attention_tc_tile_tokens(int heads, int kv_heads, int dim, int vdim, int elem, int q_tiles) {
+    if (heads <= 0 || kv_heads <= 0 || heads % kv_heads || elem != 2 || (q_tiles != 1 && q_tiles != 2)) return 0;
+    if ((dim != 64 && dim != 128) || (vdim != 64 && vdim != 128)) return 0;
+    int tb, hg;
+    atc::plan(heads / kv_heads, q_tiles, tb, hg);
+    return tb;
+}
+
+PA_API int pa_masked_attention_tc_units(int heads, int kv_heads, int q_tiles) {
+    if (heads <= 0 || kv_heads <= 0 || heads % kv_heads || (q_tiles != 1 && q_tiles != 2)) return 0;
+    int tb, hg;
+    atc::plan(heads / kv_heads, q_tiles, tb, hg);
+    return kv_heads * ((heads / kv_heads + hg - 1) / hg);
+}
+
+PA_API int pa_latent_attention_expanded(const void* d_q, int64_t q_stride, int q_off, const void* d_k, int64_t k_stride,
+                                        const void* d_latent, int64_t latent_stride, int rot_off, const void* d_v,
+                                        int64_t v_stride, int64_t kv_rows, const int32_t* d_q_tiles, int num_q_tiles, int heads,
+                                        int dim, int rot_dim, int vdim, float scale, const float* d_sink, void* d_out, int q_tiles,
+                                        pa_stream_t stream) {
+    using namespace pa::atc;
+    PA_CHECK_ARG(d_q && d_k && d_latent && d_v && d_q_tiles && d_out && num_q_tiles >= 0 && heads > 0 && kv_rows > 0 &&
+                 (q_tiles == 1 || q_tiles == 2));
+    if ((dim != 64 && dim != 128) || (vdim != 64 && vdim != 128) || rot_dim % 16 || rot_dim <= 0 || rot_dim > 64) return PA_ERR_UNSUPPORTED;
+    if (q_stride % 8 || q_off % 8 || k_stride % 8 || latent_stride % 8 || v_stride % 8 || rot_off % 8) return PA_ERR_UNSUPPORTED;
+    if (((uintptr_t)d_q | (uintptr_t)d_k | (uintptr_t)d_latent | (uintptr_t)d_v | (uintptr_t)d_out) % 16 || kv_rows >= 0x7fffff00ll)
+        return PA_ERR_UNSUPPORTED;
+    if (num_q_tiles == 0) return PA_OK;
+    Args a;
+    MaskAttnParams& p = a.p;
+    p = MaskAttnParams{};
+    p.q = d_q;
+    p.q_stride = q_stride;
+    p.q_off = q_off;
+    p.num_kv_heads = p.heads = heads;
+    p.tiles = d_q_tiles;
+    p.dim = dim + rot_dim;
+    p.vdim = vdim;
+    p.scale = scale;
+    p.out = d_out;
+    p.sink = d_sink;
+    plan(1, q_tiles, a.tb, a.hg);
+    a.hchunks = 1;
+    a.qd = dim + rot_dim;
+    a.kn = dim;
+    a.k2_col = rot_off;
+    a.upt = 1;
+    a.total_rows = (int)kv_rows;
+    CUtensorMap k, k2, v;
+    if (!make_bf16_map(&k, d_k, kv_rows, (uint64_t)heads * dim, k_stride, 64) || !make_bf16_map(&v, d_v, kv_rows, (uint64_t)heads * vdim, v_stride, 64) ||
+        !make_bf16_map(&k2, d_latent, kv_rows, (uint64_t)rot_off + rot_dim, latent_stride, 64))
+        return PA_ERR_UNSUPPORTED;
+    cudaStream_t st = as_stream(stream);
+#define PA_ATC(KB, VB)                                                                            \
+    if (dim == (KB - 1) * 64 && vdim == VB * 64)                                                  \
+        return q_tiles == 2 ? launch<KB, VB, 2, true, false>(k, k2, v, a, num_q_tiles, 0, st)     \
+                            : launch<KB, VB, 1, true, false>(k, k2, v, a, num_q_tiles, 0, st);
+    PA_ATC(2, 1) PA_ATC(2, 2) PA_ATC(3, 1) PA_ATC(3, 2)
+#undef PA_ATC
+    return PA_ERR_UNSUPPORTED;
+}
+
+PA_API int pa_attention_tc_errors(int* host_count) {
+    PA_CHECK_ARG(host_count);
+    return (int)cudaMemcpyFromSymbol(host_count, pa::atc::g_errors, sizeof(int));
+}

@@ -21,6 +21,7 @@
 //   latent_kv_append_kernel  RMS norm (per-channel gain) of the latent columns + rotation of the shared key part, written
 //                            to the row's place in the pool; optionally the norm of the query latent, or the rotation of
 //                            all heads' queries in place, in the same launch
+//   latent_gather_kernel     the cached rows of whole sequences, in order, into a plain buffer (the expanded form of prompt portions)
 //   head_linear_kernel       out[r, h, :] = x[r, h, :] . W[h]  (W [heads][K][N]), any strides
 //   latent_attention_kernel  float tile kernel, any shape, keys optionally split with a merge kernel
 //   latent_attention_mma_kernel  bfloat16 tensor-core kernel (mma.sync), see there
@@ -76,6 +77,25 @@ __global__ void rope_rows_kernel(T* __restrict__ x, int64_t stride, int off, int
     const float u = to_f32<T>(*p0), v = to_f32<T>(*p1);
     *p0 = from_f32<T>(u * c - v * s);
     *p1 = from_f32<T>(v * c + u * s);
+}
+
+// The cached rows of whole sequences, in order, into a plain buffer [rows][kd]: item = (slot, tokens, first output row), one
+// warp per row, 16 bytes a lane.  A position without a page leaves zeros.
+__global__ void latent_gather_kernel(const uint4* __restrict__ pool, const int32_t* __restrict__ table, int num_slots, int num_tiles,
+                                     int total_pages, int tile_size, int words, const int32_t* __restrict__ items, int num_items,
+                                     uint4* __restrict__ out) {
+    const int lane = threadIdx.x & 31;
+    const int* it = items + 3 * blockIdx.y;
+    const int slot = it[0], tokens = it[1], first = it[2];
+    for (int j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); j < tokens; j += gridDim.x * (blockDim.x >> 5)) {
+        int64_t src = -1;
+        if ((unsigned)slot < (unsigned)num_slots && j / tile_size < num_tiles) {
+            const int page = table[(int64_t)slot * num_tiles + j / tile_size];
+            if (page >= 0 && page < total_pages) src = (int64_t)page * tile_size + j % tile_size;
+        }
+        uint4* dst = out + ((int64_t)first + j) * words;
+        for (int w = lane; w < words; w += 32) dst[w] = src >= 0 ? pool[src * words + w] : make_uint4(0u, 0u, 0u, 0u);
+    }
 }
 
 // RMS norm of a row by one warp
@@ -1097,4 +1117,16 @@ PA_API int pa_latent_attention_sink(const void* d_q_lat, int64_t ql_row_stride, 
 PA_API int pa_latent_attention_mma_tile_tokens(int heads, int kv_rank, int rot_dim, int elem) {
     if (heads <= 0 || elem != 2 || !lm_shape_ok(kv_rank, rot_dim)) return 0;
     return kLmRows / (heads < kLmRows ? heads : kLmRows);
+}
+
+PA_API int pa_latent_gather(const void* d_pool, const int32_t* d_table, int num_slots, int num_tiles, int total_pages, int tile_size,
+                            int row_bytes, const int32_t* d_items, int num_items, int longest, void* d_out, pa_stream_t stream) {
+    PA_CHECK_ARG(d_pool && d_table && d_items && d_out && num_slots > 0 && num_tiles > 0 && total_pages > 0 && tile_size > 0);
+    PA_CHECK_ARG(num_items >= 0 && num_items <= 65535 && row_bytes > 0 && longest >= 0);
+    if (row_bytes % 16 || (uintptr_t)d_pool % 16 || (uintptr_t)d_out % 16) return PA_ERR_UNSUPPORTED;
+    if (num_items == 0 || longest == 0) return PA_OK;
+    dim3 grid((unsigned)((longest + 7) / 8), (unsigned)num_items);
+    latent_gather_kernel<<<grid, 256, 0, as_stream(stream)>>>(static_cast<const uint4*>(d_pool), d_table, num_slots, num_tiles, total_pages,
+                                                              tile_size, row_bytes / 16, d_items, num_items, static_cast<uint4*>(d_out));
+    PA_RETURN_LAUNCH_STATUS();
 }

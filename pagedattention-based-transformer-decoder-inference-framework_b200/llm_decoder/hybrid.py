@@ -267,6 +267,7 @@ class DiffAttentionMixer:
         return c.model._linear(out, self.w_o)
 
 
+EXPAND_FROM = 128         # portions at least this long run latent attention on keys and values built per head (bfloat16)
 ROPE_PAIRING = {"neighbours": 0, "halves": 1}
 
 
@@ -349,6 +350,14 @@ class LatentAttentionMixer:
         self.mma_tokens = 0
         if self.dim % 8 == 0 and qd % 8 == 0:
             self.mma_tokens = model._lib.pa_latent_attention_mma_tile_tokens(H, self.kv_rank, self.rot_dim, _ELEM[model.act_dtype])
+        # prompt portions with keys and values built per head (tcgen05): tokens per tile with two and with one query tile per CTA
+        self.tc_tokens, self.w_ukv = (0, 0), None
+        lib, elem = model._lib, _ELEM[model.act_dtype]
+        q_cols = H * qd if self.q_latent else int(self.w_in.shape[0])       # row stride of the queries: 16-byte rows
+        if (self.mma_tokens and 16 <= self.rot_dim <= 64 and self.rot_dim % 16 == 0 and self.kv_rank % 8 == 0 and q_cols % 8 == 0 and
+                lib.pa_masked_attention_tc_tile_tokens(1, 1, self.dim, self.vdim, elem, 2)):
+            self.tc_tokens = tuple(lib.pa_masked_attention_tc_tile_tokens(1, 1, self.dim, self.vdim, elem, q) for q in (2, 1))
+            self.w_ukv = model._weight_raw(torch.cat([W[prefix + "uk"], W[prefix + "uv"]], 0))        # [H * (dim + vdim)][kv_rank]
 
     def alloc_state(self, model):
         self.kv = model.states.add_kv_layer(1, self.kd, 0, _KV[model.act_dtype])
@@ -373,7 +382,24 @@ class LatentAttentionMixer:
                                   _cabi.stream()), "pa_head_linear")
         return out
 
-    def _attend(self, c, q, ql, lat, mma):
+    def _attend_expanded(self, c, q, out):
+        """The prompt portions that build the keys and values of their whole sequences: per head a key of dim + rot_dim and a value
+        of vdim columns instead of kv_rank + rot_dim and kv_rank, for one product over the cached rows."""
+        b, lib, kv, s, H = c.batch, c.lib, self.kv, _cabi.stream(), self.heads
+        pt = kv.page_table_
+        q_tiles = 2 if b.count_tiles(self.tc_tokens[0], EXPAND_FROM) * H >= c.model.sm_count else 1
+        for items, nitems, longest, rows, tiles, ntiles in b.whole_sequences(EXPAND_FROM, self.tc_tokens[2 - q_tiles]):
+            lat = c.empty(rows, self.kd)
+            _chk(lib.pa_latent_gather(kv.key_buffer_.data_ptr(), pt.device_data().data_ptr(), pt.num_beams_, pt.num_tiles_,
+                                      kv.total_pages_, kv.tile_size_, self.kd * c.elem, items.data_ptr(), nitems, longest,
+                                      lat.data_ptr(), s), "pa_latent_gather")
+            built = torch.nn.functional.linear(lat[:, :self.kv_rank], self.w_ukv)
+            _chk(lib.pa_latent_attention_expanded(q.data_ptr(), q.stride(0), 0, built.data_ptr(), built.stride(0), lat.data_ptr(),
+                                                  self.kd, self.kv_rank, built.data_ptr() + H * self.dim * c.elem, built.stride(0),
+                                                  rows, tiles.data_ptr(), ntiles, H, self.dim, self.rot_dim, self.vdim, self.scale,
+                                                  _cabi.ptr(self.sink), out.data_ptr(), q_tiles, s), "pa_latent_attention_expanded")
+
+    def _attend(self, c, q, ql, lat, mma, without=0):
         """Launch the attention kernels over this step's tiles (prompt portions, then single decoded tokens).  Returns
         False when the tensor-core kernel refuses the operands (nothing was written that the float kernel does not
         write again)."""
@@ -381,7 +407,7 @@ class LatentAttentionMixer:
         pt = kv.page_table_
         table = pt.device_data()
         rows_per_cta = 64 if mma else 32
-        for kind, group in b.query_tiles(self.mma_tokens if mma else self.tile_tokens).items():
+        for kind, group in b.query_tiles(self.mma_tokens if mma else self.tile_tokens, without=without).items():
             if group is None:
                 continue
             tiles, ntiles, longest = group
@@ -437,21 +463,26 @@ class LatentAttentionMixer:
         proj = c.model._linear(h, self.w_in)
         q = self._queries(c, proj)
         kvr = self.kv_rank
-        ql = self._head_linear(c, q, q.stride(0), self.qd, self.w_uk, self.dim, kvr)          # [H, R, kv_rank]
-        lat = c.empty(H, R, kvr)
-        if self.mma_tokens > 0 and not self._attend(c, q, ql, lat, True):
-            self.mma_tokens = 0         # a stride or an alignment the tensor-core kernel does not take: the float kernel
-        if self.mma_tokens == 0:
-            self._attend(c, q, ql, lat, False)
-        if self.gate != "head":
+        expand = EXPAND_FROM if self.w_ukv is not None and c.batch.whole_sequences(EXPAND_FROM, self.tc_tokens[0]) else 0
+        if expand and all(c.batch._expands(p, expand) for p in c.batch.portions):
+            ov = c.empty(R, H * self.vdim)
+        else:
+            ql = self._head_linear(c, q, q.stride(0), self.qd, self.w_uk, self.dim, kvr)          # [H, R, kv_rank]
+            lat = c.empty(H, R, kvr)
+            if self.mma_tokens > 0 and not self._attend(c, q, ql, lat, True, expand):
+                self.mma_tokens = 0         # a stride or an alignment the tensor-core kernel does not take: the float kernel
+            if self.mma_tokens == 0:
+                self._attend(c, q, ql, lat, False, expand)
             ov = self._head_linear(c, lat, kvr, R * kvr, self.w_uv, kvr, self.vdim, by_row=True).view(R, H * self.vdim)
+        if expand:      # its rows of ov; what the product above left there came from no query
+            self._attend_expanded(c, q, ov)
+        if self.gate != "head":
             if self.gate == "elements":
                 _chk(lib.pa_gate_rows(ov.data_ptr(), ov.stride(0), proj.data_ptr() + self.g_off * c.elem, proj.stride(0),
                                       H * self.vdim, R, ov.data_ptr(), ov.stride(0), c.elem, s), "pa_gate_rows")
             return c.model._linear(ov, self.w_o)
-        ov = self._head_linear(c, lat, kvr, R * kvr, self.w_uv, kvr, self.vdim)               # [H, R, vdim]
         og = c.empty(R, H * self.vdim)
-        _chk(lib.pa_head_gate(ov.data_ptr(), self.vdim, R * self.vdim, proj.data_ptr() + self.g_off * c.elem, proj.stride(0),
+        _chk(lib.pa_head_gate(ov.data_ptr(), H * self.vdim, self.vdim, proj.data_ptr() + self.g_off * c.elem, proj.stride(0),
                               H, self.vdim, R, og.data_ptr(), c.elem, s), "pa_head_gate")
         return c.model._linear(og, self.w_o)
 
@@ -633,6 +664,12 @@ class MaskedAttention:
             raise ValueError(f"unknown distance bias {bias!r}")
         self.tile_tokens = model._lib.pa_masked_attention_tile_tokens(self.heads, self.kv_heads)
         self.mma_tokens = model._lib.pa_masked_attention_mma_tile_tokens(self.dim, self.vdim, _ELEM[model.act_dtype])
+        # prompt portions on tcgen05: (tokens per tile, CTAs per tile, tile kind) with two and with one query tile per CTA
+        self.tc_plans = [(model._lib.pa_masked_attention_tc_tile_tokens(self.heads, self.kv_heads, self.dim, self.vdim,
+                                                                        _ELEM[model.act_dtype], q),
+                          model._lib.pa_masked_attention_tc_units(self.heads, self.kv_heads, q), kind) for q, kind in ((2, 4), (1, 5))]
+        if self.sigmoid or self.keys_as_values or self.tc_plans[0][0] == 0:
+            self.tc_plans = []
         self.alloc_state(model)
 
     def alloc_state(self, model):
@@ -704,12 +741,19 @@ class MaskedAttention:
         gate = (proj, off + self.qkv_cols) if self.gate else (None, 0)
         proj, off = self._prepare(c, proj, off)
         out = c.empty(c.R, self.heads * self.vdim)
+        if self.tc_plans:
+            # two query tiles per CTA stage every key once for 256 rows; one where that leaves SMs without a CTA
+            tokens, units, kind = self.tc_plans[0]
+            if c.batch.count_tiles(tokens, MMA_FROM) * units < c.model.sm_count:
+                tokens, units, kind = self.tc_plans[1]
+            if self._attend_tiles(c, proj, off, gate, out, tokens, kind):
+                return out
         if not self._attend_tiles(c, proj, off, gate, out, self.mma_tokens):
             self.mma_tokens = 0     # a stride or an alignment the tensor-core kernel refuses: the float kernels
             self._attend_tiles(c, proj, off, gate, out, 0)
         return out
 
-    def _attend_tiles(self, c, proj, off, gate, out, mma_tokens):
+    def _attend_tiles(self, c, proj, off, gate, out, mma_tokens, portion_kind=2):
         b, lib, kv, s = c.batch, c.lib, self.kv, _cabi.stream()
         pt = kv.page_table_
         table = pt.device_data()
@@ -719,6 +763,8 @@ class MaskedAttention:
             if group is None:
                 continue
             tiles, ntiles, _longest = group
+            if kind == 2:
+                kind = portion_kind
             # decoded tokens of a batch with at least one (token, kv head) pair per SM: heads as rows on the tensor cores
             if kind == 1 and mma_tokens and ntiles * self.kv_heads >= c.model.sm_count:
                 kind = 3

@@ -61,16 +61,19 @@ class RaggedBatch:
         self.device = device
         self._cache = {}
 
-    def query_tiles(self, tile_tokens, big_tokens=0, big_from=0):
+    def query_tiles(self, tile_tokens, big_tokens=0, big_from=0, without=0):
         """The work lists of the attention kernels: every portion cut into runs of consecutive tokens, as [n, 4] int32
         device tensors (first row, tokens, slot, first position).  Three lists, keyed by the kernel's tile kind:
         1 = portions of ONE token (decoded tokens: the streaming kernel), 2 = portions of at least `big_from` tokens in
         runs of `big_tokens` (the tensor-core kernel; none when big_tokens is 0), 0 = the rest in runs of `tile_tokens`.
-        Each comes as (tensor, count, longest context) or None."""
-        key = ("qt", tile_tokens, big_tokens, big_from)
+        Each comes as (tensor, count, longest context) or None.  without: leave out the portions that whole_sequences(without)
+        serves."""
+        key = ("qt", tile_tokens, big_tokens, big_from, without)
         if key not in self._cache:
             groups = {0: [], 1: [], 2: []}
             for p in self.portions:
+                if without and self._expands(p, without):
+                    continue
                 groups[1 if p[1] == 1 else 2 if big_tokens and p[1] >= big_from else 0].append(p)
             out = {}
             for kind, portions in groups.items():
@@ -78,7 +81,47 @@ class RaggedBatch:
                     out[kind] = None
                     continue
                 runs = _runs(portions, big_tokens if kind == 2 else tile_tokens)
+                if kind == 2:       # longest context first: the CTAs of a launch end together
+                    runs = runs[np.argsort(-(runs[:, 5] + runs[:, 1]), kind="stable")]
                 out[kind] = (self._upload(runs[:, [0, 1, 2, 5]]), len(runs), int((runs[:, 5] + runs[:, 1]).max()))
+            self._cache[key] = out
+        return self._cache[key]
+
+    def count_tiles(self, tokens, at_least):
+        """How many runs of at most `tokens` tokens the portions of at least `at_least` tokens make."""
+        key = ("ct", tokens, at_least)
+        if key not in self._cache:
+            self._cache[key] = sum(-(-p[1] // tokens) for p in self.portions if p[1] >= at_least)
+        return self._cache[key]
+
+    EXPAND_MOST = 65536         # cached tokens whose keys and values are built at a time
+
+    def _expands(self, p, at_least):
+        """Whether the keys and values of ALL tokens of a portion's sequence are worth building for its queries: `at_least` new
+        tokens, and not many times as many cached ones."""
+        return p[1] >= at_least and p[3] + p[1] <= min(16 * p[1], self.EXPAND_MOST)
+
+    def whole_sequences(self, at_least, tokens):
+        """The portions that _expands picks, in groups of at most EXPAND_MOST tokens of context: per group ([n, 3] int32 items (slot,
+        tokens, first row), n, longest, rows, [m, 4] query tiles of at most `tokens` tokens (first batch row, tokens, first row of
+        the sequence, position), m), longest context first."""
+        key = ("ws", at_least, tokens)
+        if key not in self._cache:
+            groups = []
+            for p in self.portions:
+                if not self._expands(p, at_least):
+                    continue
+                total = p[3] + p[1]
+                if not groups or groups[-1][1] + total > self.EXPAND_MOST:
+                    groups.append([[], 0])
+                groups[-1][0].append((p, groups[-1][1]))
+                groups[-1][1] += total
+            out = []
+            for members, rows in groups:
+                items = np.array([(p[2], p[3] + p[1], r) for p, r in members], dtype=np.int32)
+                runs = _runs([(p[0], p[1], r, p[3]) for p, r in members], tokens)
+                runs = runs[np.argsort(-(runs[:, 5] + runs[:, 1]), kind="stable")]
+                out.append((self._upload(items), len(items), int(items[:, 1].max()), rows, self._upload(runs[:, [0, 1, 2, 5]]), len(runs)))
             self._cache[key] = out
         return self._cache[key]
 
