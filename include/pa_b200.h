@@ -880,7 +880,7 @@ int pa_streams_add_norm(const float* d_src, int src_streams, float* d_dst, int64
  * pa_latent_gather: d_items [n][3] = slot, tokens (at most `longest`), first output row: the cached rows of whole sequences
  *   from a latent pool into d_out [rows][row_bytes].
  * pa_attention_tc_errors: how many CTAs of these kernels gave up on a wait since the library was loaded (0 unless something is
- *   broken; their rows hold NaN).  Synchronises. */
+ *   broken; their rows hold NaN).  Synchronises.  pa_moe_tc_errors: the same for the grouped expert products on tcgen05. */
 int pa_masked_attention_tc_tile_tokens(int heads, int kv_heads, int dim, int vdim, int elem, int q_tiles);
 int pa_masked_attention_tc_units(int heads, int kv_heads, int q_tiles);
 int pa_latent_attention_expanded(const void* d_q, int64_t q_stride, int q_off, const void* d_k, int64_t k_stride,
@@ -890,6 +890,7 @@ int pa_latent_attention_expanded(const void* d_q, int64_t q_stride, int q_off, c
 int pa_latent_gather(const void* d_pool, const int32_t* d_table, int num_slots, int num_tiles, int total_pages, int tile_size,
                      int row_bytes, const int32_t* d_items, int num_items, int longest, void* d_out, pa_stream_t stream);
 int pa_attention_tc_errors(int* host_count);
+int pa_moe_tc_errors(int* host_count);
 
 /* ---- token-pair embedding, block passes that add, convolved + turned + normed projections, sinks on the latent ---------
  * pa_embedding_bigram: x[r] = embed[ids[r]] * scale + bigram[b(r)] as float (tables in the activation type), b(r) =

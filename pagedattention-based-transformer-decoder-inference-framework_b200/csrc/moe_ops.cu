@@ -605,6 +605,10 @@ __global__ void __launch_bounds__(kSkWarps * 32) grouped_skinny_kernel(const bf1
     }
 }
 
+// moe_tc.cu: the tcgen05 form of the grouped products (PA_ERR_UNSUPPORTED: operands that stay on the kernels here)
+int grouped_tc_launch(int mode, const void* A, int64_t lda, const void* W, int K, int n_out, int experts, const int32_t* order,
+                      const float* a_scale, int top, const int32_t* offsets, int pairs, int act, void* out, cudaStream_t st);
+
 static bool mma_ok(const void* A, int64_t lda, const void* W, int K) {
     return K % 8 == 0 && lda % 8 == 0 && (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0;
 }
@@ -691,6 +695,8 @@ PA_API int pa_moe_gate_up_act(const void* d_h, int64_t ldh, const void* d_w_gate
         PA_RETURN_LAUNCH_STATUS();
     }
     if (elem == 2 && mma_ok(d_h, ldh, d_w_gate_up, width)) {
+        const int st = grouped_tc_launch(0, d_h, ldh, d_w_gate_up, width, ff, experts, d_order, d_sel_w, top, d_meta, pairs, act, d_act, as_stream(stream));
+        if (st != PA_ERR_UNSUPPORTED) return st;
         grouped_mma_kernel<0><<<grid, 128, 0, as_stream(stream)>>>(
             static_cast<const bf16_t*>(d_h), ldh, static_cast<const bf16_t*>(d_w_gate_up), width, ff, d_order, d_sel_w, top,
             tiles, static_cast<bf16_t*>(d_act), nullptr, act);
@@ -724,6 +730,8 @@ PA_API int pa_moe_up(const void* d_h, int64_t ldh, const void* d_w_up, int width
         PA_RETURN_LAUNCH_STATUS();
     }
     if (elem == 2 && mma_ok(d_h, ldh, d_w_up, width)) {
+        const int st = grouped_tc_launch(2, d_h, ldh, d_w_up, width, ff, experts, d_order, d_sel_w, top, d_meta, pairs, act, d_act, as_stream(stream));
+        if (st != PA_ERR_UNSUPPORTED) return st;
         grouped_mma_kernel<2><<<dim3(nt, (unsigned)((ff + 127) / 128)), 128, 0, as_stream(stream)>>>(
             static_cast<const bf16_t*>(d_h), ldh, static_cast<const bf16_t*>(d_w_up), width, ff, d_order, d_sel_w, top, tiles,
             static_cast<bf16_t*>(d_act), nullptr, act);
@@ -749,6 +757,8 @@ PA_API int pa_moe_down(const void* d_act, const void* d_w_down, int ff, int widt
         PA_RETURN_LAUNCH_STATUS();
     }
     if (elem == 2 && mma_ok(d_act, ff, d_w_down, ff)) {
+        const int st = grouped_tc_launch(1, d_act, ff, d_w_down, ff, width, experts, d_order, nullptr, 1, d_meta, pairs, 0, d_out_pairs, as_stream(stream));
+        if (st != PA_ERR_UNSUPPORTED) return st;
         dim3 g2((unsigned)pa_moe_max_tiles(pairs, experts), (unsigned)((width + 127) / 128));
         grouped_mma_kernel<1><<<g2, 128, 0, as_stream(stream)>>>(
             static_cast<const bf16_t*>(d_act), (int64_t)ff, static_cast<const bf16_t*>(d_w_down), ff, width, d_order, nullptr, 1,

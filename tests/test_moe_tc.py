@@ -1,0 +1,60 @@
+"""The tcgen05 form of the grouped expert products (csrc/moe_tc.cu) alone, against the same products in float64: experts without
+pairs, with less than a row tile and with several, output sizes that end inside a strip of 128 or 256, inner sizes that end
+inside a stage of 64, with and without a weight on the input, gate / up pairs and single products with each activation.
+
+Bound of the first product: gate, up and their product are rounded to bfloat16 (half a unit each, 2^-9 relative), relu squared and
+gate * up double a relative error: 4 * 2^-9 of the largest result, and as much again for values next to a rounding border.  The second
+product is float on bfloat16 operands: 1e-5 of sum |a| |w|."""
+import ctypes
+
+import pytest
+import torch
+
+BF = torch.bfloat16
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,experts,top,width,ff", [(700, 3, 2, 192, 264), (257, 2, 1, 64, 520), (1300, 20, 2, 136, 128), (129, 1, 1, 72, 8)])
+@pytest.mark.parametrize("act,gated,weighted", [(0, True, False), (1, True, True), (2, False, False)])
+def test_grouped_products(rows, experts, top, width, ff, act, gated, weighted):
+    from llm_decoder import _cabi
+    lib, dev, s = _cabi.lib(), torch.device("cuda"), _cabi.stream
+    g = torch.Generator().manual_seed(rows + act)
+    pairs = rows * top
+    h = torch.randn(rows, width, generator=g).to(BF)
+    wu = (torch.randn(experts, (2 if gated else 1) * ff, width, generator=g) / width ** 0.5).to(BF)
+    wd = (torch.randn(experts, width, ff, generator=g) / ff ** 0.5).to(BF)
+    ids = torch.randint(0, experts, (pairs,), generator=g)
+    if experts > 2:
+        ids[ids == 1] = 0                       # one expert without pairs
+        ids[ids == 2] = 0
+        ids[:5] = 2                             # one with five
+    sel_w = torch.rand(pairs, generator=g) + 0.1
+    idd, swd = ids.to(torch.int32).to(dev), sel_w.to(dev)
+    order = torch.empty(pairs, dtype=torch.int32, device=dev)
+    meta = torch.empty(lib.pa_moe_meta_ints(pairs, experts), dtype=torch.int32, device=dev)
+    _cabi.check(lib.pa_moe_sort(idd.data_ptr(), pairs, experts, order.data_ptr(), meta.data_ptr(), s()), "sort")
+    hd, wud, wdd = h.to(dev), wu.to(dev), wd.to(dev)
+    mid = torch.full((pairs, ff), float("nan"), device=dev, dtype=BF)
+    out = torch.full((pairs, width), float("nan"), device=dev)
+    fn = lib.pa_moe_gate_up_act if gated else lib.pa_moe_up
+    _cabi.check(fn(hd.data_ptr(), width, wud.data_ptr(), width, ff, experts, order.data_ptr(), swd.data_ptr() if weighted else None, top,
+                   meta.data_ptr(), pairs, act, mid.data_ptr(), 2, s()), "up")
+    _cabi.check(lib.pa_moe_down(mid.data_ptr(), wdd.data_ptr(), ff, width, experts, order.data_ptr(), meta.data_ptr(), pairs, out.data_ptr(), 2,
+                                s()), "down")
+    o = order.long().cpu()
+    assert sorted(o.tolist()) == list(range(pairs)) and bool((ids[o][1:] >= ids[o][:-1]).all())
+    a = h[o // top].double() * (sel_w[o].double()[:, None] if weighted else 1.0)
+    want_mid, want = torch.empty(pairs, ff, dtype=torch.float64), torch.empty(pairs, width, dtype=torch.float64)
+    bound = torch.empty(pairs, width, dtype=torch.float64)
+    f = [lambda v: v * torch.sigmoid(v), lambda v: v.clamp(min=0), lambda v: v.clamp(min=0) ** 2][act]
+    got_mid = mid.cpu()
+    for e in range(experts):
+        r = ids[o] == e
+        p = a[r] @ wu[e].double().T
+        want_mid[r] = f(p[:, :ff]) * p[:, ff:] if gated else f(p)
+        want[r], bound[r] = got_mid[r].double() @ wd[e].double().T, got_mid[r].double().abs() @ wd[e].double().abs().T
+    assert (got_mid.double() - want_mid).abs().max() < 8 * 2.0 ** -9 * want_mid.abs().max()
+    assert ((out.double().cpu()[o] - want).abs() <= 1e-5 * bound + 1e-30).all()
+    n = ctypes.c_int(-1)
+    assert lib.pa_moe_tc_errors(ctypes.byref(n)) == 0 and n.value == 0
