@@ -45,7 +45,9 @@ __device__ __forceinline__ void rt_load(const T* p, float (&f)[16 / sizeof(T)]) 
     }
 }
 
-template <typename T, bool VEC>
+// RPW: token rows per warp.  The weights cross L1 once per warp, which bounds many rows: four rows a warp (8192 rows of 2048 over
+// 8 experts 20 us, one row a warp 49 us); one where that would leave SMs without a CTA.
+template <typename T, bool VEC, int RPW>
 __global__ void __launch_bounds__(128) router_topk_kernel(const T* __restrict__ h, const float* __restrict__ w_router,
                                                           const float* __restrict__ bias,
                                                           const float* __restrict__ w_shared_gate, int rows, int width,
@@ -53,61 +55,73 @@ __global__ void __launch_bounds__(128) router_topk_kernel(const T* __restrict__ 
                                                           int ngroups, int keep, const float* __restrict__ choice_bias,
                                                           int32_t* __restrict__ sel_id, float* __restrict__ sel_w,
                                                           float* __restrict__ shared_gate) {
-    extern __shared__ float sc[];                     // [warps][experts]
+    extern __shared__ float sc[];                     // [warps][RPW][experts]
     constexpr int VN = 16 / sizeof(T);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int row = blockIdx.x * (blockDim.x >> 5) + warp;
-    if (row >= rows) return;
-    float* s = sc + warp * experts;
-    const T* hr = h + (int64_t)row * width;
+    const int row0 = (blockIdx.x * (blockDim.x >> 5) + warp) * RPW;
+    if (row0 >= rows) return;
+    const int nrow = min(RPW, rows - row0);
+    const T* hr[RPW];                                 // rows past the last one read the last one and are not written
+#pragma unroll
+    for (int q = 0; q < RPW; ++q) hr[q] = h + (int64_t)min(row0 + q, rows - 1) * width;
     const int nvec = experts + (w_shared_gate ? 1 : 0);
     for (int e0 = 0; e0 < nvec; e0 += kRtGroup) {
-        float acc[kRtGroup];
+        float acc[kRtGroup][RPW];
         const float* wr[kRtGroup];
 #pragma unroll
         for (int c = 0; c < kRtGroup; ++c) {
-            acc[c] = 0.f;
             const int e = e0 + c;
-            wr[c] = e < experts ? w_router + (int64_t)e * width : e < nvec ? w_shared_gate : nullptr;
+#pragma unroll
+            for (int q = 0; q < RPW; ++q) acc[c][q] = 0.f;
+            wr[c] = e < experts ? w_router + (int64_t)e * width : e < nvec ? w_shared_gate : w_router;
         }
-        if (VEC) {
+        if (VEC) {                                    // vectors past the last one read the first and are dropped below
             for (int j = lane * VN; j < width; j += 32 * VN) {
-                float hv[VN];
-                rt_load<T>(hr + j, hv);
+                float hv[RPW][VN];
+#pragma unroll
+                for (int q = 0; q < RPW; ++q) rt_load<T>(hr[q] + j, hv[q]);
 #pragma unroll
                 for (int c = 0; c < kRtGroup; ++c) {
-                    if (!wr[c]) continue;
 #pragma unroll
                     for (int i = 0; i < VN; i += 4) {
                         const float4 w4 = *reinterpret_cast<const float4*>(wr[c] + j + i);
-                        acc[c] = fmaf(hv[i], w4.x, acc[c]);
-                        acc[c] = fmaf(hv[i + 1], w4.y, acc[c]);
-                        acc[c] = fmaf(hv[i + 2], w4.z, acc[c]);
-                        acc[c] = fmaf(hv[i + 3], w4.w, acc[c]);
+#pragma unroll
+                        for (int q = 0; q < RPW; ++q) {
+                            acc[c][q] = fmaf(hv[q][i], w4.x, acc[c][q]);
+                            acc[c][q] = fmaf(hv[q][i + 1], w4.y, acc[c][q]);
+                            acc[c][q] = fmaf(hv[q][i + 2], w4.z, acc[c][q]);
+                            acc[c][q] = fmaf(hv[q][i + 3], w4.w, acc[c][q]);
+                        }
                     }
                 }
             }
         } else {
             for (int j = lane; j < width; j += 32) {
-                const float hv = to_f32<T>(hr[j]);
 #pragma unroll
-                for (int c = 0; c < kRtGroup; ++c)
-                    if (wr[c]) acc[c] = fmaf(hv, wr[c][j], acc[c]);
+                for (int q = 0; q < RPW; ++q) {
+                    const float hv = to_f32<T>(hr[q][j]);
+#pragma unroll
+                    for (int c = 0; c < kRtGroup; ++c) acc[c][q] = fmaf(hv, wr[c][j], acc[c][q]);
+                }
             }
         }
 #pragma unroll
         for (int c = 0; c < kRtGroup; ++c) {
             const int e = e0 + c;
             if (e >= nvec) continue;
-            const float v = warp_sum(acc[c]);
-            if (lane == 0) {
-                if (e < experts) s[e] = bias ? v + bias[e] : v;
-                else shared_gate[row] = sigmoid_f32(v);
+#pragma unroll
+            for (int q = 0; q < RPW; ++q) {
+                const float v = warp_sum(acc[c][q]);
+                if (lane != q || q >= nrow) continue;
+                if (e < experts) sc[(warp * RPW + q) * experts + e] = bias ? v + bias[e] : v;
+                else shared_gate[row0 + q] = sigmoid_f32(v);
             }
         }
     }
     __syncwarp();
-    if (lane == 0) {
+    if (lane < nrow) {                                // a lane per row
+        const int row = row0 + lane;
+        float* s = sc + (warp * RPW + lane) * experts;
         if (score_fn == 0) {
             for (int e = 0; e < experts; ++e) s[e] = sigmoid_f32(s[e]);
         } else if (score_fn == 1) {
@@ -635,16 +649,18 @@ PA_API int pa_router_topk_biased(const void* d_h, const float* d_w_router, const
     PA_CHECK_ARG(top > 0 && top <= experts && score_fn >= 0 && score_fn <= 2 && (!d_w_shared_gate || d_shared_gate));
     if (rows == 0) return PA_OK;
     if (experts > 2048) return PA_ERR_UNSUPPORTED;
-    const size_t smem = (size_t)4 * experts * sizeof(float);
+    const bool four = experts <= 512 && rows >= 16 * device_info().sm_count;
+    const size_t smem = (size_t)(four ? 16 : 4) * experts * sizeof(float);
     // 16-byte pieces: every row of the tokens and of the float weight vectors must start on a 16-byte boundary
     const bool vec = width % 8 == 0 && (uintptr_t)d_h % 16 == 0 && (uintptr_t)d_w_router % 16 == 0 &&
                      (uintptr_t)d_w_shared_gate % 16 == 0;
-#define PA_ROUTER(VEC)                                                                                                 \
-    PA_DISPATCH_ELEM(elem, (router_topk_kernel<T, VEC><<<(unsigned)((rows + 3) / 4), 128, smem, as_stream(stream)>>>(  \
+#define PA_ROUTER(VEC, RPW)                                                                                            \
+    PA_DISPATCH_ELEM(elem, (router_topk_kernel<T, VEC, RPW><<<(unsigned)((rows + 4 * RPW - 1) / (4 * RPW)), 128, smem, as_stream(stream)>>>( \
                                static_cast<const T*>(d_h), d_w_router, d_bias, d_w_shared_gate, rows, width, experts, top, \
                                score_fn, renorm, ngroups, keep, d_choice_bias, d_sel_id, d_sel_w, d_shared_gate)))
-    if (vec) PA_ROUTER(true);
-    else PA_ROUTER(false);
+    if (vec && four) PA_ROUTER(true, 4);
+    else if (vec) PA_ROUTER(true, 1);
+    else PA_ROUTER(false, 1);
 #undef PA_ROUTER
     PA_RETURN_LAUNCH_STATUS();
 }

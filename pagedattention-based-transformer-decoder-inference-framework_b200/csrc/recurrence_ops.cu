@@ -378,6 +378,66 @@ __global__ void __launch_bounds__(256) gated_norm_kernel(const float* __restrict
     }
 }
 
+// the same for groups of whole words of four columns (at most 128 NV, aligned): a lane keeps its values in registers, so y and
+// the gate are read once, 16 and 8 bytes at a time.  8192 rows of 16 groups of 128 (134 MB): 40 us, 68 us with single columns.
+template <typename T, int NV>
+__global__ void __launch_bounds__(256) gated_norm_vec_kernel(const float* __restrict__ y, int64_t rows, int inner, int groups,
+                                                             const T* __restrict__ gate, int64_t gate_stride, int gate_off,
+                                                             int gate_mode, const float* __restrict__ weight, float eps,
+                                                             T* __restrict__ out) {
+    const int lane = threadIdx.x & 31;
+    const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (w >= rows * groups) return;
+    const int64_t r = w / groups;
+    const int gsz = inner / groups, c0 = (int)(w - r * groups) * gsz;
+    const float* yr = y + r * inner + c0;
+    const T* gr = gate ? gate + r * gate_stride + gate_off + c0 : nullptr;
+    float v[NV][4], gt[NV][4];
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int j = 4 * lane + 128 * i;
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (j < gsz) a = *reinterpret_cast<const float4*>(yr + j);
+        v[i][0] = a.x; v[i][1] = a.y; v[i][2] = a.z; v[i][3] = a.w;
+        if (gr && j < gsz) {
+            if constexpr (sizeof(T) == 2) {
+                const uint2 b = *reinterpret_cast<const uint2*>(gr + j);
+                gt[i][0] = __uint_as_float(b.x << 16); gt[i][1] = __uint_as_float(b.x & 0xffff0000u);
+                gt[i][2] = __uint_as_float(b.y << 16); gt[i][3] = __uint_as_float(b.y & 0xffff0000u);
+            } else {
+                const float4 b = *reinterpret_cast<const float4*>(gr + j);
+                gt[i][0] = b.x; gt[i][1] = b.y; gt[i][2] = b.z; gt[i][3] = b.w;
+            }
+        } else {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) gt[i][c] = 0.f;
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if (gate_mode == 1) v[i][c] *= silu_f32(gt[i][c]);
+            ss = fmaf(v[i][c], v[i][c], ss);
+        }
+    }
+    ss = warp_sum(ss);
+    const float rn = 1.0f / sqrtf(ss / (float)gsz + eps);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int j = 4 * lane + 128 * i;
+        if (j >= gsz) continue;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            v[i][c] *= rn;
+            if (weight) v[i][c] *= weight[c0 + j + c];
+            if (gate_mode == 2) v[i][c] *= sigmoid_f32(gt[i][c]);
+            if (gate_mode == 3) v[i][c] *= silu_f32(gt[i][c]);
+        }
+        T* o = out + r * inner + c0 + j;
+        if constexpr (sizeof(T) == 2) *reinterpret_cast<uint2*>(o) = make_uint2(pack_bf16x2(v[i][0], v[i][1]), pack_bf16x2(v[i][2], v[i][3]));
+        else *reinterpret_cast<float4*>(o) = make_float4(v[i][0], v[i][1], v[i][2], v[i][3]);
+    }
+}
+
 // the same with one CTA per (row, group): groups of many values, or few rows
 template <typename T>
 __global__ void __launch_bounds__(256) gated_norm_block_kernel(const float* __restrict__ y, int inner, int groups,
@@ -560,6 +620,20 @@ PA_API int pa_gated_rms_norm(const float* d_y, int64_t rows, int inner, int grou
         PA_RETURN_LAUNCH_STATUS();
     }
     const int64_t threads = rows * groups * 32;
+    const int gsz = inner / groups;
+    const size_t word = (size_t)elem * 4;
+    if (gsz % 4 == 0 && (elem == 2 || elem == 4) && (uintptr_t)d_y % 16 == 0 && (uintptr_t)d_out % word == 0 &&
+        (!d_gate || ((uintptr_t)d_gate % word == 0 && gate_stride % 4 == 0 && gate_off % 4 == 0))) {
+#define PA_GNORM(NV)                                                                                                     \
+    PA_DISPATCH_ELEM(elem, (gated_norm_vec_kernel<T, NV><<<(unsigned)((threads + 255) / 256), 256, 0, as_stream(stream)>>>( \
+                               d_y, rows, inner, groups, static_cast<const T*>(d_gate), gate_stride, gate_off, gate_mode, \
+                               d_weight, eps, static_cast<T*>(d_out))))
+        if (gsz <= 128) PA_GNORM(1);
+        else if (gsz <= 256) PA_GNORM(2);
+        else PA_GNORM(4);                       // below 512 here
+#undef PA_GNORM
+        PA_RETURN_LAUNCH_STATUS();
+    }
     PA_DISPATCH_ELEM(elem, gated_norm_kernel<T><<<(unsigned)((threads + 255) / 256), 256, 0, as_stream(stream)>>>(
                                d_y, rows, inner, groups, static_cast<const T*>(d_gate), gate_stride, gate_off, gate_mode,
                                d_weight, eps, static_cast<T*>(d_out)));
