@@ -267,7 +267,7 @@ class DiffAttentionMixer:
         return c.model._linear(out, self.w_o)
 
 
-EXPAND_FROM = 128         # portions at least this long run latent attention on keys and values built per head (bfloat16)
+EXPAND_FROM = 64          # portions at least this long run latent attention on keys and values built per head (bfloat16)
 ROPE_PAIRING = {"neighbours": 0, "halves": 1}
 
 

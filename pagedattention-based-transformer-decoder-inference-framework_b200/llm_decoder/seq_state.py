@@ -97,9 +97,10 @@ class RaggedBatch:
     EXPAND_MOST = 65536         # cached tokens whose keys and values are built at a time
 
     def _expands(self, p, at_least):
-        """Whether the keys and values of ALL tokens of a portion's sequence are worth building for its queries: `at_least` new
-        tokens, and not many times as many cached ones."""
-        return p[1] >= at_least and p[3] + p[1] <= min(16 * p[1], self.EXPAND_MOST)
+        """Whether the keys and values of ALL tokens of a portion's sequence are built for its queries.  Building costs a cached
+        token as much as about 25 queries save on it (16 heads of 128, rank 512), so the length of the context does not enter, only
+        its place in the buffers."""
+        return p[1] >= at_least and p[3] + p[1] <= self.EXPAND_MOST
 
     def whole_sequences(self, at_least, tokens):
         """The portions that _expands picks, in groups of at most EXPAND_MOST tokens of context: per group ([n, 3] int32 items (slot,
