@@ -261,8 +261,32 @@ def ptr(t):
 
 
 def stream():
+    """Raw handle of the current stream of the current device."""
     import torch
-    return torch.cuda.current_stream().cuda_stream
+    if not torch.cuda.is_initialized():
+        torch.cuda.init()
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+class _Here:
+    """The guard of a device that is current already."""
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *_exc):
+        return False
+
+
+_HERE = _Here()
+
+
+def on_device(device):
+    """torch.cuda.device(device), which costs several microseconds, only where another device is current."""
+    import torch
+    if torch.cuda.is_initialized() and device.index == torch._C._cuda_getDevice():
+        return _HERE
+    return torch.cuda.device(device)
 
 
 def device_info():

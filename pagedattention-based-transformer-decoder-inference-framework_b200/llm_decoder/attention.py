@@ -192,12 +192,12 @@ class AttentionTileLauncher:
         pipe = HostPipe.get(dev) if (pipe_q or pipe_out) else None
         release_q = out_slot = None
         if pipe_q:
-            with torch.cuda.device(dev):
+            with _cabi.on_device(dev):
                 d_q, release_q = pipe.upload(q.view(B, H, D), "q")
         else:
             d_q = _to_device(q, "q", dev, torch.float32) if host_io else q
         if pipe_out:
-            with torch.cuda.device(dev):
+            with _cabi.on_device(dev):
                 d_out, out_slot = pipe.out_slot("out", (B, H, D), torch.float32)
         else:
             d_out = _stage.get("out", (B, H, D), torch.float32, dev)[1] if host_out else out
@@ -226,7 +226,7 @@ class AttentionTileLauncher:
         common = (table.data_ptr(), pt.num_beams_, pt.num_heads_, pt.num_tiles_, kv_cache.total_pages_,
                   _cabi.ptr(d_beam), _cabi.ptr(d_ctx), B, T, D, kv_cache.tile_size_, float(temperature),
                   _cabi.ptr(d_rope), _cabi.ptr(d_lse), ws.data_ptr(), ws.numel(), None)
-        with torch.cuda.device(dev):
+        with _cabi.on_device(dev):
             common = common[:-1] + (_cabi.stream(),)
             if kv_cache.dtype == "f16":
                 fn = lib.pa_paged_decode_f16_overlap if use_overlap else lib.pa_paged_decode_f16
@@ -285,7 +285,7 @@ def apply_rotary_embedding(q, k, rotary_emb, positions):
     in place with rotary_emb [T, D] (interleaved cos, sin) at token positions[row] (int32 CUDA tensor)."""
     ref = q if q is not None else k
     rows, H, D = ref.shape
-    with torch.cuda.device(ref.device):
+    with _cabi.on_device(ref.device):
         _cabi.check(_cabi.lib().pa_apply_rope_f32(_cabi.ptr(q), _cabi.ptr(k), rotary_emb.data_ptr(), positions.data_ptr(),
                                                   rows, H, D, rotary_emb.shape[0], _cabi.stream()), "pa_apply_rope_f32")
     return q, k
@@ -305,7 +305,7 @@ def paged_prefill(q, out, kv_cache, B, Tq, temperature=1.0, beam_ids=None, ctx_s
     if token_major:
         common = (pt.device_data().data_ptr(), pt.num_beams_, H, pt.num_tiles_, kv_cache.total_pages_, _cabi.ptr(beam_ids),
                   _cabi.ptr(ctx_start), B, Tq, D, kv_cache.tile_size_, float(temperature))
-        with torch.cuda.device(kv_cache.key_buffer_.device):
+        with _cabi.on_device(kv_cache.key_buffer_.device):
             if kv_cache.dtype == "f16":
                 st = lib.pa_paged_prefill_f16_tokmajor(q.data_ptr(), out.data_ptr(), kv_cache.key_buffer_.data_ptr(),
                                                        kv_cache.value_buffer_.data_ptr(), *common, _cabi.stream())
@@ -333,7 +333,7 @@ def paged_prefill(q, out, kv_cache, B, Tq, temperature=1.0, beam_ids=None, ctx_s
         ws_ptr, ws_bytes = ws.data_ptr(), ws.numel()
     common = (pt.device_data().data_ptr(), pt.num_beams_, H, pt.num_tiles_, kv_cache.total_pages_, _cabi.ptr(beam_ids),
               _cabi.ptr(ctx_start), B, Tq, D, kv_cache.tile_size_, float(temperature), ws_ptr, ws_bytes)
-    with torch.cuda.device(kv_cache.key_buffer_.device):
+    with _cabi.on_device(kv_cache.key_buffer_.device):
         if kv_cache.dtype == "f16":
             st = lib.pa_paged_prefill_f16(q.data_ptr(), out.data_ptr(), kv_cache.key_buffer_.data_ptr(),
                                           kv_cache.value_buffer_.data_ptr(), *common, _cabi.stream())
@@ -369,7 +369,7 @@ def paged_attention_filtered(q, out, kv_cache, B, T, temperature=1.0, top_k=0, t
                                               else torch.as_tensor(np.asarray(rotary_emb), dtype=torch.float32).to(dev))
     for t in (logits, attention_weights):
         assert t is None or (t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() and t.numel() == B * H * T)
-    with torch.cuda.device(dev):
+    with _cabi.on_device(dev):
         st = lib.pa_paged_attention_filtered(
             q.data_ptr(), out.data_ptr(), kv_cache.key_buffer_.data_ptr(), kv_cache.value_buffer_.data_ptr(),
             _cabi.ptr(kv_cache.k_scales_), _cabi.ptr(kv_cache.v_scales_), kind, pt.device_data().data_ptr(), pt.num_beams_, H,
@@ -388,7 +388,7 @@ def paged_decode_group(q, out, kv_cache, B, T, beam_width, temperature=1.0, beam
     H, D = pt.num_heads_, kv_cache.head_dim_
     if kv_cache.dtype == "i8":  # per-row streaming kernel through the beam indirection; shared pages served from L2
         ws = kv_cache.workspace(B)
-        with torch.cuda.device(kv_cache.key_buffer_.device):
+        with _cabi.on_device(kv_cache.key_buffer_.device):
             st = _cabi.lib().pa_paged_decode_i8_group(
                 q.data_ptr(), out.data_ptr(), kv_cache.key_buffer_.data_ptr(), kv_cache.value_buffer_.data_ptr(),
                 kv_cache.k_scales_.data_ptr(), kv_cache.v_scales_.data_ptr(), pt.device_data().data_ptr(), pt.num_beams_, H,
@@ -400,7 +400,7 @@ def paged_decode_group(q, out, kv_cache, B, T, beam_width, temperature=1.0, beam
     if kv_cache.dtype != "f16":
         raise NotImplementedError("paged_decode_group: fp16 or int8 KV pages")
     ws = kv_cache.workspace(B)
-    with torch.cuda.device(kv_cache.key_buffer_.device):
+    with _cabi.on_device(kv_cache.key_buffer_.device):
         st = _cabi.lib().pa_paged_decode_f16_group(
             q.data_ptr(), out.data_ptr(), kv_cache.key_buffer_.data_ptr(), kv_cache.value_buffer_.data_ptr(),
             pt.device_data().data_ptr(), pt.num_beams_, H, pt.num_tiles_, kv_cache.total_pages_, _cabi.ptr(beam_ids),
@@ -428,7 +428,7 @@ def paged_decode_partial(q, kv_cache, B, T, temperature=1.0, beam_ids=None, ctx_
         fn, name = lib.pa_paged_decode_f16_partial, "pa_paged_decode_f16_partial"
     else:
         raise NotImplementedError("paged_decode_partial: fp16 or int8 KV pages")
-    with torch.cuda.device(dev):
+    with _cabi.on_device(dev):
         st = fn(q.data_ptr(), pm.data_ptr(), pl.data_ptr(), po.data_ptr(), *pools, pt.device_data().data_ptr(),
                 pt.num_beams_, H, pt.num_tiles_, kv_cache.total_pages_, _cabi.ptr(beam_ids), _cabi.ptr(ctx_lens), B, T, D,
                 kv_cache.tile_size_, float(temperature), _cabi.ptr(rotary_emb), ws.data_ptr(), ws.numel(), _cabi.stream())
@@ -441,7 +441,7 @@ def lse_combine(part_m, part_l, part_o, out=None, lse_out=None):
     n_parts, rows, D = part_o.shape
     if out is None:
         out = torch.empty((rows, D), dtype=torch.float32, device=part_o.device)
-    with torch.cuda.device(part_o.device):
+    with _cabi.on_device(part_o.device):
         _cabi.check(_cabi.lib().pa_lse_combine(part_m.data_ptr(), part_l.data_ptr(), part_o.data_ptr(),
                                                n_parts, rows, D, out.data_ptr(), _cabi.ptr(lse_out),
                                                _cabi.stream()), "pa_lse_combine")

@@ -50,7 +50,7 @@ class Engine:
         dev = self.model.device
         if not batch_entries:
             return torch.empty((0, self.model.vocab), dtype=torch.float32, device=dev)
-        with torch.cuda.device(dev):
+        with _cabi.on_device(dev):
             batch = self.states.make_batch(batch_entries)
             want_rows = _to_device(torch.tensor(want, dtype=torch.int32), dev)
             return self.model.forward(batch, want_rows)

@@ -18,7 +18,7 @@ def quantize_to_int8(input, scale):
     x = input.contiguous()
     assert x.is_cuda and x.dtype == torch.float32
     q = torch.empty(x.shape, dtype=torch.int8, device=x.device)
-    with torch.cuda.device(x.device):
+    with _cabi.on_device(x.device):
         _chk(_cabi.lib().pa_quantize_i8(x.data_ptr(), x.numel(), float(scale), q.data_ptr(), _cabi.stream()),
              "pa_quantize_i8")
     return q
@@ -31,7 +31,7 @@ def batch_quantize(input, scales, dim):
     assert x.is_cuda and x.dtype == torch.float32 and s.dtype == torch.float32
     assert x.numel() == s.numel() * dim
     q = torch.empty(x.shape, dtype=torch.int8, device=x.device)
-    with torch.cuda.device(x.device):
+    with _cabi.on_device(x.device):
         _chk(_cabi.lib().pa_batch_quantize_i8(x.data_ptr(), s.data_ptr(), s.numel(), dim, q.data_ptr(),
                                               _cabi.stream()), "pa_batch_quantize_i8")
     return q
@@ -41,7 +41,7 @@ def compute_absmax(input):
     """int8_quant.cpp:30-36 -> python float."""
     x = input.contiguous()
     out = torch.empty(1, dtype=torch.float32, device=x.device)
-    with torch.cuda.device(x.device):
+    with _cabi.on_device(x.device):
         _chk(_cabi.lib().pa_absmax(x.data_ptr(), x.numel(), out.data_ptr(), _cabi.stream()), "pa_absmax")
     return float(out.item())
 
@@ -51,7 +51,7 @@ def dequantize_from_int8(input, scale):
     q = input.contiguous()
     assert q.is_cuda and q.dtype == torch.int8
     x = torch.empty(q.shape, dtype=torch.float32, device=q.device)
-    with torch.cuda.device(q.device):
+    with _cabi.on_device(q.device):
         _chk(_cabi.lib().pa_dequantize_i8(q.data_ptr(), q.numel(), float(scale), x.data_ptr(), _cabi.stream()),
              "pa_dequantize_i8")
     return x
@@ -63,7 +63,7 @@ def batch_dequantize(input, scales, dim):
     s = scales.contiguous()
     assert q.numel() == s.numel() * dim
     x = torch.empty(q.shape, dtype=torch.float32, device=q.device)
-    with torch.cuda.device(q.device):
+    with _cabi.on_device(q.device):
         _chk(_cabi.lib().pa_batch_dequantize_i8(q.data_ptr(), s.data_ptr(), s.numel(), dim, x.data_ptr(),
                                                 _cabi.stream()), "pa_batch_dequantize_i8")
     return x
@@ -73,7 +73,7 @@ def compute_minmax_scale(input):
     """int8_quant.cpp:59-64 -> python float."""
     x = input.contiguous()
     out = torch.empty(1, dtype=torch.float32, device=x.device)
-    with torch.cuda.device(x.device):
+    with _cabi.on_device(x.device):
         _chk(_cabi.lib().pa_minmax_scale(x.data_ptr(), x.numel(), out.data_ptr(), _cabi.stream()),
              "pa_minmax_scale")
     return float(out.item())
@@ -84,7 +84,7 @@ def batch_minmax_scale(input, dim):
     x = input.contiguous()
     rows = x.numel() // dim
     s = torch.empty(rows, dtype=torch.float32, device=x.device)
-    with torch.cuda.device(x.device):
+    with _cabi.on_device(x.device):
         _chk(_cabi.lib().pa_batch_minmax_scale(x.data_ptr(), rows, dim, s.data_ptr(), _cabi.stream()),
              "pa_batch_minmax_scale")
     return s
@@ -102,7 +102,7 @@ def dnnl_matmul_int8(A, B, C, BATCH, M, N, K, scaleA, scaleB, scaleC=1.0, bias=N
     if activation not in _cabi.ACT:
         return False
     try:
-        with torch.cuda.device(A.device):
+        with _cabi.on_device(A.device):
             lib = _cabi.lib()
             # split-K scratch is the caller's (stream-ordered torch allocation, released after the call is enqueued)
             need = lib.pa_gemm_i8_workspace_bytes(BATCH, M, N, K)

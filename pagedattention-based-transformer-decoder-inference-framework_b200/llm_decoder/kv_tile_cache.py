@@ -205,7 +205,7 @@ class KVTileCache:
         assert src.dtype == self.key_buffer_.dtype and src.dim() == 2 and src.stride(1) == 1
         pt = self.page_table_
         table = pt.device_data()
-        with torch.cuda.device(table.device):
+        with _cabi.on_device(table.device):
             _cabi.check(_cabi.lib().pa_kv_append_rows(
                 self.key_buffer_.data_ptr(), self.value_buffer_.data_ptr(), table.data_ptr(), pt.num_beams_,
                 pt.num_heads_, pt.num_tiles_, self.total_pages_, self.tile_size_, self.head_dim_, self.value_dim_,
@@ -336,7 +336,7 @@ class KVTileCache:
             from .attention import HostPipe
             assert new_k.is_pinned() and new_v.is_pinned(), "host new_k/new_v must be page-locked"
             pipe = HostPipe.get(table.device)
-            with torch.cuda.device(table.device):
+            with _cabi.on_device(table.device):
                 new_k, rk = pipe.upload(new_k, "new_k")
                 new_v, rv = pipe.upload(new_v, "new_v")
             releases = [rk, rv]
@@ -348,7 +348,7 @@ class KVTileCache:
         common = (table.data_ptr(), pt.num_beams_, pt.num_heads_, pt.num_tiles_, self.total_pages_,
                   self.tile_size_, self.head_dim_, new_k.data_ptr(), new_v.data_ptr(),
                   _cabi.ptr(beam_ids), positions.data_ptr(), R, _cabi.stream())
-        with torch.cuda.device(table.device):
+        with _cabi.on_device(table.device):
             if self.dtype == "f32":
                 assert new_k.dtype == torch.float32
                 st = lib.pa_kv_append_f32(self.key_buffer_.data_ptr(), self.value_buffer_.data_ptr(), *common)
@@ -362,7 +362,7 @@ class KVTileCache:
                 assert new_k.dtype == torch.float32
                 st = lib.pa_kv_append_f32_f16(self.key_buffer_.data_ptr(), self.value_buffer_.data_ptr(), *common)
         _cabi.check(st, "pa_kv_append")
-        with torch.cuda.device(table.device):
+        with _cabi.on_device(table.device):
             for rel in releases:
                 rel()
 
@@ -439,7 +439,7 @@ class KVTileCache:
         if src:
             d_src = torch.tensor(src, dtype=torch.int32).to(dev)
             d_dst = torch.tensor(dst, dtype=torch.int32).to(dev)
-            with torch.cuda.device(dev):
+            with _cabi.on_device(dev):
                 _cabi.check(_cabi.lib().pa_kv_copy_pages(
                     self.key_buffer_.data_ptr(), self.value_buffer_.data_ptr(), _cabi.ptr(self.k_scales_),
                     _cabi.ptr(self.v_scales_), d_src.data_ptr(), d_dst.data_ptr(), len(src), self.total_pages_,
@@ -458,7 +458,7 @@ class KVTileCache:
         R = rows if rows is not None else (beam_ids.numel() if beam_ids is not None else pt.num_beams_)
         dense = torch.empty((R, pt.num_heads_, pt.num_tiles_ * self.tile_size_, self.head_dim_),
                             dtype=pool.dtype, device=pool.device)
-        with torch.cuda.device(pool.device):
+        with _cabi.on_device(pool.device):
             _cabi.check(_cabi.lib().pa_kv_gather(pool.data_ptr(), dense.data_ptr(), table.data_ptr(),
                                                  pt.num_beams_, pt.num_heads_, pt.num_tiles_,
                                                  self.total_pages_, self.tile_size_, self.head_dim_,
@@ -470,10 +470,10 @@ class KVTileCache:
         """Scratch for the decode kernels (chunk counter + partials): one buffer per (cache, stream), so decode
         calls on different streams never share it; sized on the cache's own device."""
         dev = self.key_buffer_.device
-        with torch.cuda.device(dev):
+        with _cabi.on_device(dev):
             need = _cabi.lib().pa_decode_workspace_bytes(B, self.page_table_.num_heads_, self.head_dim_,
                                                          self.page_table_.num_tiles_, self.tile_size_)
-            key = torch.cuda.current_stream(dev).cuda_stream
+            key = _cabi.stream()
         ws = self._ws.get(key)
         if ws is None or ws.numel() < need:
             ws = self._ws[key] = torch.empty(need, dtype=torch.uint8, device=dev)

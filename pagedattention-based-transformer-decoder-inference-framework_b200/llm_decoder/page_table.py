@@ -36,7 +36,7 @@ class PageTable:
         self._clear_device()
 
     def _clear_device(self):
-        with torch.cuda.device(self.d_table_.device):
+        with _cabi.on_device(self.d_table_.device):
             _cabi.check(_cabi.lib().pa_page_table_clear(self.d_table_.data_ptr(), self.total_entries_,
                                                         _cabi.stream()), "pa_page_table_clear")
 
@@ -68,7 +68,7 @@ class PageTable:
         dev = self.d_table_.device
         di = torch.from_numpy(flat_idx.astype(np.int32)).to(dev)
         dp = torch.from_numpy(pages).to(dev)
-        with torch.cuda.device(dev):
+        with _cabi.on_device(dev):
             _cabi.check(_cabi.lib().pa_page_table_update(self.d_table_.data_ptr(), self.total_entries_,
                                                          di.data_ptr(), dp.data_ptr(), di.numel(),
                                                          _cabi.stream()), "pa_page_table_update")
@@ -89,7 +89,7 @@ class PageTable:
         idx = to_device(torch.tensor(list(self._pending.keys()), dtype=torch.int32), dev)
         pg = to_device(torch.tensor(list(self._pending.values()), dtype=torch.int32), dev)
         self._pending.clear()
-        with torch.cuda.device(dev):
+        with _cabi.on_device(dev):
             _cabi.check(_cabi.lib().pa_page_table_update(self.d_table_.data_ptr(), self.total_entries_,
                                                          idx.data_ptr(), pg.data_ptr(), idx.numel(),
                                                          _cabi.stream()), "pa_page_table_update")
@@ -109,7 +109,7 @@ class PageTable:
         h = torch.as_tensor(heads, dtype=torch.int32).to(dev)
         t = torch.as_tensor(tiles, dtype=torch.int32).to(dev)
         out = torch.empty_like(b)
-        with torch.cuda.device(dev):
+        with _cabi.on_device(dev):
             _cabi.check(_cabi.lib().pa_page_table_lookup(self.d_table_.data_ptr(), self.num_beams_,
                                                          self.num_heads_, self.num_tiles_, b.data_ptr(),
                                                          h.data_ptr(), t.data_ptr(), out.data_ptr(),
