@@ -892,6 +892,22 @@ int pa_latent_gather(const void* d_pool, const int32_t* d_table, int num_slots, 
 int pa_attention_tc_errors(int* host_count);
 int pa_moe_tc_errors(int* host_count);
 
+/* ---- decoded tokens with the keys cut into equal shares (masked_decode.cu) ----------------------------------------------
+ * pa_masked_decode: pa_masked_attention_gated for tiles of ONE token, bfloat16 softmax attention: the 16-key units of all
+ *   (token, kv head) pairs are one list that `workers` warps share equally, and a second kernel joins the shares of a pair.
+ *   d_q_tiles 16-byte aligned.  PA_ERR_UNSUPPORTED: head sizes other than 64 and 128, values that are the keys, more than 4096
+ *   tokens, pages that are not a multiple of 16 tokens, or an alignment.
+ * pa_masked_decode_workers: a worker count for tokens with at most `longest` keys (any 1 .. 8 * SMs is served). */
+int pa_masked_decode_workers(int num_tokens, int heads, int kv_heads, int64_t longest);
+size_t pa_masked_decode_workspace_bytes(int num_tokens, int heads, int kv_heads, int vdim, int workers);
+int pa_masked_decode(const void* d_q, int64_t q_stride, int q_off, const void* d_k_pool, const void* d_v_pool,
+                     const int32_t* d_table, int num_slots, int num_kv_heads, int num_tiles, int total_pages, int tile_size,
+                     const int32_t* d_q_tiles, int num_q_tiles, int heads, int dim, int vdim, float scale, float softcap,
+                     int mask_kind, int mask_size, int mask_keep, int bias_kind, const float* d_bias, int bias_len,
+                     const float* d_head_scale, const float* d_sink, const float* d_out_rot, const float* d_head_bias,
+                     const void* d_gate, int64_t gate_stride, int gate_off, void* d_out, int workers, void* d_workspace,
+                     size_t workspace_bytes, pa_stream_t stream);
+
 /* ---- token-pair embedding, block passes that add, convolved + turned + normed projections, sinks on the latent ---------
  * pa_embedding_bigram: x[r] = embed[ids[r]] * scale + bigram[b(r)] as float (tables in the activation type), b(r) =
  *   (prev_ids[r] * mul_prev + ids[r] * mul_cur) mod buckets, or row `buckets` (the table has buckets + 1 rows) where

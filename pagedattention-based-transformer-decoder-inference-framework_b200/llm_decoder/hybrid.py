@@ -670,6 +670,8 @@ class MaskedAttention:
                           model._lib.pa_masked_attention_tc_units(self.heads, self.kv_heads, q), kind) for q, kind in ((2, 4), (1, 5))]
         if self.sigmoid or self.keys_as_values or self.tc_plans[0][0] == 0:
             self.tc_plans = []
+        # the same forms and sizes: decoded tokens with their keys cut into equal shares
+        self.shares = bool(self.tc_plans)
         self.alloc_state(model)
 
     def alloc_state(self, model):
@@ -765,6 +767,8 @@ class MaskedAttention:
             tiles, ntiles, _longest = group
             if kind == 2:
                 kind = portion_kind
+            if kind == 1 and self.shares and self._decode(c, proj, off, gate, out, tiles, ntiles, _longest, out_rot):
+                continue
             # decoded tokens of a batch with at least one (token, kv head) pair per SM: heads as rows on the tensor cores
             if kind == 1 and mma_tokens and ntiles * self.kv_heads >= c.model.sm_count:
                 kind = 3
@@ -781,6 +785,25 @@ class MaskedAttention:
             if kind >= 2 and st == _cabi.PA_ERR_UNSUPPORTED:
                 return False
             _chk(st, "pa_masked_attention_gated")
+        return True
+
+    def _decode(self, c, proj, off, gate, out, tiles, ntiles, longest, out_rot):
+        """Tiles of one token on pa_masked_decode; False where it does not take the operands."""
+        lib, kv = c.lib, self.kv
+        pt = kv.page_table_
+        workers = lib.pa_masked_decode_workers(ntiles, self.heads, self.kv_heads, min(longest, self.mask_size + self.mask_keep + 32)
+                                               if self.mask_kind else longest)
+        ws = c.empty(lib.pa_masked_decode_workspace_bytes(ntiles, self.heads, self.kv_heads, self.vdim, workers), dtype=torch.uint8)
+        st = lib.pa_masked_decode(proj.data_ptr(), proj.stride(0), off, kv.key_buffer_.data_ptr(), kv.value_buffer_.data_ptr(),
+                                  pt.device_data().data_ptr(), pt.num_beams_, pt.num_heads_, pt.num_tiles_, kv.total_pages_, kv.tile_size_,
+                                  tiles.data_ptr(), ntiles, self.heads, self.dim, self.vdim, self.scale, self.softcap, self.mask_kind,
+                                  self.mask_size, self.mask_keep, self.bias_kind, _cabi.ptr(self.bias), self.bias_len,
+                                  _cabi.ptr(self.head_scale), _cabi.ptr(self.sink), _cabi.ptr(out_rot), _cabi.ptr(self.head_bias),
+                                  _cabi.ptr(gate[0]), gate[0].stride(0) if gate[0] is not None else 0, gate[1], out.data_ptr(), workers,
+                                  ws.data_ptr(), ws.numel(), _cabi.stream())
+        if st == _cabi.PA_ERR_UNSUPPORTED:
+            return False
+        _chk(st, "pa_masked_decode")
         return True
 
     def project_out(self, c, heads_out):
