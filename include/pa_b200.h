@@ -908,6 +908,19 @@ int pa_masked_decode(const void* d_q, int64_t q_stride, int q_off, const void* d
                      const void* d_gate, int64_t gate_stride, int gate_off, void* d_out, int workers, void* d_workspace,
                      size_t workspace_bytes, pa_stream_t stream);
 
+/* pa_latent_decode: pa_latent_attention_sink for tiles of ONE token, bfloat16 (latent_decode.cu): the 32-key units of all tokens are
+ *   one list that `workers` CTAs share equally, and a second kernel joins the shares of a token.  d_q_tiles 16-byte aligned.
+ *   PA_ERR_UNSUPPORTED: kv_rank other than 128, 256, 384, 512, rot_dim above 64 or not a multiple of 8, more than 4096 tokens, pages
+ *   that are not a multiple of 16 tokens, or an alignment.
+ * pa_latent_decode_workers: a worker count for tokens with at most `longest` keys (any 1 .. SMs is served). */
+int pa_latent_decode_workers(int num_tokens, int heads, int64_t longest);
+size_t pa_latent_decode_workspace_bytes(int num_tokens, int heads, int kv_rank, int workers);
+int pa_latent_decode(const void* d_q_lat, int64_t ql_row_stride, int64_t ql_head_stride, const void* d_q_rot, int64_t qr_row_stride,
+                     int64_t qr_head_stride, const void* d_pool, const int32_t* d_table, int num_slots, int num_tiles, int total_pages,
+                     int tile_size, const int32_t* d_q_tiles, int num_q_tiles, int heads, int kv_rank, int rot_dim, float scale,
+                     const float* d_sink, void* d_out, int64_t o_row_stride, int64_t o_head_stride, int workers, void* d_workspace,
+                     size_t workspace_bytes, pa_stream_t stream);
+
 /* ---- token-pair embedding, block passes that add, convolved + turned + normed projections, sinks on the latent ---------
  * pa_embedding_bigram: x[r] = embed[ids[r]] * scale + bigram[b(r)] as float (tables in the activation type), b(r) =
  *   (prev_ids[r] * mul_prev + ids[r] * mul_cur) mod buckets, or row `buckets` (the table has buckets + 1 rows) where

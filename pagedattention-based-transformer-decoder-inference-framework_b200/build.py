@@ -19,7 +19,7 @@ CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libpa_b200.so")
 OUT_CORE = os.path.join(HERE, "libpa_b200_core.so")
 CORE = ("page_table.cu", "decoder_ops.cu", "linear_tf32x3.cu", "sampling.cu", "seq_ops.cu", "diff_attention.cu",
-        "latent_attention.cu", "masked_attention.cu", "attention_tc.cu", "masked_decode.cu", "recurrence_ops.cu", "moe_ops.cu", "moe_tc.cu")
+        "latent_attention.cu", "masked_attention.cu", "attention_tc.cu", "masked_decode.cu", "latent_decode.cu", "recurrence_ops.cu", "moe_ops.cu", "moe_tc.cu")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 
 FLAGS = [

@@ -412,6 +412,17 @@ class LatentAttentionMixer:
                 continue
             tiles, ntiles, longest = group
             ws = None
+            if kind == 1 and mma and kvr % 128 == 0:    # decoded tokens: their keys in equal shares, where that kernel takes the operands
+                workers = lib.pa_latent_decode_workers(ntiles, H, longest)
+                ws = c.empty(lib.pa_latent_decode_workspace_bytes(ntiles, H, kvr, workers), dtype=torch.uint8)
+                st = lib.pa_latent_decode(ql.data_ptr(), kvr, R * kvr, q.data_ptr() + self.dim * c.elem, q.stride(0), self.qd,
+                                          kv.key_buffer_.data_ptr(), table.data_ptr(), pt.num_beams_, pt.num_tiles_, kv.total_pages_,
+                                          kv.tile_size_, tiles.data_ptr(), ntiles, H, kvr, self.rot_dim, self.scale, _cabi.ptr(self.sink),
+                                          lat.data_ptr(), kvr, R * kvr, workers, ws.data_ptr(), ws.numel(), s)
+                if st != _cabi.PA_ERR_UNSUPPORTED:
+                    _chk(st, "pa_latent_decode")
+                    continue
+                ws = None
             nsplit = latent_key_splits(ntiles * math.ceil(H / rows_per_cta), longest, c.model.sm_count)
             if nsplit > 1:
                 ws = c.empty(lib.pa_latent_attention_workspace_bytes(ntiles, H, kvr, nsplit), dtype=torch.uint8)
