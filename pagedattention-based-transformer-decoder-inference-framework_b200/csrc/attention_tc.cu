@@ -20,9 +20,11 @@
 // O share the reference, so O / l does not depend on it): rows are rescaled a few times instead of once per tile.
 //
 // What bounds it: per 64 keys and 128 rows 4096 / 16 = 512 cycles of ex2 on the MUFU against 512 (dim 128) to 640 (dim 192)
-// cycles of tensor pipe; two tiles per CTA keep both busy at once.  Measured, 4 x 2048 tokens causal: 16 query / 4 kv heads of 128
-// paged 123 us = 560 TFLOP/s (mma.sync kernel 918 us); latent attention at 16 heads of 128 + 64 / 128, five ragged portions
-// 129 us, and 38 us for gathering the rows and building keys and values (absorbed form on mma.sync 1360 us).
+// cycles of tensor pipe; two tiles per CTA keep both busy at once.  A step takes about 2300 cycles: the exponentials of both tiles
+// (1600 with their adds and conversions) and the hand-offs between pipes (tiles of 128 keys, which have half as many but no
+// second score buffer, took 150 us where this takes 123; query rows by TMA and no wait but the scores' own gave 123 -> 110).  Measured, 4 x 2048 tokens causal: 16 query / 4 kv heads of 128
+// paged 110 us = 620 TFLOP/s (mma.sync kernel 918 us); latent attention at 16 heads of 128 + 64 / 128, five ragged portions
+// 110 us, and 38 us for gathering the rows and building keys and values (absorbed form on mma.sync 1360 us).
 //
 // Every wait is bounded: on a protocol error the CTA raises a flag (pa_attention_tc_errors), waits for its copies, frees its
 // TMEM and leaves NaN in its rows.
@@ -39,7 +41,6 @@ constexpr int QT = 128, KT = 64;
 struct Args {
     MaskAttnParams p;
     int tb, hg, hchunks;     // tokens per head block, heads per CTA, head chunks per kv head
-    int qd;                  // columns of a query (multiple of 16); query of head h at q_off + h * qd
     int kn;                  // dense: key columns per head (multiple of 64); the shared block starts at k2_col of its buffer
     int k2_col;
     int upt;                 // paged: 16-token units per page
@@ -58,9 +59,10 @@ constexpr size_t smem_for(int kb, int vb, int nq) {
 }
 
 // KB / VB: blocks of 64 columns of a key / a value; MOD: the score has more than a factor (soft cap or distance bias)
-template <int KB, int VB, int NQ, bool DENSE, bool MOD>
+// QD: columns of a query (the last block may be part of one)
+template <int KB, int VB, int NQ, bool DENSE, bool MOD, int QD>
 __global__ void __launch_bounds__(threads_for(NQ), NQ == 1 && KB < 3 ? 2 : 1)
-attention_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmK2,
+attention_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmK2,
                     const __grid_constant__ CUtensorMap tmV, const Args a) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     constexpr int ST = stages_for(KB, NQ), NBAR = nbar_for(KB, NQ), TMEM_COLS = NQ * 256, D = VB * 64;
@@ -95,7 +97,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
                 mbar_init(p_full(x, b), QT);
                 mbar_init(o_full(x, b), 1);
             }
-            mbar_init(q_ready(x), QT);
+            mbar_init(q_ready(x), QT + 1);
         }
         asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(fail_sm), "r"(0u) : "memory");
         mbar_fence_init();
@@ -136,9 +138,24 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
     tc_fence_after();
     uint32_t tmem_base;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
+    const bool whole = ntok == a.tb;        // no box of query rows reaches past the work item's
 
     if (warp == W_PROD) {
         if (elect_one()) {
+            for (int x = 0; x < NQ; ++x) {  // 64 rows of one head x 64 columns a box
+                const int nb = whole ? min(2, ((hend - h0) * a.tb - x * QT) / 64) : 0;      // blocks of 64 rows with a head
+                if (nb <= 0) {
+                    mbar_arrive_cnt(q_ready(x));
+                    continue;
+                }
+                mbar_arrive_expect_tx(q_ready(x), nb * KB * 8192);
+                for (int b = 0; b < nb; ++b) {
+                    const int r = x * QT + b * 64, col = p.q_off + (h0 + r / a.tb) * QD;
+#pragma unroll
+                    for (int kb = 0; kb < KB; ++kb)
+                        tma_load_2d(q_sm + x * Q_BYTES + kb * (QT * 128) + b * 8192, &tmQ, col + kb * 64, row0 + r % a.tb, q_ready(x));
+                }
+            }
             const int32_t* trow = DENSE ? nullptr : p.table + ((int64_t)slot * p.num_kv_heads + g) * p.num_tiles;
             const bool slot_ok = DENSE || (unsigned)slot < (unsigned)p.num_slots;
             int pgn[4];
@@ -200,13 +217,12 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
         }
     } else if (warp >= W_MMA) {
         constexpr uint32_t kIdescS = idesc_f16(QT, KT, 0, 0, 1), kIdescO = idesc_f16(QT, D, 0, 1, 1);
-        const int x = warp - W_MMA, ntx = nts[x], kmx = kmaxs[x], ksteps_q = a.qd >> 4;
+        const int x = warp - W_MMA, ntx = nts[x], kmx = kmaxs[x];
         auto issue_S = [&](int i, int stage) {
             if (elect_one()) {
                 const uint32_t st = kv_sm + stage * STAGE, qx = q_sm + x * Q_BYTES;
 #pragma unroll
-                for (int ks = 0; ks < KB * 4; ++ks) {
-                    if (ks >= ksteps_q) break;
+                for (int ks = 0; ks < QD / 16; ++ks) {
                     const uint64_t da = make_desc(qx + (ks >> 2) * (QT * 128) + (ks & 3) * 32, 16, 1024);
                     const uint64_t db = make_desc(st + (ks >> 2) * (KT * 128) + (ks & 3) * 32, 16, 1024);
                     umma_f16(tmem_base + x * 2 * KT + (i & 1) * KT, da, db, kIdescS, ks > 0 ? 1u : 0u);
@@ -275,18 +291,28 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
         const int qpos = tok < nw ? pos0 + tok : -1;
         const int nt = nts[x], kmax = kmaxs[x];
         const uint32_t lane_base = (uint32_t)(qtr * 32) << 16;
-        if (nt > 0) {
+        if (nt > 0 && whole) mbar_arrive_cnt(q_ready(x));
+        if (nt > 0 && !whole) {
             // the warp's query rows into the swizzled K-major A tile
-            const bf16_t* qsrc = static_cast<const bf16_t*>(p.q) + p.q_off + (int64_t)head * a.qd;
+            const bf16_t* qsrc = static_cast<const bf16_t*>(p.q) + p.q_off + (int64_t)head * QD;
             const uint32_t qx = q_sm + x * Q_BYTES;
-            const int chunks = a.qd >> 3;
-#pragma unroll 4
-            for (int idx = lane; idx < 32 * chunks; idx += 32) {
-                const int r = idx / chunks, c = idx - r * chunks, rr = qtr * 32 + r;
-                uint4 v = make_uint4(0u, 0u, 0u, 0u);
-                if (tokw + r < nw) v = __ldg(reinterpret_cast<const uint4*>(qsrc + (int64_t)(row0 + tokw + r) * p.q_stride) + c);
-                const uint32_t addr = qx + (c >> 3) * (QT * 128) + rr * 128 + (((c & 7) ^ (rr & 7)) << 4);
-                asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+            constexpr int CH = QD / 8, PER = CH <= 32 ? 8 : 4;     // 16-byte pieces of a row; loads in flight per lane
+#pragma unroll 1
+            for (int i0 = 0; i0 < 32 * CH; i0 += 32 * PER) {
+                uint4 v[PER];
+#pragma unroll
+                for (int j = 0; j < PER; ++j) {
+                    const int idx = i0 + j * 32 + lane, r = idx / CH, c = idx % CH;
+                    v[j] = make_uint4(0u, 0u, 0u, 0u);
+                    if (r < 32 && tokw + r < nw) v[j] = __ldg(reinterpret_cast<const uint4*>(qsrc + (int64_t)(row0 + tokw + r) * p.q_stride) + c);
+                }
+#pragma unroll
+                for (int j = 0; j < PER; ++j) {
+                    const int idx = i0 + j * 32 + lane, r = idx / CH, c = idx % CH, rr = qtr * 32 + r;
+                    if (r >= 32) continue;
+                    const uint32_t addr = qx + (c >> 3) * (QT * 128) + rr * 128 + (((c & 7) ^ (rr & 7)) << 4);
+                    asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(v[j].x), "r"(v[j].y), "r"(v[j].z), "r"(v[j].w) : "memory");
+                }
             }
             fence_proxy_async();
             mbar_arrive_cnt(q_ready(x));
@@ -305,26 +331,17 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
         float m_ref = -INFINITY, l_run = 0.f;
         const uint32_t s_addr = tmem_base + lane_base + x * 2 * KT;
         const uint32_t o_addr = tmem_base + lane_base + NQ * 2 * KT + x * D;
-        int oc[2] = {0, 0};
-        auto ensure_pv = [&](int tp) {      // P.V(tp) is complete; phases are consumed in order, at most two tiles late
-            const int b = tp & 1, k = tp >> 1;
-            if (oc[b] <= k) {
-                wait(o_full(x, b), (uint32_t)(k & 1));
-                oc[b] = k + 1;
-            }
-        };
+        // P.V(t) is complete.  Unambiguous without consuming every phase: S(i) follows P.V(i - 2) on the pipe, so by the time a
+        // thread works on tile i the barrier of P.V(i - 1) is in the phase asked for or just past it.
+        auto pv_done = [&](int t) { wait(o_full(x, t & 1), (uint32_t)((t >> 1) & 1)); };
         int st_i = 0;
-        uint32_t st_ph = 0;
 #pragma unroll 1
         for (int i = 0; i < nt; ++i) {
             const int sb = i & 1, kp0 = steps.step(i) * KT;
-            uint32_t mapped = 15u;
-            if (!DENSE) {
-                wait(kv_full(st_i), st_ph);     // long complete: makes the producer's note about this stage visible
-                asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(mapped) : "r"(meta_sm + st_i * 4) : "memory");
-            }
             wait(s_full(x, sb), (uint32_t)((i >> 1) & 1));
             tc_fence_after();
+            uint32_t mapped = 15u;      // the producer's note about this stage, older than the scores
+            if (!DENSE) asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(mapped) : "r"(meta_sm + st_i * 4) : "memory");
             uint32_t sr[2][32];
             tmem_ld32(s_addr + sb * KT, sr[0]);
             tmem_ld32(s_addr + sb * KT + 32, sr[1]);
@@ -371,9 +388,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
                 w[k] = pack_bf16x2(e0, e1);
             }
             const bool dead = m_ref == -INFINITY;       // nothing visible yet: the exponents above are NaN
-            if (i >= 2) ensure_pv(i - 2);
             if (__any_sync(0xffffffffu, corr != 1.f)) {
-                if (i > 0) ensure_pv(i - 1);
+                if (i > 0) pv_done(i - 1);
                 tc_fence_after();
 #pragma unroll
                 for (int c4 = 0; c4 < D / 32; ++c4) {
@@ -396,14 +412,10 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
             tmem_wait_st();
             tc_fence_before();
             mbar_arrive_cnt(p_full(x, sb));
-            if (++st_i == ST) {
-                st_i = 0;
-                st_ph ^= 1u;
-            }
+            if (++st_i == ST) st_i = 0;
         }
         if (nt > 0) {
-            if (nt > 1) ensure_pv(nt - 2);
-            ensure_pv(nt - 1);
+            pv_done(nt - 1);
             tc_fence_after();
             float inv = 1.0f / l_run;
             if (p.sink) {                               // the reference maximum is in the log2 domain
@@ -469,16 +481,16 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_consta
     }
 }
 
-template <int KB, int VB, int NQ, bool DENSE, bool MOD>
-static int launch(const CUtensorMap& k, const CUtensorMap& k2, const CUtensorMap& v, const Args& a, int ntiles, size_t extra,
+template <int KB, int VB, int NQ, bool DENSE, bool MOD, int QD = KB * 64>
+static int launch(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& k2, const CUtensorMap& v, const Args& a, int ntiles, size_t extra,
                   cudaStream_t st) {
     const size_t smem = smem_for(KB, VB, NQ) + extra;
     const int64_t ctas = (int64_t)ntiles * a.p.num_kv_heads * a.hchunks;
     if (ctas > 0x7fffffff) return PA_ERR_INVALID_ARG;
-    auto kern = attention_tc_kernel<KB, VB, NQ, DENSE, MOD>;
+    auto kern = attention_tc_kernel<KB, VB, NQ, DENSE, MOD, QD>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    kern<<<(unsigned)ctas, threads_for(NQ), smem, st>>>(k, k2, v, a);
+    kern<<<(unsigned)ctas, threads_for(NQ), smem, st>>>(q, k, k2, v, a);
     PA_RETURN_LAUNCH_STATUS();
 }
 
@@ -513,19 +525,20 @@ int masked_attention_tc_launch(const MaskAttnParams& p, int ntiles, int q_tiles,
     a.p = p;
     plan(p.heads / p.num_kv_heads, q_tiles, a.tb, a.hg);
     a.hchunks = (p.heads / p.num_kv_heads + a.hg - 1) / a.hg;
-    a.qd = p.dim;
     a.kn = a.k2_col = 0;
     a.upt = p.tile_size / 16;
     a.total_rows = (int)rows;
     const size_t extra = p.bias_kind == 2 ? (size_t)p.bias_len * a.hg * 4 : 0;
     if (extra > 40 * 1024) return PA_ERR_UNSUPPORTED;
-    CUtensorMap k, v;
+    // the number of query rows is not known here: boxes are only taken of rows that a work item has
+    CUtensorMap q, k, v;
+    if (!make_bf16_map(&q, p.q, 0x7fffffff, p.q_off + (int64_t)p.heads * p.dim, p.q_stride, 64)) return PA_ERR_UNSUPPORTED;
     if (!make_bf16_map(&k, p.k_pool, rows, p.dim, p.dim, 16) || !make_bf16_map(&v, p.v_pool, rows, p.vdim, p.vdim, 16)) return PA_ERR_UNSUPPORTED;
 #define PA_ATC(KB, VB)                                                                                            \
     if (p.dim == KB * 64 && p.vdim == VB * 64) {                                                                  \
         if (q_tiles == 2)                                                                                         \
-            return mod ? launch<KB, VB, 2, false, true>(k, k, v, a, ntiles, extra, st) : launch<KB, VB, 2, false, false>(k, k, v, a, ntiles, extra, st); \
-        return mod ? launch<KB, VB, 1, false, true>(k, k, v, a, ntiles, extra, st) : launch<KB, VB, 1, false, false>(k, k, v, a, ntiles, extra, st); \
+            return mod ? launch<KB, VB, 2, false, true>(q, k, k, v, a, ntiles, extra, st) : launch<KB, VB, 2, false, false>(q, k, k, v, a, ntiles, extra, st); \
+        return mod ? launch<KB, VB, 1, false, true>(q, k, k, v, a, ntiles, extra, st) : launch<KB, VB, 1, false, false>(q, k, k, v, a, ntiles, extra, st); \
     }
     PA_ATC(1, 1) PA_ATC(1, 2) PA_ATC(2, 1) PA_ATC(2, 2)
 #undef PA_ATC
@@ -579,21 +592,23 @@ PA_API int pa_latent_attention_expanded(const void* d_q, int64_t q_stride, int q
     p.sink = d_sink;
     plan(1, q_tiles, a.tb, a.hg);
     a.hchunks = 1;
-    a.qd = dim + rot_dim;
     a.kn = dim;
     a.k2_col = rot_off;
     a.upt = 1;
     a.total_rows = (int)kv_rows;
-    CUtensorMap k, k2, v;
+    CUtensorMap q, k, k2, v;
+    if (!make_bf16_map(&q, d_q, 0x7fffffff, q_off + (int64_t)heads * p.dim, q_stride, 64)) return PA_ERR_UNSUPPORTED;
     if (!make_bf16_map(&k, d_k, kv_rows, (uint64_t)heads * dim, k_stride, 64) || !make_bf16_map(&v, d_v, kv_rows, (uint64_t)heads * vdim, v_stride, 64) ||
         !make_bf16_map(&k2, d_latent, kv_rows, (uint64_t)rot_off + rot_dim, latent_stride, 64))
         return PA_ERR_UNSUPPORTED;
     cudaStream_t st = as_stream(stream);
-#define PA_ATC(KB, VB)                                                                            \
-    if (dim == (KB - 1) * 64 && vdim == VB * 64)                                                  \
-        return q_tiles == 2 ? launch<KB, VB, 2, true, false>(k, k2, v, a, num_q_tiles, 0, st)     \
-                            : launch<KB, VB, 1, true, false>(k, k2, v, a, num_q_tiles, 0, st);
-    PA_ATC(2, 1) PA_ATC(2, 2) PA_ATC(3, 1) PA_ATC(3, 2)
+#define PA_ATC(KB, VB, ROT)                                                                       \
+    if (dim == (KB - 1) * 64 && vdim == VB * 64 && rot_dim == ROT)                                \
+        return q_tiles == 2 ? launch<KB, VB, 2, true, false, (KB - 1) * 64 + ROT>(q, k, k2, v, a, num_q_tiles, 0, st)     \
+                            : launch<KB, VB, 1, true, false, (KB - 1) * 64 + ROT>(q, k, k2, v, a, num_q_tiles, 0, st);
+#define PA_ATC_ROT(ROT) PA_ATC(2, 1, ROT) PA_ATC(2, 2, ROT) PA_ATC(3, 1, ROT) PA_ATC(3, 2, ROT)
+    PA_ATC_ROT(16) PA_ATC_ROT(32) PA_ATC_ROT(48) PA_ATC_ROT(64)
+#undef PA_ATC_ROT
 #undef PA_ATC
     return PA_ERR_UNSUPPORTED;
 }

@@ -633,17 +633,9 @@ __global__ void __launch_bounds__(threads_for(KV, NQ, MW), (NQ == 1 && KV == 0) 
         float m_ref = -INFINITY, l_run = 0.f;  // reference maximum of this row (see the header), running sum
         const uint32_t s_addr = tmem_base + lane_base + x * 2 * KT;
         const uint32_t o_addr = tmem_base + lane_base + NQ * 2 * KT + x * D;
-        // P.V(t') completion: tile t' -> barrier t' & 1, phase t' >> 1.  Every thread consumes the phases of each
-        // barrier in order and at the latest two tiles late (P.V(t') can only be issued after this thread's own
-        // arrival on p_full(t'), so the barrier is never more than one phase ahead of what is waited for).
-        int oc[2] = {0, 0};
-        auto ensure_pv = [&](int tp) {
-            const int bsel = tp & 1, k = tp >> 1;
-            if (oc[bsel] <= k) {
-                mbar_wait_wd(o_full(x, bsel), (uint32_t)(k & 1));
-                oc[bsel] = k + 1;
-            }
-        };
+        // P.V(t') is complete.  Unambiguous without consuming every phase: S(i) follows P.V(i - 2) on the pipe, so by the time a
+        // thread works on tile i the barrier of P.V(i - 1) is in the phase asked for or just past it.
+        auto pv_done = [&](int tp) { mbar_wait_wd(o_full(x, tp & 1), (uint32_t)((tp >> 1) & 1)); };
         int pgn[4];  // page ids of the next tile's 4 units
         auto load_pages = [&](int tile) {
 #pragma unroll
@@ -743,10 +735,9 @@ __global__ void __launch_bounds__(threads_for(KV, NQ, MW), (NQ == 1 && KV == 0) 
             if (qtr == 0) PROBE(x, i, 3);
             const bool dead = m_ref == -INFINITY;  // nothing visible yet (padding rows of the last query tile)
             if (qtr == 0) PROBE(x, i, 4);
-            if (i >= 2) ensure_pv(i - 2);  // complete since S(i) was written: keeps the phase bookkeeping tight
             if (__any_sync(0xffffffffu, corr != 1.f)) {  // warp-collective TMEM access; lanes that keep their
                 // reference multiply by 1.  P.V(i-1) must be complete before O is rescaled.
-                if (i > 0) ensure_pv(i - 1);
+                if (i > 0) pv_done(i - 1);
                 tc_fence_after();
 #pragma unroll
                 for (int c4 = 0; c4 < D / 32; ++c4) {
@@ -780,8 +771,7 @@ __global__ void __launch_bounds__(threads_for(KV, NQ, MW), (NQ == 1 && KV == 0) 
         }
         PROBE_CTA(4);
         if (nt > 0) {
-            if (nt > 1) ensure_pv(nt - 2);
-            ensure_pv(nt - 1);
+            pv_done(nt - 1);
             PROBE_CTA(5);
             tc_fence_after();
             const float inv = 1.f / (l_run + 1e-6f);  // softmax_lut.cpp:224 epsilon (App. A D4)
