@@ -382,13 +382,13 @@ class LatentAttentionMixer:
                                   _cabi.stream()), "pa_head_linear")
         return out
 
-    def _attend_expanded(self, c, q, out):
+    def _attend_expanded(self, c, q, out, at_least):
         """The prompt portions that build the keys and values of their whole sequences: per head a key of dim + rot_dim and a value
         of vdim columns instead of kv_rank + rot_dim and kv_rank, for one product over the cached rows."""
         b, lib, kv, s, H = c.batch, c.lib, self.kv, _cabi.stream(), self.heads
         pt = kv.page_table_
-        q_tiles = 2 if b.count_tiles(self.tc_tokens[0], EXPAND_FROM) * H >= c.model.sm_count else 1
-        for items, nitems, longest, rows, tiles, ntiles in b.whole_sequences(EXPAND_FROM, self.tc_tokens[2 - q_tiles]):
+        q_tiles = 2 if b.count_tiles(self.tc_tokens[0], at_least) * H >= c.model.sm_count else 1
+        for items, nitems, longest, rows, tiles, ntiles in b.whole_sequences(at_least, self.tc_tokens[2 - q_tiles]):
             lat = c.empty(rows, self.kd)
             _chk(lib.pa_latent_gather(kv.key_buffer_.data_ptr(), pt.device_data().data_ptr(), pt.num_beams_, pt.num_tiles_,
                                       kv.total_pages_, kv.tile_size_, self.kd * c.elem, items.data_ptr(), nitems, longest,
@@ -474,7 +474,7 @@ class LatentAttentionMixer:
         proj = c.model._linear(h, self.w_in)
         q = self._queries(c, proj)
         kvr = self.kv_rank
-        expand = EXPAND_FROM if self.w_ukv is not None and c.batch.whole_sequences(EXPAND_FROM, self.tc_tokens[0]) else 0
+        expand = c.batch.expand_from(EXPAND_FROM) if self.w_ukv is not None else 0
         if expand and all(c.batch._expands(p, expand) for p in c.batch.portions):
             ov = c.empty(R, H * self.vdim)
         else:
@@ -486,7 +486,7 @@ class LatentAttentionMixer:
                 self._attend(c, q, ql, lat, False, expand)
             ov = self._head_linear(c, lat, kvr, R * kvr, self.w_uv, kvr, self.vdim, by_row=True).view(R, H * self.vdim)
         if expand:      # its rows of ov; what the product above left there came from no query
-            self._attend_expanded(c, q, ov)
+            self._attend_expanded(c, q, ov, expand)
         if self.gate != "head":
             if self.gate == "elements":
                 _chk(lib.pa_gate_rows(ov.data_ptr(), ov.stride(0), proj.data_ptr() + self.g_off * c.elem, proj.stride(0),

@@ -102,6 +102,15 @@ class RaggedBatch:
         its place in the buffers."""
         return p[1] >= at_least and p[3] + p[1] <= self.EXPAND_MOST
 
+    def expand_from(self, tokens):
+        """From how many new tokens on the portions build keys and values: `tokens` where all of them have that many, else twice as
+        many where some do (the others run beside them, with products over every row), else 0."""
+        key = ("ef", tokens)
+        if key not in self._cache:
+            self._cache[key] = (tokens if all(self._expands(p, tokens) for p in self.portions) else
+                                2 * tokens if any(self._expands(p, 2 * tokens) for p in self.portions) else 0)
+        return self._cache[key]
+
     def whole_sequences(self, at_least, tokens):
         """The portions that _expands picks, in groups of at most EXPAND_MOST tokens of context: per group ([n, 3] int32 items (slot,
         tokens, first row), n, longest, rows, [m, 4] query tiles of at most `tokens` tokens (first batch row, tokens, first row of
@@ -168,6 +177,63 @@ class RaggedBatch:
             a, b = _to_device(a, self.device), _to_device(b, self.device)
             self._cache[key] = (a[0], a[1], b[0], b[1], len(cs))
         return self._cache[key]
+
+
+class DecodeBatch(RaggedBatch):
+    """The description of a step that decodes ONE token of each of n sequences, in device buffers that stay: everything about such
+    a step but the sequences' tokens, slots and positions is the same every time, so the next step writes those into the same
+    places (fill) and the launches of one step serve for all (engine.DecodeSteps).  longest: an upper bound of the sequences'
+    lengths, which the launches are sized for."""
+
+    def __init__(self, n, longest, device, prev_ids):
+        self.rows = self.num_seqs = n
+        self.portions = [(r, 1, 0, 0) for r in range(n)]
+        self.device, self.longest = device, longest
+        # ids, slot, position, previous row, previous token, portion: first row, length, slot | query tiles [n, 4] | portion items
+        # [n, 6] | chunk items [n, 4] | first chunk, chunks
+        self._host = np.zeros(24 * n, dtype=np.int32)
+        self._dev = torch.zeros(24 * n, dtype=torch.int32, device=device)
+        row = np.arange(n, dtype=np.int32)
+        f, h = self._fields(self._dev), self._fields(self._host)
+        self.ids, self.row_slot, self.row_pos, self.row_prev, prev, self.seq_start, self.seq_len, self.seq_slot = f["rows"]
+        self.prev_ids = prev if prev_ids else None
+        h["rows"][3], h["rows"][5], h["rows"][6] = -1, row, 1
+        h["tiles"][:, 0], h["tiles"][:, 1] = row, 1
+        h["items"][:, 0], h["items"][:, 1], h["items"][:, 4] = row, 1, 1
+        h["chunks"][:, 0], h["chunks"][:, 1] = row, 1
+        h["runs"][0], h["runs"][1] = row, 1
+        self._h, self._f = h, f
+
+    def _fields(self, a):
+        n = self.rows
+        return dict(rows=a[:8 * n].reshape(8, n), tiles=a[8 * n:12 * n].reshape(n, 4), items=a[12 * n:18 * n].reshape(n, 6),
+                    chunks=a[18 * n:22 * n].reshape(n, 4), runs=a[22 * n:].reshape(2, n))
+
+    def fill(self, ids, slots, pos, prev):
+        h = self._h
+        h["rows"][0], h["rows"][1], h["rows"][2], h["rows"][4], h["rows"][7] = ids, slots, pos, prev, slots
+        h["tiles"][:, 2], h["tiles"][:, 3] = slots, pos
+        h["items"][:, 2], h["items"][:, 5] = slots, pos
+        h["chunks"][:, 2] = slots
+        _to_device(torch.from_numpy(self._host), self.device, self._dev)
+
+    def query_tiles(self, tile_tokens, big_tokens=0, big_from=0, without=0):
+        return {0: None, 1: (self._f["tiles"], self.rows, self.longest), 2: None}
+
+    def chunk_items(self, chunk):
+        return self._f["chunks"], self.rows, self._f["runs"][0], self._f["runs"][1]
+
+    def portion_items(self, chunk):
+        return self._f["items"], self.rows
+
+    def count_tiles(self, tokens, at_least):
+        return 0
+
+    def expand_from(self, tokens):
+        return 0
+
+    def scan_chunks(self, chunk):
+        raise RuntimeError("a decoded token is no long portion")
 
 
 class SequenceStateCache:
@@ -250,6 +316,22 @@ class SequenceStateCache:
         del self._len[slot]
         self._last.pop(slot, None)
         self._free_slots.append(slot)
+
+    def advance(self, entries):
+        """extend by one token per entry [(slot, [token])], each slot at most once: the tokens, slots, positions and previous tokens
+        (-1: none, or not tracked) as lists."""
+        if len({slot for slot, _toks in entries}) != len(entries):
+            raise ValueError("a sequence may appear once per step")
+        ids, slots, pos, prev = [], [], [], []
+        for slot, toks in entries:
+            t = int(toks[0])
+            pos.append(self.extend(slot, 1))
+            ids.append(t)
+            slots.append(slot)
+            prev.append(self._last.get(slot, -1) if self.track_tokens else -1)
+            if self.track_tokens:
+                self._last[slot] = t
+        return ids, slots, pos, prev
 
     # ---- batch description ------------------------------------------------------------------------------------------
     def make_batch(self, entries):

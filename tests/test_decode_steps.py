@@ -1,0 +1,95 @@
+"""Decode steps replayed from CUDA graphs (llm_decoder.engine.DecodeSteps) against the same steps run launch by launch: the same
+kernels on the same numbers, so the logits agree to the last bit except where a kernel's work split depends on the bound of the
+lengths (bfloat16 sums in another order: 2e-2 of the logits' spread, as for this precision elsewhere)."""
+import pytest
+import torch
+
+from oracle import dubarax_ref, namudra_ref, tiradra_ref
+
+
+def _pair(config, W, **kw):
+    """Two engines over equal models; the second never captures."""
+    import llm_decoder as ld
+    a, b = (ld.Engine(ld.HybridDecoder(config, W, "bfloat16", **kw)) for _ in range(2))
+    a._decode.PATIENCE = 2
+    b._decode.serves = lambda *_a: False
+    return a, b
+
+
+def _config(name):
+    if name == "tiradra":
+        R = tiradra_ref
+        c = R.make_config([R.attention_layer(dim=64, heads=4, kv_heads=2), R.latent_layer()], loop={"start": 0, "stop": 2, "times": 2})
+    elif name == "namudra":
+        R = namudra_ref
+        c = R.make_config([R.retention_layer(ff=32)], streams=2)
+    else:
+        R = dubarax_ref
+        c = R.make_config([R.attention_layer(mlp=R.moe_mlp()), R.mamba_layer(mlp=R.moe_mlp())])
+    return c, R.random_weights(c, 3)
+
+
+def _close(x, y):
+    assert torch.isfinite(x).all() and (x - y).abs().max() < 2e-2 * y.abs().max(), (x - y).abs().max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", ["tiradra", "namudra", "dubarax"])
+def test_replayed_steps_equal_launched_ones(name):
+    """Requests of unequal length decode together, some end and others take their slots, the number of sequences changes, a step is
+    skipped by one of them, and the lengths cross the bound of 256."""
+    config, W = _config(name)
+    a, b = _pair(config, W, max_tokens=2048, max_seqs=4)
+    g = torch.Generator().manual_seed(1)
+    tok = lambda n=1: torch.randint(0, config["vocab"], (n,), generator=g).tolist()  # noqa: E731
+    both = lambda entries: (a.step(entries), b.step(entries))  # noqa: E731
+    _close(*both([(0, tok(7), [6]), (1, tok(250), [249]), (2, tok(1), [0])]))
+    for k in range(12):
+        _close(*both([(i, tok(), [0]) for i in (0, 1, 2)]))
+    assert a._decode._graphs
+    for e in (a, b):
+        e.finish(0)
+    _close(*both([(3, tok(30), [29]), (1, tok(), [0])]))            # a prompt beside a decoded token: launched
+    for k in range(4):
+        _close(*both([(i, tok(), [0]) for i in (3, 1, 2)]))         # the slot of request 0
+        _close(*both([(i, tok(), [0]) for i in (2, 3)]))
+        x, y = both([(i, tok(), [0] if i == 2 else []) for i in (2, 3)])
+        assert x.shape[0] == 1
+        _close(x, y)
+    with pytest.raises(ValueError):
+        a.step([(2, [1], [1])])
+
+
+@pytest.mark.gpu
+def test_replaced_weights_hooks_and_streams():
+    """A weight replaced by another tensor, or given other storage, is seen by the next step; results of earlier steps stay; steps on
+    changing streams keep their order; a hook makes steps run launch by launch."""
+    config, W = _config("tiradra")
+    a, b = _pair(config, W, max_tokens=512, max_seqs=2)
+    step = lambda t: (a.step([(0, [t], [0]), (1, [t + 1], [0])]), b.step([(0, [t], [0]), (1, [t + 1], [0])]))  # noqa: E731
+    first = [step(t) for t in range(4)]
+    kept = [x.clone() for x, _y in first]
+    for m in (a.model, b.model):
+        m.head = m.head * 0.5
+    x, y = step(5)
+    _close(x, y)
+    for _ in range(4):
+        _close(*step(6))
+    for m in (a.model, b.model):
+        m.head.data = m.head.data * 3.0
+    for _ in range(4):
+        _close(*step(7))
+    for m in (a.model, b.model):
+        m.head.mul_(0.25)                       # in place: the graph reads the new numbers
+    _close(*step(8))
+    assert all(torch.equal(p, x) for p, (x, _y) in zip(kept, first))
+    s = torch.cuda.Stream()
+    for k in range(6):
+        s.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(s if k % 2 else torch.cuda.current_stream()):
+            _close(*step(9 + k))
+        torch.cuda.current_stream().wait_stream(s)
+    calls = []
+    a.model.layer_hook = b.model.layer_hook = lambda x: calls.append(1)
+    _close(*step(20))
+    assert calls
