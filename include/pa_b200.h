@@ -853,6 +853,15 @@ int pa_decay_scan_rotated(const void* d_q, int64_t q_stride, int q_off, const vo
                           float* d_state, float* d_out, int64_t out_stride, const int32_t* d_items, int num_items,
                           const int32_t* d_seq_chunk0, const int32_t* d_seq_nchunks, const int32_t* d_seq_slot, int num_seqs,
                           int chunked, void* d_workspace, size_t workspace_bytes, int elem, pa_stream_t stream);
+/* pa_decay_scan_rotated for items of at most chunk_tokens tokens (0: unknown): chunks of up to 64 tokens with a constant decay, no
+ * activation, bfloat16 rows and a 64 x 64 or 64 x 128 state are folded and replayed as matrix products. */
+int pa_decay_scan_chunked(const void* d_q, int64_t q_stride, int q_off, const void* d_k, int64_t k_stride, int k_off,
+                          const void* d_v, int64_t v_stride, int v_off, int heads, int groups, int dim, int vdim, int act,
+                          const float* d_decay, const void* d_dt, int64_t dt_stride, int dt_off, const float* d_dt_bias,
+                          const float* d_a_log, const float* d_skip, const float* d_rope, int rot_dims, float k_scale,
+                          float* d_state, float* d_out, int64_t out_stride, const int32_t* d_items, int num_items,
+                          const int32_t* d_seq_chunk0, const int32_t* d_seq_nchunks, const int32_t* d_seq_slot, int num_seqs,
+                          int chunked, void* d_workspace, size_t workspace_bytes, int elem, int chunk_tokens, pa_stream_t stream);
 int pa_rope_rows_paired(void* d_x, int64_t stride, int off, int head_stride, int heads, int dims, const float* d_table,
                         int pairing, int rows, int elem, pa_stream_t stream);
 int pa_latent_norm_append(void* d_pool, const int32_t* d_table, int num_slots, int num_tiles, int total_pages,

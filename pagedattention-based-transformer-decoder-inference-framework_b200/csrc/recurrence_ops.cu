@@ -310,6 +310,273 @@ __global__ void __launch_bounds__(kDsMaxThreads) decay_scan_kernel(const DecaySc
     if (MODE == 1 && threadIdx.x == 0 && blockIdx.z == 0) dst[sz] = total;
 }
 
+// ---- fold and replay of chunks of up to 64 tokens as matrix products (constant decays, bfloat16 rows) -----------------------
+// With a constant decay d the tokens of a chunk need no walk:  fold   S = sum_t d^(n-1-t) k_t v_t^T
+//                                                             replay o_t = sum_{s<=t} d^(t-s) (q_t . k_s) v_s + d^(t+1) S0^T q_t
+// and both run on the tensor cores (mma.sync m16n8k16, float accumulators) WITHOUT giving up float operands: every float factor
+// (rotated q and k, weighted k, the scores with their decays, the incoming state) is the sum of three bfloat16 numbers, 24 bits
+// of it, and a product of two such factors keeps the six terms that reach 2^-24; the value rows are bfloat16 as they come.  One CTA
+// of four warps per (chunk, head); a warp has 16 rows of the result.
+// What bounds it: issue of ldmatrix and mma.sync.  4 x 2048 tokens, 16 heads of 64 x 128: fold 60 us, replay 146 us; the
+// walk on the float pipe 141 and 231 us.  Error of the layer against float64 4.3e-3 either way (rounding of the result).
+constexpr int kDmTokens = 64, kDmDim = 64, kDmLd = kDmDim + 8, kDmThreads = 128;
+
+__device__ __forceinline__ void dm_split(float x, bf16_t (&b)[3]) {
+    b[0] = __float2bfloat16_rn(x);
+    float r = isfinite(x) ? x - __bfloat162float(b[0]) : 0.f;
+    b[1] = __float2bfloat16_rn(r);
+    r -= __bfloat162float(b[1]);
+    b[2] = __float2bfloat16_rn(r);
+}
+// two neighbouring columns split into three planes `plane` elements apart
+__device__ __forceinline__ void dm_store2(bf16_t* dst, int plane, float x, float y) {
+    bf16_t a[3], b[3];
+    dm_split(x, a);
+    dm_split(y, b);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        __nv_bfloat162 v;
+        v.x = a[i];
+        v.y = b[i];
+        *reinterpret_cast<__nv_bfloat162*>(dst + i * plane) = v;
+    }
+}
+// rows of q or k of one head: rotated (halves), times f(token), zeros past the chunk's end
+template <typename F>
+__device__ __forceinline__ void dm_stage(const DecayScanParams& p, const bf16_t* src, int64_t stride, int row0, int n, bf16_t* dst, F f) {
+    const int half = p.rope ? p.rot_dims >> 1 : 0;
+    constexpr int U = 8;                                    // pieces of two columns whose loads are in flight together
+#pragma unroll 1
+    for (int i0 = 0; i0 < kDmTokens * kDmDim / 2; i0 += U * kDmThreads) {
+        uint32_t xw[U], yw[U];
+        float4 cs[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int idx = i0 + u * kDmThreads + threadIdx.x, t = idx / (kDmDim / 2), d = idx % (kDmDim / 2) * 2;
+            const bool ok = t < n;
+            const bf16_t* r = src + (int64_t)(row0 + (ok ? t : 0)) * stride;
+            xw[u] = ok ? *reinterpret_cast<const uint32_t*>(r + d) : 0u;
+            yw[u] = ok && d < half ? *reinterpret_cast<const uint32_t*>(r + d + half) : 0u;
+            cs[u] = make_float4(1.f, 0.f, 1.f, 0.f);
+            if (ok && d < half) cs[u] = *reinterpret_cast<const float4*>(p.rope + ((int64_t)(row0 + t) * half + d) * 2);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int idx = i0 + u * kDmThreads + threadIdx.x, t = idx / (kDmDim / 2), d = idx % (kDmDim / 2) * 2;
+            if (d >= half && d < 2 * half) continue;        // the partners of the first half
+            const float w = t < n ? f(t) : 0.f;
+            const float x0 = __uint_as_float(xw[u] << 16), x1 = __uint_as_float(xw[u] & 0xffff0000u);
+            const float y0 = __uint_as_float(yw[u] << 16), y1 = __uint_as_float(yw[u] & 0xffff0000u);
+            if (d < half)
+                dm_store2(dst + t * kDmLd + d + half, kDmTokens * kDmLd, (y0 * cs[u].x + x0 * cs[u].y) * w, (y1 * cs[u].z + x1 * cs[u].w) * w);
+            dm_store2(dst + t * kDmLd + d, kDmTokens * kDmLd, (x0 * cs[u].x - y0 * cs[u].y) * w, (x1 * cs[u].z - y1 * cs[u].w) * w);
+        }
+    }
+}
+template <int VD>
+__device__ __forceinline__ void dm_stage_values(const DecayScanParams& p, int h, int row0, int n, bf16_t* dst) {
+    const bf16_t* vb = static_cast<const bf16_t*>(p.v) + p.v_off + (int64_t)h * VD;
+#pragma unroll
+    for (int i = 0; i < kDmTokens * VD / 8 / kDmThreads; ++i) {
+        const int idx = i * kDmThreads + threadIdx.x, t = idx / (VD / 8), c = idx % (VD / 8) * 8;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (t < n) v = *reinterpret_cast<const uint4*>(vb + (int64_t)(row0 + t) * p.v_stride + c);
+        *reinterpret_cast<uint4*>(dst + t * (VD + 8) + c) = v;
+    }
+}
+// d^0 .. d^64
+__device__ __forceinline__ void dm_powers(float d, float* pw) {
+    for (int j = threadIdx.x; j <= kDmTokens; j += blockDim.x) {
+        double r = 1.0, b = d;
+        for (int e = j; e; e >>= 1, b *= b)
+            if (e & 1) r *= b;
+        pw[j] = (float)r;
+    }
+}
+// o[n-tile] += A (16 x 16, fragment a) . B: 16 rows of a [.][ld] matrix from row k0, all VD columns
+template <int VD>
+__device__ __forceinline__ void dm_rows_product(float (&o)[VD / 8][4], const uint32_t (&a)[4], const bf16_t* B, int ld, int k0, int lane) {
+#pragma unroll
+    for (int np = 0; np < VD / 16; ++np) {
+        uint32_t b0, b1, b2, b3;
+        ldsm_x4_trans(smem_u32(B + (k0 + (lane & 7) + ((lane >> 3) & 1) * 8) * ld + np * 16 + (lane >> 4) * 8), b0, b1, b2, b3);
+        mma_bf16_16816(o[2 * np], a, b0, b1);
+        mma_bf16_16816(o[2 * np + 1], a, b2, b3);
+    }
+}
+
+template <int VD>
+__global__ void __launch_bounds__(kDmThreads) decay_fold_mma_kernel(const DecayScanParams p) {
+    extern __shared__ __align__(16) unsigned char dm_smem[];
+    bf16_t* Ks = reinterpret_cast<bf16_t*>(dm_smem);                  // [3][64][kDmLd]
+    bf16_t* Vs = Ks + 3 * kDmTokens * kDmLd;                          // [64][VD + 8]
+    __shared__ float pw[kDmTokens + 1];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = blockIdx.y, g = h / (p.heads / p.groups);
+    const int* it = p.items + 4 * blockIdx.x;
+    const int row0 = it[0], n = it[1];
+    dm_powers(p.decay[h], pw);
+    dm_stage_values<VD>(p, h, row0, n, Vs);
+    __syncthreads();
+    dm_stage(p, static_cast<const bf16_t*>(p.k) + p.k_off + (int64_t)g * kDmDim, p.k_stride, row0, n, Ks,
+             [&](int t) { return pw[n - 1 - t] * p.k_scale; });
+    __syncthreads();
+    float o[VD / 8][4];
+#pragma unroll
+    for (int i = 0; i < VD / 8; ++i)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) o[i][c] = 0.f;
+#pragma unroll
+    for (int x = 2; x >= 0; --x)                                      // the small terms first
+#pragma unroll
+        for (int ks = 0; ks < kDmTokens; ks += 16) {
+            uint32_t a[4];                                            // rows = dimensions, read across the tokens' rows
+            ldsm_x4_trans(smem_u32(Ks + (x * kDmTokens + ks + (lane & 7) + (lane >> 4) * 8) * kDmLd + warp * 16 + ((lane >> 3) & 1) * 8), a[0],
+                          a[1], a[2], a[3]);
+            dm_rows_product<VD>(o, a, Vs, VD + 8, ks, lane);
+        }
+    const int64_t sz = (int64_t)kDmDim * VD;
+    float* dst = p.part + ((int64_t)blockIdx.x * p.heads + h) * (sz + 1);
+#pragma unroll
+    for (int i = 0; i < VD / 8; ++i)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) dst[(warp * 16 + (lane >> 2) + (c >> 1) * 8) * VD + i * 8 + 2 * (lane & 3) + (c & 1)] = o[i][c];
+    if (threadIdx.x == 0) dst[sz] = pw[n];
+}
+
+template <int VD>
+__global__ void __launch_bounds__(kDmThreads, 2) decay_replay_mma_kernel(const DecayScanParams p) {
+    extern __shared__ __align__(16) unsigned char dm_smem[];
+    bf16_t* Ks = reinterpret_cast<bf16_t*>(dm_smem);                  // [3][64][kDmLd]
+    bf16_t* Vs = Ks + 3 * kDmTokens * kDmLd;                          // [64][VD + 8]
+    bf16_t* Ss = Vs + kDmTokens * (VD + 8);                           // [3][64][VD + 8]: first the queries, then the incoming state
+    __shared__ float pw[kDmTokens + 1];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = blockIdx.y, g = h / (p.heads / p.groups);
+    const int* it = p.items + 4 * blockIdx.x;
+    const int row0 = it[0], n = it[1];
+    dm_powers(p.decay[h], pw);
+    dm_stage_values<VD>(p, h, row0, n, Vs);
+    dm_stage(p, static_cast<const bf16_t*>(p.k) + p.k_off + (int64_t)g * kDmDim, p.k_stride, row0, n, Ks, [&](int) { return p.k_scale; });
+    dm_stage(p, static_cast<const bf16_t*>(p.q) + p.q_off + (int64_t)g * kDmDim, p.q_stride, row0, n, Ss, [](int) { return 1.f; });
+    __syncthreads();
+    uint32_t qf[3][kDmDim / 16][4];
+#pragma unroll
+    for (int x = 0; x < 3; ++x)
+#pragma unroll
+        for (int ks = 0; ks < kDmDim / 16; ++ks)
+            ldsm_x4(smem_u32(Ss + (x * kDmTokens + warp * 16 + (lane & 15)) * kDmLd + ks * 16 + (lane >> 4) * 8), qf[x][ks][0], qf[x][ks][1],
+                    qf[x][ks][2], qf[x][ks][3]);
+    __syncthreads();
+    const int64_t sz = (int64_t)kDmDim * VD;
+    const float* S0 = p.part + ((int64_t)blockIdx.x * p.heads + h) * (sz + 1);
+#pragma unroll 1
+    for (int i0 = 0; i0 < kDmDim * VD / 2; i0 += 16 * kDmThreads) {
+        float x[16], y[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) {
+            const int at = (i0 + u * kDmThreads + threadIdx.x) * 2;
+            x[u] = S0[at];
+            y[u] = S0[at + 1];
+        }
+#pragma unroll
+        for (int u = 0; u < 16; ++u) {
+            const int idx = i0 + u * kDmThreads + threadIdx.x, d = idx / (VD / 2), c = idx % (VD / 2) * 2;
+            dm_store2(Ss + d * (VD + 8) + c, kDmDim * (VD + 8), x[u], y[u]);
+        }
+    }
+    // scores of this warp's tokens against the keys up to them
+    float s[kDmTokens / 8][4];
+#pragma unroll
+    for (int i = 0; i < kDmTokens / 8; ++i)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) s[i][c] = 0.f;
+#pragma unroll
+    for (int np = 0; np < kDmTokens / 16; ++np) {
+        if (np > warp) break;
+#pragma unroll
+        for (int ks = 0; ks < kDmDim / 16; ++ks)
+#pragma unroll
+            for (int y = 2; y >= 0; --y) {
+                uint32_t b0, b1, b2, b3;
+                ldsm_x4(smem_u32(Ks + (y * kDmTokens + np * 16 + (lane & 7) + ((lane >> 4) << 3)) * kDmLd + ks * 16 + ((lane >> 3) & 1) * 8), b0,
+                        b1, b2, b3);
+#pragma unroll
+                for (int x = 2 - y; x >= 0; --x) {
+                    mma_bf16_16816(s[2 * np], qf[x][ks], b0, b1);
+                    mma_bf16_16816(s[2 * np + 1], qf[x][ks], b2, b3);
+                }
+            }
+    }
+    __syncthreads();                                                  // the state is staged
+    float o[VD / 8][4];
+#pragma unroll
+    for (int i = 0; i < VD / 8; ++i)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) o[i][c] = 0.f;
+#pragma unroll
+    for (int y = 2; y >= 0; --y)
+#pragma unroll
+        for (int x = 2 - y; x >= 0; --x)
+#pragma unroll
+            for (int ks = 0; ks < kDmDim / 16; ++ks) dm_rows_product<VD>(o, qf[x][ks], Ss + y * kDmDim * (VD + 8), VD + 8, ks * 16, lane);
+    const int t0 = warp * 16 + (lane >> 2);
+    const float in0 = pw[t0 + 1], in1 = pw[t0 + 9];
+#pragma unroll
+    for (int i = 0; i < VD / 8; ++i) {
+        o[i][0] *= in0;
+        o[i][1] *= in0;
+        o[i][2] *= in1;
+        o[i][3] *= in1;
+    }
+#pragma unroll
+    for (int kk = 0; kk < kDmTokens / 16; ++kk) {
+        if (kk > warp) break;
+        uint32_t a[3][4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {                                 // rows g, g + 8, then the second eight keys
+            const int i = 2 * kk + (j >> 1), r = j & 1;
+            bf16_t u[3], w[3];
+            const int dist = t0 + 8 * r - (i * 8 + 2 * (lane & 3));
+            dm_split(dist >= 0 ? s[i][2 * r] * pw[dist] : 0.f, u);
+            dm_split(dist >= 1 ? s[i][2 * r + 1] * pw[dist - 1] : 0.f, w);
+#pragma unroll
+            for (int x = 0; x < 3; ++x) {
+                __nv_bfloat162 v;
+                v.x = u[x];
+                v.y = w[x];
+                a[x][j] = *reinterpret_cast<const uint32_t*>(&v);
+            }
+        }
+#pragma unroll
+        for (int x = 2; x >= 0; --x) dm_rows_product<VD>(o, a[x], Vs, VD + 8, kk * 16, lane);
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const int t = t0 + 8 * r;
+        if (t >= n) continue;
+        float* dst = p.out + (int64_t)(row0 + t) * p.out_stride + (int64_t)h * VD + 2 * (lane & 3);
+#pragma unroll
+        for (int i = 0; i < VD / 8; ++i) *reinterpret_cast<float2*>(dst + i * 8) = make_float2(o[i][2 * r], o[i][2 * r + 1]);
+    }
+}
+
+// Whether the chunks run as matrix products: chunks of at most 64 tokens, bfloat16 rows, a constant decay, no activation, states of
+// 64 x 64 or 64 x 128, and rows whose staged pieces are aligned.
+static bool dm_ok(const DecayScanParams& p, int chunk_tokens, int elem) {
+    return chunk_tokens > 0 && chunk_tokens <= kDmTokens && elem == 2 && !p.dt && !p.act && !p.skip && p.dim == kDmDim &&
+           (p.vdim == 64 || p.vdim == 128) && p.rot_dims % 4 == 0 && (uintptr_t)p.rope % 16 == 0 && p.q_stride % 2 == 0 && p.q_off % 2 == 0 &&
+           (uintptr_t)p.q % 4 == 0 && p.k_stride % 2 == 0 && p.k_off % 2 == 0 && (uintptr_t)p.k % 4 == 0 && p.v_stride % 8 == 0 &&
+           p.v_off % 8 == 0 && (uintptr_t)p.v % 16 == 0 && p.out_stride % 2 == 0 && (uintptr_t)p.out % 8 == 0;
+}
+template <int VD, bool REPLAY>
+static int dm_launch(const DecayScanParams& p, int num_items, cudaStream_t st) {
+    const size_t smem = sizeof(bf16_t) * (3 * kDmTokens * kDmLd + kDmTokens * (VD + 8) + (REPLAY ? 3 * kDmDim * (VD + 8) : 0));
+    auto kern = REPLAY ? decay_replay_mma_kernel<VD> : decay_fold_mma_kernel<VD>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    kern<<<dim3((unsigned)num_items, (unsigned)p.heads), kDmThreads, smem, st>>>(p);
+    PA_RETURN_LAUNCH_STATUS();
+}
+
 // Chain pass of the chunked scan: per (portion, head, state element) walk the portion's chunks in order from the state
 // slot; every chunk's folded state is replaced by its INCOMING state, and the slot gets the state after the last chunk.
 __global__ void __launch_bounds__(256) decay_chunk_chain_kernel(float* __restrict__ part, int heads, int64_t sz,
@@ -573,6 +840,19 @@ PA_API int pa_decay_scan_rotated(const void* d_q, int64_t q_stride, int q_off, c
                          const int32_t* d_items, int num_items, const int32_t* d_seq_chunk0, const int32_t* d_seq_nchunks,
                          const int32_t* d_seq_slot, int num_seqs, int chunked, void* d_workspace, size_t workspace_bytes,
                          int elem, pa_stream_t stream) {
+    return pa_decay_scan_chunked(d_q, q_stride, q_off, d_k, k_stride, k_off, d_v, v_stride, v_off, heads, groups, dim, vdim, act, d_decay, d_dt,
+                                 dt_stride, dt_off, d_dt_bias, d_a_log, d_skip, d_rope, rot_dims, k_scale, d_state, d_out, out_stride, d_items,
+                                 num_items, d_seq_chunk0, d_seq_nchunks, d_seq_slot, num_seqs, chunked, d_workspace, workspace_bytes, elem, 0,
+                                 stream);
+}
+
+PA_API int pa_decay_scan_chunked(const void* d_q, int64_t q_stride, int q_off, const void* d_k, int64_t k_stride, int k_off,
+                         const void* d_v, int64_t v_stride, int v_off, int heads, int groups, int dim, int vdim, int act,
+                         const float* d_decay, const void* d_dt, int64_t dt_stride, int dt_off, const float* d_dt_bias,
+                         const float* d_a_log, const float* d_skip, const float* d_rope, int rot_dims, float k_scale, float* d_state, float* d_out, int64_t out_stride,
+                         const int32_t* d_items, int num_items, const int32_t* d_seq_chunk0, const int32_t* d_seq_nchunks,
+                         const int32_t* d_seq_slot, int num_seqs, int chunked, void* d_workspace, size_t workspace_bytes,
+                         int elem, int chunk_tokens, pa_stream_t stream) {
     PA_CHECK_ARG(d_q && d_k && d_v && d_state && d_out && d_items && num_items >= 0);
     PA_CHECK_ARG(heads > 0 && groups > 0 && heads % groups == 0 && dim > 0 && vdim > 0);
     PA_CHECK_ARG(d_dt ? (d_dt_bias && d_a_log) : d_decay != nullptr);
@@ -598,10 +878,17 @@ PA_API int pa_decay_scan_rotated(const void* d_q, int64_t q_stride, int q_off, c
     }
     PA_CHECK_ARG(d_seq_chunk0 && d_seq_nchunks && d_seq_slot && num_seqs > 0);
     if (!d_workspace || workspace_bytes < pa_decay_scan_workspace_bytes(num_items, heads, dim, vdim)) return PA_ERR_WORKSPACE;
-    PA_DS(1);
+    const bool products = dm_ok(p, chunk_tokens, elem);
+    if (products) {
+        const int rc = vdim == 64 ? dm_launch<64, false>(p, num_items, st) : dm_launch<128, false>(p, num_items, st);
+        if (rc != PA_OK) return rc;
+    } else {
+        PA_DS(1);
+    }
     const int64_t sz = (int64_t)dim * vdim;
     dim3 grid((unsigned)((sz + 255) / 256), (unsigned)heads, (unsigned)num_seqs);
     decay_chunk_chain_kernel<<<grid, 256, 0, st>>>(p.part, heads, sz, d_seq_chunk0, d_seq_nchunks, d_seq_slot, d_state);
+    if (products) return vdim == 64 ? dm_launch<64, true>(p, num_items, st) : dm_launch<128, true>(p, num_items, st);
     PA_DS(2);
 #undef PA_DS
     PA_RETURN_LAUNCH_STATUS();

@@ -196,6 +196,9 @@ _SIGS = {
     "pa_decay_scan_rotated": ([_vp, _i64, _i32, _vp, _i64, _i32, _vp, _i64, _i32, _i32, _i32, _i32, _i32, _i32, _vp, _vp, _i64,
                                _i32, _vp, _vp, _vp, _vp, _i32, _f32, _vp, _vp, _i64, _vp, _i32, _vp, _vp, _vp, _i32, _i32, _vp,
                                _sz, _i32, _vp], _i32),
+    "pa_decay_scan_chunked": ([_vp, _i64, _i32, _vp, _i64, _i32, _vp, _i64, _i32, _i32, _i32, _i32, _i32, _i32, _vp, _vp, _i64,
+                               _i32, _vp, _vp, _vp, _vp, _i32, _f32, _vp, _vp, _i64, _vp, _i32, _vp, _vp, _vp, _i32, _i32, _vp,
+                               _sz, _i32, _i32, _vp], _i32),
     "pa_rope_rows_paired": ([_vp, _i64, _i32, _i32, _i32, _i32, _vp, _i32, _i32, _i32, _vp], _i32),
     "pa_latent_norm_append": ([_vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _vp, _i64, _i32, _vp, _f32, _vp, _i32,
                                _i32, _vp, _vp, _i64, _vp, _vp, _i32, _i32, _vp], _i32),

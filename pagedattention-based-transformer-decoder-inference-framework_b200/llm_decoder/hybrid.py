@@ -832,13 +832,13 @@ def decay_scan(c, state, out, heads, groups, dim, vdim, q, k, v, act=0, decay=No
     ws = None
     if chunked:
         ws = c.empty(lib.pa_decay_scan_workspace_bytes(n, heads, dim, vdim), dtype=torch.uint8)
-    _chk(lib.pa_decay_scan_rotated(
+    _chk(lib.pa_decay_scan_chunked(
         q[0].data_ptr(), q[0].stride(0), q[1], k[0].data_ptr(), k[0].stride(0), k[1], v[0].data_ptr(), v[0].stride(0), v[1],
         heads, groups, dim, vdim, act, _cabi.ptr(decay), dt[0].data_ptr() if dt else None, dt[0].stride(0) if dt else 0,
         dt[1] if dt else 0, _cabi.ptr(dt_bias), _cabi.ptr(a_log), _cabi.ptr(skip), _cabi.ptr(rope), rot_dims, k_scale,
         state.data_ptr(), out.data_ptr(), out.stride(0), items.data_ptr(), n, s0.data_ptr(), sn.data_ptr(),
         b.seq_slot.data_ptr(), b.num_seqs, 1 if chunked else 0, _cabi.ptr(ws), ws.numel() if ws is not None else 0, c.elem,
-        _cabi.stream()), "pa_decay_scan_rotated")
+        DECAY_CHUNK if chunked else 0, _cabi.stream()), "pa_decay_scan_chunked")
 
 
 class DecayLinearAttention:
