@@ -10,11 +10,13 @@ are fed in chunks under a per-step token budget next to the running requests' si
 of every request whose last fed token ended its prompt (or was a decoded token) is sampled on the device with the
 framework's samplers (greedy pa_argmax_f32; temperature / top-k / top-p through llm_decoder.sampling)."""
 import collections
+import types
 
 import torch
 
 from . import _cabi
 from .host_stage import to_device as _to_device
+from .hybrid import HybridDecoder
 from .seq_state import DecodeBatch
 
 
@@ -35,7 +37,8 @@ class DecodeSteps:
 
     def serves(self, entries, wanted_rows):
         m = self.model
-        return (len(entries) <= self.SEQS and m.act_dtype == torch.bfloat16 and m.device.type == "cuda" and m.layer_hook is None and
+        return (type(m) is HybridDecoder and len(entries) <= self.SEQS and m.act_dtype == torch.bfloat16 and m.device.type == "cuda" and
+                m.layer_hook is None and
                 len(wanted_rows) == len(entries) and all(len(t) == 1 for _s, t in entries) and
                 not torch.cuda.is_current_stream_capturing())
 
@@ -79,6 +82,8 @@ class DecodeSteps:
                 self._seen.clear()
             self._seen[key] = self._seen.get(key, 0) + 1
             return None
+        if g is None and any(isinstance(v, (types.FunctionType, types.MethodType)) for _d, _n, items in self._watched()[0] for _k, v, _p in items):
+            return None         # a function put in the place of a method may do more than launch kernels
         if g is None:
             g = dict(batch=DecodeBatch(len(entries), bound, m.device, st.track_tokens), graph=None, stream=None, event=torch.cuda.Event())
         stream = torch.cuda.current_stream(m.device)
@@ -88,7 +93,11 @@ class DecodeSteps:
         for kv in st._tables:
             kv.page_table_.flush()              # no update of a table belongs into the graph
         if g["graph"] is None:
-            self._capture(g, stream)
+            try:
+                self._capture(g, stream)
+            except RuntimeError:        # memory, or a library call that cannot be captured: this kind stays with launches
+                self._seen[key] = -(1 << 60)
+                return m.forward(g["batch"], torch.arange(g["batch"].rows, dtype=torch.int32, device=m.device))
             self._graphs[key] = g
             while len(self._graphs) > self.MOST:
                 self._graphs.popitem(last=False)

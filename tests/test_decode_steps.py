@@ -93,3 +93,24 @@ def test_replaced_weights_hooks_and_streams():
     a.model.layer_hook = b.model.layer_hook = lambda x: calls.append(1)
     _close(*step(20))
     assert calls
+
+
+@pytest.mark.gpu
+def test_functions_in_place_of_methods_and_failed_captures():
+    """A method replaced on the instance is called in every step; a capture that fails leaves the step to launches."""
+    config, W = _config("tiradra")
+    a, b = _pair(config, W, max_tokens=256, max_seqs=1)
+    calls, real = [], a.model._linear
+    a.model._linear = lambda *args, **kw: (calls.append(1), real(*args, **kw))[1]
+    for k in range(6):
+        n = len(calls)
+        _close(a.step([(0, [k], [0])]), b.step([(0, [k], [0])]))
+        assert len(calls) > n
+    del a.model._linear
+
+    def fails(*_a):
+        raise RuntimeError("no capture")
+    a._decode._capture = fails
+    for k in range(6):
+        _close(a.step([(0, [k + 9], [0])]), b.step([(0, [k + 9], [0])]))
+    assert not a._decode._graphs
