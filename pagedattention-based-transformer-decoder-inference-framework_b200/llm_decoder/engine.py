@@ -24,16 +24,35 @@ class DecodeSteps:
     """Steps that decode one token of each of n sequences, as CUDA graphs: such a step is some dozens of launches of a few
     microseconds each, and issuing them takes several times as long as running them (8 sequences, 4 layers of width 1024: 1.0 ms
     launch by launch, 0.3 ms replayed).  A graph belongs to a number of sequences and a bound of their lengths (a power of two).
-    A capture costs 6 to 30 ms, so the first PATIENCE steps of a kind run launch by launch; from then on a step writes its tokens,
-    slots and positions into the graph's buffers and replays it.
+    A capture costs as much as 6 to 30 launched steps, so the first PATIENCE steps of a kind run launch by launch; from then on a
+    step writes its tokens, slots and positions into the graph's buffers and replays it.  Where more kinds come up than graphs are kept,
+    captures stay rare: one in GAP steps at most, a graph gives way only after IDLE steps without a replay, and a kind that was captured
+    before has to come up twice as often as the last time.
 
     A graph holds the addresses of the model's weights and caches.  It keeps those tensors alive, and before every replay every
     attribute of the model, its layers, their parts and the caches has to be the very object it was at the capture: anything that
     was replaced since makes the step run launch by launch and be captured anew."""
-    MOST, SEQS, PATIENCE = 8, 256, 16       # graphs kept; sequences of a step; steps of a kind before it is captured
+    MOST, SEQS = 8, 256                     # graphs kept; sequences of a step
+    PATIENCE, GAP, IDLE = 16, 64, 256       # in steps, see above
 
     def __init__(self, model):
-        self.model, self._graphs, self._seen, self._side = model, collections.OrderedDict(), {}, None
+        self.model, self._side = model, None
+        self._graphs = collections.OrderedDict()        # kind -> graph, the one whose replay is longest ago first
+        self._seen, self._caught = {}, {}               # kind -> launched steps since its last capture; captures
+        self._now, self._last = 0, None                 # steps so far; the step of the last capture
+
+    def _due(self, key):
+        """Whether a step of a kind without a graph captures one."""
+        seen = self._seen.get(key, 0)
+        due = (seen >= self.PATIENCE << min(self._caught.get(key, 0), 20) and
+               (self._last is None or self._now - self._last >= self.GAP) and
+               (len(self._graphs) < self.MOST or self._now - next(iter(self._graphs.values()))["used"] >= self.IDLE))
+        if not due:
+            if len(self._seen) > 64 * self.MOST:        # kinds that came up now and then
+                self._seen.clear()
+                self._caught.clear()
+            self._seen[key] = seen + 1
+        return due
 
     def serves(self, entries, wanted_rows):
         m = self.model
@@ -72,15 +91,12 @@ class DecodeSteps:
         while bound < longest:
             bound *= 2
         key = (len(entries), bound)
+        self._now += 1
         g = self._graphs.get(key)
         if g is not None and not self._same(g["watched"]):
             del self._graphs[key]
             g = None
-            self._seen.pop(key, None)
-        if g is None and self._seen.get(key, 0) < self.PATIENCE:
-            if len(self._seen) > 64 * self.MOST:        # kinds that came up now and then
-                self._seen.clear()
-            self._seen[key] = self._seen.get(key, 0) + 1
+        if g is None and not self._due(key):
             return None
         if g is None and any(isinstance(v, (types.FunctionType, types.MethodType)) for _d, _n, items in self._watched()[0] for _k, v, _p in items):
             return None         # a function put in the place of a method may do more than launch kernels
@@ -98,10 +114,12 @@ class DecodeSteps:
             except RuntimeError:        # memory, or a library call that cannot be captured: this kind stays with launches
                 self._seen[key] = -(1 << 60)
                 return m.forward(g["batch"], torch.arange(g["batch"].rows, dtype=torch.int32, device=m.device))
-            self._graphs[key] = g
-            while len(self._graphs) > self.MOST:
+            while len(self._graphs) >= self.MOST:
                 self._graphs.popitem(last=False)
+            self._graphs[key], self._last = g, self._now
+            self._seen[key], self._caught[key] = 0, self._caught.get(key, 0) + 1
         self._graphs.move_to_end(key)
+        g["used"] = self._now
         g["graph"].replay()
         out = g["logits"].clone()
         g["event"].record(stream)

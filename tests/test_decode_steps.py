@@ -1,6 +1,8 @@
 """Decode steps replayed from CUDA graphs (llm_decoder.engine.DecodeSteps) against the same steps run launch by launch: the same
 kernels on the same numbers, so the logits agree to the last bit except where a kernel's work split depends on the bound of the
 lengths (bfloat16 sums in another order: 2e-2 of the logits' spread, as for this precision elsewhere)."""
+import random
+
 import pytest
 import torch
 
@@ -114,3 +116,60 @@ def test_functions_in_place_of_methods_and_failed_captures():
     for k in range(6):
         _close(a.step([(0, [k + 9], [0])]), b.step([(0, [k + 9], [0])]))
     assert not a._decode._graphs
+
+
+class _Held:
+    """Stands in for streams, events, graphs and batches: takes every call and has every attribute."""
+    rows = 1
+
+    def __getattr__(self, _name):
+        return _Held()
+
+    def __call__(self, *_a, **_kw):
+        return _Held()
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *_exc):
+        return False
+
+
+def _host_only(monkeypatch):
+    """DecodeSteps over stand-ins: its bookkeeping without a GPU.  The current stream is steps.on, captures are noted in steps.noted."""
+    from llm_decoder import engine
+    steps = engine.DecodeSteps(_Held())
+    steps.on, steps.noted, steps.now = _Held(), [], 0
+    monkeypatch.setattr(torch.cuda, "Event", lambda *_a: _Held())
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda *_a: steps.on)
+    monkeypatch.setattr(engine, "DecodeBatch", lambda *_a: _Held())
+    steps.model.device, steps.model.runs = torch.device("cpu"), []
+    st = steps.model.states = _Held()
+    st.length, st.advance, st._tables, st.track_tokens = lambda _s: 100, lambda _e: (), [], False
+    steps._lane = _Held()
+    steps._watched = lambda: ([], ())
+    steps._same = lambda _w: True
+    steps._capture = lambda g, _stream: (steps.noted.append(steps.now), g.update(graph=_Held(), logits=torch.zeros(1), want=None, watched=None))
+    return steps
+
+
+@pytest.mark.parametrize("kinds", [9, 21, 64])
+@pytest.mark.parametrize("order", ["in turn", "at random", "walk"])
+def test_captures_of_many_kinds_are_few(monkeypatch, kinds, order):
+    """Numbers of sequences that change from step to step, more of them than graphs are kept: a capture costs up to 30 launched steps, so
+    no more than one in 64 steps captures, none where the kept ones keep coming back, and kept ones are replayed."""
+    steps = _host_only(monkeypatch)
+    r, n, replayed = random.Random(3), kinds // 2, 0
+    for steps.now in range(6000):
+        if order == "in turn":
+            n = steps.now % kinds
+        elif order == "at random":
+            n = r.randrange(kinds)
+        elif r.random() < 0.2:
+            n = min(max(n + r.choice((-1, 1)), 0), kinds - 1)
+        replayed += steps.step([(i, [0]) for i in range(n + 1)]) is not None
+    caught = steps.noted
+    assert len(steps._graphs) <= steps.MOST
+    assert order != "in turn" or len(caught) == steps.MOST
+    assert all(b - a >= 64 for a, b in zip(caught, caught[1:])), caught
+    assert replayed > 6000 * min(1.0, steps.MOST / kinds) * 0.5, replayed
