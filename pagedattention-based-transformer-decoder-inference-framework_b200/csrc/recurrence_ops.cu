@@ -319,17 +319,24 @@ __global__ void __launch_bounds__(kDsMaxThreads) decay_scan_kernel(const DecaySc
 // of four warps per (chunk, head); a warp has 16 rows of the result.
 // What bounds it: issue of ldmatrix and mma.sync.  4 x 2048 tokens, 16 heads of 64 x 128: fold 60 us, replay 146 us; the
 // walk on the float pipe 141 and 231 us.  Error of the layer against float64 4.3e-3 either way (rounding of the result).
+// A product adds zero times what a walk never meets (later tokens' values) and takes an infinity apart into planes.  So a chunk whose
+// operands or incoming state hold a number that is not finite, or so large that a sum of products could overflow, is walked
+// by the same CTA (dm_walk), as is a decay above one.
 constexpr int kDmTokens = 64, kDmDim = 64, kDmLd = kDmDim + 8, kDmThreads = 128;
+constexpr float kDmMost = 68719476736.f;      // 2^36: 64 x 64 products of three such numbers stay below 2^120
+constexpr uint32_t kDmMostBf16 = 0x5180u;     // the bits of 2^36 as bfloat16
 
 __device__ __forceinline__ void dm_split(float x, bf16_t (&b)[3]) {
     b[0] = __float2bfloat16_rn(x);
-    float r = isfinite(x) ? x - __bfloat162float(b[0]) : 0.f;
+    const float hi = __bfloat162float(b[0]);
+    float r = isfinite(hi) ? x - hi : 0.f;
     b[1] = __float2bfloat16_rn(r);
     r -= __bfloat162float(b[1]);
     b[2] = __float2bfloat16_rn(r);
 }
-// two neighbouring columns split into three planes `plane` elements apart
-__device__ __forceinline__ void dm_store2(bf16_t* dst, int plane, float x, float y) {
+// two neighbouring columns split into three planes `plane` elements apart; big: either is not below kDmMost
+__device__ __forceinline__ void dm_store2(bf16_t* dst, int plane, float x, float y, bool& big) {
+    big |= !(fabsf(x) < kDmMost) || !(fabsf(y) < kDmMost);
     bf16_t a[3], b[3];
     dm_split(x, a);
     dm_split(y, b);
@@ -343,7 +350,7 @@ __device__ __forceinline__ void dm_store2(bf16_t* dst, int plane, float x, float
 }
 // rows of q or k of one head: rotated (halves), times f(token), zeros past the chunk's end
 template <typename F>
-__device__ __forceinline__ void dm_stage(const DecayScanParams& p, const bf16_t* src, int64_t stride, int row0, int n, bf16_t* dst, F f) {
+__device__ __forceinline__ void dm_stage(const DecayScanParams& p, const bf16_t* src, int64_t stride, int row0, int n, bf16_t* dst, bool& big, F f) {
     const int half = p.rope ? p.rot_dims >> 1 : 0;
     constexpr int U = 8;                                    // pieces of two columns whose loads are in flight together
 #pragma unroll 1
@@ -368,21 +375,25 @@ __device__ __forceinline__ void dm_stage(const DecayScanParams& p, const bf16_t*
             const float x0 = __uint_as_float(xw[u] << 16), x1 = __uint_as_float(xw[u] & 0xffff0000u);
             const float y0 = __uint_as_float(yw[u] << 16), y1 = __uint_as_float(yw[u] & 0xffff0000u);
             if (d < half)
-                dm_store2(dst + t * kDmLd + d + half, kDmTokens * kDmLd, (y0 * cs[u].x + x0 * cs[u].y) * w, (y1 * cs[u].z + x1 * cs[u].w) * w);
-            dm_store2(dst + t * kDmLd + d, kDmTokens * kDmLd, (x0 * cs[u].x - y0 * cs[u].y) * w, (x1 * cs[u].z - y1 * cs[u].w) * w);
+                dm_store2(dst + t * kDmLd + d + half, kDmTokens * kDmLd, (y0 * cs[u].x + x0 * cs[u].y) * w, (y1 * cs[u].z + x1 * cs[u].w) * w, big);
+            dm_store2(dst + t * kDmLd + d, kDmTokens * kDmLd, (x0 * cs[u].x - y0 * cs[u].y) * w, (x1 * cs[u].z - y1 * cs[u].w) * w, big);
         }
     }
 }
 template <int VD>
-__device__ __forceinline__ void dm_stage_values(const DecayScanParams& p, int h, int row0, int n, bf16_t* dst) {
+__device__ __forceinline__ void dm_stage_values(const DecayScanParams& p, int h, int row0, int n, bf16_t* dst, bool& big) {
     const bf16_t* vb = static_cast<const bf16_t*>(p.v) + p.v_off + (int64_t)h * VD;
+    uint32_t top = 0u;                  // the largest magnitudes, as bits
 #pragma unroll
     for (int i = 0; i < kDmTokens * VD / 8 / kDmThreads; ++i) {
         const int idx = i * kDmThreads + threadIdx.x, t = idx / (VD / 8), c = idx % (VD / 8) * 8;
         uint4 v = make_uint4(0u, 0u, 0u, 0u);
         if (t < n) v = *reinterpret_cast<const uint4*>(vb + (int64_t)(row0 + t) * p.v_stride + c);
         *reinterpret_cast<uint4*>(dst + t * (VD + 8) + c) = v;
+        top = __vmaxu2(__vmaxu2(top, __vmaxu2(v.x & 0x7fff7fffu, v.y & 0x7fff7fffu)),
+                            __vmaxu2(v.z & 0x7fff7fffu, v.w & 0x7fff7fffu));
     }
+    big |= (top & 0xffffu) >= kDmMostBf16 || (top >> 16) >= kDmMostBf16;
 }
 // d^0 .. d^64
 __device__ __forceinline__ void dm_powers(float d, float* pw) {
@@ -405,6 +416,35 @@ __device__ __forceinline__ void dm_rows_product(float (&o)[VD / 8][4], const uin
     }
 }
 
+// The chunk token by token, a thread per column of the state: Ks, Qs [3][64][kDmLd] rotated and scaled rows in planes, Vs [64][VD + 8].
+// S0: the incoming state (null: zeros); Qs null: no outputs; end: where the state after the chunk goes (or null).
+template <int VD>
+__device__ __noinline__ void dm_walk(const bf16_t* Ks, const bf16_t* Vs, const bf16_t* Qs, int n, float a, const float* S0, float* out,
+                                     int64_t out_stride, float* end) {
+    const int c = threadIdx.x;
+    if (c >= VD) return;
+    auto whole = [](const bf16_t* x) {          // the three planes of a number, whose sum is exact
+        return (__bfloat162float(x[2 * kDmTokens * kDmLd]) + __bfloat162float(x[kDmTokens * kDmLd])) + __bfloat162float(x[0]);
+    };
+    float S[kDmDim];
+#pragma unroll
+    for (int d = 0; d < kDmDim; ++d) S[d] = S0 ? S0[(int64_t)d * VD + c] : 0.f;
+    for (int t = 0; t < n; ++t) {
+        const float x = __bfloat162float(Vs[t * (VD + 8) + c]);
+        float o = 0.f;
+#pragma unroll
+        for (int d = 0; d < kDmDim; ++d) {
+            S[d] = fmaf(a, S[d], whole(Ks + t * kDmLd + d) * x);
+            if (Qs) o = fmaf(S[d], whole(Qs + t * kDmLd + d), o);
+        }
+        if (Qs) out[t * out_stride + c] = o;
+    }
+    if (end) {
+#pragma unroll
+        for (int d = 0; d < kDmDim; ++d) end[(int64_t)d * VD + c] = S[d];
+    }
+}
+
 template <int VD>
 __global__ void __launch_bounds__(kDmThreads) decay_fold_mma_kernel(const DecayScanParams p) {
     extern __shared__ __align__(16) unsigned char dm_smem[];
@@ -414,12 +454,22 @@ __global__ void __launch_bounds__(kDmThreads) decay_fold_mma_kernel(const DecayS
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = blockIdx.y, g = h / (p.heads / p.groups);
     const int* it = p.items + 4 * blockIdx.x;
     const int row0 = it[0], n = it[1];
-    dm_powers(p.decay[h], pw);
-    dm_stage_values<VD>(p, h, row0, n, Vs);
+    const float decay = p.decay[h];
+    const bf16_t* kb = static_cast<const bf16_t*>(p.k) + p.k_off + (int64_t)g * kDmDim;
+    const int64_t sz = (int64_t)kDmDim * VD;
+    float* dst = p.part + ((int64_t)blockIdx.x * p.heads + h) * (sz + 1);
+    bool big = !(fabsf(decay) <= 1.f);
+    dm_powers(decay, pw);
+    dm_stage_values<VD>(p, h, row0, n, Vs, big);
     __syncthreads();
-    dm_stage(p, static_cast<const bf16_t*>(p.k) + p.k_off + (int64_t)g * kDmDim, p.k_stride, row0, n, Ks,
-             [&](int t) { return pw[n - 1 - t] * p.k_scale; });
-    __syncthreads();
+    dm_stage(p, kb, p.k_stride, row0, n, Ks, big, [&](int t) { return pw[n - 1 - t] * p.k_scale; });
+    if (threadIdx.x == 0) dst[sz] = pw[n];
+    if (__syncthreads_or(big)) {
+        dm_stage(p, kb, p.k_stride, row0, n, Ks, big, [&](int) { return p.k_scale; });
+        __syncthreads();
+        dm_walk<VD>(Ks, Vs, nullptr, n, decay, nullptr, nullptr, 0, dst);
+        return;
+    }
     float o[VD / 8][4];
 #pragma unroll
     for (int i = 0; i < VD / 8; ++i)
@@ -434,13 +484,10 @@ __global__ void __launch_bounds__(kDmThreads) decay_fold_mma_kernel(const DecayS
                           a[1], a[2], a[3]);
             dm_rows_product<VD>(o, a, Vs, VD + 8, ks, lane);
         }
-    const int64_t sz = (int64_t)kDmDim * VD;
-    float* dst = p.part + ((int64_t)blockIdx.x * p.heads + h) * (sz + 1);
 #pragma unroll
     for (int i = 0; i < VD / 8; ++i)
 #pragma unroll
         for (int c = 0; c < 4; ++c) dst[(warp * 16 + (lane >> 2) + (c >> 1) * 8) * VD + i * 8 + 2 * (lane & 3) + (c & 1)] = o[i][c];
-    if (threadIdx.x == 0) dst[sz] = pw[n];
 }
 
 template <int VD>
@@ -453,10 +500,13 @@ __global__ void __launch_bounds__(kDmThreads, 2) decay_replay_mma_kernel(const D
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = blockIdx.y, g = h / (p.heads / p.groups);
     const int* it = p.items + 4 * blockIdx.x;
     const int row0 = it[0], n = it[1];
-    dm_powers(p.decay[h], pw);
-    dm_stage_values<VD>(p, h, row0, n, Vs);
-    dm_stage(p, static_cast<const bf16_t*>(p.k) + p.k_off + (int64_t)g * kDmDim, p.k_stride, row0, n, Ks, [&](int) { return p.k_scale; });
-    dm_stage(p, static_cast<const bf16_t*>(p.q) + p.q_off + (int64_t)g * kDmDim, p.q_stride, row0, n, Ss, [](int) { return 1.f; });
+    const float decay = p.decay[h];
+    const bf16_t* qb = static_cast<const bf16_t*>(p.q) + p.q_off + (int64_t)g * kDmDim;
+    bool big = !(fabsf(decay) <= 1.f);
+    dm_powers(decay, pw);
+    dm_stage_values<VD>(p, h, row0, n, Vs, big);
+    dm_stage(p, static_cast<const bf16_t*>(p.k) + p.k_off + (int64_t)g * kDmDim, p.k_stride, row0, n, Ks, big, [&](int) { return p.k_scale; });
+    dm_stage(p, qb, p.q_stride, row0, n, Ss, big, [](int) { return 1.f; });
     __syncthreads();
     uint32_t qf[3][kDmDim / 16][4];
 #pragma unroll
@@ -480,7 +530,7 @@ __global__ void __launch_bounds__(kDmThreads, 2) decay_replay_mma_kernel(const D
 #pragma unroll
         for (int u = 0; u < 16; ++u) {
             const int idx = i0 + u * kDmThreads + threadIdx.x, d = idx / (VD / 2), c = idx % (VD / 2) * 2;
-            dm_store2(Ss + d * (VD + 8) + c, kDmDim * (VD + 8), x[u], y[u]);
+            dm_store2(Ss + d * (VD + 8) + c, kDmDim * (VD + 8), x[u], y[u], big);
         }
     }
     // scores of this warp's tokens against the keys up to them
@@ -506,7 +556,12 @@ __global__ void __launch_bounds__(kDmThreads, 2) decay_replay_mma_kernel(const D
                 }
             }
     }
-    __syncthreads();                                                  // the state is staged
+    if (__syncthreads_or(big)) {                                      // the state is staged
+        dm_stage(p, qb, p.q_stride, row0, n, Ss, big, [](int) { return 1.f; });
+        __syncthreads();
+        dm_walk<VD>(Ks, Vs, Ss, n, decay, S0, p.out + (int64_t)row0 * p.out_stride + (int64_t)h * VD, p.out_stride, nullptr);
+        return;
+    }
     float o[VD / 8][4];
 #pragma unroll
     for (int i = 0; i < VD / 8; ++i)

@@ -74,3 +74,66 @@ def test_fold_and_replay(heads, groups, vdim, rot_dims):
     top = [want.abs().max().item()] + [S.abs().max().item() for S in states64]
     for a, b, t in zip(*off, top):
         assert a <= 2 * b + 2.0 ** -22 * t, off
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("vdim,groups", [(64, 2), (128, 1)])
+@pytest.mark.parametrize("where", ["value", "nan value", "key", "query", "state", "large"])
+def test_values_that_are_not_finite(vdim, groups, where):
+    """An infinity or NaN in one token, or in the incoming state, reaches the outputs and states that the walk lets it reach and no others;
+    large finite numbers give what the walk gives.
+
+    Bound for what stays finite: both are float sums of up to 128 terms whose magnitudes add up to at most 2^11 here (2^-24 each), or to
+    2^6 times the column's largest number where that is large: 2^-13 and 2^-18 of it."""
+    from llm_decoder import _cabi
+    from llm_decoder.seq_state import SequenceStateCache
+    lib, dev, dim, heads, rot_dims = _cabi.lib(), torch.device("cuda"), 64, 2, 32
+    g = torch.Generator().manual_seed(vdim + len(where))
+    lens = [300, 70, 3]
+    R, cols = sum(lens), 2 * groups * dim + heads * vdim
+    states = SequenceStateCache(len(lens), 4096, 16, dev)
+    st = states.add_state(heads * dim * vdim)
+    slots = [states.alloc() for _ in lens]
+    batch = states.make_batch([(s, [0] * n) for s, n in zip(slots, lens)])
+    start = torch.randn(st.shape, generator=g)
+    X = torch.randn(R, cols, generator=g).to(torch.bfloat16)
+    v0, inf = 2 * groups * dim, float("inf")
+    if where == "value":
+        X[70, v0 + 5], X[77, v0 + 5], X[311, v0 + vdim + 3], X[372, v0] = inf, -inf, -inf, inf
+    elif where == "nan value":
+        X[20, v0 + 9], X[369, v0 + vdim] = float("nan"), float("nan")
+    elif where == "key":
+        X[130, groups * dim + 7], X[301, groups * dim + 40] = inf, float("nan")
+    elif where == "query":
+        X[200, 3], X[5, 50] = -inf, float("nan")
+    elif where == "state":
+        start[slots[0], 17], start[slots[1], dim * vdim + 4], start[slots[2], 2] = inf, float("nan"), -inf
+    else:
+        X[64:70, v0 + 1], X[305, groups * dim + 2], start[slots[2], 9] = 1e30, -1e25, 3e38
+    decay = torch.tensor([0.9, 0.25])
+    ang = torch.rand(R, rot_dims // 2, generator=g) * 6.0
+    Xd, decayd, roped = X.to(dev), decay.to(dev), torch.stack([torch.cos(ang), torch.sin(ang)], -1).to(dev).contiguous()
+    items, n, s0, sn = batch.chunk_items(64)
+    ws = torch.empty(lib.pa_decay_scan_workspace_bytes(n, heads, dim, vdim), dtype=torch.uint8, device=dev)
+    got = []
+    for chunk_tokens in (64, 0):            # as products, and walked
+        st.copy_(start)
+        out = torch.full((R, heads * vdim), float("nan"), device=dev)
+        assert lib.pa_decay_scan_chunked(
+            Xd.data_ptr(), Xd.stride(0), 0, Xd.data_ptr(), Xd.stride(0), groups * dim, Xd.data_ptr(), Xd.stride(0), v0, heads, groups, dim, vdim, 0,
+            decayd.data_ptr(), None, 0, 0, None, None, None, roped.data_ptr(), rot_dims, 0.125, st.data_ptr(), out.data_ptr(), out.stride(0),
+            items.data_ptr(), n, s0.data_ptr(), sn.data_ptr(), batch.seq_slot.data_ptr(), batch.num_seqs, 1, ws.data_ptr(), ws.numel(), 2,
+            chunk_tokens, _cabi.stream()) == 0
+        got.append((out.cpu().reshape(R, heads, vdim), st.cpu().reshape(len(lens), heads, dim, vdim)[slots].transpose(1, 2)))
+    for a, b in zip(*got):                  # outputs [token, head, column], states [sequence, dimension, head, column]
+        assert torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(torch.isinf(a), torch.isinf(b))
+        assert torch.equal(a[torch.isinf(a)], b[torch.isinf(b)])
+        ok = torch.isfinite(b)
+        zero = torch.zeros_like(a)
+        a, b = torch.where(ok, a, zero).double(), torch.where(ok, b, zero).double()
+        r0 = 0
+        for m in (lens if a.shape[0] == R else [1] * len(lens)):
+            x, y = a[r0:r0 + m], b[r0:r0 + m]
+            top = y.abs().cummax(0).values if m > 1 else y.abs().amax(1, keepdim=True)
+            assert ((x - y).abs() <= 2.0 ** -18 * top + 2.0 ** -13).all(), ((x - y).abs() / (top + 1e-30)).max()
+            r0 += m
