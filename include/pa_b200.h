@@ -40,6 +40,8 @@ int pa_version(void);
 const char* pa_error_string(int status);
 /* sm count / compute capability of the current device. */
 int pa_device_info(int* sm_count, int* cc_major, int* cc_minor);
+/* A stream of its own on the current device, which no pool hands out a second time (non-blocking; lives as long as the process). */
+int pa_stream_create(pa_stream_t* stream);
 
 /* ------------------------------------------------------------- page table */
 /* kv_cache/page_table.cpp:14-26,41-47  PageTable::init / clear:

@@ -259,6 +259,14 @@ PA_API int pa_device_info(int* sm_count, int* cc_major, int* cc_minor) {
     return PA_OK;
 }
 
+PA_API int pa_stream_create(pa_stream_t* stream) {
+    PA_CHECK_ARG(stream);
+    cudaStream_t s = nullptr;
+    const cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+    if (e == cudaSuccess) *stream = (pa_stream_t)s;
+    return (int)e;
+}
+
 PA_API int pa_page_table_clear(int32_t* d_table, int64_t n_entries, pa_stream_t stream) {
     PA_CHECK_ARG(d_table && n_entries >= 0);
     if (n_entries == 0) return PA_OK;

@@ -25,6 +25,7 @@ _SIGS = {
     "pa_version": ([], _i32),
     "pa_error_string": ([_i32], C.c_char_p),
     "pa_device_info": ([C.POINTER(_i32)] * 3, _i32),
+    "pa_stream_create": ([C.POINTER(_vp)], _i32),
     "pa_page_table_clear": ([_vp, _i64, _vp], _i32),
     "pa_page_table_update": ([_vp, _i64, _vp, _vp, _i32, _vp], _i32),
     "pa_page_table_lookup": ([_vp, _i32, _i32, _i32, _vp, _vp, _vp, _vp, _i32, _vp], _i32),

@@ -10,6 +10,8 @@ are fed in chunks under a per-step token budget next to the running requests' si
 of every request whose last fed token ended its prompt (or was a decoded token) is sampled on the device with the
 framework's samplers (greedy pa_argmax_f32; temperature / top-k / top-p through llm_decoder.sampling)."""
 import collections
+import ctypes
+import threading
 import types
 
 import torch
@@ -18,6 +20,38 @@ from . import _cabi
 from .host_stage import to_device as _to_device
 from .hybrid import HybridDecoder
 from .seq_state import DecodeBatch
+
+
+class _Lane:
+    """A stream that graphs are captured on, and the order of their replays.  The vendor products captured on a stream share the
+    library's scratch of that stream, so the replays of a lane follow one another, whatever streams they are issued on; and a lane's stream
+    is nobody else's, so that no launched product uses that scratch.  An engine has a lane of its own up to the EACH-th of a device."""
+    EACH = 8
+    _lock, _lanes, _next = threading.Lock(), {}, {}
+
+    def __init__(self, device):
+        raw = ctypes.c_void_p()
+        _cabi.check(_cabi.lib().pa_stream_create(ctypes.byref(raw)), "pa_stream_create")
+        self.side, self.lock = torch.cuda.ExternalStream(raw.value, device=device), threading.Lock()
+        self._event, self._stream = torch.cuda.Event(), None
+
+    @classmethod
+    def of(cls, device):
+        with cls._lock:
+            at = torch.cuda.current_device()
+            lanes, i = cls._lanes.setdefault(at, []), cls._next.get(at, 0)
+            cls._next[at] = i + 1
+            if len(lanes) < cls.EACH:
+                lanes.append(cls(device))
+            return lanes[i % cls.EACH]
+
+    def before(self, stream):
+        if self._stream is not None and self._stream != stream:
+            stream.wait_event(self._event)
+
+    def after(self, stream):
+        self._event.record(stream)
+        self._stream = stream
 
 
 class DecodeSteps:
@@ -36,7 +70,7 @@ class DecodeSteps:
     PATIENCE, GAP, IDLE = 16, 64, 256       # in steps, see above
 
     def __init__(self, model):
-        self.model, self._side = model, None
+        self.model, self._lane = model, None
         self._graphs = collections.OrderedDict()        # kind -> graph, the one whose replay is longest ago first
         self._seen, self._caught = {}, {}               # kind -> launched steps since its last capture; captures
         self._now, self._last = 0, None                 # steps so far; the step of the last capture
@@ -100,47 +134,48 @@ class DecodeSteps:
             return None
         if g is None and any(isinstance(v, (types.FunctionType, types.MethodType)) for _d, _n, items in self._watched()[0] for _k, v, _p in items):
             return None         # a function put in the place of a method may do more than launch kernels
+        if self._lane is None:
+            self._lane = _Lane.of(m.device)
         if g is None:
-            g = dict(batch=DecodeBatch(len(entries), bound, m.device, st.track_tokens), graph=None, stream=None, event=torch.cuda.Event())
+            g = dict(batch=DecodeBatch(len(entries), bound, m.device, st.track_tokens), graph=None, stream=None)
         stream = torch.cuda.current_stream(m.device)
-        if g["stream"] is not None and g["stream"] != stream:
-            stream.wait_event(g["event"])       # the last replay, on another stream, still reads the buffers
-        g["batch"].fill(*st.advance(entries))
-        for kv in st._tables:
-            kv.page_table_.flush()              # no update of a table belongs into the graph
-        if g["graph"] is None:
-            try:
-                self._capture(g, stream)
-            except RuntimeError:        # memory, or a library call that cannot be captured: this kind stays with launches
-                self._seen[key] = -(1 << 60)
-                return m.forward(g["batch"], torch.arange(g["batch"].rows, dtype=torch.int32, device=m.device))
-            while len(self._graphs) >= self.MOST:
-                self._graphs.popitem(last=False)
-            self._graphs[key], self._last = g, self._now
-            self._seen[key], self._caught[key] = 0, self._caught.get(key, 0) + 1
-        self._graphs.move_to_end(key)
-        g["used"] = self._now
-        g["graph"].replay()
-        out = g["logits"].clone()
-        g["event"].record(stream)
-        g["stream"] = stream
+        with self._lane.lock:
+            self._lane.before(stream)           # the last replay, on another stream, still reads the buffers
+            if g["stream"] != stream:           # ... and this one may when the graph is dropped
+                g["stream"] = stream
+                g["batch"].used_on(stream)
+            g["batch"].fill(*st.advance(entries))
+            for kv in st._tables:
+                kv.page_table_.flush()          # no update of a table belongs into the graph
+            if g["graph"] is None:
+                try:
+                    self._capture(g, stream)
+                except RuntimeError:        # memory, or a library call that cannot be captured: this kind stays with launches
+                    self._seen[key] = -(1 << 60)
+                    return m.forward(g["batch"], g["batch"].seq_start)
+                while len(self._graphs) >= self.MOST:
+                    self._graphs.popitem(last=False)
+                self._graphs[key], self._last = g, self._now
+                self._seen[key], self._caught[key] = 0, self._caught.get(key, 0) + 1
+            self._graphs.move_to_end(key)
+            g["used"] = self._now
+            g["graph"].replay()
+            out = g["logits"].clone()
+            self._lane.after(stream)
         return out
 
     def _capture(self, g, stream):
         m = self.model
-        want = torch.arange(g["batch"].rows, dtype=torch.int32, device=m.device)
-        if self._side is None:
-            self._side = torch.cuda.Stream(m.device)
-        side, graph = self._side, torch.cuda.CUDAGraph()
+        side, graph = self._lane.side, torch.cuda.CUDAGraph()
         side.wait_stream(stream)
         with torch.cuda.stream(side):
             graph.capture_begin(capture_error_mode="thread_local")
             try:
-                logits = m.forward(g["batch"], want)
+                logits = m.forward(g["batch"], g["batch"].seq_start)
             finally:
                 graph.capture_end()
         stream.wait_stream(side)
-        g.update(graph=graph, logits=logits, want=want, watched=self._watched())
+        g.update(graph=graph, logits=logits, watched=self._watched())
 
 
 class Engine:

@@ -217,6 +217,9 @@ class DecodeBatch(RaggedBatch):
         h["chunks"][:, 2] = slots
         _to_device(torch.from_numpy(self._host), self.device, self._dev)
 
+    def used_on(self, stream):
+        self._dev.record_stream(stream)
+
     def query_tiles(self, tile_tokens, big_tokens=0, big_from=0, without=0):
         return {0: None, 1: (self._f["tiles"], self.rows, self.longest), 2: None}
 

@@ -173,3 +173,54 @@ def test_captures_of_many_kinds_are_few(monkeypatch, kinds, order):
     assert order != "in turn" or len(caught) == steps.MOST
     assert all(b - a >= 64 for a, b in zip(caught, caught[1:])), caught
     assert replayed > 6000 * min(1.0, steps.MOST / kinds) * 0.5, replayed
+
+
+def test_replays_of_an_engine_follow_one_another(monkeypatch):
+    """All graphs of an engine share the scratch of the stream they were captured on: a replay waits for the last one on another stream,
+    of whatever kind, and the buffers a replay reads are kept for the streams that replay."""
+    from llm_decoder import engine
+    steps = _host_only(monkeypatch)
+    steps.PATIENCE = steps.GAP = 0
+    log, held = [], []
+
+    class Stream:
+        def wait_event(self, event):
+            log.append(("wait", self, event.by))
+
+    class Event:
+        by = None
+
+        def record(self, stream):
+            self.by = stream
+
+    class Batch(_Held):
+        def __init__(self, *_a):
+            self.streams = []
+            held.append(self)
+
+        def used_on(self, stream):
+            self.streams.append(stream)
+    monkeypatch.setattr(torch.cuda, "Event", Event)
+    monkeypatch.setattr(engine, "DecodeBatch", Batch)
+    lane = object.__new__(engine._Lane)
+    lane.side, lane.lock, lane._event, lane._stream = _Held(), _Held(), Event(), None
+    steps._lane = lane
+    a, b = Stream(), Stream()
+    for steps.on, n in ((a, 1), (a, 2), (b, 1), (b, 1), (b, 2), (a, 2), (a, 1)):
+        assert steps.step([(i, [0]) for i in range(n)]) is not None
+    assert log == [("wait", b, a), ("wait", a, b)]
+    assert held[0].streams == [a, b, a] and held[1].streams == [a, b, a]
+
+
+@pytest.mark.gpu
+def test_capture_streams_are_nobody_elses():
+    """No stream that a program gets is one that graphs were captured on, and engines capture on different ones."""
+    config, W = _config("tiradra")
+    sides = []
+    for _ in range(3):
+        a, b = _pair(config, W, max_tokens=64, max_seqs=1)
+        for k in range(5):
+            _close(a.step([(0, [k], [0])]), b.step([(0, [k], [0])]))
+        sides.append(a._decode._lane.side.cuda_stream)
+    assert len(set(sides)) == 3
+    assert not set(sides) & {torch.cuda.Stream().cuda_stream for _ in range(70)}
