@@ -150,7 +150,8 @@ class DecodeSteps:
             if g["graph"] is None:
                 try:
                     self._capture(g, stream)
-                except RuntimeError:        # memory, or a library call that cannot be captured: this kind stays with launches
+                except Exception:           # memory, a call that cannot be captured: this kind stays with launches, which raise
+                                            # what was not the capture's fault
                     self._seen[key] = -(1 << 60)
                     return m.forward(g["batch"], g["batch"].seq_start)
                 while len(self._graphs) >= self.MOST:

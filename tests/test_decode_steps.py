@@ -224,3 +224,52 @@ def test_capture_streams_are_nobody_elses():
         sides.append(a._decode._lane.side.cuda_stream)
     assert len(set(sides)) == 3
     assert not set(sides) & {torch.cuda.Stream().cuda_stream for _ in range(70)}
+
+
+@pytest.mark.parametrize("kind", [RuntimeError, ValueError, AssertionError, KeyError])
+def test_any_error_of_a_capture_leaves_the_step_to_launches(monkeypatch, kind):
+    """The sequences have advanced by then: the step runs launch by launch, once, and its kind is not captured again."""
+    steps = _host_only(monkeypatch)
+    steps.PATIENCE = steps.GAP = 0
+    advanced = []
+    steps.model.states.advance = lambda entries: advanced.append(entries) or ()
+    steps.model.forward = lambda *_a: "launched"
+
+    def fails(*_a):
+        steps.noted.append(1)
+        raise kind("no capture")
+    steps._capture = fails
+    assert steps.step([(0, [1])]) == "launched"
+    assert steps.step([(0, [1])]) is None and len(advanced) == 1 and len(steps.noted) == 1
+
+    def broken(*_a):
+        raise kind("neither")
+    steps.model.forward = broken
+    with pytest.raises(kind):
+        steps.step([(0, [1]), (1, [1])])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", [RuntimeError, ValueError])
+def test_a_capture_that_stops_half_way(monkeypatch, kind):
+    """An error in the middle of a real capture ends it; this and all later steps give the launched results, and another kind of step is
+    captured and replayed."""
+    from llm_decoder.hybrid import HybridDecoder
+    config, W = _config("tiradra")
+    a, b = _pair(config, W, max_tokens=256, max_seqs=2)
+    a._decode.GAP = 0
+    real, raised = HybridDecoder._linear, []
+
+    def linear(self, *args, **kw):
+        if torch.cuda.is_current_stream_capturing():
+            raised.append(len(raised))
+            if len(raised) == 4:
+                raise kind("in the middle")
+        return real(self, *args, **kw)
+    monkeypatch.setattr(HybridDecoder, "_linear", linear)
+    for k in range(6):
+        _close(a.step([(0, [k], [0])]), b.step([(0, [k], [0])]))
+    assert len(raised) == 4 and not a._decode._graphs
+    for k in range(6):
+        _close(a.step([(i, [k + i], [0]) for i in (0, 1)]), b.step([(i, [k + i], [0]) for i in (0, 1)]))
+    assert len(a._decode._graphs) == 1
