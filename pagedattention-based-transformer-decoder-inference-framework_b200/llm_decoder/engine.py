@@ -214,7 +214,9 @@ class Engine:
         if not batch_entries:
             return torch.empty((0, self.model.vocab), dtype=torch.float32, device=dev)
         with _cabi.on_device(dev):
-            if self._decode.serves(batch_entries, want) and want == list(range(row0)):
+            if self._decode.model is not self.model:
+                self._decode = DecodeSteps(self.model)
+            if self.model.states is self.states and self._decode.serves(batch_entries, want) and want == list(range(row0)):
                 logits = self._decode.step(batch_entries)
                 if logits is not None:
                     return logits

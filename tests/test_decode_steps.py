@@ -273,3 +273,32 @@ def test_a_capture_that_stops_half_way(monkeypatch, kind):
     for k in range(6):
         _close(a.step([(i, [k + i], [0]) for i in (0, 1)]), b.step([(i, [k + i], [0]) for i in (0, 1)]))
     assert len(a._decode._graphs) == 1
+
+
+def test_a_model_put_in_the_place_of_another(monkeypatch):
+    """Steps run on the engine's model and states of the moment."""
+    import contextlib
+    import llm_decoder as ld
+    from llm_decoder import engine
+    monkeypatch.setattr(engine._cabi, "on_device", lambda _d: contextlib.nullcontext())
+
+    class Model:
+        def __init__(self, name, states):
+            self.device, self.vocab, self.states, self.name = torch.device("cpu"), 3, states, name
+
+        def forward(self, *_a):
+            return self.name
+
+    class Steps(engine.DecodeSteps):
+        def serves(self, *_a):
+            return True
+
+        def step(self, _entries):
+            return self.model.name
+    states = _Held()
+    states.alloc = lambda: 0
+    e = ld.Engine(Model("first", states))
+    e._decode = Steps(e.model)
+    assert e.step([(0, [1], [0])]) == "first"
+    e.model = Model("second", states)
+    assert e.step([(0, [1], [0])]) == "second"
