@@ -9,6 +9,10 @@
 // share belongs to the next pair or the next worker, so no two meet.  A second kernel, resident before the first ends
 // (programmatic dependent launch), joins the shares of each pair and applies sink, turn and gate.
 //
+// The softmax weights enter the second product as bfloat16 for batches that give every SM a pair, as in masked_attention.cu's
+// kernel with heads as rows; smaller batches, whose streaming kernel keeps them float, keep them float here too: three
+// bfloat16 numbers add up to the 24 bits of a weight, for three products instead of one.
+//
 // What bounds it: HBM.  Eight workers x 3 stages x 8 KB per SM are in flight, as in the streaming kernel of paged_decode.cu; a unit
 // costs a warp about 150 instructions.  64 tokens, 16 query / 4 kv heads of 128, 2048 keys (268 MB): 56 us = 4.8 TB/s and 4 us for the
 // join (heads as rows without a key split, masked_attention_mma_decode_kernel: 91 us); 8 tokens, 2 kv heads, 400 keys: 10 us
@@ -44,7 +48,8 @@ __device__ __forceinline__ int find_tile(const int* pre, int n, int64_t f, int p
     return lo;
 }
 
-template <int DIM, int VDIM>
+// FLOAT_W: the weights of the second product are float (see above)
+template <int DIM, int VDIM, bool FLOAT_W>
 __global__ void __launch_bounds__(kWarps * 32, 1) masked_decode_kernel(const __grid_constant__ CUtensorMap tmK,
                                                                        const __grid_constant__ CUtensorMap tmV, const Args a) {
     constexpr int KB = DIM / 64, VB = VDIM / 64, STAGE = (KB + VB) * 2048, NT = VDIM / 8;
@@ -269,18 +274,62 @@ __global__ void __launch_bounds__(kWarps * 32, 1) masked_decode_kernel(const __g
                 s[n][c] = exp2f(s[n][c] - ref[c >> 1]);
                 l[c >> 1] += s[n][c];
             }
-        const uint32_t pf[4] = {pack_bf16x2(s[0][0], s[0][1]), pack_bf16x2(s[0][2], s[0][3]), pack_bf16x2(s[1][0], s[1][1]),
-                                pack_bf16x2(s[1][2], s[1][3])};
-        {
-            const int r = (lane & 7) + ((lane >> 3) & 1) * 8;
+        const int vr = (lane & 7) + ((lane >> 3) & 1) * 8;
+        auto load_values = [&](int np, uint32_t (&b)[4]) {
+            ldsm_x4_trans(vs_sm + (np >> 2) * 2048 + vr * 128 + ((((np & 3) * 2 + (lane >> 4)) ^ (vr & 7)) << 4), b[0], b[1], b[2], b[3]);
+        };
+        if constexpr (!FLOAT_W) {
+            const uint32_t pf[4] = {pack_bf16x2(s[0][0], s[0][1]), pack_bf16x2(s[0][2], s[0][3]), pack_bf16x2(s[1][0], s[1][1]),
+                                    pack_bf16x2(s[1][2], s[1][3])};
 #pragma unroll
             for (int np = 0; np < NT / 2; ++np) {
-                const int c = (np & 3) * 2 + (lane >> 4);
-                uint32_t b0, b1, b2, b3;
-                ldsm_x4_trans(vs_sm + (np >> 2) * 2048 + r * 128 + ((c ^ (r & 7)) << 4), b0, b1, b2, b3);
-                mma_bf16_16816(o[2 * np], pf, b0, b1);
-                mma_bf16_16816(o[2 * np + 1], pf, b2, b3);
+                uint32_t b[4];
+                load_values(np, b);
+                mma_bf16_16816(o[2 * np], pf, b[0], b[1]);
+                mma_bf16_16816(o[2 * np + 1], pf, b[2], b[3]);
             }
+        } else {
+            uint32_t pf[3][4], vf[NT / 2][4];   // plane i of the weights: what the planes before it left
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                float x = s[j >> 1][2 * (j & 1)], y = s[j >> 1][2 * (j & 1) + 1];
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    pf[i][j] = pack_bf16x2(x, y);
+                    x -= __uint_as_float(pf[i][j] << 16);
+                    y -= __uint_as_float(pf[i][j] & 0xffff0000u);
+                }
+            }
+#pragma unroll
+            for (int np = 0; np < NT / 2; ++np) load_values(np, vf[np]);
+            auto weigh = [&](const uint32_t (&w)[4]) {
+#pragma unroll
+                for (int np = 0; np < NT / 2; ++np) {
+                    mma_bf16_16816(o[2 * np], w, vf[np][0], vf[np][1]);
+                    mma_bf16_16816(o[2 * np + 1], w, vf[np][2], vf[np][3]);
+                }
+            };
+            // a value that is not finite meets the first plane alone: a zero of the others would make NaN of an infinity
+            const __nv_bfloat162 zero = __floats2bfloat162_rn(0.f, 0.f);
+            __nv_bfloat162 probe = zero;        // 0 x value, summed up: NaN if any is not finite
+#pragma unroll
+            for (int np = 0; np < NT / 2; ++np)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) probe = __hfma2(*reinterpret_cast<const __nv_bfloat162*>(&vf[np][j]), zero, probe);
+            const bool apart = __any_sync(0xffffffffu, __hisnan(probe.x) || __hisnan(probe.y));
+            if (apart) {
+                weigh(pf[0]);
+#pragma unroll
+                for (int np = 0; np < NT / 2; ++np)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const uint32_t v = vf[np][j];
+                        vf[np][j] = ((v & 0x7f80u) == 0x7f80u ? 0u : v & 0xffffu) | ((v & 0x7f800000u) == 0x7f800000u ? 0u : v & 0xffff0000u);
+                    }
+            }
+            weigh(pf[2]);                       // the small terms first
+            weigh(pf[1]);
+            if (!apart) weigh(pf[0]);
         }
         __syncwarp();                   // every lane has read the stage
         issue();                        // refills it
@@ -332,8 +381,8 @@ __global__ void __launch_bounds__(128) masked_decode_join_kernel(const Args a) {
 #pragma unroll
             for (int i = 0; i < NV; i += 2) {
                 const float2 x = *reinterpret_cast<const float2*>(s + 2 + lane * NV + i);
-                v[k][i] = x.x;
-                v[k][i + 1] = x.y;
+                v[k][i] = w + k <= w1 ? x.x : 0.f;      // 0 x infinity = NaN
+                v[k][i + 1] = w + k <= w1 ? x.y : 0.f;
             }
         }
 #pragma unroll
@@ -367,14 +416,14 @@ __global__ void __launch_bounds__(128) masked_decode_join_kernel(const Args a) {
 
 static size_t pre_bytes(int ntiles) { return ((size_t)(ntiles + 1) * sizeof(int) + 15) / 16 * 16; }
 
-template <int DIM, int VDIM>
+template <int DIM, int VDIM, bool FLOAT_W>
 static int launch(const CUtensorMap& k, const CUtensorMap& v, const Args& a, cudaStream_t st) {
     const size_t smem = (size_t)kWarps * kStages * ((DIM + VDIM) / 64 * 2048 + 8) + (a.ntiles + 1) * 4 + 1024;
-    cudaError_t e = cudaFuncSetAttribute(masked_decode_kernel<DIM, VDIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(masked_decode_kernel<DIM, VDIM, FLOAT_W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     const int sms = device_info().sm_count;
     const int grid = a.workers < sms ? a.workers : sms;
-    masked_decode_kernel<DIM, VDIM><<<grid, kWarps * 32, smem, st>>>(k, v, a);
+    masked_decode_kernel<DIM, VDIM, FLOAT_W><<<grid, kWarps * 32, smem, st>>>(k, v, a);
     e = cudaGetLastError();
     if (e != cudaSuccess) return (int)e;
     const int64_t warps = (int64_t)a.ntiles * a.p.num_kv_heads * a.hch * a.rows;
@@ -454,6 +503,12 @@ PA_API int pa_masked_decode(const void* d_q, int64_t q_stride, int q_off, const 
     CUtensorMap k, v;
     if (!tc::make_bf16_map(&k, d_k_pool, rows, dim, dim, 16) || !tc::make_bf16_map(&v, d_v_pool, rows, vdim, vdim, 16)) return PA_ERR_UNSUPPORTED;
     cudaStream_t st = as_stream(stream);
-    if (dim == 64) return vdim == 64 ? launch<64, 64>(k, v, a, st) : launch<64, 128>(k, v, a, st);
-    return vdim == 64 ? launch<128, 64>(k, v, a, st) : launch<128, 128>(k, v, a, st);
+    // bfloat16 weights where masked_attention.cu's kernel with heads as rows would serve the batch: a pair per SM, 16-byte query rows
+    const bool rows16 = q_stride % 8 == 0 && q_off % 8 == 0 && (uintptr_t)d_q % 16 == 0;
+    const bool float_w = !rows16 || (int64_t)num_q_tiles * num_kv_heads < device_info().sm_count;
+#define PA_MDEC(D, V)                                                                                             \
+    if (dim == D && vdim == V) return float_w ? launch<D, V, true>(k, v, a, st) : launch<D, V, false>(k, v, a, st)
+    PA_MDEC(64, 64); PA_MDEC(64, 128); PA_MDEC(128, 64); PA_MDEC(128, 128);
+#undef PA_MDEC
+    return PA_ERR_UNSUPPORTED;
 }

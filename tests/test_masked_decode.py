@@ -96,3 +96,52 @@ def test_shares_of_decoded_tokens(heads, kv_heads, dim, vdim, mask, size, keep, 
         assert torch.isfinite(out.float()).all()
         err = (out.double().cpu() - want.reshape(n, -1)).abs().max().item()
         assert err < 1.1 * 2.0 ** -8 * max(v.abs().max().item() for v in V) * (1.42 if turn is not None else 1.0), (workers, err)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(8, 2, 128, 128), (20, 1, 64, 128), (4, 4, 128, 64)])
+@pytest.mark.parametrize("stride", [0, 2])
+def test_weights_of_small_batches_are_float(heads, kv_heads, dim, vdim, stride):
+    """With fewer (token, kv head) pairs than SMs, and for query rows that are not 16-byte aligned, the softmax weights keep the 24 bits of a
+    float in the second product, as in the streaming kernel.
+
+    Bound: the result is rounded to bfloat16 once (2^-8 of itself); scores of up to 8 are float sums (error 2^-20, so the weights' too), as
+    are the weighted sums: 2^-16 max |v| covers them.  Weights rounded to bfloat16 are off by up to 2^-8 max |v|."""
+    from llm_decoder import _cabi
+    from llm_decoder.seq_state import SequenceStateCache
+    lib, dev = _cabi.lib(), torch.device("cuda")
+    g = torch.Generator().manual_seed(heads + dim + stride)
+    pos = [2, 6, 15, 16, 40, 300]
+    n, per, scale = len(pos), heads // kv_heads, dim ** -0.5 * 1.5
+    if stride:                                  # enough pairs for an SM each, rows of queries at 4-byte places
+        pos = (pos * 200)[:max(1, 160 // kv_heads) + 1]
+        n = len(pos)
+    states = SequenceStateCache(n, sum(c + 17 for c in pos), 16, dev)
+    kv = states.add_kv_layer(kv_heads, dim, vdim, "bf16")
+    slots = [states.alloc() for _ in range(n)]
+    batch = states.make_batch([(s, [0] * (c + 1)) for s, c in zip(slots, pos)])
+    KV = torch.randn(batch.rows, kv_heads * (dim + vdim), generator=g).to(BF)
+    V = KV[:, kv_heads * dim:].clone()
+    KV[1, kv_heads * dim + 3], KV[3, -1] = float("inf"), float("nan")       # of the first and the second token: they stay in their columns
+    kv.append_rows(KV.to(dev), 0, kv_heads * dim, batch.row_slot, batch.row_pos)
+    Q = torch.randn(n, heads * dim + 8 + stride, generator=g).to(BF)
+    want, r0 = torch.zeros(n, heads, vdim, dtype=torch.float64), 0
+    for i, c in enumerate(pos):
+        x = KV[r0:r0 + c + 1].double()
+        k, v = x[:, :kv_heads * dim].reshape(c + 1, kv_heads, dim), x[:, kv_heads * dim:].reshape(c + 1, kv_heads, vdim)
+        q = Q[i, stride:stride + heads * dim].double().reshape(kv_heads, per, dim)
+        want[i] = torch.einsum("ghj,jgv->ghv", torch.softmax(torch.einsum("ghd,jgd->ghj", q, k) * scale, -1), v).reshape(heads, vdim)
+        r0 += c + 1
+    tiles = torch.tensor([[i, 1, s, c] for i, (s, c) in enumerate(zip(slots, pos))], dtype=torch.int32, device=dev)
+    Qd, pt = Q.to(dev), kv.page_table_
+    for workers in (1, lib.pa_masked_decode_workers(n, heads, kv_heads, 301)):
+        ws = torch.empty(lib.pa_masked_decode_workspace_bytes(n, heads, kv_heads, vdim, workers), dtype=torch.uint8, device=dev)
+        out = torch.full((n, heads * vdim), float("nan"), dtype=BF, device=dev)
+        assert lib.pa_masked_decode(
+            Qd.data_ptr(), Qd.stride(0), stride, kv.key_buffer_.data_ptr(), kv.value_buffer_.data_ptr(), pt.device_data().data_ptr(),
+            pt.num_beams_, pt.num_heads_, pt.num_tiles_, kv.total_pages_, kv.tile_size_, tiles.data_ptr(), n, heads, dim, vdim, scale, 0.0, 0, 0, 0,
+            0, None, 0, None, None, None, None, None, 0, 0, out.data_ptr(), workers, ws.data_ptr(), ws.numel(), _cabi.stream()) == 0
+        got, fin = out.double().cpu().reshape(want.shape), torch.isfinite(want)
+        assert torch.equal(torch.nan_to_num(got[~fin], 7.0), torch.nan_to_num(want[~fin], 7.0)), (workers, got[~fin], want[~fin])
+        err = (got - want)[fin].abs() - 2.0 ** -8 * want[fin].abs()
+        assert err.max().item() < 2.0 ** -16 * V.abs().max().item(), (workers, err.max().item())
