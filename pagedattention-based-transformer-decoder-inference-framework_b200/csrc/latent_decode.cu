@@ -7,11 +7,12 @@
 // serves both products: for the scores a warp takes 8 keys and half of the columns, the partial scores meet in shared memory
 // behind the one barrier of a step, every warp keeps the softmax of all 32 keys, and for the weighted sums a warp owns an
 // eighth of the latent columns -- nothing is computed twice but the 16 x 32 exponentials.  Shares that end inside a token are
-// joined by a second kernel; share w of pair p goes to slot p + w (see masked_decode.cu).
+// joined by a second kernel (decode_shares.cuh).
 //
 // What bounds it: HBM, 180 KB in flight per SM; the chain of a step (scores, exchange, exponentials, weighted sums) is the
 // rest.  64 tokens, 16 heads, rank 512 + 64, 2048 keys (151 MB): 49 us = 3.1 TB/s (latent_attention_mma_kernel with two key splits
 // and its merge: 70 + 8 us); 8 tokens, 8 heads, rank 256 + 32, 400 keys: 7.5 us (13.6 us).
+#include "decode_shares.cuh"
 #include "mma_utils.cuh"
 #include "seq_common.cuh"
 #include "tcgen05_utils.cuh"
@@ -19,7 +20,8 @@
 namespace pa {
 namespace ldec {
 
-constexpr int kUnit = 32, kRows = 16, kConsumers = 8, kThreads = (kConsumers + 1) * 32, kMostTiles = 4096;
+// at least two units a share: opening and closing one costs about as much as that
+constexpr int kUnit = 32, kRows = 16, kConsumers = 8, kThreads = (kConsumers + 1) * 32, kLeast = 2;
 constexpr int kSLd = 40;                // row stride of the score exchange (floats): two rows apart do not share banks
 
 __host__ __device__ constexpr int blocks_for(int kvr) { return kvr / 64 + 1; }      // 64-column blocks of a row; the last is the rotated part
@@ -42,16 +44,6 @@ struct Args {
     int* pre;                   // [ntiles + 1] units of one pair of every token, summed up
     float* part;                // [slots][rows][2 + kv_rank]: maximum (log2), sum, weighted sums
 };
-
-__device__ __forceinline__ int find_tile(const int* pre, int n, int64_t f, int pairs) {
-    int lo = 0, hi = n;
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if ((int64_t)pre[mid] * pairs <= f) lo = mid;
-        else hi = mid;
-    }
-    return lo;
-}
 
 template <int KVR>
 __global__ void __launch_bounds__(kThreads, 1) latent_decode_kernel(const __grid_constant__ CUtensorMap tmP, const Args a) {
@@ -78,31 +70,15 @@ __global__ void __launch_bounds__(kThreads, 1) latent_decode_kernel(const __grid
         fail_word = 0;
         mbar_fence_init();
     }
-    for (int t = threadIdx.x; t < a.ntiles; t += blockDim.x) pre[t + 1] = (__ldg(a.tiles + 4 * t + 3) + kUnit) / kUnit;
-    __syncthreads();
-    if (warp == 0) {
-        int run = 0;
-        for (int t0 = 0; t0 < a.ntiles; t0 += 32) {
-            int n = t0 + lane < a.ntiles ? pre[t0 + lane + 1] : 0;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, n, o);
-                if (lane >= o) n += v;
-            }
-            if (t0 + lane < a.ntiles) pre[t0 + lane + 1] = run + n;
-            run += __shfl_sync(0xffffffffu, n, 31);
-        }
-        if (lane == 0) pre[0] = 0;
-    }
-    __syncthreads();
+    shares::count_units(pre, a.ntiles, [&](int t) { return (__ldg(a.tiles + 4 * t + 3) + kUnit) / kUnit; });
     if (blockIdx.x == 0)
         for (int t = threadIdx.x; t <= a.ntiles; t += blockDim.x) a.pre[t] = pre[t];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     const int w = blockIdx.x, pairs = a.hch;
     const int64_t total = (int64_t)pre[a.ntiles] * pairs;
-    const int64_t shares = min((int64_t)a.workers, total);     // every share has a unit
-    const int64_t f_lo = w < shares ? total * w / shares : 0, f_hi = w < shares ? total * (w + 1) / shares : 0;
+    const int64_t ns = shares::count(total, a.workers, kLeast);
+    const int64_t f_lo = w < ns ? total * w / ns : 0, f_hi = w < ns ? total * (w + 1) / ns : 0;
     if (f_lo >= f_hi) return;
 
     if (warp == kConsumers) {
@@ -110,7 +86,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_decode_kernel(const __grid
         auto row_of = [&](int64_t f0) -> int {
             const int64_t f = f0 + (lane >> 1);
             if (f >= f_hi) return -1;
-            const int t = find_tile(pre, a.ntiles, f, pairs), per = pre[t + 1] - pre[t];
+            const int t = shares::find_token(pre, a.ntiles, f, pairs), per = pre[t + 1] - pre[t];
             const int u = (int)(f - (int64_t)pre[t] * pairs) % per, j = u * kUnit + (lane & 1) * 16;
             const int4 tl = __ldg(reinterpret_cast<const int4*>(a.tiles) + t);
             const int pt = j / a.tile_size;
@@ -150,7 +126,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_decode_kernel(const __grid
     // ---- consumers
     const int nkey = (warp & 3) * 8, kg = warp >> 2;            // scores: these 8 keys, this half of the columns
     const int p0 = kg ? KPH : 0, np_mine = kg ? KP - KPH : KPH;
-    int t = find_tile(pre, a.ntiles, f_lo, pairs), per = pre[t + 1] - pre[t], pr, u;
+    int t = shares::find_token(pre, a.ntiles, f_lo, pairs), per = pre[t + 1] - pre[t], pr, u;
     {
         const int rem = (int)(f_lo - (int64_t)pre[t] * pairs);
         pr = rem / per;
@@ -338,10 +314,10 @@ __global__ void __launch_bounds__(128) latent_decode_join_kernel(const Args a) {
     if (wid >= a.ntiles * a.hch * a.rows) return;
     const int r = wid % a.rows, pair = wid / a.rows, t = pair / a.hch, pr = pair % a.hch, head = pr * kRows + r;
     if (head >= a.heads) return;
-    const int64_t total = (int64_t)a.pre[a.ntiles] * a.hch, shares = min((int64_t)a.workers, total);
+    const int64_t total = (int64_t)a.pre[a.ntiles] * a.hch, ns = shares::count(total, a.workers, kLeast);
     const int per = a.pre[t + 1] - a.pre[t];
     const int64_t f0 = (int64_t)a.pre[t] * a.hch + (int64_t)pr * per, f1 = f0 + per - 1;
-    const int w0 = (int)(((f0 + 1) * shares - 1) / total), w1 = (int)(((f1 + 1) * shares - 1) / total);
+    const int w0 = (int)(((f0 + 1) * ns - 1) / total), w1 = (int)(((f1 + 1) * ns - 1) / total);
     const int ld = 2 + KVR;
     const float* src = a.part + (((int64_t)pair + w0) * a.rows + r) * ld;
     const int64_t step = (int64_t)a.rows * ld;
@@ -383,8 +359,6 @@ __global__ void __launch_bounds__(128) latent_decode_join_kernel(const Args a) {
     for (int i = 0; i < NV; ++i) *reinterpret_cast<uint32_t*>(dst + 2 * lane + 64 * i) = pack_bf16x2(acc[i].x * inv, acc[i].y * inv);
 }
 
-static size_t pre_bytes(int ntiles) { return ((size_t)(ntiles + 1) * sizeof(int) + 15) / 16 * 16; }
-
 template <int KVR>
 static int launch(const CUtensorMap& m, const Args& a, cudaStream_t st) {
     const size_t smem = (size_t)stages_for(KVR) * (stage_bytes(KVR) + 16) + (a.ntiles + 1) * 4 + 1024;
@@ -413,16 +387,14 @@ using namespace pa;
 
 PA_API int pa_latent_decode_workers(int num_tokens, int heads, int64_t longest) {
     if (num_tokens <= 0 || heads <= 0 || longest <= 0) return 0;
-    // at least two units a worker: opening and closing a share costs about as much as that
     const int64_t units = (int64_t)num_tokens * ((heads + ldec::kRows - 1) / ldec::kRows) * ((longest + ldec::kUnit - 1) / ldec::kUnit);
-    const int64_t w = (units + 1) / 2, most = device_info().sm_count;
-    return (int)(w < most ? w : most);
+    return (int)shares::count(units, device_info().sm_count, ldec::kLeast);
 }
 
 PA_API size_t pa_latent_decode_workspace_bytes(int num_tokens, int heads, int kv_rank, int workers) {
     if (num_tokens <= 0 || heads <= 0 || kv_rank <= 0 || workers <= 0) return 0;
     const int hch = (heads + ldec::kRows - 1) / ldec::kRows, rows = heads < ldec::kRows ? heads : ldec::kRows;
-    return ldec::pre_bytes(num_tokens) + ((size_t)num_tokens * hch + workers) * rows * (2 + kv_rank) * sizeof(float);
+    return shares::pre_bytes(num_tokens) + ((size_t)num_tokens * hch + workers) * rows * (2 + kv_rank) * sizeof(float);
 }
 
 PA_API int pa_latent_decode(const void* d_q_lat, int64_t ql_row_stride, int64_t ql_head_stride, const void* d_q_rot,
@@ -436,7 +408,7 @@ PA_API int pa_latent_decode(const void* d_q_lat, int64_t ql_row_stride, int64_t 
     if (num_q_tiles == 0) return PA_OK;
     const int64_t rows = (int64_t)total_pages * tile_size;
     const int kd = kv_rank + rot_dim;
-    if (kv_rank % 128 || kv_rank > 512 || rot_dim % 8 || rot_dim > 64 || tile_size % 16 || num_q_tiles > kMostTiles || rows >= 0x7fffff00ll)
+    if (kv_rank % 128 || kv_rank > 512 || rot_dim % 8 || rot_dim > 64 || tile_size % 16 || num_q_tiles > shares::kMostTokens || rows >= 0x7fffff00ll)
         return PA_ERR_UNSUPPORTED;
     if (((uintptr_t)d_pool | (uintptr_t)d_q_tiles | (uintptr_t)d_workspace) % 16 || ((uintptr_t)d_q_lat | (uintptr_t)d_q_rot | (uintptr_t)d_out) % 4 ||
         (ql_row_stride | ql_head_stride | qr_row_stride | qr_head_stride | o_row_stride | o_head_stride) % 2)
@@ -451,7 +423,7 @@ PA_API int pa_latent_decode(const void* d_q_lat, int64_t ql_row_stride, int64_t 
     a.rows = heads < kRows ? heads : kRows; a.rot_dim = rot_dim; a.workers = workers; a.total_rows = (int)rows; a.scale = scale;
     a.sink = d_sink; a.out = static_cast<bf16_t*>(d_out); a.o_rs = o_row_stride; a.o_hs = o_head_stride;
     a.pre = static_cast<int*>(d_workspace);
-    a.part = reinterpret_cast<float*>(static_cast<char*>(d_workspace) + pre_bytes(num_q_tiles));
+    a.part = reinterpret_cast<float*>(static_cast<char*>(d_workspace) + shares::pre_bytes(num_q_tiles));
     CUtensorMap m;
     if (!tc::make_bf16_map(&m, d_pool, rows, kd, kd, 16)) return PA_ERR_UNSUPPORTED;
     cudaStream_t st = as_stream(stream);

@@ -5,8 +5,7 @@
 // worker with an equal contiguous share of that list, whatever the lengths of the sequences: it streams its units through a
 // ring of its own (TMA boxes of 16 keys x 64 columns, SWIZZLE_128B, page ids 32 units ahead), the query heads of the kv head
 // are the rows of mma.sync m16n8k16 products (up to 16, the rest zero), and where its share leaves a (token, kv head) pair it
-// writes the pair's running maximum, sum and weighted sum.  Share w of pair p goes to slot p + w: walking the list, every new
-// share belongs to the next pair or the next worker, so no two meet.  A second kernel, resident before the first ends
+// writes the pair's running maximum, sum and weighted sum (decode_shares.cuh).  A second kernel, resident before the first ends
 // (programmatic dependent launch), joins the shares of each pair and applies sink, turn and gate.
 //
 // The softmax weights enter the second product as bfloat16 for batches that give every SM a pair, as in masked_attention.cu's
@@ -17,6 +16,7 @@
 // costs a warp about 150 instructions.  64 tokens, 16 query / 4 kv heads of 128, 2048 keys (268 MB): 56 us = 4.8 TB/s and 4 us for the
 // join (heads as rows without a key split, masked_attention_mma_decode_kernel: 91 us); 8 tokens, 2 kv heads, 400 keys: 10 us
 // (streaming kernel, one CTA per pair: 38 us).
+#include "decode_shares.cuh"
 #include "masked_attention.cuh"
 #include "mma_utils.cuh"
 #include "tcgen05_utils.cuh"
@@ -24,7 +24,8 @@
 namespace pa {
 namespace mdec {
 
-constexpr int kWarps = 8, kStages = 3, kUnit = 16, kRows = 16, kMostTiles = 4096;
+// at least four units a share: opening and closing one costs about as much as that
+constexpr int kWarps = 8, kStages = 3, kUnit = 16, kRows = 16, kLeast = 4;
 
 struct Args {
     MaskAttnParams p;
@@ -37,17 +38,6 @@ struct Args {
 __device__ __forceinline__ int tile_units(const MaskAttnParams& p, int pos) {
     return ma_steps(p, ma_first_key(p, pos), pos + 1, kUnit).count;
 }
-// the token whose pairs hold unit f (pre[] * pairs is the first unit of a token's pairs)
-__device__ __forceinline__ int find_tile(const int* pre, int n, int64_t f, int pairs) {
-    int lo = 0, hi = n;
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if ((int64_t)pre[mid] * pairs <= f) lo = mid;
-        else hi = mid;
-    }
-    return lo;
-}
-
 // FLOAT_W: the weights of the second product are float (see above)
 template <int DIM, int VDIM, bool FLOAT_W>
 __global__ void __launch_bounds__(kWarps * 32, 1) masked_decode_kernel(const __grid_constant__ CUtensorMap tmK,
@@ -67,23 +57,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) masked_decode_kernel(const __g
         mbar_fence_init();
     }
     if (threadIdx.x == 0) fail_word = 0;
-    for (int t = threadIdx.x; t < a.ntiles; t += blockDim.x) pre[t + 1] = tile_units(p, __ldg(p.tiles + 4 * t + 3));
-    __syncthreads();
-    if (warp == 0) {
-        int run = 0;
-        for (int t0 = 0; t0 < a.ntiles; t0 += 32) {
-            int n = t0 + lane < a.ntiles ? pre[t0 + lane + 1] : 0;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, n, o);
-                if (lane >= o) n += v;
-            }
-            if (t0 + lane < a.ntiles) pre[t0 + lane + 1] = run + n;
-            run += __shfl_sync(0xffffffffu, n, 31);
-        }
-        if (lane == 0) pre[0] = 0;
-    }
-    __syncthreads();
+    shares::count_units(pre, a.ntiles, [&](int t) { return tile_units(p, __ldg(p.tiles + 4 * t + 3)); });
     if (blockIdx.x == 0)
         for (int t = threadIdx.x; t <= a.ntiles; t += blockDim.x) a.pre[t] = pre[t];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -91,14 +65,14 @@ __global__ void __launch_bounds__(kWarps * 32, 1) masked_decode_kernel(const __g
     const int w = warp * gridDim.x + blockIdx.x;
     const int pairs = p.num_kv_heads * a.hch, hpg = p.heads / p.num_kv_heads;
     const int64_t total = (int64_t)pre[a.ntiles] * pairs;
-    const int64_t shares = min((int64_t)a.workers, total);     // every share has a unit: none is read that was not written
-    const int64_t f_lo = w < shares ? total * w / shares : 0, f_hi = w < shares ? total * (w + 1) / shares : 0;
+    const int64_t ns = shares::count(total, a.workers, kLeast);
+    const int64_t f_lo = w < ns ? total * w / ns : 0, f_hi = w < ns ? total * (w + 1) / ns : 0;
     if (f_lo >= f_hi) return;
 
     // ---- the copies: unit f's rows in the pools, 32 units at a time
     auto rows_of = [&](int64_t f) -> int {
         if (f >= f_hi) return -1;
-        const int t = find_tile(pre, a.ntiles, f, pairs), per = pre[t + 1] - pre[t];
+        const int t = shares::find_token(pre, a.ntiles, f, pairs), per = pre[t + 1] - pre[t];
         const int rem = (int)(f - (int64_t)pre[t] * pairs), g = rem / per / a.hch, u = rem % per;
         const int4 tl = __ldg(reinterpret_cast<const int4*>(p.tiles) + t);
         const MaSteps st = ma_steps(p, ma_first_key(p, tl.w), tl.w + 1, kUnit);
@@ -137,7 +111,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) masked_decode_kernel(const __g
     for (int s = 0; s < kStages; ++s) issue();
 
     // ---- the pair at hand
-    int t = find_tile(pre, a.ntiles, f_lo, pairs);
+    int t = shares::find_token(pre, a.ntiles, f_lo, pairs);
     int per = pre[t + 1] - pre[t], pr, u;       // units of a pair of token t, pair within the token, unit within the pair
     {
         const int rem = (int)(f_lo - (int64_t)pre[t] * pairs);
@@ -358,8 +332,8 @@ __global__ void __launch_bounds__(128) masked_decode_join_kernel(const Args a) {
     const int64_t total = (int64_t)a.pre[a.ntiles] * pairs;
     const int per = a.pre[t + 1] - a.pre[t];
     const int64_t f0 = (int64_t)a.pre[t] * pairs + (int64_t)pr * per, f1 = f0 + per - 1;
-    const int64_t shares = min((int64_t)a.workers, total);
-    const int w0 = (int)(((f0 + 1) * shares - 1) / total), w1 = (int)(((f1 + 1) * shares - 1) / total);
+    const int64_t ns = shares::count(total, a.workers, kLeast);
+    const int w0 = (int)(((f0 + 1) * ns - 1) / total), w1 = (int)(((f1 + 1) * ns - 1) / total);
     const int ld = 2 + VDIM;
     const float* src = a.part + (((int64_t)pair + w0) * a.rows + r) * ld;
     const int64_t step = (int64_t)a.rows * ld;
@@ -414,8 +388,6 @@ __global__ void __launch_bounds__(128) masked_decode_join_kernel(const Args a) {
     }
 }
 
-static size_t pre_bytes(int ntiles) { return ((size_t)(ntiles + 1) * sizeof(int) + 15) / 16 * 16; }
-
 template <int DIM, int VDIM, bool FLOAT_W>
 static int launch(const CUtensorMap& k, const CUtensorMap& v, const Args& a, cudaStream_t st) {
     const size_t smem = (size_t)kWarps * kStages * ((DIM + VDIM) / 64 * 2048 + 8) + (a.ntiles + 1) * 4 + 1024;
@@ -447,16 +419,14 @@ using namespace pa;
 PA_API int pa_masked_decode_workers(int num_tokens, int heads, int kv_heads, int64_t longest) {
     if (num_tokens <= 0 || kv_heads <= 0 || heads <= 0 || heads % kv_heads || longest <= 0) return 0;
     const int hch = (heads / kv_heads + mdec::kRows - 1) / mdec::kRows;
-    // at least four units a worker: opening and closing a share costs about as much as that
     const int64_t units = (int64_t)num_tokens * kv_heads * hch * ((longest + mdec::kUnit - 1) / mdec::kUnit), most = mdec::kWarps * device_info().sm_count;
-    const int64_t w = (units + 3) / 4;
-    return (int)(w < most ? w : most);
+    return (int)shares::count(units, (int)most, mdec::kLeast);
 }
 
 PA_API size_t pa_masked_decode_workspace_bytes(int num_tokens, int heads, int kv_heads, int vdim, int workers) {
     if (num_tokens <= 0 || kv_heads <= 0 || heads <= 0 || heads % kv_heads || vdim <= 0 || workers <= 0) return 0;
     const int hpg = heads / kv_heads, hch = (hpg + mdec::kRows - 1) / mdec::kRows, rows = hpg < mdec::kRows ? hpg : mdec::kRows;
-    return mdec::pre_bytes(num_tokens) + ((size_t)num_tokens * kv_heads * hch + workers) * rows * (2 + vdim) * sizeof(float);
+    return shares::pre_bytes(num_tokens) + ((size_t)num_tokens * kv_heads * hch + workers) * rows * (2 + vdim) * sizeof(float);
 }
 
 PA_API int pa_masked_decode(const void* d_q, int64_t q_stride, int q_off, const void* d_k_pool, const void* d_v_pool,
@@ -475,7 +445,7 @@ PA_API int pa_masked_decode(const void* d_q, int64_t q_stride, int q_off, const 
     PA_CHECK_ARG(bias_kind >= 0 && bias_kind <= 2 && (bias_kind == 0 || d_bias) && (bias_kind != 2 || bias_len > 0));
     if (num_q_tiles == 0) return PA_OK;
     const int64_t rows = (int64_t)total_pages * tile_size;
-    if ((dim != 64 && dim != 128) || (vdim != 64 && vdim != 128) || d_k_pool == d_v_pool || num_q_tiles > kMostTiles || tile_size % 16 ||
+    if ((dim != 64 && dim != 128) || (vdim != 64 && vdim != 128) || d_k_pool == d_v_pool || num_q_tiles > shares::kMostTokens || tile_size % 16 ||
         rows >= 0x7fffff00ll)
         return PA_ERR_UNSUPPORTED;
     if (((uintptr_t)d_k_pool | (uintptr_t)d_v_pool | (uintptr_t)d_q_tiles | (uintptr_t)d_workspace) % 16 || (uintptr_t)d_q % 4 ||
@@ -499,7 +469,7 @@ PA_API int pa_masked_decode(const void* d_q, int64_t q_stride, int q_off, const 
     a.workers = workers;
     a.total_rows = (int)rows;
     a.pre = static_cast<int*>(d_workspace);
-    a.part = reinterpret_cast<float*>(static_cast<char*>(d_workspace) + pre_bytes(num_q_tiles));
+    a.part = reinterpret_cast<float*>(static_cast<char*>(d_workspace) + shares::pre_bytes(num_q_tiles));
     CUtensorMap k, v;
     if (!tc::make_bf16_map(&k, d_k_pool, rows, dim, dim, 16) || !tc::make_bf16_map(&v, d_v_pool, rows, vdim, vdim, 16)) return PA_ERR_UNSUPPORTED;
     cudaStream_t st = as_stream(stream);

@@ -57,7 +57,7 @@ class _Lane:
 class DecodeSteps:
     """Steps that decode one token of each of n sequences, as CUDA graphs: such a step is some dozens of launches of a few
     microseconds each, and issuing them takes several times as long as running them (8 sequences, 4 layers of width 1024: 1.0 ms
-    launch by launch, 0.3 ms replayed).  A graph belongs to a number of sequences and a bound of their lengths (a power of two).
+    launch by launch, 0.3 ms replayed).  A graph belongs to a number of sequences and a bound of their lengths (see _bound).
     A capture costs as much as 6 to 30 launched steps, so the first PATIENCE steps of a kind run launch by launch; from then on a
     step writes its tokens, slots and positions into the graph's buffers and replays it.  Where more kinds come up than graphs are kept,
     captures stay rare: one in GAP steps at most, a graph gives way only after IDLE steps without a replay, and a kind that was captured
@@ -95,6 +95,18 @@ class DecodeSteps:
                 len(wanted_rows) == len(entries) and all(len(t) == 1 for _s, t in entries) and
                 not torch.cuda.is_current_stream_capturing())
 
+    def _bound(self, longest):
+        """The bound of the lengths that the launches of a graph are made for: a power of two from 512 on.  Equal shares of the keys
+        follow from the lengths alone, so these launches give the bits of launches made for the exact lengths; the kernels that cut
+        keys by the longest context do so from 513 keys on, by its multiples of 256 and up to 64 of them: where a layer runs on
+        those, the bound lies between the same multiples."""
+        if 512 < longest < 64 * 256 and any(getattr(mixer, "cuts_keys", False) for _L, mixer, _pass in self.model.runs):
+            return longest // 256 * 256 + 255
+        bound = 512
+        while bound < longest:
+            bound *= 2
+        return bound
+
     def _watched(self):
         """What a forward pass reads: [(owner's dict, its size, [(key, value, address of a tensor)])] and the runs."""
         seen, out = set(), []
@@ -120,10 +132,7 @@ class DecodeSteps:
     def step(self, entries):
         """Logits [n, vocab] of the step, or None where it is to run launch by launch."""
         m, st = self.model, self.model.states
-        longest = max((st.length(s) for s, _t in entries), default=0) + 1
-        bound = 256
-        while bound < longest:
-            bound *= 2
+        bound = self._bound(max((st.length(s) for s, _t in entries), default=0) + 1)
         key = (len(entries), bound)
         self._now += 1
         g = self._graphs.get(key)

@@ -211,6 +211,7 @@ class DiffAttentionMixer:
     """Differential attention with grouped key/value heads over a paged pool of its own (KVTileCache with key rows
     of 2 * dim and value rows of vdim)."""
     kind = "attention"
+    cuts_keys = True        # a decoded token's keys are cut by the longest context of the step
 
     def __init__(self, model, prefix, cfg, W):
         self.heads, self.kv_heads = int(cfg["heads"]), int(cfg["kv_heads"])
@@ -267,6 +268,7 @@ class DiffAttentionMixer:
         return c.model._linear(out, self.w_o)
 
 
+SHARE_TOKENS = 4096       # decoded tokens of a step that the kernels with equal shares of the keys serve
 EXPAND_FROM = 64          # portions at least this long run latent attention on keys and values built per head (bfloat16)
 ROPE_PAIRING = {"neighbours": 0, "halves": 1}
 
@@ -350,6 +352,7 @@ class LatentAttentionMixer:
         self.mma_tokens = 0
         if self.dim % 8 == 0 and qd % 8 == 0:
             self.mma_tokens = model._lib.pa_latent_attention_mma_tile_tokens(H, self.kv_rank, self.rot_dim, _ELEM[model.act_dtype])
+        self.shares = self.mma_tokens > 0 and self.kv_rank % 128 == 0       # decoded tokens with their keys in equal shares
         # prompt portions with keys and values built per head (tcgen05): tokens per tile with two and with one query tile per CTA
         self.tc_tokens, self.w_ukv = (0, 0), None
         lib, elem = model._lib, _ELEM[model.act_dtype]
@@ -358,6 +361,11 @@ class LatentAttentionMixer:
                 lib.pa_masked_attention_tc_tile_tokens(1, 1, self.dim, self.vdim, elem, 2)):
             self.tc_tokens = tuple(lib.pa_masked_attention_tc_tile_tokens(1, 1, self.dim, self.vdim, elem, q) for q in (2, 1))
             self.w_ukv = model._weight_raw(torch.cat([W[prefix + "uk"], W[prefix + "uv"]], 0))        # [H * (dim + vdim)][kv_rank]
+
+    @property
+    def cuts_keys(self):
+        """Whether a decoded token's keys are cut by the longest context of the step (shares follow from all lengths alone)."""
+        return not (self.shares and self.mma_tokens)
 
     def alloc_state(self, model):
         self.kv = model.states.add_kv_layer(1, self.kd, 0, _KV[model.act_dtype])
@@ -412,7 +420,7 @@ class LatentAttentionMixer:
                 continue
             tiles, ntiles, longest = group
             ws = None
-            if kind == 1 and mma and kvr % 128 == 0:    # decoded tokens: their keys in equal shares, where that kernel takes the operands
+            if kind == 1 and mma and self.shares:       # where that kernel takes the operands
                 workers = lib.pa_latent_decode_workers(ntiles, H, longest)
                 ws = c.empty(lib.pa_latent_decode_workspace_bytes(ntiles, H, kvr, workers), dtype=torch.uint8)
                 st = lib.pa_latent_decode(ql.data_ptr(), kvr, R * kvr, q.data_ptr() + self.dim * c.elem, q.stride(0), self.qd,
@@ -422,7 +430,7 @@ class LatentAttentionMixer:
                 if st != _cabi.PA_ERR_UNSUPPORTED:
                     _chk(st, "pa_latent_decode")
                     continue
-                ws = None
+                ws, self.shares = None, ntiles > SHARE_TOKENS       # more tokens than it serves in this step, or never
             nsplit = latent_key_splits(ntiles * math.ceil(H / rows_per_cta), longest, c.model.sm_count)
             if nsplit > 1:
                 ws = c.empty(lib.pa_latent_attention_workspace_bytes(ntiles, H, kvr, nsplit), dtype=torch.uint8)
@@ -813,6 +821,7 @@ class MaskedAttention:
                                   _cabi.ptr(gate[0]), gate[0].stride(0) if gate[0] is not None else 0, gate[1], out.data_ptr(), workers,
                                   ws.data_ptr(), ws.numel(), _cabi.stream())
         if st == _cabi.PA_ERR_UNSUPPORTED:
+            self.shares = ntiles > SHARE_TOKENS         # more tokens than it serves in this step, or never
             return False
         _chk(st, "pa_masked_decode")
         return True

@@ -183,7 +183,7 @@ class DecodeBatch(RaggedBatch):
     """The description of a step that decodes ONE token of each of n sequences, in device buffers that stay: everything about such
     a step but the sequences' tokens, slots and positions is the same every time, so the next step writes those into the same
     places (fill) and the launches of one step serve for all (engine.DecodeSteps).  longest: an upper bound of the sequences'
-    lengths, which the launches are sized for."""
+    lengths, which the launches are sized for (and cut as for the lengths themselves, see engine.DecodeSteps)."""
 
     def __init__(self, n, longest, device, prev_ids):
         self.rows = self.num_seqs = n

@@ -6,7 +6,7 @@ import random
 import pytest
 import torch
 
-from oracle import dubarax_ref, namudra_ref, tiradra_ref
+from oracle import domilix_ref, dubarax_ref, gunulorn_ref, hybrid_ref, namudra_ref, tiradra_ref
 
 
 def _pair(config, W, **kw):
@@ -116,6 +116,52 @@ def test_functions_in_place_of_methods_and_failed_captures():
     for k in range(6):
         _close(a.step([(0, [k + 9], [0])]), b.step([(0, [k + 9], [0])]))
     assert not a._decode._graphs
+
+
+def _design(name):
+    """A model of every design, with the head sizes of the shared-out kernels where the design has such layers, and without."""
+    if name == "megusun":
+        R = hybrid_ref
+        c = R.make_config([R.attention_layer(mlp=R.moe_mlp()), R.mingru_layer(mlp=R.dense_mlp())])
+    elif name == "domilix":
+        R = domilix_ref
+        c = R.make_config([R.latent_layer(mlp=R.dense_mlp()), R.latent_layer(heads=20, dim=16, rot_dim=16, kv_rank=128, mlp=R.moe_mlp()),
+                           R.latent_layer(kv_from=0, mlp=R.dense_mlp())])
+    elif name == "gunulorn":
+        R = gunulorn_ref
+        c = R.make_config([R.conv_layer(dim=64, vdim=128, mlp=R.dense_mlp()), R.window_layer(dim=64, vdim=64, mlp=R.moe_mlp()),
+                           R.conv_layer(mlp=R.dense_mlp())])
+    elif name == "dubarax":
+        R = dubarax_ref
+        c = R.make_config([R.attention_layer(dim=64, vdim=64, window=300, mlp=R.moe_mlp()), R.parallel_layer(mlp=R.moe_mlp()), R.mamba_layer(mlp=R.moe_mlp())])
+    elif name == "namudra":
+        R = namudra_ref
+        c = R.make_config([R.window_layer(), R.latent_layer(), R.latent_layer(dim=16, rot_dim=16, kv_rank=256), R.retention_layer(dim=64, vdim=64)])
+    else:
+        R = tiradra_ref
+        c = R.make_config([R.attention_layer(dim=128, heads=4, kv_heads=2), R.latent_layer(dim=16, rot_dim=16, kv_rank=128), R.latent_layer()])
+    return c, R.random_weights(c, 5)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", ["megusun", "domilix", "dubarax", "gunulorn", "namudra", "tiradra"])
+def test_a_replayed_step_gives_the_bits_of_a_launched_one(name):
+    """A request's logits do not depend on how many steps of a kind the engine has run: contexts of unequal length, past the bounds from
+    which kernels cut their keys, growing over a multiple of 256 and of 512."""
+    config, W = _design(name)
+    a, b = _pair(config, W, max_tokens=4096, max_seqs=4)
+    a._decode.GAP = 0
+    g = torch.Generator().manual_seed(2)
+    tok = lambda n=1: torch.randint(0, config["vocab"], (n,), generator=g).tolist()  # noqa: E731
+    both = lambda entries: (a.step(entries), b.step(entries))  # noqa: E731
+    both([(0, tok(762), [761]), (1, tok(90), [89]), (2, tok(20), [19]), (3, tok(506), [505])])
+    replays = 0
+    for ids in ((0, 1, 2), (3,), (3, 1)):
+        for k in range(12):
+            x, y = both([(i, tok(), [0]) for i in ids])
+            assert torch.equal(x, y), (ids, k, (x - y).abs().max())
+        replays += sum(k[0] == len(ids) for k in a._decode._graphs)
+    assert replays >= 3
 
 
 class _Held:
