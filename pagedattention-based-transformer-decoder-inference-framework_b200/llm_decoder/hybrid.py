@@ -270,6 +270,7 @@ class DiffAttentionMixer:
 
 SHARE_TOKENS = 4096       # decoded tokens of a step that the kernels with equal shares of the keys serve
 EXPAND_FROM = 64          # portions at least this long run latent attention on keys and values built per head (bfloat16)
+EXPAND_BYTES = 128 << 20  # ... in buffers of this size, or of what the other form takes for the step's rows
 ROPE_PAIRING = {"neighbours": 0, "halves": 1}
 
 
@@ -354,13 +355,13 @@ class LatentAttentionMixer:
             self.mma_tokens = model._lib.pa_latent_attention_mma_tile_tokens(H, self.kv_rank, self.rot_dim, _ELEM[model.act_dtype])
         self.shares = self.mma_tokens > 0 and self.kv_rank % 128 == 0       # decoded tokens with their keys in equal shares
         # prompt portions with keys and values built per head (tcgen05): tokens per tile with two and with one query tile per CTA
-        self.tc_tokens, self.w_ukv = (0, 0), None
+        self.tc_tokens = None
         lib, elem = model._lib, _ELEM[model.act_dtype]
         q_cols = H * qd if self.q_latent else int(self.w_in.shape[0])       # row stride of the queries: 16-byte rows
         if (self.mma_tokens and 16 <= self.rot_dim <= 64 and self.rot_dim % 16 == 0 and self.kv_rank % 8 == 0 and q_cols % 8 == 0 and
                 lib.pa_masked_attention_tc_tile_tokens(1, 1, self.dim, self.vdim, elem, 2)):
             self.tc_tokens = tuple(lib.pa_masked_attention_tc_tile_tokens(1, 1, self.dim, self.vdim, elem, q) for q in (2, 1))
-            self.w_ukv = model._weight_raw(torch.cat([W[prefix + "uk"], W[prefix + "uv"]], 0))        # [H * (dim + vdim)][kv_rank]
+            self.w_uv = model._weight_raw(W[prefix + "uv"].reshape(H, self.vdim, self.kv_rank)).transpose(1, 2)     # the same, by output channel
 
     @property
     def cuts_keys(self):
@@ -390,24 +391,34 @@ class LatentAttentionMixer:
                                   _cabi.stream()), "pa_head_linear")
         return out
 
-    def _attend_expanded(self, c, q, out, at_least):
+    def _expand_rows(self, c):
+        """How many cached rows have their keys and values built at a time: what fits the memory that queries and weighted sums of
+        kv_rank columns per head would take for this step's rows, or EXPAND_BYTES where that is more, so that a step needs no more
+        than EXPAND_BYTES on top of what it needs without building them."""
+        room = max(EXPAND_BYTES, 2 * self.heads * c.R * self.kv_rank * c.elem)
+        return min(room // ((self.heads * (self.dim + self.vdim) + self.kd) * c.elem), c.batch.EXPAND_MOST)
+
+    def _attend_expanded(self, c, q, out, at_least, most):
         """The prompt portions that build the keys and values of their whole sequences: per head a key of dim + rot_dim and a value
-        of vdim columns instead of kv_rank + rot_dim and kv_rank, for one product over the cached rows."""
+        of vdim columns instead of kv_rank + rot_dim and kv_rank, for two products over the cached rows."""
         b, lib, kv, s, H = c.batch, c.lib, self.kv, _cabi.stream(), self.heads
         pt = kv.page_table_
         q_tiles = 2 if b.count_tiles(self.tc_tokens[0], at_least) * H >= c.model.sm_count else 1
-        for items, nitems, longest, rows, tiles, ntiles in b.whole_sequences(at_least, self.tc_tokens[2 - q_tiles]):
+        for items, nitems, longest, rows, tiles, ntiles in b.whole_sequences(at_least, self.tc_tokens[2 - q_tiles], most):
             lat = c.empty(rows, self.kd)
             _chk(lib.pa_latent_gather(kv.key_buffer_.data_ptr(), pt.device_data().data_ptr(), pt.num_beams_, pt.num_tiles_,
                                       kv.total_pages_, kv.tile_size_, self.kd * c.elem, items.data_ptr(), nitems, longest,
                                       lat.data_ptr(), s), "pa_latent_gather")
-            built = torch.nn.functional.linear(lat[:, :self.kv_rank], self.w_ukv)
-            _chk(lib.pa_latent_attention_expanded(q.data_ptr(), q.stride(0), 0, built.data_ptr(), built.stride(0), lat.data_ptr(),
-                                                  self.kd, self.kv_rank, built.data_ptr() + H * self.dim * c.elem, built.stride(0),
-                                                  rows, tiles.data_ptr(), ntiles, H, self.dim, self.rot_dim, self.vdim, self.scale,
-                                                  _cabi.ptr(self.sink), out.data_ptr(), q_tiles, s), "pa_latent_attention_expanded")
+            # both are views of what the other form reads: w_uk as it lies, w_uv is kept by output channel for this product
+            keys = torch.nn.functional.linear(lat[:, :self.kv_rank], self.w_uk.reshape(H * self.dim, self.kv_rank))
+            values = torch.nn.functional.linear(lat[:, :self.kv_rank], self.w_uv.transpose(1, 2).reshape(H * self.vdim, self.kv_rank))
+            _chk(lib.pa_latent_attention_expanded(q.data_ptr(), q.stride(0), 0, keys.data_ptr(), H * self.dim, lat.data_ptr(), self.kd,
+                                                  self.kv_rank, values.data_ptr(), H * self.vdim, rows, tiles.data_ptr(), ntiles, H,
+                                                  self.dim, self.rot_dim, self.vdim, self.scale, _cabi.ptr(self.sink), out.data_ptr(),
+                                                  q_tiles, s), "pa_latent_attention_expanded")
+            del lat, keys, values       # before the next group's
 
-    def _attend(self, c, q, ql, lat, mma, without=0):
+    def _attend(self, c, q, ql, lat, mma, without=None):
         """Launch the attention kernels over this step's tiles (prompt portions, then single decoded tokens).  Returns
         False when the tensor-core kernel refuses the operands (nothing was written that the float kernel does not
         write again)."""
@@ -482,19 +493,22 @@ class LatentAttentionMixer:
         proj = c.model._linear(h, self.w_in)
         q = self._queries(c, proj)
         kvr = self.kv_rank
-        expand = c.batch.expand_from(EXPAND_FROM) if self.w_ukv is not None else 0
-        if expand and all(c.batch._expands(p, expand) for p in c.batch.portions):
+        most = self._expand_rows(c) if self.tc_tokens else 0
+        expand = c.batch.expand_from(EXPAND_FROM, most) if most else 0
+        without = (expand, most) if expand else None
+        if expand and all(c.batch._expands(p, *without) for p in c.batch.portions):
             ov = c.empty(R, H * self.vdim)
         else:
             ql = self._head_linear(c, q, q.stride(0), self.qd, self.w_uk, self.dim, kvr)          # [H, R, kv_rank]
             lat = c.empty(H, R, kvr)
-            if self.mma_tokens > 0 and not self._attend(c, q, ql, lat, True, expand):
+            if self.mma_tokens > 0 and not self._attend(c, q, ql, lat, True, without):
                 self.mma_tokens = 0         # a stride or an alignment the tensor-core kernel does not take: the float kernel
             if self.mma_tokens == 0:
-                self._attend(c, q, ql, lat, False, expand)
+                self._attend(c, q, ql, lat, False, without)
             ov = self._head_linear(c, lat, kvr, R * kvr, self.w_uv, kvr, self.vdim, by_row=True).view(R, H * self.vdim)
+            del ql, lat
         if expand:      # its rows of ov; what the product above left there came from no query
-            self._attend_expanded(c, q, ov, expand)
+            self._attend_expanded(c, q, ov, expand, most)
         if self.gate != "head":
             if self.gate == "elements":
                 _chk(lib.pa_gate_rows(ov.data_ptr(), ov.stride(0), proj.data_ptr() + self.g_off * c.elem, proj.stride(0),

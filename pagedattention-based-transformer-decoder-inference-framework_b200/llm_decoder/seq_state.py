@@ -66,13 +66,13 @@ class RaggedBatch:
         device tensors (first row, tokens, slot, first position).  Three lists, keyed by the kernel's tile kind:
         1 = portions of ONE token (decoded tokens: the streaming kernel), 2 = portions of at least `big_from` tokens in
         runs of `big_tokens` (the tensor-core kernel; none when big_tokens is 0), 0 = the rest in runs of `tile_tokens`.
-        Each comes as (tensor, count, longest context) or None.  without: leave out the portions that whole_sequences(without)
-        serves."""
+        Each comes as (tensor, count, longest context) or None.  without: (at_least, most), leave out the portions that
+        whole_sequences serves with these."""
         key = ("qt", tile_tokens, big_tokens, big_from, without)
         if key not in self._cache:
             groups = {0: [], 1: [], 2: []}
             for p in self.portions:
-                if without and self._expands(p, without):
+                if without and self._expands(p, *without):
                     continue
                 groups[1 if p[1] == 1 else 2 if big_tokens and p[1] >= big_from else 0].append(p)
             out = {}
@@ -96,33 +96,33 @@ class RaggedBatch:
 
     EXPAND_MOST = 65536         # cached tokens whose keys and values are built at a time
 
-    def _expands(self, p, at_least):
+    def _expands(self, p, at_least, most=EXPAND_MOST):
         """Whether the keys and values of ALL tokens of a portion's sequence are built for its queries.  Building costs a cached
         token as much as about 25 queries save on it (16 heads of 128, rank 512), so the length of the context does not enter, only
-        its place in the buffers."""
-        return p[1] >= at_least and p[3] + p[1] <= self.EXPAND_MOST
+        its place in buffers of `most` tokens."""
+        return p[1] >= at_least and p[3] + p[1] <= most
 
-    def expand_from(self, tokens):
+    def expand_from(self, tokens, most=EXPAND_MOST):
         """From how many new tokens on the portions build keys and values: `tokens` where all of them have that many, else twice as
         many where some do (the others run beside them, with products over every row), else 0."""
-        key = ("ef", tokens)
+        key = ("ef", tokens, most)
         if key not in self._cache:
-            self._cache[key] = (tokens if all(self._expands(p, tokens) for p in self.portions) else
-                                2 * tokens if any(self._expands(p, 2 * tokens) for p in self.portions) else 0)
+            self._cache[key] = (tokens if all(self._expands(p, tokens, most) for p in self.portions) else
+                                2 * tokens if any(self._expands(p, 2 * tokens, most) for p in self.portions) else 0)
         return self._cache[key]
 
-    def whole_sequences(self, at_least, tokens):
-        """The portions that _expands picks, in groups of at most EXPAND_MOST tokens of context: per group ([n, 3] int32 items (slot,
+    def whole_sequences(self, at_least, tokens, most=EXPAND_MOST):
+        """The portions that _expands picks, in groups of at most `most` tokens of context: per group ([n, 3] int32 items (slot,
         tokens, first row), n, longest, rows, [m, 4] query tiles of at most `tokens` tokens (first batch row, tokens, first row of
         the sequence, position), m), longest context first."""
-        key = ("ws", at_least, tokens)
+        key = ("ws", at_least, tokens, most)
         if key not in self._cache:
             groups = []
             for p in self.portions:
-                if not self._expands(p, at_least):
+                if not self._expands(p, at_least, most):
                     continue
                 total = p[3] + p[1]
-                if not groups or groups[-1][1] + total > self.EXPAND_MOST:
+                if not groups or groups[-1][1] + total > most:
                     groups.append([[], 0])
                 groups[-1][0].append((p, groups[-1][1]))
                 groups[-1][1] += total
@@ -232,7 +232,7 @@ class DecodeBatch(RaggedBatch):
     def count_tiles(self, tokens, at_least):
         return 0
 
-    def expand_from(self, tokens):
+    def expand_from(self, tokens, most=0):
         return 0
 
     def scan_chunks(self, chunk):
