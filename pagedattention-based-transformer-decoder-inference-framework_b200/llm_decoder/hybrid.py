@@ -778,11 +778,12 @@ class MaskedAttention:
         out = c.empty(c.R, self.heads * self.vdim)
         if self.tc_plans:
             # two query tiles per CTA stage every key once for 256 rows; one where that leaves SMs without a CTA
-            tokens, units, kind = self.tc_plans[0]
+            tokens, units, kind = plan = self.tc_plans[0]
             if c.batch.count_tiles(tokens, MMA_FROM) * units < c.model.sm_count:
-                tokens, units, kind = self.tc_plans[1]
+                tokens, units, kind = plan = self.tc_plans[-1]
             if self._attend_tiles(c, proj, off, gate, out, tokens, kind):
                 return out
+            self.tc_plans = [p for p in self.tc_plans if p != plan]     # a page size, a stride or a bias table it does not take
         if not self._attend_tiles(c, proj, off, gate, out, self.mma_tokens):
             self.mma_tokens = 0     # a stride or an alignment the tensor-core kernel refuses: the float kernels
             self._attend_tiles(c, proj, off, gate, out, 0)

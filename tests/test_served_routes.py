@@ -79,3 +79,20 @@ def test_memory_of_built_keys_and_values():
     eng.step([(0, [1] * 64, [])])
     most = hybrid.EXPAND_BYTES + 3 * 2 * 64 * H * (kvr + 192 + 128) * 2 + (16 << 20)
     assert torch.cuda.max_memory_allocated() - before < most, (torch.cuda.max_memory_allocated() - before, most)
+
+
+@pytest.mark.gpu
+def test_a_refused_plan_is_not_asked_again():
+    """Pages of 8 tokens: the tcgen05 kernel does not serve them.  The portions of later steps run once, on the kernel that does, and give
+    what pages of 16 give (2e-2 of the logits' spread: bfloat16 sums in another order)."""
+    import llm_decoder as ld
+    from oracle import tiradra_ref as R
+    config = R.make_config([R.attention_layer(heads=4, kv_heads=2, dim=64, vdim=128)])
+    W = R.random_weights(config, 2)
+    engines = [ld.Engine(ld.HybridDecoder(config, W, "bfloat16", max_tokens=512, max_seqs=2, tile_size=t)) for t in (8, 16)]
+    for step in ([(0, 40)], [(0, 1), (1, 130)], [(0, 30), (1, 1)], [(0, 1), (1, 17)]):
+        entries = [(r, [(7 * k + r) % 71 for k in range(n)], [n - 1]) for r, n in step]
+        x, y = (e.step(entries) for e in engines)
+        assert (x - y).abs().max() < 2e-2 * y.abs().max()
+    eight, sixteen = (e.model.layers[0].mixer.core for e in engines)
+    assert eight.tc_plans == [] and eight.mma_tokens and len(sixteen.tc_plans) == 2
