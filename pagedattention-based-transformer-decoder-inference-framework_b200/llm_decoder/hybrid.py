@@ -269,7 +269,14 @@ class DiffAttentionMixer:
 
 
 SHARE_TOKENS = 4096       # decoded tokens of a step that the kernels with equal shares of the keys serve
-EXPAND_FROM = 64          # portions at least this long run latent attention on keys and values built per head (bfloat16)
+# Portions at least this long run latent attention on keys and values built per head (bfloat16), and as long as EXPAND_WORK / kv_rank:
+# what building saves grows with the rank.  GPU time of a layer, the other form over this one, 16 heads of 128 + 64 (64 + 32):
+#   rank 64    64 tokens 0.82 to 1.07 (0.85 to 1.08)   128 tokens 0.93 to 1.07 (0.99 to 1.07)   512 and more 1.7 to 2.2 (2.1 to 2.6)
+#   rank 128   64 tokens 0.89 to 1.09 (0.91 to 1.17)   128 tokens 1.05 to 1.14 (1.14 to 1.21)
+#   rank 256   64 tokens 0.94 to 1.33 (0.98 to 1.43)   128 tokens 1.16 to 1.30 (1.34 to 1.41)
+#   rank 512   64 tokens 1.05 to 1.58 (1.07 to 1.77)   128 tokens 1.37 to 1.55 (1.65 to 1.78)
+# (1, 4 and 16 sequences, 0 to 1024 cached tokens; the lowest where nothing is cached).
+EXPAND_FROM, EXPAND_WORK = 64, 16384
 EXPAND_BYTES = 128 << 20  # ... in buffers of this size, or of what the other form takes for the step's rows
 ROPE_PAIRING = {"neighbours": 0, "halves": 1}
 
@@ -360,6 +367,7 @@ class LatentAttentionMixer:
         q_cols = H * qd if self.q_latent else int(self.w_in.shape[0])       # row stride of the queries: 16-byte rows
         if (self.mma_tokens and 16 <= self.rot_dim <= 64 and self.rot_dim % 16 == 0 and self.kv_rank % 8 == 0 and q_cols % 8 == 0 and
                 lib.pa_masked_attention_tc_tile_tokens(1, 1, self.dim, self.vdim, elem, 2)):
+            self.expand_from = max(EXPAND_FROM, -(-EXPAND_WORK // self.kv_rank))
             self.tc_tokens = tuple(lib.pa_masked_attention_tc_tile_tokens(1, 1, self.dim, self.vdim, elem, q) for q in (2, 1))
             self.w_uv = model._weight_raw(W[prefix + "uv"].reshape(H, self.vdim, self.kv_rank)).transpose(1, 2)     # the same, by output channel
 
@@ -494,7 +502,7 @@ class LatentAttentionMixer:
         q = self._queries(c, proj)
         kvr = self.kv_rank
         most = self._expand_rows(c) if self.tc_tokens else 0
-        expand = c.batch.expand_from(EXPAND_FROM, most) if most else 0
+        expand = c.batch.expand_from(self.expand_from, most) if most else 0
         without = (expand, most) if expand else None
         if expand and all(c.batch._expands(p, *without) for p in c.batch.portions):
             ov = c.empty(R, H * self.vdim)

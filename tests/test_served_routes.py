@@ -96,3 +96,22 @@ def test_a_refused_plan_is_not_asked_again():
         assert (x - y).abs().max() < 2e-2 * y.abs().max()
     eight, sixteen = (e.model.layers[0].mixer.core for e in engines)
     assert eight.tc_plans == [] and eight.mma_tokens and len(sixteen.tc_plans) == 2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kv_rank,tokens", [(64, 256), (128, 128), (256, 64)])
+def test_small_ranks_build_keys_for_long_portions_only(monkeypatch, kv_rank, tokens):
+    """A portion one token short of the line stays on the other form; both sides agree with the oracle."""
+    import llm_decoder as ld
+    from llm_decoder import hybrid
+    R = tiradra_ref
+    config = R.make_config([R.latent_layer(heads=2, dim=64, rot_dim=16, vdim=64, kv_rank=kv_rank)])
+    W = R.random_weights(config, 3)
+    eng, built, real = ld.Engine(ld.HybridDecoder(config, W, "bfloat16", max_tokens=1024, max_seqs=2)), [], hybrid.LatentAttentionMixer._attend_expanded
+    monkeypatch.setattr(hybrid.LatentAttentionMixer, "_attend_expanded", lambda self, *a: (built.append(1), real(self, *a))[1])
+    rnd = random.Random(kv_rank)
+    for r, n in ((0, tokens - 1), (1, tokens)):
+        toks = [rnd.randrange(config["vocab"]) for _ in range(n)]
+        x, y = eng.step([(r, toks, list(range(n)))]).double().cpu(), R.forward(config, W, toks)
+        assert ((x - y).pow(2).mean(-1).sqrt() / y.pow(2).mean(-1).sqrt()).median().item() < BF16_TOL
+        assert len(built) == r
