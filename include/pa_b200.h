@@ -890,8 +890,8 @@ int pa_streams_add_norm(const float* d_src, int src_streams, float* d_dst, int64
  *   q_tiles)), first row of the sequence in the key buffers, position.  d_out [rows][heads * vdim].
  * pa_latent_gather: d_items [n][3] = slot, tokens (at most `longest`), first output row: the cached rows of whole sequences
  *   from a latent pool into d_out [rows][row_bytes].
- * pa_attention_tc_errors: how many CTAs of these kernels gave up on a wait since the library was loaded (0 unless something is
- *   broken; their rows hold NaN).  Synchronises.  pa_moe_tc_errors: the same for the grouped expert products on tcgen05. */
+ * pa_attention_tc_errors: how often one of these kernels, pa_masked_decode or pa_latent_decode gave up on a wait since the library was
+ *   loaded (0 unless something is broken; the rows of that CTA or share hold NaN).  Synchronises.  pa_moe_tc_errors: the same for the grouped expert products on tcgen05. */
 int pa_masked_attention_tc_tile_tokens(int heads, int kv_heads, int dim, int vdim, int elem, int q_tiles);
 int pa_masked_attention_tc_units(int heads, int kv_heads, int q_tiles);
 int pa_latent_attention_expanded(const void* d_q, int64_t q_stride, int q_off, const void* d_k, int64_t k_stride,
@@ -918,6 +918,14 @@ int pa_masked_decode(const void* d_q, int64_t q_stride, int q_off, const void* d
                      const float* d_head_scale, const float* d_sink, const float* d_out_rot, const float* d_head_bias,
                      const void* d_gate, int64_t gate_stride, int gate_off, void* d_out, int workers, void* d_workspace,
                      size_t workspace_bytes, pa_stream_t stream);
+/* with a limit of the kernel's waits (0: nothing is requested, so that the first wait runs out and all rows are NaN) */
+int pa_masked_decode_polls(const void* d_q, int64_t q_stride, int q_off, const void* d_k_pool, const void* d_v_pool,
+                           const int32_t* d_table, int num_slots, int num_kv_heads, int num_tiles, int total_pages, int tile_size,
+                           const int32_t* d_q_tiles, int num_q_tiles, int heads, int dim, int vdim, float scale, float softcap,
+                           int mask_kind, int mask_size, int mask_keep, int bias_kind, const float* d_bias, int bias_len,
+                           const float* d_head_scale, const float* d_sink, const float* d_out_rot, const float* d_head_bias,
+                           const void* d_gate, int64_t gate_stride, int gate_off, void* d_out, int workers, void* d_workspace,
+                           size_t workspace_bytes, int polls, pa_stream_t stream);
 
 /* pa_latent_decode: pa_latent_attention_sink for tiles of ONE token, bfloat16 (latent_decode.cu): the 32-key units of all tokens are
  *   one list that `workers` CTAs share equally, and a second kernel joins the shares of a token.  d_q_tiles 16-byte aligned.
@@ -931,6 +939,11 @@ int pa_latent_decode(const void* d_q_lat, int64_t ql_row_stride, int64_t ql_head
                      int tile_size, const int32_t* d_q_tiles, int num_q_tiles, int heads, int kv_rank, int rot_dim, float scale,
                      const float* d_sink, void* d_out, int64_t o_row_stride, int64_t o_head_stride, int workers, void* d_workspace,
                      size_t workspace_bytes, pa_stream_t stream);
+int pa_latent_decode_polls(const void* d_q_lat, int64_t ql_row_stride, int64_t ql_head_stride, const void* d_q_rot, int64_t qr_row_stride,
+                           int64_t qr_head_stride, const void* d_pool, const int32_t* d_table, int num_slots, int num_tiles, int total_pages,
+                           int tile_size, const int32_t* d_q_tiles, int num_q_tiles, int heads, int kv_rank, int rot_dim, float scale,
+                           const float* d_sink, void* d_out, int64_t o_row_stride, int64_t o_head_stride, int workers, void* d_workspace,
+                           size_t workspace_bytes, int polls, pa_stream_t stream);
 
 /* ---- token-pair embedding, block passes that add, convolved + turned + normed projections, sinks on the latent ---------
  * pa_embedding_bigram: x[r] = embed[ids[r]] * scale + bigram[b(r)] as float (tables in the activation type), b(r) =

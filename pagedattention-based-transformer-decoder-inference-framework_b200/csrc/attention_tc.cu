@@ -211,8 +211,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                 }
             }
             if (failed()) {     // let the copies in flight land before the CTA's shared memory goes away
-                for (int b = 0; b < ST; ++b)
-                    for (uint32_t n = 0; n < 4096 && !mbar_try_wait(kv_full(b), b < s ? ph ^ 1u : ph); ++n) __nanosleep(256);
+                for (int b = 0; b < ST; ++b) tc_let_land(kv_full(b), b < s ? ph ^ 1u : ph);
             }
         }
     } else if (warp >= W_MMA) {
@@ -511,6 +510,9 @@ static void plan(int hpg, int q_tiles, int& tb, int& hg) {
 
 }  // namespace atc
 
+int masked_decode_errors(int* host_count);
+int latent_decode_errors(int* host_count);
+
 int masked_attention_tc_launch(const MaskAttnParams& p, int ntiles, int q_tiles, cudaStream_t st) {
     using namespace atc;
     const bool mod = p.softcap > 0.f || p.bias_kind != 0 || p.head_bias;
@@ -615,5 +617,10 @@ PA_API int pa_latent_attention_expanded(const void* d_q, int64_t q_stride, int q
 
 PA_API int pa_attention_tc_errors(int* host_count) {
     PA_CHECK_ARG(host_count);
-    return (int)cudaMemcpyFromSymbol(host_count, pa::atc::g_errors, sizeof(int));
+    int n = 0, masked = 0, latent = 0;
+    int rc = (int)cudaMemcpyFromSymbol(&n, pa::atc::g_errors, sizeof(int));
+    if (rc == PA_OK) rc = masked_decode_errors(&masked);
+    if (rc == PA_OK) rc = latent_decode_errors(&latent);
+    *host_count = n + masked + latent;
+    return rc;
 }

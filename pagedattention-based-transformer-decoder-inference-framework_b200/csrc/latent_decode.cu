@@ -37,6 +37,7 @@ struct Args {
     int num_slots, num_tiles, total_pages, tile_size;
     const int32_t* tiles;
     int ntiles, heads, hch, rows, rot_dim, workers, total_rows;
+    uint32_t polls;             // of a wait
     float scale;
     const float* sink;
     bf16_t* out;
@@ -44,6 +45,8 @@ struct Args {
     int* pre;                   // [ntiles + 1] units of one pair of every token, summed up
     float* part;                // [slots][rows][2 + kv_rank]: maximum (log2), sum, weighted sums
 };
+
+__device__ int g_errors;
 
 template <int KVR>
 __global__ void __launch_bounds__(kThreads, 1) latent_decode_kernel(const __grid_constant__ CUtensorMap tmP, const Args a) {
@@ -103,8 +106,8 @@ __global__ void __launch_bounds__(kThreads, 1) latent_decode_kernel(const __grid
                 nxt = row_of(f + 16);
             }
             const int r0 = __shfl_sync(0xffffffffu, cur, (o & 15) * 2), r1 = __shfl_sync(0xffffffffu, cur, (o & 15) * 2 + 1);
-            tc::tc_wait(empty(s), ph, fail_sm);
-            if (elect_one()) {
+            if (!__all_sync(0xffffffffu, tc::tc_wait(empty(s), ph, fail_sm))) break;
+            if (a.polls && elect_one()) {       // 0: a wait that is to run out
                 meta[s] = (r0 >= 0 ? 1u : 0u) | (r1 >= 0 ? 2u : 0u);
                 const uint32_t st = base + s * STAGE;
                 mbar_arrive_expect_tx(full(s), STAGE);
@@ -179,7 +182,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_decode_kernel(const __grid
             float* dst = a.part + (slot * a.rows + r) * ld;
             if (warp == 0 && (lane & 3) == 0) {
                 dst[0] = m[i];
-                dst[1] = s;
+                dst[1] = tc::tc_failed(fail_sm) ? __int_as_float(0x7fc00000) : s;       // a wait of some warp ran out before this pair's end
             }
 #pragma unroll
             for (int n = 0; n < NT; ++n)
@@ -202,7 +205,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_decode_kernel(const __grid
             open_pair();
         }
         const uint32_t st = base + stage * STAGE;
-        tc::tc_wait(full(stage), phase, fail_sm);
+        if (!tc::tc_wait(full(stage), phase, fail_sm, a.polls)) tc::tc_let_land(full(stage), phase);      // run out: on over whatever is there
         const uint32_t mapped = meta[stage];
         const int j0 = u * kUnit, valid = qpos + 1 - j0;
         // scores of this warp's keys over its columns
@@ -302,6 +305,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_decode_kernel(const __grid
         }
     }
     close_pair();
+    if (threadIdx.x == 0 && tc::tc_failed(fail_sm)) atomicAdd(&g_errors, 1);
 }
 
 // One warp per (pair, row); a lane has columns 2 lane + 64 i and the next.
@@ -397,12 +401,17 @@ PA_API size_t pa_latent_decode_workspace_bytes(int num_tokens, int heads, int kv
     return shares::pre_bytes(num_tokens) + ((size_t)num_tokens * hch + workers) * rows * (2 + kv_rank) * sizeof(float);
 }
 
-PA_API int pa_latent_decode(const void* d_q_lat, int64_t ql_row_stride, int64_t ql_head_stride, const void* d_q_rot,
+namespace pa {
+int latent_decode_errors(int* host_count) { return (int)cudaMemcpyFromSymbol(host_count, ldec::g_errors, sizeof(int)); }
+}  // namespace pa
+
+PA_API int pa_latent_decode_polls(const void* d_q_lat, int64_t ql_row_stride, int64_t ql_head_stride, const void* d_q_rot,
                             int64_t qr_row_stride, int64_t qr_head_stride, const void* d_pool, const int32_t* d_table, int num_slots,
                             int num_tiles, int total_pages, int tile_size, const int32_t* d_q_tiles, int num_q_tiles, int heads,
                             int kv_rank, int rot_dim, float scale, const float* d_sink, void* d_out, int64_t o_row_stride,
-                            int64_t o_head_stride, int workers, void* d_workspace, size_t workspace_bytes, pa_stream_t stream) {
+                            int64_t o_head_stride, int workers, void* d_workspace, size_t workspace_bytes, int polls, pa_stream_t stream) {
     using namespace pa::ldec;
+    PA_CHECK_ARG(polls >= 0);
     PA_CHECK_ARG(d_q_lat && (d_q_rot || rot_dim == 0) && d_pool && d_table && d_q_tiles && d_out && num_q_tiles >= 0);
     PA_CHECK_ARG(num_slots > 0 && num_tiles > 0 && total_pages > 0 && tile_size > 0 && heads > 0 && kv_rank > 0 && rot_dim >= 0 && workers > 0);
     if (num_q_tiles == 0) return PA_OK;
@@ -421,6 +430,7 @@ PA_API int pa_latent_decode(const void* d_q_lat, int64_t ql_row_stride, int64_t 
     a.table = d_table; a.num_slots = num_slots; a.num_tiles = num_tiles; a.total_pages = total_pages; a.tile_size = tile_size;
     a.tiles = d_q_tiles; a.ntiles = num_q_tiles; a.heads = heads; a.hch = (heads + kRows - 1) / kRows;
     a.rows = heads < kRows ? heads : kRows; a.rot_dim = rot_dim; a.workers = workers; a.total_rows = (int)rows; a.scale = scale;
+    a.polls = (uint32_t)polls;
     a.sink = d_sink; a.out = static_cast<bf16_t*>(d_out); a.o_rs = o_row_stride; a.o_hs = o_head_stride;
     a.pre = static_cast<int*>(d_workspace);
     a.part = reinterpret_cast<float*>(static_cast<char*>(d_workspace) + shares::pre_bytes(num_q_tiles));
@@ -431,4 +441,14 @@ PA_API int pa_latent_decode(const void* d_q_lat, int64_t ql_row_stride, int64_t 
     if (kv_rank == 256) return launch<256>(m, a, st);
     if (kv_rank == 384) return launch<384>(m, a, st);
     return launch<512>(m, a, st);
+}
+
+PA_API int pa_latent_decode(const void* d_q_lat, int64_t ql_row_stride, int64_t ql_head_stride, const void* d_q_rot,
+                            int64_t qr_row_stride, int64_t qr_head_stride, const void* d_pool, const int32_t* d_table, int num_slots,
+                            int num_tiles, int total_pages, int tile_size, const int32_t* d_q_tiles, int num_q_tiles, int heads,
+                            int kv_rank, int rot_dim, float scale, const float* d_sink, void* d_out, int64_t o_row_stride,
+                            int64_t o_head_stride, int workers, void* d_workspace, size_t workspace_bytes, pa_stream_t stream) {
+    return pa_latent_decode_polls(d_q_lat, ql_row_stride, ql_head_stride, d_q_rot, qr_row_stride, qr_head_stride, d_pool, d_table, num_slots,
+                                  num_tiles, total_pages, tile_size, d_q_tiles, num_q_tiles, heads, kv_rank, rot_dim, scale, d_sink, d_out,
+                                  o_row_stride, o_head_stride, workers, d_workspace, workspace_bytes, (int)pa::tc::kPolls, stream);
 }

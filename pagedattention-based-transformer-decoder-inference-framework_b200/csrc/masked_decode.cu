@@ -31,9 +31,12 @@ struct Args {
     MaskAttnParams p;
     int ntiles, hch, workers, rows;     // hch: chunks of 16 query heads per kv head; rows: query rows of a pair that are real
     int total_rows;
+    uint32_t polls;                     // of a wait
     int* pre;                           // [ntiles + 1] units of one pair of every token, summed up
     float* part;                        // [slots][rows][2 + vdim]: maximum (log2), sum, weighted sums
 };
+
+__device__ int g_errors;
 
 __device__ __forceinline__ int tile_units(const MaskAttnParams& p, int pos) {
     return ma_steps(p, ma_first_key(p, pos), pos + 1, kUnit).count;
@@ -94,7 +97,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) masked_decode_kernel(const __g
         }
         const int row = __shfl_sync(0xffffffffu, rows_cur, o & 31);
         mapped = row >= 0 ? mapped | 1u << is_stage : mapped & ~(1u << is_stage);
-        if (elect_one()) {
+        if (a.polls && elect_one()) {   // 0: a wait that is to run out
             const uint32_t st = ring + is_stage * STAGE, bar = bar0 + is_stage * 8;
             const int r = row >= 0 ? row : a.total_rows;        // no page: a box of zeros
             mbar_arrive_expect_tx(bar, STAGE);
@@ -170,7 +173,8 @@ __global__ void __launch_bounds__(kWarps * 32, 1) masked_decode_kernel(const __g
     open_pair();
     int stage = 0;
     uint32_t phase = 0;
-    for (int64_t f = f_lo; f < f_hi; ++f) {
+    int64_t f = f_lo;
+    for (; f < f_hi; ++f) {
         if (u == per) {
             close_pair();
             u = 0;
@@ -182,7 +186,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) masked_decode_kernel(const __g
             open_pair();
         }
         const uint32_t ks_sm = ring + stage * STAGE, vs_sm = ks_sm + KB * 2048;
-        tc::tc_wait(bar0 + stage * 8, phase, fail_sm);
+        if (!__all_sync(0xffffffffu, tc::tc_wait(bar0 + stage * 8, phase, fail_sm, a.polls))) break;
         const bool has = mapped >> stage & 1u;
         const int j0 = steps.step(u) * kUnit, valid = qpos + 1 - j0;
         if (valid < kUnit) {            // value rows past the query's own position may hold anything (0 x NaN = NaN)
@@ -313,6 +317,24 @@ __global__ void __launch_bounds__(kWarps * 32, 1) masked_decode_kernel(const __g
             phase ^= 1u;
         }
     }
+    if (f < f_hi) {                     // a wait ran out: the copies that were requested land, and the pairs from here on get NaN
+        for (int64_t i = f; i < f_is; ++i) {
+            const int at = stage + (int)(i - f);
+            tc::tc_let_land(bar0 + at % kStages * 8, at < kStages ? phase : phase ^ 1u);
+        }
+        if (lane == 0) atomicAdd(&g_errors, 1);
+        for (f += per - u; f < f_hi; f += per) {
+            l[0] = l[1] = __int_as_float(0x7fc00000);
+            close_pair();
+            if (++pr == pairs) {
+                pr = 0;
+                ++t;
+                per = pre[t + 1] - pre[t];
+            }
+            open_pair();
+        }
+        l[0] = l[1] = __int_as_float(0x7fc00000);
+    }
     close_pair();
 }
 
@@ -429,14 +451,19 @@ PA_API size_t pa_masked_decode_workspace_bytes(int num_tokens, int heads, int kv
     return shares::pre_bytes(num_tokens) + ((size_t)num_tokens * kv_heads * hch + workers) * rows * (2 + vdim) * sizeof(float);
 }
 
-PA_API int pa_masked_decode(const void* d_q, int64_t q_stride, int q_off, const void* d_k_pool, const void* d_v_pool,
+namespace pa {
+int masked_decode_errors(int* host_count) { return (int)cudaMemcpyFromSymbol(host_count, mdec::g_errors, sizeof(int)); }
+}  // namespace pa
+
+PA_API int pa_masked_decode_polls(const void* d_q, int64_t q_stride, int q_off, const void* d_k_pool, const void* d_v_pool,
                             const int32_t* d_table, int num_slots, int num_kv_heads, int num_tiles, int total_pages, int tile_size,
                             const int32_t* d_q_tiles, int num_q_tiles, int heads, int dim, int vdim, float scale, float softcap,
                             int mask_kind, int mask_size, int mask_keep, int bias_kind, const float* d_bias, int bias_len,
                             const float* d_head_scale, const float* d_sink, const float* d_out_rot, const float* d_head_bias,
                             const void* d_gate, int64_t gate_stride, int gate_off, void* d_out, int workers, void* d_workspace,
-                            size_t workspace_bytes, pa_stream_t stream) {
+                            size_t workspace_bytes, int polls, pa_stream_t stream) {
     using namespace pa::mdec;
+    PA_CHECK_ARG(polls >= 0);
     PA_CHECK_ARG(mask_keep >= 0 && (mask_keep == 0 || mask_kind == 1) && (!d_out_rot || vdim % 2 == 0));
     PA_CHECK_ARG(d_q && d_k_pool && d_v_pool && d_table && d_q_tiles && d_out && num_q_tiles >= 0);
     PA_CHECK_ARG(num_slots > 0 && num_kv_heads > 0 && num_tiles > 0 && total_pages > 0 && tile_size > 0);
@@ -468,6 +495,7 @@ PA_API int pa_masked_decode(const void* d_q, int64_t q_stride, int q_off, const 
     a.rows = hpg < kRows ? hpg : kRows;
     a.workers = workers;
     a.total_rows = (int)rows;
+    a.polls = (uint32_t)polls;
     a.pre = static_cast<int*>(d_workspace);
     a.part = reinterpret_cast<float*>(static_cast<char*>(d_workspace) + shares::pre_bytes(num_q_tiles));
     CUtensorMap k, v;
@@ -481,4 +509,17 @@ PA_API int pa_masked_decode(const void* d_q, int64_t q_stride, int q_off, const 
     PA_MDEC(64, 64); PA_MDEC(64, 128); PA_MDEC(128, 64); PA_MDEC(128, 128);
 #undef PA_MDEC
     return PA_ERR_UNSUPPORTED;
+}
+
+PA_API int pa_masked_decode(const void* d_q, int64_t q_stride, int q_off, const void* d_k_pool, const void* d_v_pool,
+                            const int32_t* d_table, int num_slots, int num_kv_heads, int num_tiles, int total_pages, int tile_size,
+                            const int32_t* d_q_tiles, int num_q_tiles, int heads, int dim, int vdim, float scale, float softcap,
+                            int mask_kind, int mask_size, int mask_keep, int bias_kind, const float* d_bias, int bias_len,
+                            const float* d_head_scale, const float* d_sink, const float* d_out_rot, const float* d_head_bias,
+                            const void* d_gate, int64_t gate_stride, int gate_off, void* d_out, int workers, void* d_workspace,
+                            size_t workspace_bytes, pa_stream_t stream) {
+    return pa_masked_decode_polls(d_q, q_stride, q_off, d_k_pool, d_v_pool, d_table, num_slots, num_kv_heads, num_tiles, total_pages, tile_size,
+                                  d_q_tiles, num_q_tiles, heads, dim, vdim, scale, softcap, mask_kind, mask_size, mask_keep, bias_kind, d_bias,
+                                  bias_len, d_head_scale, d_sink, d_out_rot, d_head_bias, d_gate, gate_stride, gate_off, d_out, workers,
+                                  d_workspace, workspace_bytes, (int)pa::tc::kPolls, stream);
 }

@@ -84,14 +84,21 @@ __device__ __forceinline__ bool tc_failed(uint32_t fail_sm) {
     asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(f) : "r"(fail_sm) : "memory");
     return f != 0;
 }
-__device__ __forceinline__ void tc_wait(uint32_t bar, uint32_t parity, uint32_t fail_sm) {
+// true: the phase is complete.  polls: how often it may be asked for in vain before the wait has run out.
+constexpr uint32_t kPolls = 1u << 25;
+__device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, uint32_t fail_sm, uint32_t polls = kPolls) {
     uint32_t n = 0;
     while (!mbar_try_wait(bar, parity)) {
-        if ((++n & 255u) == 0 && (n > (1u << 25) || tc_failed(fail_sm))) {
+        if (++n > polls || ((n & 255u) == 0 && tc_failed(fail_sm))) {
             asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(fail_sm), "r"(1u) : "memory");
-            return;
+            return false;
         }
     }
+    return true;
+}
+// copies that were requested land in shared memory, so it has to outlive them, also where a wait ran out: up to a second here
+__device__ __forceinline__ void tc_let_land(uint32_t bar, uint32_t parity) {
+    for (uint32_t n = 0; n < 4096 && !mbar_try_wait(bar, parity); ++n) __nanosleep(256);
 }
 
 // [rows][cols] bfloat16, rows `stride` elements apart; box = box_rows x 64 columns (128 bytes), SWIZZLE_128B

@@ -126,6 +126,10 @@ _SIGS = {
     "pa_masked_decode_workspace_bytes": ([_i32, _i32, _i32, _i32, _i32], _sz),
     "pa_masked_decode": ([_vp, _i64, _i32, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _vp, _i32, _i32, _i32, _i32, _f32, _f32, _i32,
                           _i32, _i32, _i32, _vp, _i32, _vp, _vp, _vp, _vp, _vp, _i64, _i32, _vp, _i32, _vp, _sz, _vp], _i32),
+    "pa_masked_decode_polls": ([_vp, _i64, _i32, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _vp, _i32, _i32, _i32, _i32, _f32, _f32, _i32,
+                                _i32, _i32, _i32, _vp, _i32, _vp, _vp, _vp, _vp, _vp, _i64, _i32, _vp, _i32, _vp, _sz, _i32, _vp], _i32),
+    "pa_latent_decode_polls": ([_vp, _i64, _i64, _vp, _i64, _i64, _vp, _vp, _i32, _i32, _i32, _i32, _vp, _i32, _i32, _i32, _i32, _f32, _vp,
+                                _vp, _i64, _i64, _i32, _vp, _sz, _i32, _vp], _i32),
     "pa_latent_decode_workers": ([_i32, _i32, _i64], _i32),
     "pa_latent_decode_workspace_bytes": ([_i32, _i32, _i32, _i32], _sz),
     "pa_latent_decode": ([_vp, _i64, _i64, _vp, _i64, _i64, _vp, _vp, _i32, _i32, _i32, _i32, _vp, _i32, _i32, _i32, _i32, _f32, _vp, _vp,

@@ -1,0 +1,83 @@
+"""Kernels whose waits run out (the limit of a wait is an argument; with 0 nothing is requested, so that the first wait runs out): the call
+returns, its rows are NaN and never plausible numbers, the count of waits that ran out goes up, and the next call is served.  In processes
+of their own, since other tests ask for a count of zero."""
+import os
+import subprocess
+import sys
+
+import pytest
+import torch
+
+BF = torch.bfloat16
+
+
+def _count(fn):
+    import ctypes
+    n = ctypes.c_int(-1)
+    assert fn(ctypes.byref(n)) == 0
+    return n.value
+
+
+def masked_decode():
+    from llm_decoder import _cabi
+    from llm_decoder.seq_state import SequenceStateCache
+    lib, dev, H, G, D, pos = _cabi.lib(), torch.device("cuda"), 8, 2, 128, [0, 30, 700, 5, 2000]
+    for copies in (1, 30):                      # float and bfloat16 weights
+        tokens = pos * copies
+        n = len(tokens)
+        st = SequenceStateCache(n, sum(tokens) + 32 * n, 16, dev)
+        kv = st.add_kv_layer(G, D, D, "bf16")
+        slots = [st.alloc() for _ in tokens]
+        b = st.make_batch([(s, [0] * (c + 1)) for s, c in zip(slots, tokens)])
+        kv.append_rows(torch.randn(b.rows, 2 * G * D, device=dev).to(BF), 0, G * D, b.row_slot, b.row_pos)
+        tiles = torch.tensor([[i, 1, s, c] for i, (s, c) in enumerate(zip(slots, tokens))], dtype=torch.int32, device=dev)
+        q, pt = torch.randn(n, H * D, device=dev).to(BF), kv.page_table_
+        workers = lib.pa_masked_decode_workers(n, H, G, 2001)
+        ws = torch.empty(lib.pa_masked_decode_workspace_bytes(n, H, G, D, workers), dtype=torch.uint8, device=dev)
+        for polls in (0, 1 << 25):
+            out, before = torch.zeros(n, H * D, dtype=BF, device=dev), _count(lib.pa_attention_tc_errors)
+            assert lib.pa_masked_decode_polls(
+                q.data_ptr(), H * D, 0, kv.key_buffer_.data_ptr(), kv.value_buffer_.data_ptr(), pt.device_data().data_ptr(), pt.num_beams_,
+                pt.num_heads_, pt.num_tiles_, kv.total_pages_, 16, tiles.data_ptr(), n, H, D, D, 0.1, 0.0, 0, 0, 0, 0, None, 0, None, None, None,
+                None, None, 0, 0, out.data_ptr(), workers, ws.data_ptr(), ws.numel(), polls, _cabi.stream()) == 0
+            ran_out = _count(lib.pa_attention_tc_errors) - before
+            assert torch.isnan(out.float()).all() and ran_out > 0 if polls == 0 else torch.isfinite(out.float()).all() and ran_out == 0
+
+
+def latent_decode():
+    from llm_decoder import _cabi
+    from llm_decoder.seq_state import SequenceStateCache
+    lib, dev, H, kvr, rot, pos = _cabi.lib(), torch.device("cuda"), 20, 256, 32, [0, 30, 300, 5, 90, 40]
+    n, kd = len(pos), kvr + rot
+    st = SequenceStateCache(n, sum(pos) + 32 * n, 16, dev)
+    kv = st.add_kv_layer(1, kd, 0, "bf16")
+    slots = [st.alloc() for _ in pos]
+    st.make_batch([(s, [0] * (c + 1)) for s, c in zip(slots, pos)])
+    kv.key_buffer_.normal_()
+    tiles = torch.tensor([[i, 1, s, c] for i, (s, c) in enumerate(zip(slots, pos))], dtype=torch.int32, device=dev)
+    ql, qr, pt = torch.randn(H, n, kvr, device=dev).to(BF), torch.randn(n, H * rot, device=dev).to(BF), kv.page_table_
+    for workers in (lib.pa_latent_decode_workers(n, H, 301), 7):
+        ws = torch.empty(lib.pa_latent_decode_workspace_bytes(n, H, kvr, workers), dtype=torch.uint8, device=dev)
+        for polls in (0, 1 << 25):
+            out, before = torch.zeros(H, n, kvr, dtype=BF, device=dev), _count(lib.pa_attention_tc_errors)
+            assert lib.pa_latent_decode_polls(
+                ql.data_ptr(), kvr, n * kvr, qr.data_ptr(), H * rot, rot, kv.key_buffer_.data_ptr(), pt.device_data().data_ptr(), pt.num_beams_,
+                pt.num_tiles_, kv.total_pages_, 16, tiles.data_ptr(), n, H, kvr, rot, 0.1, None, out.data_ptr(), kvr, n * kvr, workers, ws.data_ptr(),
+                ws.numel(), polls, _cabi.stream()) == 0
+            ran_out = _count(lib.pa_attention_tc_errors) - before
+            assert torch.isnan(out.float()).all() and ran_out > 0 if polls == 0 else torch.isfinite(out.float()).all() and ran_out == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", ["masked_decode", "latent_decode"])
+def test_rows_of_waits_that_run_out(case):
+    r = subprocess.run([sys.executable, os.path.abspath(__file__), case], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip().endswith("done"), r.stdout + r.stderr
+
+
+if __name__ == "__main__":
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    sys.path.insert(0, os.path.join(root, "pagedattention-based-transformer-decoder-inference-framework_b200"))
+    globals()[sys.argv[1]]()
+    torch.cuda.synchronize()
+    print("done")
