@@ -902,6 +902,11 @@ int pa_latent_gather(const void* d_pool, const int32_t* d_table, int num_slots, 
                      int row_bytes, const int32_t* d_items, int num_items, int longest, void* d_out, pa_stream_t stream);
 int pa_attention_tc_errors(int* host_count);
 int pa_moe_tc_errors(int* host_count);
+/* the grouped products on tcgen05 alone (mode 0: gate and up, 1: down, 2: up; operands as in pa_moe_gate_up_act, pa_moe_down and pa_moe_up)
+ * with a limit of the kernel's waits (0: nothing is requested, so that the first wait runs out and all rows are NaN).  PA_ERR_UNSUPPORTED: see there. */
+int pa_moe_grouped_polls(int mode, const void* d_a, int64_t lda, const void* d_w, int K, int n_out, int experts, const int32_t* d_order,
+                         const float* d_a_scale, int top, const int32_t* d_meta, int pairs, int act, void* d_out, int polls,
+                         pa_stream_t stream);
 
 /* ---- decoded tokens with the keys cut into equal shares (masked_decode.cu) ----------------------------------------------
  * pa_masked_decode: pa_masked_attention_gated for tiles of ONE token, bfloat16 softmax attention: the 16-key units of all

@@ -621,7 +621,8 @@ __global__ void __launch_bounds__(kSkWarps * 32) grouped_skinny_kernel(const bf1
 
 // moe_tc.cu: the tcgen05 form of the grouped products (PA_ERR_UNSUPPORTED: operands that stay on the kernels here)
 int grouped_tc_launch(int mode, const void* A, int64_t lda, const void* W, int K, int n_out, int experts, const int32_t* order,
-                      const float* a_scale, int top, const int32_t* offsets, int pairs, int act, void* out, cudaStream_t st);
+                      const float* a_scale, int top, const int32_t* offsets, int pairs, int act, void* out, cudaStream_t st,
+                      int polls = 1 << 25);
 
 static bool mma_ok(const void* A, int64_t lda, const void* W, int K) {
     return K % 8 == 0 && lda % 8 == 0 && (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0;

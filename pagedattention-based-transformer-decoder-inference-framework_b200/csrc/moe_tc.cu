@@ -16,7 +16,8 @@
 // 96 B per cycle and leave it at the same rate.  Measured, 16384 pairs of 8 experts, width 2048, ff 1024: gate / up 178 us = 770
 // TFLOP/s, down 67 us = 1030 TFLOP/s (mma.sync kernels of moe_ops.cu: 530 and 294 us).
 //
-// Every wait is bounded: on a protocol error the CTA raises a flag (pa_moe_tc_errors), lets its copies land and frees its TMEM.
+// Every wait is bounded: on a protocol error the CTA raises a flag (pa_moe_tc_errors), lets its copies land, frees its TMEM and
+// writes NaN into the rows of its tiles from there on.
 #include "seq_common.cuh"
 #include "tcgen05_utils.cuh"
 
@@ -38,6 +39,7 @@ struct Args {
     const int32_t* offsets;     // [experts + 1]
     bf16_t* out;                // MODE 0, 2: [pairs][n_out], sorted order
     float* out_f32;             // MODE 1: [pairs][n_out], (row, choice) order
+    uint32_t polls;             // of a wait
 };
 
 __device__ int g_errors;
@@ -125,12 +127,11 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         if (elect_one()) {
             int s = 0;
             uint32_t ph = 1;
-            while (w.next() && !tc_failed(fail_sm)) {
+            while (a.polls && w.next() && !tc_failed(fail_sm)) {       // 0: waits that are to run out, nothing is requested
                 const int n0 = w.strip * (MODE == 0 ? BN / 2 : BN);
                 const int r1 = w.e * w_rows + n0, r2 = r1 + (MODE == 0 ? a.n_out : BN / 2);
                 for (int kt = 0; kt < nk; ++kt) {
-                    tc_wait(empty(s), ph, fail_sm);
-                    if (tc_failed(fail_sm)) break;
+                    if (!tc_wait(empty(s), ph, fail_sm, a.polls)) break;
                     const uint32_t st = base + s * STAGE;
                     mbar_arrive_expect_tx(full(s), MODE == 1 ? STAGE : B_BYTES);
                     tma_load_2d(st + A_BYTES, &tmW, kt * BK, r1, full(s));
@@ -148,12 +149,14 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         constexpr uint32_t kIdesc = idesc_f16(BM, BN, 0, 0, 1);
         int s = 0, j = 0;
         uint32_t ph = 0;
-        for (; w.next(); ++j) {
+        bool ok = true;         // false: a wait ran out, and no further product is issued
+        for (; ok && w.next(); ++j) {
             const int b = j & 1;
-            tc_wait(tempty(b), ((uint32_t)(j >> 1) & 1u) ^ 1u, fail_sm);
+            ok = __all_sync(0xffffffffu, tc_wait(tempty(b), ((uint32_t)(j >> 1) & 1u) ^ 1u, fail_sm, a.polls));
             tc_fence_after();
-            for (int kt = 0; kt < nk; ++kt) {
-                tc_wait(full(s), ph, fail_sm);
+            for (int kt = 0; ok && kt < nk; ++kt) {
+                ok = __all_sync(0xffffffffu, tc_wait(full(s), ph, fail_sm, a.polls));
+                if (!ok) break;
                 tc_fence_after();
                 if (elect_one()) {
                     const uint32_t st = base + s * STAGE;
@@ -186,14 +189,19 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 pair = __ldg(a.order + w.m0 + row);
                 if (MODE != 1) sc = __ldg(a.a_scale + pair);
             }
-            tc_wait(tfull(b), (uint32_t)(j >> 1) & 1u, fail_sm);
+            tc_wait(tfull(b), (uint32_t)(j >> 1) & 1u, fail_sm, a.polls);
             tc_fence_after();
+            const bool lost = tc_failed(fail_sm);       // some wait of the CTA ran out: NaN from here on
             const uint32_t acc = tmem_base + ((uint32_t)(qtr * 32) << 16) + b * BN;
             for (int c0 = 0; c0 < cols; c0 += ECOLS) {
                 if (MODE == 1) {
                     uint32_t v[32];
                     tmem_ld32(acc + c0, v);
                     tmem_wait_ld();
+                    if (lost) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) v[i] = 0x7fc00000u;
+                    }
 #pragma unroll
                     for (int p = 0; p < 8; ++p)
                         asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(ebuf + lane * 128 + ((p ^ (lane & 7)) << 4)),
@@ -213,7 +221,8 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                                 f[e] = act_f32(round_bf16(__uint_as_float(v[8 * p + e]) * sc), a.act);
                                 if (MODE == 0) f[e] *= round_bf16(__uint_as_float(u[8 * p + e]) * sc);
                             }
-                            const uint4 o = bf16x8_pack(f);
+                            uint4 o = bf16x8_pack(f);
+                            if (lost) o = make_uint4(0x7fc07fc0u, 0x7fc07fc0u, 0x7fc07fc0u, 0x7fc07fc0u);
                             asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(ebuf + lane * 128 + (((hf * 4 + p) ^ (lane & 7)) << 4)),
                                          "r"(o.x), "r"(o.y), "r"(o.z), "r"(o.w) : "memory");
                         }
@@ -254,7 +263,7 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 src[i] = r < w.rows ? a.A + (int64_t)(__ldg(a.order + w.m0 + r) / a.top) * a.lda + piece * 8 : nullptr;
             }
             for (int kt = 0; kt < nk; ++kt) {
-                tc_wait(empty(s), ph, fail_sm);
+                tc_wait(empty(s), ph, fail_sm, a.polls);
                 const uint32_t st = base + s * STAGE;
                 const bool in_k = kt * BK + piece * 8 < a.K;
 #pragma unroll
@@ -311,7 +320,7 @@ static int launch(const CUtensorMap& tmA, const CUtensorMap& tmW, const Args& a,
 // mode 0: gate / up pairs, 1: down (rows scattered to (row, choice) order as float), 2: up.  PA_ERR_UNSUPPORTED: the caller's other
 // kernels serve these operands.
 int grouped_tc_launch(int mode, const void* A, int64_t lda, const void* W, int K, int n_out, int experts, const int32_t* order,
-                      const float* a_scale, int top, const int32_t* offsets, int pairs, int act, void* out, cudaStream_t st) {
+                      const float* a_scale, int top, const int32_t* offsets, int pairs, int act, void* out, cudaStream_t st, int polls) {
     using namespace mtc;
     const int64_t w_rows = (int64_t)experts * n_out * (mode == 0 ? 2 : 1);
     if (K % 8 || n_out % 8 || experts > kMostExperts || w_rows >= 0x7fffff00ll || (uintptr_t)out % 16) return PA_ERR_UNSUPPORTED;
@@ -322,13 +331,22 @@ int grouped_tc_launch(int mode, const void* A, int64_t lda, const void* W, int K
     if (mode == 1 && !make_bf16_map(&tmA, A, pairs, K, lda, BM)) return PA_ERR_UNSUPPORTED;
     const int strip = mode == 0 ? BN / 2 : BN;
     Args a{static_cast<const bf16_t*>(A), lda, K, n_out, experts, top, act, (n_out + strip - 1) / strip, order, a_scale, offsets,
-           static_cast<bf16_t*>(out), static_cast<float*>(out)};
+           static_cast<bf16_t*>(out), static_cast<float*>(out), (uint32_t)polls};
     return mode == 0 ? launch<0>(tmA, tmW, a, pairs, st) : mode == 1 ? launch<1>(tmA, tmW, a, pairs, st) : launch<2>(tmA, tmW, a, pairs, st);
 }
 
 }  // namespace pa
 
 using namespace pa;
+
+PA_API int pa_moe_grouped_polls(int mode, const void* d_a, int64_t lda, const void* d_w, int K, int n_out, int experts, const int32_t* d_order,
+                                const float* d_a_scale, int top, const int32_t* d_meta, int pairs, int act, void* d_out, int polls,
+                                pa_stream_t stream) {
+    PA_CHECK_ARG(mode >= 0 && mode <= 2 && d_a && d_w && d_order && d_meta && d_out && K > 0 && n_out > 0 && experts > 0 && top > 0 && pairs >= 0 &&
+                 act >= 0 && act <= 2 && polls >= 0);
+    if (pairs == 0) return PA_OK;
+    return grouped_tc_launch(mode, d_a, lda, d_w, K, n_out, experts, d_order, d_a_scale, top, d_meta, pairs, act, d_out, as_stream(stream), polls);
+}
 
 PA_API int pa_moe_tc_errors(int* host_count) {
     PA_CHECK_ARG(host_count);

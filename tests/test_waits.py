@@ -68,8 +68,28 @@ def latent_decode():
             assert torch.isnan(out.float()).all() and ran_out > 0 if polls == 0 else torch.isfinite(out.float()).all() and ran_out == 0
 
 
+def grouped():
+    from llm_decoder import _cabi
+    lib, dev, rows, experts, top, width, ff = _cabi.lib(), torch.device("cuda"), 700, 3, 2, 192, 264
+    g, pairs = torch.Generator().manual_seed(1), 1400
+    ids = torch.randint(0, experts, (pairs,), generator=g).to(torch.int32).to(dev)
+    order, meta = torch.empty(pairs, dtype=torch.int32, device=dev), torch.empty(lib.pa_moe_meta_ints(pairs, experts), dtype=torch.int32, device=dev)
+    assert lib.pa_moe_sort(ids.data_ptr(), pairs, experts, order.data_ptr(), meta.data_ptr(), _cabi.stream()) == 0
+    h, mid = torch.randn(rows, width, device=dev).to(BF), torch.randn(pairs, ff, device=dev).to(BF)
+    wu, wd = torch.randn(experts, 2 * ff, width, device=dev).to(BF), torch.randn(experts, width, ff, device=dev).to(BF)
+    for mode, a, w, K, n_out, t in ((0, h, wu, width, ff, top), (1, mid, wd, ff, width, 1), (2, h, wu[:, :ff].contiguous(), width, ff, top)):
+        for act in (0, 1) if mode != 1 else (0,):
+            for polls in (0, 1 << 25):
+                out = torch.zeros(pairs, n_out, device=dev, dtype=torch.float32 if mode == 1 else BF)
+                before = _count(lib.pa_moe_tc_errors)
+                assert lib.pa_moe_grouped_polls(mode, a.data_ptr(), K, w.data_ptr(), K, n_out, experts, order.data_ptr(), None, t, meta.data_ptr(),
+                                                pairs, act, out.data_ptr(), polls, _cabi.stream()) == 0
+                ran_out = _count(lib.pa_moe_tc_errors) - before
+                assert torch.isnan(out.float()).all() and ran_out > 0 if polls == 0 else torch.isfinite(out.float()).all() and ran_out == 0
+
+
 @pytest.mark.gpu
-@pytest.mark.parametrize("case", ["masked_decode", "latent_decode"])
+@pytest.mark.parametrize("case", ["masked_decode", "latent_decode", "grouped"])
 def test_rows_of_waits_that_run_out(case):
     r = subprocess.run([sys.executable, os.path.abspath(__file__), case], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.strip().endswith("done"), r.stdout + r.stderr
