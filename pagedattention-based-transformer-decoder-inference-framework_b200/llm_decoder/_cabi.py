@@ -285,6 +285,16 @@ def stream():
     return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
+def lost_waits():
+    """How many waits of this process's kernels ran out since the library was loaded (0 unless something is broken: the rows they were for
+    hold NaN).  Synchronises."""
+    total, n = 0, C.c_int(0)
+    for fn in (lib().pa_attention_tc_errors, lib().pa_moe_tc_errors):
+        check(fn(C.byref(n)), "lost waits")
+        total += n.value
+    return total
+
+
 class _Here:
     """The guard of a device that is current already."""
 

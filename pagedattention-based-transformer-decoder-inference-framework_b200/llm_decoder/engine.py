@@ -257,6 +257,7 @@ class Scheduler:
         self.running = []
         self.done = {}
         self._next = 0
+        self._lost = self._lost_waits()
         self._gen = None
         if self.top_k > 0 or self.top_p < 1.0:
             self._gen = torch.Generator(device=engine.model.device)
@@ -269,6 +270,13 @@ class Scheduler:
         self._next += 1
         self.waiting.append(_Request(rid, prompt, max_new_tokens))
         return rid
+
+    def _lost_waits(self):
+        dev = self.engine.model.device
+        if dev.type != "cuda":
+            return 0
+        with _cabi.on_device(dev):
+            return _cabi.lost_waits()
 
     def _tiles(self, n):
         ts = self.engine.states.tile_size
@@ -327,9 +335,12 @@ class Scheduler:
         logits = self.engine.step(entries)
         if owners:
             ids = self._sample(logits).cpu().tolist()
-            for r, t in zip(owners, ids):
+            ended = [len(r.out) + 1 >= r.max_new or int(t) == self.eos for r, t in zip(owners, ids)]
+            if any(ended) and self._lost_waits() != self._lost:     # asked before tokens are handed out: the GPU is idle here anyway
+                raise RuntimeError("a kernel gave up on a wait: logits of this run are not valid")
+            for r, t, end in zip(owners, ids, ended):
                 r.out.append(int(t))
-                if len(r.out) >= r.max_new or int(t) == self.eos:
+                if end:
                     self.engine.finish(r.rid)
                     self.done[r.rid] = r.prompt + r.out
                     self.running.remove(r)

@@ -348,3 +348,28 @@ def test_a_model_put_in_the_place_of_another(monkeypatch):
     assert e.step([(0, [1], [0])]) == "first"
     e.model = Model("second", states)
     assert e.step([(0, [1], [0])]) == "second"
+
+
+def test_a_run_with_lost_waits_hands_out_no_tokens(monkeypatch):
+    """The scheduler asks for waits that ran out before it hands out a request's tokens."""
+    import contextlib
+    import llm_decoder as ld
+    from llm_decoder import engine
+    lost = [5]
+    monkeypatch.setattr(engine._cabi, "lost_waits", lambda: lost[0])
+    monkeypatch.setattr(engine._cabi, "on_device", lambda _d: contextlib.nullcontext())
+    monkeypatch.setattr(ld.Scheduler, "_sample", lambda _self, logits: torch.zeros(logits.shape[0], dtype=torch.int32))
+    e = _Held()
+    e.model, e.states = _Held(), _Held()
+    e.model.device, e.states.max_seqs, e.states.tile_size = torch.device("cuda"), 4, 16
+    e.has, e.states.free_tokens = lambda _r: False, lambda: 1 << 20
+    e.step = lambda entries: torch.zeros(sum(len(w) for _r, _t, w in entries), 7)
+    s = ld.Scheduler(e)
+    rid = s.add_request([1, 2, 3], 4)
+    assert s.run()[rid] == [1, 2, 3, 0, 0, 0, 0]        # lost before this scheduler was made
+    rid = s.add_request([1, 2], 3)
+    s.step()
+    lost[0] += 1
+    with pytest.raises(RuntimeError):
+        s.run()
+    assert rid not in s.done
