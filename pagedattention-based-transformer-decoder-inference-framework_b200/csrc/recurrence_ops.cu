@@ -317,14 +317,13 @@ __global__ void __launch_bounds__(kDsMaxThreads) decay_scan_kernel(const DecaySc
 // (rotated q and k, weighted k, the scores with their decays, the incoming state) is the sum of three bfloat16 numbers, 24 bits
 // of it, and a product of two such factors keeps the six terms that reach 2^-24; the value rows are bfloat16 as they come.  One CTA
 // of four warps per (chunk, head); a warp has 16 rows of the result.
-// What bounds it: issue of ldmatrix and mma.sync.  4 x 2048 tokens, 16 heads of 64 x 128: fold 60 us, replay 146 us; the
+// What bounds it: issue of ldmatrix and mma.sync.  4 x 2048 tokens, 16 heads of 64 x 128: fold 62 us, replay 154 us; the
 // walk on the float pipe 141 and 231 us.  Error of the layer against float64 4.3e-3 either way (rounding of the result).
 // A product adds zero times what a walk never meets (later tokens' values) and takes an infinity apart into planes.  So a chunk whose
 // operands or incoming state hold a number that is not finite, or so large that a sum of products could overflow, is walked
-// by the same CTA (dm_walk), as is a decay above one.
+// by the same CTA (dm_walk), as is a decay above one.  Looking for such numbers costs 2 us in the fold and 8 us in the replay.
 constexpr int kDmTokens = 64, kDmDim = 64, kDmLd = kDmDim + 8, kDmThreads = 128;
 constexpr float kDmMost = 68719476736.f;      // 2^36: 64 x 64 products of three such numbers stay below 2^120
-constexpr uint32_t kDmMostBf16 = 0x5180u;     // the bits of 2^36 as bfloat16
 
 __device__ __forceinline__ void dm_split(float x, bf16_t (&b)[3]) {
     b[0] = __float2bfloat16_rn(x);
@@ -334,9 +333,13 @@ __device__ __forceinline__ void dm_split(float x, bf16_t (&b)[3]) {
     r -= __bfloat162float(b[1]);
     b[2] = __float2bfloat16_rn(r);
 }
-// two neighbouring columns split into three planes `plane` elements apart; big: either is not below kDmMost
-__device__ __forceinline__ void dm_store2(bf16_t* dst, int plane, float x, float y, bool& big) {
-    big |= !(fabsf(x) < kDmMost) || !(fabsf(y) < kDmMost);
+// the largest magnitudes seen, or NaN
+__device__ __forceinline__ void dm_note(__nv_bfloat162& top, uint32_t pair) {
+    top = __hmax2_nan(top, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&pair)));
+}
+__device__ __forceinline__ bool dm_big(__nv_bfloat162 top) { return !(__low2float(top) < kDmMost) || !(__high2float(top) < kDmMost); }
+// two neighbouring columns split into three planes `plane` elements apart
+__device__ __forceinline__ void dm_store2(bf16_t* dst, int plane, float x, float y, __nv_bfloat162& top) {
     bf16_t a[3], b[3];
     dm_split(x, a);
     dm_split(y, b);
@@ -345,13 +348,16 @@ __device__ __forceinline__ void dm_store2(bf16_t* dst, int plane, float x, float
         __nv_bfloat162 v;
         v.x = a[i];
         v.y = b[i];
-        *reinterpret_cast<__nv_bfloat162*>(dst + i * plane) = v;
+        const uint32_t bits = *reinterpret_cast<const uint32_t*>(&v);
+        if (i == 0) dm_note(top, bits);
+        *reinterpret_cast<uint32_t*>(dst + i * plane) = bits;
     }
 }
 // rows of q or k of one head: rotated (halves), times f(token), zeros past the chunk's end
 template <typename F>
-__device__ __forceinline__ void dm_stage(const DecayScanParams& p, const bf16_t* src, int64_t stride, int row0, int n, bf16_t* dst, bool& big, F f) {
-    const int half = p.rope ? p.rot_dims >> 1 : 0;
+__device__ __forceinline__ void dm_stage(const float* rope, int rot_dims, const bf16_t* src, int64_t stride, int row0, int n, bf16_t* dst,
+                                         __nv_bfloat162& top, F f) {
+    const int half = rope ? rot_dims >> 1 : 0;
     constexpr int U = 8;                                    // pieces of two columns whose loads are in flight together
 #pragma unroll 1
     for (int i0 = 0; i0 < kDmTokens * kDmDim / 2; i0 += U * kDmThreads) {
@@ -365,7 +371,7 @@ __device__ __forceinline__ void dm_stage(const DecayScanParams& p, const bf16_t*
             xw[u] = ok ? *reinterpret_cast<const uint32_t*>(r + d) : 0u;
             yw[u] = ok && d < half ? *reinterpret_cast<const uint32_t*>(r + d + half) : 0u;
             cs[u] = make_float4(1.f, 0.f, 1.f, 0.f);
-            if (ok && d < half) cs[u] = *reinterpret_cast<const float4*>(p.rope + ((int64_t)(row0 + t) * half + d) * 2);
+            if (ok && d < half) cs[u] = *reinterpret_cast<const float4*>(rope + ((int64_t)(row0 + t) * half + d) * 2);
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -375,25 +381,25 @@ __device__ __forceinline__ void dm_stage(const DecayScanParams& p, const bf16_t*
             const float x0 = __uint_as_float(xw[u] << 16), x1 = __uint_as_float(xw[u] & 0xffff0000u);
             const float y0 = __uint_as_float(yw[u] << 16), y1 = __uint_as_float(yw[u] & 0xffff0000u);
             if (d < half)
-                dm_store2(dst + t * kDmLd + d + half, kDmTokens * kDmLd, (y0 * cs[u].x + x0 * cs[u].y) * w, (y1 * cs[u].z + x1 * cs[u].w) * w, big);
-            dm_store2(dst + t * kDmLd + d, kDmTokens * kDmLd, (x0 * cs[u].x - y0 * cs[u].y) * w, (x1 * cs[u].z - y1 * cs[u].w) * w, big);
+                dm_store2(dst + t * kDmLd + d + half, kDmTokens * kDmLd, (y0 * cs[u].x + x0 * cs[u].y) * w, (y1 * cs[u].z + x1 * cs[u].w) * w, top);
+            dm_store2(dst + t * kDmLd + d, kDmTokens * kDmLd, (x0 * cs[u].x - y0 * cs[u].y) * w, (x1 * cs[u].z - y1 * cs[u].w) * w, top);
         }
     }
 }
 template <int VD>
-__device__ __forceinline__ void dm_stage_values(const DecayScanParams& p, int h, int row0, int n, bf16_t* dst, bool& big) {
+__device__ __forceinline__ void dm_stage_values(const DecayScanParams& p, int h, int row0, int n, bf16_t* dst, __nv_bfloat162& top) {
     const bf16_t* vb = static_cast<const bf16_t*>(p.v) + p.v_off + (int64_t)h * VD;
-    uint32_t top = 0u;                  // the largest magnitudes, as bits
 #pragma unroll
     for (int i = 0; i < kDmTokens * VD / 8 / kDmThreads; ++i) {
         const int idx = i * kDmThreads + threadIdx.x, t = idx / (VD / 8), c = idx % (VD / 8) * 8;
         uint4 v = make_uint4(0u, 0u, 0u, 0u);
         if (t < n) v = *reinterpret_cast<const uint4*>(vb + (int64_t)(row0 + t) * p.v_stride + c);
         *reinterpret_cast<uint4*>(dst + t * (VD + 8) + c) = v;
-        top = __vmaxu2(__vmaxu2(top, __vmaxu2(v.x & 0x7fff7fffu, v.y & 0x7fff7fffu)),
-                            __vmaxu2(v.z & 0x7fff7fffu, v.w & 0x7fff7fffu));
+        dm_note(top, v.x);
+        dm_note(top, v.y);
+        dm_note(top, v.z);
+        dm_note(top, v.w);
     }
-    big |= (top & 0xffffu) >= kDmMostBf16 || (top >> 16) >= kDmMostBf16;
 }
 // d^0 .. d^64
 __device__ __forceinline__ void dm_powers(float d, float* pw) {
@@ -416,11 +422,16 @@ __device__ __forceinline__ void dm_rows_product(float (&o)[VD / 8][4], const uin
     }
 }
 
-// The chunk token by token, a thread per column of the state: Ks, Qs [3][64][kDmLd] rotated and scaled rows in planes, Vs [64][VD + 8].
-// S0: the incoming state (null: zeros); Qs null: no outputs; end: where the state after the chunk goes (or null).
+// The chunk token by token, a thread per column of the state.  Ks, Qs: [3][64][kDmLd] rotated and scaled rows in planes, of which `staged`
+// (times `scale`) is brought in first, Vs: [64][VD + 8].  S0: the incoming state (null: zeros); Qs null: no outputs; end: where the state
+// after the chunk goes (or null).  Out of line: the products around it keep their registers.
 template <int VD>
-__device__ __noinline__ void dm_walk(const bf16_t* Ks, const bf16_t* Vs, const bf16_t* Qs, int n, float a, const float* S0, float* out,
+__device__ __noinline__ void dm_walk(const float* rope, int rot_dims, const bf16_t* src, int64_t stride, int row0, int n, bf16_t* staged, float scale,
+                                     const bf16_t* Ks, const bf16_t* Vs, const bf16_t* Qs, float a, const float* S0, float* out,
                                      int64_t out_stride, float* end) {
+    __nv_bfloat162 top = __float2bfloat162_rn(0.f);
+    dm_stage(rope, rot_dims, src, stride, row0, n, staged, top, [&](int) { return scale; });
+    __syncthreads();
     const int c = threadIdx.x;
     if (c >= VD) return;
     auto whole = [](const bf16_t* x) {          // the three planes of a number, whose sum is exact
@@ -458,16 +469,14 @@ __global__ void __launch_bounds__(kDmThreads) decay_fold_mma_kernel(const DecayS
     const bf16_t* kb = static_cast<const bf16_t*>(p.k) + p.k_off + (int64_t)g * kDmDim;
     const int64_t sz = (int64_t)kDmDim * VD;
     float* dst = p.part + ((int64_t)blockIdx.x * p.heads + h) * (sz + 1);
-    bool big = !(fabsf(decay) <= 1.f);
+    __nv_bfloat162 top = __float2bfloat162_rn(fabsf(decay) <= 1.f ? 0.f : kDmMost);
     dm_powers(decay, pw);
-    dm_stage_values<VD>(p, h, row0, n, Vs, big);
+    dm_stage_values<VD>(p, h, row0, n, Vs, top);
     __syncthreads();
-    dm_stage(p, kb, p.k_stride, row0, n, Ks, big, [&](int t) { return pw[n - 1 - t] * p.k_scale; });
+    dm_stage(p.rope, p.rot_dims, kb, p.k_stride, row0, n, Ks, top, [&](int t) { return pw[n - 1 - t] * p.k_scale; });
     if (threadIdx.x == 0) dst[sz] = pw[n];
-    if (__syncthreads_or(big)) {
-        dm_stage(p, kb, p.k_stride, row0, n, Ks, big, [&](int) { return p.k_scale; });
-        __syncthreads();
-        dm_walk<VD>(Ks, Vs, nullptr, n, decay, nullptr, nullptr, 0, dst);
+    if (__syncthreads_or(dm_big(top))) {
+        dm_walk<VD>(p.rope, p.rot_dims, kb, p.k_stride, row0, n, Ks, p.k_scale, Ks, Vs, nullptr, decay, nullptr, nullptr, 0, dst);
         return;
     }
     float o[VD / 8][4];
@@ -497,16 +506,17 @@ __global__ void __launch_bounds__(kDmThreads, 2) decay_replay_mma_kernel(const D
     bf16_t* Vs = Ks + 3 * kDmTokens * kDmLd;                          // [64][VD + 8]
     bf16_t* Ss = Vs + kDmTokens * (VD + 8);                           // [3][64][VD + 8]: first the queries, then the incoming state
     __shared__ float pw[kDmTokens + 1];
+    __shared__ int big[kDmThreads / 32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = blockIdx.y, g = h / (p.heads / p.groups);
     const int* it = p.items + 4 * blockIdx.x;
     const int row0 = it[0], n = it[1];
     const float decay = p.decay[h];
     const bf16_t* qb = static_cast<const bf16_t*>(p.q) + p.q_off + (int64_t)g * kDmDim;
-    bool big = !(fabsf(decay) <= 1.f);
+    __nv_bfloat162 top = __float2bfloat162_rn(fabsf(decay) <= 1.f ? 0.f : kDmMost);
     dm_powers(decay, pw);
-    dm_stage_values<VD>(p, h, row0, n, Vs, big);
-    dm_stage(p, static_cast<const bf16_t*>(p.k) + p.k_off + (int64_t)g * kDmDim, p.k_stride, row0, n, Ks, big, [&](int) { return p.k_scale; });
-    dm_stage(p, qb, p.q_stride, row0, n, Ss, big, [](int) { return 1.f; });
+    dm_stage_values<VD>(p, h, row0, n, Vs, top);
+    dm_stage(p.rope, p.rot_dims, static_cast<const bf16_t*>(p.k) + p.k_off + (int64_t)g * kDmDim, p.k_stride, row0, n, Ks, top, [&](int) { return p.k_scale; });
+    dm_stage(p.rope, p.rot_dims, qb, p.q_stride, row0, n, Ss, top, [](int) { return 1.f; });
     __syncthreads();
     uint32_t qf[3][kDmDim / 16][4];
 #pragma unroll
@@ -530,9 +540,11 @@ __global__ void __launch_bounds__(kDmThreads, 2) decay_replay_mma_kernel(const D
 #pragma unroll
         for (int u = 0; u < 16; ++u) {
             const int idx = i0 + u * kDmThreads + threadIdx.x, d = idx / (VD / 2), c = idx % (VD / 2) * 2;
-            dm_store2(Ss + d * (VD + 8) + c, kDmDim * (VD + 8), x[u], y[u], big);
+            dm_store2(Ss + d * (VD + 8) + c, kDmDim * (VD + 8), x[u], y[u], top);
         }
     }
+    const bool big_w = __any_sync(0xffffffffu, dm_big(top));
+    if (lane == 0) big[warp] = big_w;
     // scores of this warp's tokens against the keys up to them
     float s[kDmTokens / 8][4];
 #pragma unroll
@@ -556,12 +568,7 @@ __global__ void __launch_bounds__(kDmThreads, 2) decay_replay_mma_kernel(const D
                 }
             }
     }
-    if (__syncthreads_or(big)) {                                      // the state is staged
-        dm_stage(p, qb, p.q_stride, row0, n, Ss, big, [](int) { return 1.f; });
-        __syncthreads();
-        dm_walk<VD>(Ks, Vs, Ss, n, decay, S0, p.out + (int64_t)row0 * p.out_stride + (int64_t)h * VD, p.out_stride, nullptr);
-        return;
-    }
+    __syncthreads();                                                  // the state is staged
     float o[VD / 8][4];
 #pragma unroll
     for (int i = 0; i < VD / 8; ++i)
@@ -611,6 +618,12 @@ __global__ void __launch_bounds__(kDmThreads, 2) decay_replay_mma_kernel(const D
         float* dst = p.out + (int64_t)(row0 + t) * p.out_stride + (int64_t)h * VD + 2 * (lane & 3);
 #pragma unroll
         for (int i = 0; i < VD / 8; ++i) *reinterpret_cast<float2*>(dst + i * 8) = make_float2(o[i][2 * r], o[i][2 * r + 1]);
+    }
+    __syncthreads();
+    if (big[0] | big[1] | big[2] | big[3]) {
+        dm_walk<VD>(p.rope, p.rot_dims, qb, p.q_stride, row0, n, Ss, 1.f, Ks, Vs, Ss, decay, S0,
+                    p.out + (int64_t)row0 * p.out_stride + (int64_t)h * VD, p.out_stride, nullptr);
+        return;
     }
 }
 
