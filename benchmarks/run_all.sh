@@ -1,8 +1,7 @@
 #!/bin/bash
-# One-GPU sweep of every benchmark of the repo; JSON lines land in gpurun_out/r01_sweep/.
-#   gpurun --timeout 1500 -- 'bash benchmarks/run_all.sh'
+# One-GPU sweep of every benchmark of the repo; JSON lines land in the folder given (default: sweep_out).
 set -u
-OUT=gpurun_out/r01_sweep
+OUT=${1:-sweep_out}
 mkdir -p $OUT
 python -m pytest tests -m gpu -q --timeout 300 > $OUT/pytest_gpu.log 2>&1; tail -1 $OUT/pytest_gpu.log
 python __graft_entry__.py smoke > $OUT/smoke.log 2>&1; tail -1 $OUT/smoke.log
