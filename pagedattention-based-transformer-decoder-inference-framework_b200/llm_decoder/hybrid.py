@@ -369,7 +369,10 @@ class LatentAttentionMixer:
                 lib.pa_masked_attention_tc_tile_tokens(1, 1, self.dim, self.vdim, elem, 2)):
             self.expand_from = max(EXPAND_FROM, -(-EXPAND_WORK // self.kv_rank))
             self.tc_tokens = tuple(lib.pa_masked_attention_tc_tile_tokens(1, 1, self.dim, self.vdim, elem, q) for q in (2, 1))
-            self.w_uv = model._weight_raw(W[prefix + "uv"].reshape(H, self.vdim, self.kv_rank)).transpose(1, 2)     # the same, by output channel
+            # [H * (dim + vdim)][kv_rank], for one product over the cached rows; w_uk and w_uv, which the other form reads, are views of it
+            self.w_ukv = model._weight_raw(torch.cat([W[prefix + "uk"], W[prefix + "uv"]], 0))
+            self.w_uk = self.w_ukv[:H * self.dim].view(H, self.dim, self.kv_rank)
+            self.w_uv = self.w_ukv[H * self.dim:].view(H, self.vdim, self.kv_rank).transpose(1, 2)
 
     @property
     def cuts_keys(self):
@@ -408,7 +411,7 @@ class LatentAttentionMixer:
 
     def _attend_expanded(self, c, q, out, at_least, most):
         """The prompt portions that build the keys and values of their whole sequences: per head a key of dim + rot_dim and a value
-        of vdim columns instead of kv_rank + rot_dim and kv_rank, for two products over the cached rows."""
+        of vdim columns instead of kv_rank + rot_dim and kv_rank, for one product over the cached rows."""
         b, lib, kv, s, H = c.batch, c.lib, self.kv, _cabi.stream(), self.heads
         pt = kv.page_table_
         q_tiles = 2 if b.count_tiles(self.tc_tokens[0], at_least) * H >= c.model.sm_count else 1
@@ -417,14 +420,12 @@ class LatentAttentionMixer:
             _chk(lib.pa_latent_gather(kv.key_buffer_.data_ptr(), pt.device_data().data_ptr(), pt.num_beams_, pt.num_tiles_,
                                       kv.total_pages_, kv.tile_size_, self.kd * c.elem, items.data_ptr(), nitems, longest,
                                       lat.data_ptr(), s), "pa_latent_gather")
-            # both are views of what the other form reads: w_uk as it lies, w_uv is kept by output channel for this product
-            keys = torch.nn.functional.linear(lat[:, :self.kv_rank], self.w_uk.reshape(H * self.dim, self.kv_rank))
-            values = torch.nn.functional.linear(lat[:, :self.kv_rank], self.w_uv.transpose(1, 2).reshape(H * self.vdim, self.kv_rank))
-            _chk(lib.pa_latent_attention_expanded(q.data_ptr(), q.stride(0), 0, keys.data_ptr(), H * self.dim, lat.data_ptr(), self.kd,
-                                                  self.kv_rank, values.data_ptr(), H * self.vdim, rows, tiles.data_ptr(), ntiles, H,
-                                                  self.dim, self.rot_dim, self.vdim, self.scale, _cabi.ptr(self.sink), out.data_ptr(),
-                                                  q_tiles, s), "pa_latent_attention_expanded")
-            del lat, keys, values       # before the next group's
+            built = torch.nn.functional.linear(lat[:, :self.kv_rank], self.w_ukv)
+            _chk(lib.pa_latent_attention_expanded(q.data_ptr(), q.stride(0), 0, built.data_ptr(), built.stride(0), lat.data_ptr(),
+                                                  self.kd, self.kv_rank, built.data_ptr() + H * self.dim * c.elem, built.stride(0),
+                                                  rows, tiles.data_ptr(), ntiles, H, self.dim, self.rot_dim, self.vdim, self.scale,
+                                                  _cabi.ptr(self.sink), out.data_ptr(), q_tiles, s), "pa_latent_attention_expanded")
+            del lat, built  # before the next group's
 
     def _attend(self, c, q, ql, lat, mma, without=None):
         """Launch the attention kernels over this step's tiles (prompt portions, then single decoded tokens).  Returns
@@ -501,7 +502,7 @@ class LatentAttentionMixer:
         proj = c.model._linear(h, self.w_in)
         q = self._queries(c, proj)
         kvr = self.kv_rank
-        most = self._expand_rows(c) if self.tc_tokens else 0
+        most = self._expand_rows(c) if self.tc_tokens and c.batch.longest_portion >= self.expand_from else 0
         expand = c.batch.expand_from(self.expand_from, most) if most else 0
         without = (expand, most) if expand else None
         if expand and all(c.batch._expands(p, *without) for p in c.batch.portions):

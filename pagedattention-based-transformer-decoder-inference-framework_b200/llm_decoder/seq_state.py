@@ -52,6 +52,7 @@ class RaggedBatch:
         self.rows = len(ids)
         self.num_seqs = len(seq_start)
         self.portions = portions                      # host list of (first row, length, slot, first position)
+        self.longest_portion = max(seq_len, default=0)
         dev_rows = _to_device(host, device)
         self.ids, self.row_slot, self.row_pos, self.row_prev = dev_rows[0], dev_rows[1], dev_rows[2], dev_rows[3]
         self.prev_ids = dev_rows[4] if prev_ids is not None else None
@@ -187,7 +188,7 @@ class DecodeBatch(RaggedBatch):
 
     def __init__(self, n, longest, device, prev_ids):
         self.rows = self.num_seqs = n
-        self.portions = [(r, 1, 0, 0) for r in range(n)]
+        self.portions, self.longest_portion = [(r, 1, 0, 0) for r in range(n)], 1
         self.device, self.longest = device, longest
         # ids, slot, position, previous row, previous token, portion: first row, length, slot | query tiles [n, 4] | portion items
         # [n, 6] | chunk items [n, 4] | first chunk, chunks
