@@ -19,10 +19,11 @@
 // O keeps a per-row reference maximum that is raised only when a tile exceeds it by more than 2^8 (P stays below 2^8, and l and
 // O share the reference, so O / l does not depend on it): rows are rescaled a few times instead of once per tile.
 //
-// What bounds it: per 64 keys and 128 rows 4096 / 16 = 512 cycles of ex2 on the MUFU against 512 (dim 128) to 640 (dim 192)
-// cycles of tensor pipe; two tiles per CTA keep both busy at once.  A step takes about 2300 cycles: the exponentials of both tiles
-// (1600 with their adds and conversions) and the hand-offs between pipes (tiles of 128 keys, which have half as many but no
-// second score buffer, took 150 us where this takes 123; query rows by TMA and no wait but the scores' own gave 123 -> 110).  Measured, 4 x 2048 tokens causal: 16 query / 4 kv heads of 128
+// What bounds it: the hand-offs between the pipes and the exponentials.  Per 64 keys and 128 rows 8192 / 16 = 512 cycles of ex2 on the
+// MUFU stand against 512 (dim 128) to 640 (dim 192) cycles of tensor pipe, and two tiles per CTA could keep both busy at
+// once; a step takes about 2300 cycles, 1600 of them the exponentials of both tiles with their adds and conversions (tiles of
+// 128 keys, which have half as many hand-offs but no second score buffer, took 150 us where this takes 123; query rows by TMA
+// and no wait but the scores' own gave 123 -> 110).  Measured, 4 x 2048 tokens causal: 16 query / 4 kv heads of 128
 // paged 110 us = 620 TFLOP/s (mma.sync kernel 918 us); latent attention at 16 heads of 128 + 64 / 128, five ragged portions
 // 110 us, and 38 us for gathering the rows and building keys and values (absorbed form on mma.sync 1360 us).
 //

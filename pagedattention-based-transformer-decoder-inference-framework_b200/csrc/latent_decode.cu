@@ -9,8 +9,8 @@
 // eighth of the latent columns -- nothing is computed twice but the 16 x 32 exponentials.  Shares that end inside a token are
 // joined by a second kernel (decode_shares.cuh).
 //
-// What bounds it: HBM, 180 KB in flight per SM; the chain of a step (scores, exchange, exponentials, weighted sums) is the
-// rest.  64 tokens, 16 heads, rank 512 + 64, 2048 keys (151 MB): 49 us = 3.1 TB/s (latent_attention_mma_kernel with two key splits
+// What bounds it: the chain of a step (scores, exchange, exponentials, weighted sums), which all eight warps walk together; HBM
+// is busy 39 % of the time with 180 KB in flight per SM.  64 tokens, 16 heads, rank 512 + 64, 2048 keys (151 MB): 49 us = 3.1 TB/s (latent_attention_mma_kernel with two key splits
 // and its merge: 70 + 8 us); 8 tokens, 8 heads, rank 256 + 32, 400 keys: 7.5 us (13.6 us).
 #include "decode_shares.cuh"
 #include "mma_utils.cuh"
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(kThreads, 1) latent_decode_kernel(const __grid
             open_pair();
         }
         const uint32_t st = base + stage * STAGE;
-        if (!tc::tc_wait(full(stage), phase, fail_sm, a.polls)) tc::tc_let_land(full(stage), phase);      // run out: on over whatever is there
+        tc::tc_wait(full(stage), phase, fail_sm, a.polls);     // if it runs out, on over whatever is there: close_pair leaves NaN
         const uint32_t mapped = meta[stage];
         const int j0 = u * kUnit, valid = qpos + 1 - j0;
         // scores of this warp's keys over its columns
@@ -305,7 +305,10 @@ __global__ void __launch_bounds__(kThreads, 1) latent_decode_kernel(const __grid
         }
     }
     close_pair();
-    if (threadIdx.x == 0 && tc::tc_failed(fail_sm)) atomicAdd(&g_errors, 1);
+    if (threadIdx.x == 0 && tc::tc_failed(fail_sm)) {       // the copies that were requested land before the shared memory goes
+        for (int b = 0; b < ST; ++b) tc::tc_let_land(full(b), b < stage ? phase : phase ^ 1u);
+        atomicAdd(&g_errors, 1);
+    }
 }
 
 // One warp per (pair, row); a lane has columns 2 lane + 64 i and the next.

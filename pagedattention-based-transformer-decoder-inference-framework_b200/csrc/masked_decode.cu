@@ -12,8 +12,8 @@
 // kernel with heads as rows; smaller batches, whose streaming kernel keeps them float, keep them float here too: three
 // bfloat16 numbers add up to the 24 bits of a weight, for three products instead of one.
 //
-// What bounds it: HBM.  Eight workers x 3 stages x 8 KB per SM are in flight, as in the streaming kernel of paged_decode.cu; a unit
-// costs a warp about 150 instructions.  64 tokens, 16 query / 4 kv heads of 128, 2048 keys (268 MB): 56 us = 4.8 TB/s and 4 us for the
+// What bounds it: HBM (busy 59 % of the time, with eight workers x 3 stages x 8 KB per SM in flight) and the chain of a unit in a warp,
+// eight of which an SM has.  64 tokens, 16 query / 4 kv heads of 128, 2048 keys (268 MB): 56 us = 4.8 TB/s and 4 us for the
 // join (heads as rows without a key split, masked_attention_mma_decode_kernel: 91 us); 8 tokens, 2 kv heads, 400 keys: 10 us
 // (streaming kernel, one CTA per pair: 38 us).
 #include "decode_shares.cuh"
@@ -24,8 +24,10 @@
 namespace pa {
 namespace mdec {
 
-// at least four units a share: opening and closing one costs about as much as that
-constexpr int kWarps = 8, kStages = 3, kUnit = 16, kRows = 16, kLeast = 4;
+// At least two units a share (GPU time with 2 / 3 / 4, kernel and join, each launched alone: 8 tokens of 128 to 640 keys, 2 kv heads 15.8 /
+// 20.6 / 21.4 us, 4 x 300 keys, 4 kv heads 14.9 / 17.5 / 20.8 us, 20 x 300, 2 kv heads 15.8 / 19.3 / 19.9 us, 1 x 2000, 4 kv heads 20.3 /
+// 19.8 / 21.4 us): a short chain per warp is worth more sums to join.
+constexpr int kWarps = 8, kStages = 3, kUnit = 16, kRows = 16, kLeast = 2;
 
 struct Args {
     MaskAttnParams p;
