@@ -13,8 +13,8 @@
 // A routing weight on the expert's input is applied to the accumulated product, which is linear in it.
 //
 // What bounds it: what one SM takes in.  A stage (64 columns) is 4 x M128 N256 K16 = 512 cycles of tensor pipe, and its 48 KB would
-// have to come at 96 B per cycle; about 50 are seen, and the pipe is busy 36 % of the time.  Measured, 16384 pairs of 8 experts, width 2048, ff 1024: gate / up 178 us = 770
-// TFLOP/s, down 67 us = 1030 TFLOP/s (mma.sync kernels of moe_ops.cu: 530 and 294 us).
+// have to come at 96 B per cycle; about 50 are seen, and the pipe is busy 36 % of the time.  Measured, 16384 pairs of 8 experts,
+// width 2048, ff 1024: gate / up 178 us = 770 TFLOP/s, down 67 us = 1030 TFLOP/s (mma.sync kernels of moe_ops.cu: 530 and 294 us).
 //
 // Every wait is bounded: on a protocol error the CTA raises a flag (pa_moe_tc_errors), lets its copies land, frees its TMEM and
 // writes NaN into the rows of its tiles from there on.
