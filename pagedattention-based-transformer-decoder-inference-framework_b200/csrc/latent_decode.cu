@@ -10,7 +10,7 @@
 // joined by a second kernel (decode_shares.cuh).
 //
 // What bounds it: the chain of a step (scores, exchange, exponentials, weighted sums), which all eight warps walk together; HBM
-// is busy 39 % of the time with 180 KB in flight per SM.  64 tokens, 16 heads, rank 512 + 64, 2048 keys (151 MB): 49 us = 3.1 TB/s
+// is busy 40 % of the time with 180 KB in flight per SM.  64 tokens, 16 heads, rank 512 + 64, 2048 keys (151 MB): 49 us = 3.1 TB/s
 // (latent_attention_mma_kernel with two key splits and its merge: 70 + 8 us); 8 tokens, 8 heads, rank 256 + 32, 400 keys: 8.7 us
 // (13.6 us).
 #include "decode_shares.cuh"

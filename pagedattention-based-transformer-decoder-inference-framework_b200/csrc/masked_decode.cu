@@ -12,7 +12,7 @@
 // kernel with heads as rows; smaller batches, whose streaming kernel keeps them float, keep them float here too: three
 // bfloat16 numbers add up to the 24 bits of a weight, for three products instead of one.
 //
-// What bounds it: HBM (busy 59 % of the time, with eight workers x 3 stages x 8 KB per SM in flight) and the chain of a unit in a warp,
+// What bounds it: HBM (busy 57 % of the time, with eight workers x 3 stages x 8 KB per SM in flight) and the chain of a unit in a warp,
 // eight of which an SM has.  64 tokens, 16 query / 4 kv heads of 128, 2048 keys (268 MB): 56 us = 4.8 TB/s and 4 us for the
 // join (heads as rows without a key split, masked_attention_mma_decode_kernel: 91 us); 8 tokens, 2 kv heads, 400 keys: 8.5 us
 // (streaming kernel, one CTA per pair: 38 us).
