@@ -165,6 +165,113 @@ __global__ void latent_kv_append_kernel(T* __restrict__ pool, const int32_t* __r
     for (int d = rot_dims + lane; d < rot_dim; d += 32) dst[kv_rank + d] = s[kv_rank + d];   // unrotated remainder
 }
 
+// The same for bfloat16 rows of whole 16-byte words (see latent_append): a lane has eight neighbouring columns per step and
+// keeps its part of a row in registers between the sum of squares and the scaling, so a row is read once, all of it in flight
+// together.  A rotation has its pairs within a word (neighbours) or in two words of one lane (halves).
+// What bounds it: the latency of a row's chain (slot and position, page, row).  Rank 512 + 64, 16 heads' queries turned: 5800 rows
+// 17.6 us, 64 rows 4.4 us (element by element 24.7 and 9.2 us).
+constexpr int kLaWords = 4;             // 16-byte words of a row per lane: rows of up to 1024 columns
+
+__device__ __forceinline__ void rms_row_words(const bf16_t* __restrict__ s, int width, float eps, const float* __restrict__ gain,
+                                              bf16_t* __restrict__ dst, int lane) {
+    uint4 v[kLaWords];
+#pragma unroll
+    for (int i = 0; i < kLaWords; ++i) {
+        const int d = (lane + 32 * i) * 8;
+        v[i] = d < width ? *reinterpret_cast<const uint4*>(s + d) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < kLaWords; ++i) {
+        float f[8];
+        bf16x8_unpack(v[i], f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) ss = fmaf(f[e], f[e], ss);
+    }
+    const float rn = 1.0f / sqrtf(warp_sum(ss) / (float)width + eps);
+    if (!dst) return;
+#pragma unroll
+    for (int i = 0; i < kLaWords; ++i) {
+        const int d = (lane + 32 * i) * 8;
+        if (d >= width) continue;
+        const float4 g0 = __ldg(reinterpret_cast<const float4*>(gain + d)), g1 = __ldg(reinterpret_cast<const float4*>(gain + d + 4));
+        const float g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+        float f[8];
+        bf16x8_unpack(v[i], f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] = f[e] * rn * g[e];
+        *reinterpret_cast<uint4*>(dst + d) = bf16x8_pack(f);
+    }
+}
+
+// word i of a row's rotated part, src -> dst (which may be the same): half = rot_dims / 2 pairs, tab = their (cos, sin)
+__device__ __forceinline__ void turn_words(const bf16_t* src, bf16_t* dst, const float* __restrict__ tab, int half, int pairing, int i) {
+    if (pairing == 0) {                 // four neighbouring pairs
+        float f[8];
+        bf16x8_unpack(*reinterpret_cast<const uint4*>(src + 8 * i), f);
+        const float4 a = __ldg(reinterpret_cast<const float4*>(tab) + 2 * i), b = __ldg(reinterpret_cast<const float4*>(tab) + 2 * i + 1);
+        const float c[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int e = 0; e < 8; e += 2) {
+            const float u = f[e], v = f[e + 1];
+            f[e] = u * c[e] - v * c[e + 1];
+            f[e + 1] = v * c[e] + u * c[e + 1];
+        }
+        *reinterpret_cast<uint4*>(dst + 8 * i) = bf16x8_pack(f);
+    } else {                            // eight pairs: a word of either half
+        float f[8], h[8];
+        bf16x8_unpack(*reinterpret_cast<const uint4*>(src + 8 * i), f);
+        bf16x8_unpack(*reinterpret_cast<const uint4*>(src + half + 8 * i), h);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const float2 c = __ldg(reinterpret_cast<const float2*>(tab) + 8 * i + e);
+            const float u = f[e], v = h[e];
+            f[e] = u * c.x - v * c.y;
+            h[e] = v * c.x + u * c.y;
+        }
+        *reinterpret_cast<uint4*>(dst + 8 * i) = bf16x8_pack(f);
+        *reinterpret_cast<uint4*>(dst + half + 8 * i) = bf16x8_pack(h);
+    }
+}
+
+__global__ void __launch_bounds__(256) latent_kv_append_words_kernel(
+    bf16_t* __restrict__ pool, const int32_t* __restrict__ table, int num_slots, int num_tiles, int total_pages, int tile_size, int kv_rank,
+    int rot_dim, int rot_dims, const bf16_t* src, int64_t src_stride, int c_off, const float* __restrict__ gain, float eps,
+    const float* __restrict__ rope, const int32_t* __restrict__ row_slot, const int32_t* __restrict__ row_pos, int rows, int pairing,
+    int units, int q_off, int q_rank, const float* __restrict__ q_gain, bf16_t* q_out, int64_t q_out_stride, int turn_q, int heads,
+    int q_head_stride) {
+    const int lane = threadIdx.x & 31;
+    const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (w >= (int64_t)rows * units) return;
+    const int64_t r = w / units;
+    const int half = rot_dims / 2, turns = pairing == 0 ? rot_dims / 8 : half / 8;      // steps of one row's rotation
+    const float* tab = rope + r * rot_dims;
+    if (w % units == 1) {
+        if (!turn_q) {
+            rms_row_words(src + r * src_stride + q_off, q_rank, eps, q_gain, q_out + r * q_out_stride, lane);
+            return;
+        }
+        bf16_t* q = q_out + r * q_out_stride + q_off;
+        for (int i = lane; i < heads * turns; i += 32) {
+            bf16_t* x = q + (int64_t)(i / turns) * q_head_stride;
+            turn_words(x, x, tab, half, pairing, i % turns);
+        }
+        return;
+    }
+    const int slot = row_slot[r], pos = row_pos[r];
+    const bf16_t* s = src + r * src_stride + c_off;
+    bf16_t* dst = nullptr;
+    if (pos >= 0 && pos / tile_size < num_tiles && (unsigned)slot < (unsigned)num_slots) {
+        const int page = table[(int64_t)slot * num_tiles + pos / tile_size];
+        if (page >= 0 && page < total_pages) dst = pool + ((int64_t)page * tile_size + pos % tile_size) * (kv_rank + rot_dim);
+    }
+    rms_row_words(s, kv_rank, eps, gain, dst, lane);        // reads its row while the page is looked up
+    if (!dst) return;
+    for (int i = lane; i < turns; i += 32) turn_words(s + kv_rank, dst + kv_rank, tab, half, pairing, i);
+    for (int d = rot_dims + 8 * lane; d < rot_dim; d += 256)        // unrotated remainder
+        *reinterpret_cast<uint4*>(dst + kv_rank + d) = *reinterpret_cast<const uint4*>(s + kv_rank + d);
+}
+
 // RMS norm of `width` columns of strided rows with a per-channel gain (the query latent)
 template <typename T>
 __global__ void rms_rows_kernel(const T* __restrict__ src, int64_t src_stride, int off, int width, float eps,
@@ -922,6 +1029,18 @@ static int latent_append(void* d_pool, const int32_t* d_table, int num_slots, in
     if (rows == 0) return PA_OK;
     const int units = d_q_out ? 2 : 1;
     const int64_t threads = (int64_t)rows * units * 32;
+    // whole words: every column range starts and ends on a boundary of eight elements (halves that are rotated: each of them)
+    const int step = pairing == 0 ? 8 : 16;
+    const bool q_words = !d_q_out || (q_out_stride % 8 == 0 && q_off % 8 == 0 &&
+                                      (turn_q ? q_head_stride % 8 == 0 : q_rank % 8 == 0 && q_rank <= kLaWords * 256 && (uintptr_t)d_q_gain % 16 == 0));
+    if (elem == 2 && q_words && kv_rank % 8 == 0 && kv_rank <= kLaWords * 256 && rot_dim % 8 == 0 && rot_dims % step == 0 && src_stride % 8 == 0 &&
+        c_off % 8 == 0 && ((uintptr_t)d_pool | (uintptr_t)d_src | (uintptr_t)d_gain | (uintptr_t)d_rope_table | (uintptr_t)d_q_out) % 16 == 0) {
+        latent_kv_append_words_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, as_stream(stream)>>>(
+            static_cast<bf16_t*>(d_pool), d_table, num_slots, num_tiles, total_pages, tile_size, kv_rank, rot_dim, rot_dims,
+            static_cast<const bf16_t*>(d_src), src_stride, c_off, d_gain, eps, d_rope_table, d_row_slot, d_row_pos, rows, pairing, units,
+            q_off, q_rank, d_q_gain, static_cast<bf16_t*>(d_q_out), q_out_stride, turn_q, heads, q_head_stride);
+        PA_RETURN_LAUNCH_STATUS();
+    }
     PA_DISPATCH_ELEM(elem, latent_kv_append_kernel<T><<<(unsigned)((threads + 255) / 256), 256, 0, as_stream(stream)>>>(
                                static_cast<T*>(d_pool), d_table, num_slots, num_tiles, total_pages, tile_size, kv_rank,
                                rot_dim, rot_dims, static_cast<const T*>(d_src), src_stride, c_off, d_gain, eps,

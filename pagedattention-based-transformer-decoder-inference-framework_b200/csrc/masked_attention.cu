@@ -28,6 +28,7 @@
 //
 // Pools: K pages [total_pages][tile_size][dim], V pages [total_pages][tile_size][vdim]; a (slot, kv head, tile) entry
 // of the page table names the page of both (appended by pa_kv_append_rows).
+#include "f32x2.cuh"
 #include "masked_attention.cuh"
 
 namespace pa {
@@ -528,6 +529,193 @@ __global__ void __launch_bounds__(kCaThreads, EPL == 4 && TAPS <= 4 ? 5 : 1) con
     }
 }
 
+// The same for many items of bfloat16 rows of whole 16-byte words, heads of at most 128: a unit is LANES lanes with eight columns
+// each, a CTA has one item and kCaThreads / LANES of its units.  Tokens go two at a time: their sums of squares are reduced
+// together, so that one chain of shuffles serves two rows, and the raw rows of the four after them are on their way meanwhile.
+// The turns of sixteen tokens are staged in shared memory, where all units of the CTA read them.
+// What bounds it: instructions and occupancy (128 registers); 4 x 2048 tokens, 16 + 2 x 4 heads of 128, four taps (100 MB): 37 us
+// = 2.7 TB/s, the form above 52 us.  64 decoded tokens: 6.5 and 3.9 us, so that few items stay with the form above (ca_dispatch).
+// the same as pairs
+template <typename T, int EPL>
+__device__ __forceinline__ void ca_word_pairs(const CaWord<T, EPL>& r, uint64_t (&f)[EPL / 2]) {
+    float x[EPL];
+    ca_word_unpack<T, EPL>(r, x);
+#pragma unroll
+    for (int i = 0; i < EPL / 2; ++i) f[i] = f32x2::pack2(x[2 * i], x[2 * i + 1]);
+}
+template <int EPL>
+__device__ __forceinline__ void ca_load_pairs(const float* __restrict__ p, uint64_t (&f)[EPL / 2]) {
+    float x[EPL];
+    ca_load_floats<EPL>(p, x);
+#pragma unroll
+    for (int i = 0; i < EPL / 2; ++i) f[i] = f32x2::pack2(x[2 * i], x[2 * i + 1]);
+}
+
+constexpr int kCaTurns = 16;        // tokens whose turns are staged together
+
+template <int LANES, int TAPS>
+__global__ void __launch_bounds__(kCaThreads, 4) conv_rope_norm_append_words_kernel(const ConvAppendParams p) {
+    typedef bf16_t T;
+    constexpr int EPL = 8, kAhead = 4, kGroup = 2, kUnits = kCaThreads / LANES;
+    __shared__ __align__(16) float turns[kCaTurns * EPL * LANES];
+    const int lane = threadIdx.x & (LANES - 1);
+    const int units = p.heads + (p.k_pool ? 2 * p.kv_heads : 0), groups = (units + kUnits - 1) / kUnits;
+    const int item = blockIdx.x / groups, unit_at = blockIdx.x % groups * kUnits + threadIdx.x / LANES;
+    // every thread stays to the end (barriers; the sums over a unit's lanes are warp shuffles); lanes past the last unit or past
+    // a head's size read its first columns and write nothing
+    const bool unit_ok = unit_at < units;
+    const int unit = unit_ok ? unit_at : 0;
+    const int* it = p.items + 6 * item;
+    const int row0 = it[0], n = it[1], off = it[3], plen = it[4], pos0 = it[5];
+    const int kind = unit < p.heads ? 0 : unit < p.heads + p.kv_heads ? 1 : 2;       // query, key, value
+    const int g = kind == 0 ? 0 : unit - p.heads - (kind - 1) * p.kv_heads;
+    const int size = kind == 2 ? p.vdim : p.dim;
+    const bool slot_ok = (unsigned)it[2] < (unsigned)p.num_slots;
+    const bool live = unit_ok && lane * EPL < size && slot_ok;
+    const int slot = slot_ok ? it[2] : 0;
+    const int d = lane * EPL < size ? lane * EPL : 0;
+    const int ch0 = (kind == 0 ? unit * p.dim : p.heads * p.dim + (kind == 1 ? g * p.dim : p.kv_heads * p.dim + g * p.vdim)) + d;
+    const int stride = (int)p.in_stride;
+    const T* in = static_cast<const T*>(p.in) + p.in_off + ch0 + (int64_t)row0 * stride;
+    const int taps = p.w ? p.taps : 1;
+    float* st = taps > 1 ? p.state + (int64_t)slot * (taps - 1) * p.channels + ch0 : nullptr;
+    const int turned = kind < 2 ? min(EPL, max(0, p.rot_dims - d)) : 0;      // columns of this lane that are rotated
+    const bool norm = kind < 2 && p.norm;
+    const float inv_size = 1.0f / (float)size;
+
+    CaWord<T, EPL> nxt[kAhead];
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) nxt[i] = ca_word_load<T, EPL>(in + (int64_t)min(i, n - 1) * stride);
+    uint64_t wt[TAPS][EPL / 2], win[TAPS][EPL / 2];    // pairs of columns; win: ring, token t in place t % TAPS
+#pragma unroll
+    for (int b = 0; b < TAPS; ++b)
+#pragma unroll
+        for (int c = 0; c < EPL / 2; ++c) {
+            wt[b][c] = p.w || b ? 0ull : f32x2::pack2(1.f, 1.f);
+            win[b][c] = 0ull;
+        }
+    if (p.w) {
+#pragma unroll
+        for (int b = 0; b < TAPS; ++b)
+            if (b < taps) ca_load_pairs<EPL>(p.w + (int64_t)b * p.channels + ch0, wt[b]);
+    }
+#pragma unroll
+    for (int b = 1; b < TAPS; ++b)
+        if (b < taps) {
+            const int t = off - b;                     // offset within the portion
+            if (t >= 0) ca_word_pairs<T, EPL>(ca_word_load<T, EPL>(in - (int64_t)b * stride), win[TAPS - b]);
+            else ca_load_pairs<EPL>(st + (int64_t)(taps - 1 + t) * p.channels, win[TAPS - b]);
+        }
+    // destination of the current token's row (null: not stored), and its place in its page
+    T* dst = kind == 0 ? static_cast<T*>(p.q_out) + (int64_t)row0 * p.q_out_stride + ch0 : nullptr;
+    const int64_t dstep = kind == 0 ? p.q_out_stride : size;
+    int tile = 0, at = 0;
+    auto look_up = [&]() {
+        const int page = tile < p.num_tiles ? p.table[((int64_t)slot * p.kv_heads + g) * p.num_tiles + tile] : -1;
+        dst = page >= 0 && page < p.total_pages
+                  ? static_cast<T*>(kind == 1 ? p.k_pool : p.v_pool) + ((int64_t)page * p.tile_size + at) * size + d : nullptr;
+    };
+    if (kind && pos0 >= 0) {
+        tile = pos0 / p.tile_size;
+        at = pos0 - tile * p.tile_size;
+        look_up();
+    }
+
+    // the token in place `place` of the window from its raw row and its turns; returns its sum of squares over this lane's columns
+    auto convolve = [&](int place, const CaWord<T, EPL>& raw, const float* cs, uint64_t (&y)[EPL / 2]) {
+        uint64_t (&now)[EPL / 2] = win[place];
+        ca_word_pairs<T, EPL>(raw, now);
+#pragma unroll
+        for (int c = 0; c < EPL / 2; ++c) {
+            y[c] = f32x2::mul2(wt[0][c], now[c]);
+#pragma unroll
+            for (int b = 1; b < TAPS; ++b) y[c] = f32x2::fma2(wt[b][c], win[(place + TAPS - b) % TAPS][c], y[c]);
+        }
+#pragma unroll
+        for (int c = 0; c < EPL; c += 4)
+            if (c < turned) {
+                const float4 a = *reinterpret_cast<const float4*>(cs + c);
+                float u, v;
+                f32x2::unpack2(y[c / 2], u, v);
+                y[c / 2] = f32x2::fma2(y[c / 2], f32x2::pack2(a.x, a.x), f32x2::mul2(f32x2::pack2(-v, u), f32x2::pack2(a.y, a.y)));
+                f32x2::unpack2(y[c / 2 + 1], u, v);
+                y[c / 2 + 1] = f32x2::fma2(y[c / 2 + 1], f32x2::pack2(a.z, a.z), f32x2::mul2(f32x2::pack2(-v, u), f32x2::pack2(a.w, a.w)));
+            }
+        uint64_t sq = 0ull;
+#pragma unroll
+        for (int c = 0; c < EPL / 2; ++c) sq = f32x2::fma2(y[c], y[c], sq);
+        float s0, s1;
+        f32x2::unpack2(sq, s0, s1);
+        return lane * EPL < size ? s0 + s1 : 0.f;
+    };
+    auto store = [&](const uint64_t (&y)[EPL / 2], float ss) {
+        float z[EPL];
+        const float rn = norm ? rsqrtf(fmaf(ss, inv_size, p.eps)) : 1.f;
+#pragma unroll
+        for (int c = 0; c < EPL / 2; ++c) f32x2::unpack2(f32x2::mul2(y[c], f32x2::pack2(rn, rn)), z[2 * c], z[2 * c + 1]);
+        if (live && dst) ca_word_store<T, EPL>(dst, z);
+    };
+
+    for (int t0 = 0; t0 < n; t0 += kAhead) {  // n is the CTA's
+        if (p.rot_dims > 0 && t0 % kCaTurns == 0) {    // kAhead divides kCaTurns
+            if (t0) __syncthreads();
+            const int m = min(kCaTurns, n - t0) * (p.rot_dims / 4);
+            const float4* src = reinterpret_cast<const float4*>(p.rope + (int64_t)(row0 + t0) * p.rot_dims);
+            for (int i = threadIdx.x; i < m; i += kCaThreads) reinterpret_cast<float4*>(turns)[i] = __ldg(src + i);
+            __syncthreads();
+        }
+#pragma unroll
+        for (int j = 0; j < kAhead; j += kGroup) {
+            const int t = t0 + j;
+            if (t >= n) break;
+            uint64_t y[kGroup][EPL / 2];
+            float ss[kGroup] = {};
+#pragma unroll
+            for (int i = 0; i < kGroup; ++i) {
+                if (t + i >= n) break;                 // the same for the whole CTA
+                ss[i] = convolve((j + i) % TAPS, nxt[j + i], turns + ((t + i) % kCaTurns) * p.rot_dims + d, y[i]);
+                if (t + i + kAhead < n) nxt[j + i] = ca_word_load<T, EPL>(in + (int64_t)(t + i + kAhead) * stride);
+            }
+            if (p.norm) {                              // the same for every lane of a warp
+#pragma unroll
+                for (int o = LANES / 2; o > 0; o >>= 1)
+#pragma unroll
+                    for (int i = 0; i < kGroup; ++i) ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], o);
+            }
+#pragma unroll
+            for (int i = 0; i < kGroup; ++i) {
+                if (t + i >= n) break;
+                store(y[i], ss[i]);
+                if (dst) dst += dstep;
+                if (kind && ++at == p.tile_size) {
+                    at = 0;
+                    ++tile;
+                    if (t + i + 1 < n) look_up();
+                }
+            }
+        }
+    }
+
+    if (!live || off != 0 || taps <= 1) return;
+    for (int j = 0; j < taps - 1; ++j) {               // rows older than the portion move up within the slot
+        const int t = plen - (taps - 1) + j;
+        float f[EPL];
+        if (t >= 0) ca_word_unpack<T, EPL>(ca_word_load<T, EPL>(in + (int64_t)t * stride), f);
+        else ca_load_floats<EPL>(st + (int64_t)(taps - 1 + t) * p.channels, f);
+        ca_word_store<float, EPL>(st + (int64_t)j * p.channels, f);
+    }
+}
+
+template <int LANES>
+static int ca_launch_words(const ConvAppendParams& p, cudaStream_t st) {
+    constexpr int kUnits = kCaThreads / LANES;
+    const int units = p.heads + (p.k_pool ? 2 * p.kv_heads : 0);
+    const unsigned grid = (unsigned)((int64_t)p.num_items * ((units + kUnits - 1) / kUnits));
+    if ((p.w ? p.taps : 1) <= 1) conv_rope_norm_append_words_kernel<LANES, 1><<<grid, kCaThreads, 0, st>>>(p);
+    else conv_rope_norm_append_words_kernel<LANES, 4><<<grid, kCaThreads, 0, st>>>(p);
+    PA_RETURN_LAUNCH_STATUS();
+}
+
 template <typename T, int EPL, int LANES>
 static int ca_launch_vec(const ConvAppendParams& p, cudaStream_t st) {
     const int units = p.heads + (p.k_pool ? 2 * p.kv_heads : 0);
@@ -553,6 +741,16 @@ static int ca_launch(const ConvAppendParams& p, cudaStream_t st) {
 template <typename T>
 static int ca_dispatch(const ConvAppendParams& p, cudaStream_t st) {
     const int n = p.k_pool && p.vdim > p.dim ? p.vdim : p.dim;
+    if constexpr (sizeof(T) == 2) {
+        // from as many units on as the form with a warp each does not hold at once (four warps a CTA, five CTAs an SM): up to there
+        // its items all run side by side, and it is the faster one (24 units an item, 64 items 10.8 and 11.4 us, 128 items 18.1 and
+        // 13.2, 512 items 53 and 38)
+        const int64_t units = (int64_t)p.num_items * (p.heads + (p.k_pool ? 2 * p.kv_heads : 0));
+        if (p.words == 8 && (p.w ? p.taps : 1) <= 4 && n <= 128 && units > 20 * device_info().sm_count) {
+            if (n <= 64) return ca_launch_words<8>(p, st);
+            return ca_launch_words<16>(p, st);
+        }
+    }
     if (p.words >= 4 && n <= 128) {
         if (n <= 32) return ca_launch_vec<T, 4, 8>(p, st);
         if (n <= 64) return ca_launch_vec<T, 4, 16>(p, st);
