@@ -649,6 +649,12 @@ int pa_moe_gate_up_act(const void* d_h, int64_t ldh, const void* d_w_gate_up, in
 int pa_moe_up(const void* d_h, int64_t ldh, const void* d_w_up, int width, int ff, int experts,
               const int32_t* d_order, const float* d_sel_w, int top, const int32_t* d_meta, int pairs, int act,
               void* d_act, int elem, pa_stream_t stream);
+/* pa_moe_gate_up_act (gated 1) or pa_moe_up (0) with scratch for the rows of the pairs in sorted order, which the products of large
+ * batches read faster than scattered ones: pa_moe_sorted_rows_bytes (0: the launch has no use for it; d_rows may be NULL). */
+size_t pa_moe_sorted_rows_bytes(int pairs, int experts, int width, int elem);
+int pa_moe_up_sorted(const void* d_h, int64_t ldh, const void* d_w, int gated, int width, int ff, int experts, const int32_t* d_order,
+                     const float* d_sel_w, int top, const int32_t* d_meta, int pairs, int act, void* d_act, void* d_rows,
+                     size_t rows_bytes, int elem, pa_stream_t stream);
 /* out_pairs[row * top + choice] = W_down[e] act[i] as float, weights [experts][width][ff]. */
 int pa_moe_down(const void* d_act, const void* d_w_down, int ff, int width, int experts, const int32_t* d_order,
                 const int32_t* d_meta, int pairs, float* d_out_pairs, int elem, pa_stream_t stream);

@@ -622,7 +622,8 @@ __global__ void __launch_bounds__(kSkWarps * 32) grouped_skinny_kernel(const bf1
 // moe_tc.cu: the tcgen05 form of the grouped products (PA_ERR_UNSUPPORTED: operands that stay on the kernels here)
 int grouped_tc_launch(int mode, const void* A, int64_t lda, const void* W, int K, int n_out, int experts, const int32_t* order,
                       const float* a_scale, int top, const int32_t* offsets, int pairs, int act, void* out, cudaStream_t st,
-                      int polls = 1 << 25);
+                      int polls = 1 << 25, void* rows = nullptr);
+bool grouped_tc_pairs_up(int pairs, int experts);
 
 static bool mma_ok(const void* A, int64_t lda, const void* W, int K) {
     return K % 8 == 0 && lda % 8 == 0 && (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0;
@@ -696,9 +697,9 @@ PA_API int pa_moe_sort(const int32_t* d_sel_id, int pairs, int experts, int32_t*
     PA_RETURN_LAUNCH_STATUS();
 }
 
-PA_API int pa_moe_gate_up_act(const void* d_h, int64_t ldh, const void* d_w_gate_up, int width, int ff, int experts,
-                              const int32_t* d_order, const float* d_sel_w, int top, const int32_t* d_meta, int pairs,
-                              int act, void* d_act, int elem, pa_stream_t stream) {
+static int moe_gate_up(const void* d_h, int64_t ldh, const void* d_w_gate_up, int width, int ff, int experts, const int32_t* d_order,
+                       const float* d_sel_w, int top, const int32_t* d_meta, int pairs, int act, void* d_act, void* d_rows, int elem,
+                       pa_stream_t stream) {
     PA_CHECK_ARG(d_h && d_w_gate_up && d_order && d_meta && d_act && width > 0 && ff > 0 && experts > 0 && top > 0);
     PA_CHECK_ARG(act >= 0 && act <= 2);
     if (pairs <= 0) return PA_OK;
@@ -712,7 +713,7 @@ PA_API int pa_moe_gate_up_act(const void* d_h, int64_t ldh, const void* d_w_gate
         PA_RETURN_LAUNCH_STATUS();
     }
     if (elem == 2 && mma_ok(d_h, ldh, d_w_gate_up, width)) {
-        const int st = grouped_tc_launch(0, d_h, ldh, d_w_gate_up, width, ff, experts, d_order, d_sel_w, top, d_meta, pairs, act, d_act, as_stream(stream));
+        const int st = grouped_tc_launch(0, d_h, ldh, d_w_gate_up, width, ff, experts, d_order, d_sel_w, top, d_meta, pairs, act, d_act, as_stream(stream), 1 << 25, d_rows);
         if (st != PA_ERR_UNSUPPORTED) return st;
         grouped_mma_kernel<0><<<grid, 128, 0, as_stream(stream)>>>(
             static_cast<const bf16_t*>(d_h), ldh, static_cast<const bf16_t*>(d_w_gate_up), width, ff, d_order, d_sel_w, top,
@@ -725,6 +726,12 @@ PA_API int pa_moe_gate_up_act(const void* d_h, int64_t ldh, const void* d_w_gate
     PA_RETURN_LAUNCH_STATUS();
 }
 
+PA_API int pa_moe_gate_up_act(const void* d_h, int64_t ldh, const void* d_w_gate_up, int width, int ff, int experts,
+                              const int32_t* d_order, const float* d_sel_w, int top, const int32_t* d_meta, int pairs,
+                              int act, void* d_act, int elem, pa_stream_t stream) {
+    return moe_gate_up(d_h, ldh, d_w_gate_up, width, ff, experts, d_order, d_sel_w, top, d_meta, pairs, act, d_act, nullptr, elem, stream);
+}
+
 PA_API int pa_moe_gate_up(const void* d_h, int64_t ldh, const void* d_w_gate_up, int width, int ff, int experts,
                           const int32_t* d_order, const float* d_sel_w, int top, const int32_t* d_meta, int pairs,
                           void* d_act, int elem, pa_stream_t stream) {
@@ -732,9 +739,9 @@ PA_API int pa_moe_gate_up(const void* d_h, int64_t ldh, const void* d_w_gate_up,
                               stream);
 }
 
-PA_API int pa_moe_up(const void* d_h, int64_t ldh, const void* d_w_up, int width, int ff, int experts,
-                     const int32_t* d_order, const float* d_sel_w, int top, const int32_t* d_meta, int pairs, int act,
-                     void* d_act, int elem, pa_stream_t stream) {
+static int moe_up(const void* d_h, int64_t ldh, const void* d_w_up, int width, int ff, int experts, const int32_t* d_order,
+                  const float* d_sel_w, int top, const int32_t* d_meta, int pairs, int act, void* d_act, void* d_rows, int elem,
+                  pa_stream_t stream) {
     PA_CHECK_ARG(d_h && d_w_up && d_order && d_meta && d_act && width > 0 && ff > 0 && experts > 0 && top > 0);
     PA_CHECK_ARG(act >= 0 && act <= 2);
     if (pairs <= 0) return PA_OK;
@@ -747,7 +754,7 @@ PA_API int pa_moe_up(const void* d_h, int64_t ldh, const void* d_w_up, int width
         PA_RETURN_LAUNCH_STATUS();
     }
     if (elem == 2 && mma_ok(d_h, ldh, d_w_up, width)) {
-        const int st = grouped_tc_launch(2, d_h, ldh, d_w_up, width, ff, experts, d_order, d_sel_w, top, d_meta, pairs, act, d_act, as_stream(stream));
+        const int st = grouped_tc_launch(2, d_h, ldh, d_w_up, width, ff, experts, d_order, d_sel_w, top, d_meta, pairs, act, d_act, as_stream(stream), 1 << 25, d_rows);
         if (st != PA_ERR_UNSUPPORTED) return st;
         grouped_mma_kernel<2><<<dim3(nt, (unsigned)((ff + 127) / 128)), 128, 0, as_stream(stream)>>>(
             static_cast<const bf16_t*>(d_h), ldh, static_cast<const bf16_t*>(d_w_up), width, ff, d_order, d_sel_w, top, tiles,
@@ -758,6 +765,25 @@ PA_API int pa_moe_up(const void* d_h, int64_t ldh, const void* d_w_up, int width
                                static_cast<const T*>(d_h), ldh, static_cast<const T*>(d_w_up), width, ff, d_order, d_sel_w, top,
                                tiles, static_cast<T*>(d_act), nullptr, act));
     PA_RETURN_LAUNCH_STATUS();
+}
+
+PA_API int pa_moe_up(const void* d_h, int64_t ldh, const void* d_w_up, int width, int ff, int experts,
+                     const int32_t* d_order, const float* d_sel_w, int top, const int32_t* d_meta, int pairs, int act,
+                     void* d_act, int elem, pa_stream_t stream) {
+    return moe_up(d_h, ldh, d_w_up, width, ff, experts, d_order, d_sel_w, top, d_meta, pairs, act, d_act, nullptr, elem, stream);
+}
+
+PA_API size_t pa_moe_sorted_rows_bytes(int pairs, int experts, int width, int elem) {
+    return elem == 2 && pairs > 0 && experts > 0 && width > 0 && !skinny_ok(pairs, experts) && grouped_tc_pairs_up(pairs, experts)
+               ? (size_t)pairs * width * 2 : 0;
+}
+
+PA_API int pa_moe_up_sorted(const void* d_h, int64_t ldh, const void* d_w, int gated, int width, int ff, int experts, const int32_t* d_order,
+                            const float* d_sel_w, int top, const int32_t* d_meta, int pairs, int act, void* d_act, void* d_rows,
+                            size_t rows_bytes, int elem, pa_stream_t stream) {
+    PA_CHECK_ARG(gated == 0 || gated == 1);
+    if (d_rows && rows_bytes < pa_moe_sorted_rows_bytes(pairs, experts, width, elem)) return PA_ERR_WORKSPACE;
+    return (gated ? moe_gate_up : moe_up)(d_h, ldh, d_w, width, ff, experts, d_order, d_sel_w, top, d_meta, pairs, act, d_act, d_rows, elem, stream);
 }
 
 PA_API int pa_moe_down(const void* d_act, const void* d_w_down, int ff, int width, int experts, const int32_t* d_order,

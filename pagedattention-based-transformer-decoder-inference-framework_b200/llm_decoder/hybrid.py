@@ -1171,9 +1171,11 @@ class MoEFF:
         _chk(lib.pa_moe_sort(sel_id.data_ptr(), pairs, self.experts, order.data_ptr(), meta.data_ptr(), s), "pa_moe_sort")
         act = c.empty(pairs, self.ff)
         in_w = sel_w.data_ptr() if self.weight_on == "input" else None
-        _chk((lib.pa_moe_gate_up_act if self.gated else lib.pa_moe_up)(
-            h.data_ptr(), h.stride(0), self.w_gate_up.data_ptr(), wdt, self.ff, self.experts, order.data_ptr(), in_w,
-            self.top, meta.data_ptr(), pairs, self.act, act.data_ptr(), c.elem, s), "pa_moe_gate_up_act / pa_moe_up")
+        nb = lib.pa_moe_sorted_rows_bytes(pairs, self.experts, wdt, c.elem)
+        rows = c.empty(nb, dtype=torch.uint8) if nb else None
+        _chk(lib.pa_moe_up_sorted(h.data_ptr(), h.stride(0), self.w_gate_up.data_ptr(), 1 if self.gated else 0, wdt, self.ff,
+                                  self.experts, order.data_ptr(), in_w, self.top, meta.data_ptr(), pairs, self.act, act.data_ptr(),
+                                  _cabi.ptr(rows), nb, c.elem, s), "pa_moe_up_sorted")
         routed = c.empty(pairs, wdt, **f32)
         _chk(lib.pa_moe_down(act.data_ptr(), self.w_down.data_ptr(), self.ff, wdt, self.experts, order.data_ptr(),
                              meta.data_ptr(), pairs, routed.data_ptr(), c.elem, s), "pa_moe_down")

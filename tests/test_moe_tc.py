@@ -14,7 +14,9 @@ BF = torch.bfloat16
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("rows,experts,top,width,ff", [(700, 3, 2, 192, 264), (257, 2, 1, 64, 520), (1300, 20, 2, 136, 128), (129, 1, 1, 72, 8)])
+@pytest.mark.parametrize("rows,experts,top,width,ff", [(700, 3, 2, 192, 264), (257, 2, 1, 64, 520), (1300, 20, 2, 136, 128), (129, 1, 1, 72, 8),
+                                                        # from 6144 pairs and 256 an expert on also by pairs of CTAs, tiles of 256
+                                                        (6144, 1, 1, 72, 8), (3300, 3, 2, 136, 264), (3205, 24, 2, 320, 136)])
 @pytest.mark.parametrize("act,gated,weighted", [(0, True, False), (1, True, True), (2, False, False)])
 def test_grouped_products(rows, experts, top, width, ff, act, gated, weighted):
     from llm_decoder import _cabi
@@ -40,6 +42,14 @@ def test_grouped_products(rows, experts, top, width, ff, act, gated, weighted):
     fn = lib.pa_moe_gate_up_act if gated else lib.pa_moe_up
     _cabi.check(fn(hd.data_ptr(), width, wud.data_ptr(), width, ff, experts, order.data_ptr(), swd.data_ptr() if weighted else None, top,
                    meta.data_ptr(), pairs, act, mid.data_ptr(), 2, s()), "up")
+    nb = lib.pa_moe_sorted_rows_bytes(pairs, experts, width, 2)
+    assert (nb > 0) == (pairs >= 6144)
+    if nb:                      # the same through sorted rows, by pairs of CTAs: the same sums
+        rows_ws, mid2 = torch.empty(nb, dtype=torch.uint8, device=dev), torch.full_like(mid, float("nan"))
+        _cabi.check(lib.pa_moe_up_sorted(hd.data_ptr(), width, wud.data_ptr(), 1 if gated else 0, width, ff, experts, order.data_ptr(),
+                                         swd.data_ptr() if weighted else None, top, meta.data_ptr(), pairs, act, mid2.data_ptr(),
+                                         rows_ws.data_ptr(), nb, 2, s()), "sorted")
+        assert torch.equal(mid, mid2)
     _cabi.check(lib.pa_moe_down(mid.data_ptr(), wdd.data_ptr(), ff, width, experts, order.data_ptr(), meta.data_ptr(), pairs, out.data_ptr(), 2,
                                 s()), "down")
     o = order.long().cpu()
@@ -58,3 +68,27 @@ def test_grouped_products(rows, experts, top, width, ff, act, gated, weighted):
     assert ((out.double().cpu()[o] - want).abs() <= 1e-5 * bound + 1e-30).all()
     n = ctypes.c_int(-1)
     assert lib.pa_moe_tc_errors(ctypes.byref(n)) == 0 and n.value == 0
+
+
+@pytest.mark.gpu
+def test_waits_of_a_pair_of_ctas():
+    """Pairs of CTAs whose waits run out leave NaN and are counted, and the next launch is whole."""
+    from llm_decoder import _cabi
+    lib, dev, s = _cabi.lib(), torch.device("cuda"), _cabi.stream
+    g = torch.Generator().manual_seed(5)
+    pairs, experts, K, n_out = 6200, 2, 136, 264
+    a, w = torch.randn(pairs, K, generator=g).to(BF).to(dev), torch.randn(experts, n_out, K, generator=g).to(BF).to(dev)
+    ids = torch.randint(0, experts, (pairs,), generator=g, dtype=torch.int32).to(dev)
+    order = torch.empty(pairs, dtype=torch.int32, device=dev)
+    meta = torch.empty(lib.pa_moe_meta_ints(pairs, experts), dtype=torch.int32, device=dev)
+    _cabi.check(lib.pa_moe_sort(ids.data_ptr(), pairs, experts, order.data_ptr(), meta.data_ptr(), s()), "sort")
+    out, counts = [], []
+    for polls in (1 << 25, 0, 1 << 25):
+        o, n = torch.zeros(pairs, n_out, device=dev), ctypes.c_int()
+        assert lib.pa_moe_grouped_polls(1, a.data_ptr(), K, w.data_ptr(), K, n_out, experts, order.data_ptr(), None, 1, meta.data_ptr(), pairs, 0,
+                                        o.data_ptr(), polls, s()) == 0
+        assert lib.pa_moe_tc_errors(ctypes.byref(n)) == 0
+        out.append(o)
+        counts.append(n.value)
+    assert counts[1] > counts[0] and counts[2] == counts[1]
+    assert bool(torch.isnan(out[1]).all()) and torch.equal(out[0], out[2]) and not bool(torch.isnan(out[0]).any())
