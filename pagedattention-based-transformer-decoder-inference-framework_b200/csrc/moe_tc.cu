@@ -441,10 +441,11 @@ static int launch(const CUtensorMap& tmA, const CUtensorMap& tmW, const Args& a,
     return (int)cudaLaunchKernelEx(&cfg, grouped_tc_kernel<MODE, CTAS>, tmA, tmW, a);
 }
 
-// the token rows of the pairs in sorted order, 16 bytes a thread
-__global__ void __launch_bounds__(256) sorted_rows_kernel(const uint4* __restrict__ A, int64_t lda, const int32_t* __restrict__ order, int top, int pairs,
-                                                          int words, uint4* __restrict__ out) {
-    const int64_t i0 = (int64_t)blockIdx.x * 256 + threadIdx.x, n = (int64_t)pairs * words, step = (int64_t)gridDim.x * 256;
+// The token rows of the pairs in sorted order, 16 bytes a thread.  *count: how many pairs the sort gave a place; a pair whose id belongs
+// to no expert (an identity output) has none, so order and out end there and may hold anything behind.
+__global__ void __launch_bounds__(256) sorted_rows_kernel(const uint4* __restrict__ A, int64_t lda, const int32_t* __restrict__ order, int top,
+                                                          const int32_t* __restrict__ count, int words, uint4* __restrict__ out) {
+    const int64_t i0 = (int64_t)blockIdx.x * 256 + threadIdx.x, n = (int64_t)__ldg(count) * words, step = (int64_t)gridDim.x * 256;
     for (int64_t i = i0; i < n; i += 4 * step) {
         uint4 v[4];
 #pragma unroll
@@ -481,7 +482,7 @@ int grouped_tc_launch(int mode, const void* A, int64_t lda, const void* W, int K
     if (mode != 1 && pair) {
         if (!make_bf16_map(&tmA, rows, pairs, K, K, BM)) return PA_ERR_UNSUPPORTED;
         const int64_t blocks = ((int64_t)pairs * (K / 8) + 1023) / 1024, most = 8 * device_info().sm_count;
-        sorted_rows_kernel<<<(unsigned)(blocks < most ? blocks : most), 256, 0, st>>>(static_cast<const uint4*>(A), lda / 8, order, top, pairs, K / 8,
+        sorted_rows_kernel<<<(unsigned)(blocks < most ? blocks : most), 256, 0, st>>>(static_cast<const uint4*>(A), lda / 8, order, top, offsets + experts, K / 8,
                                                                                       static_cast<uint4*>(rows));
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return (int)e;

@@ -92,3 +92,33 @@ def test_waits_of_a_pair_of_ctas():
         counts.append(n.value)
     assert counts[1] > counts[0] and counts[2] == counts[1]
     assert bool(torch.isnan(out[1]).all()) and torch.equal(out[0], out[2]) and not bool(torch.isnan(out[0]).any())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("gated", [True, False])
+def test_pairs_without_an_expert(gated):
+    """Ids of no expert (a router's identity outputs) have no place in the sorted order: the copy of the rows ends where the sort did."""
+    from llm_decoder import _cabi
+    lib, dev, s = _cabi.lib(), torch.device("cuda"), _cabi.stream
+    g = torch.Generator().manual_seed(9)
+    rows, top, experts, width, ff = 3600, 2, 4, 136, 264
+    pairs = rows * top
+    ids = torch.randint(0, experts + 2, (pairs,), generator=g, dtype=torch.int32).to(dev)
+    order = torch.zeros(pairs, dtype=torch.int32, device=dev)           # its end, which the sort leaves alone, names a row that there is
+    meta = torch.empty(lib.pa_moe_meta_ints(pairs, experts), dtype=torch.int32, device=dev)
+    _cabi.check(lib.pa_moe_sort(ids.data_ptr(), pairs, experts, order.data_ptr(), meta.data_ptr(), s()), "sort")
+    count = int((ids < experts).sum())
+    assert int(meta[experts]) == count < pairs
+    h = torch.randn(rows, width, generator=g).to(BF).to(dev)
+    w = (torch.randn(experts, (2 if gated else 1) * ff, width, generator=g) / width ** 0.5).to(BF).to(dev)
+    nb = lib.pa_moe_sorted_rows_bytes(pairs, experts, width, 2)
+    assert nb == pairs * width * 2
+    scratch = torch.full((pairs, width), 7.5, dtype=BF, device=dev)
+    out = []
+    for ws in (scratch, None):
+        o = torch.full((pairs, ff), 3.25, dtype=BF, device=dev)
+        _cabi.check(lib.pa_moe_up_sorted(h.data_ptr(), width, w.data_ptr(), 1 if gated else 0, width, ff, experts, order.data_ptr(), None, top,
+                                         meta.data_ptr(), pairs, 1, o.data_ptr(), _cabi.ptr(ws), nb if ws is not None else 0, 2, s()), "sorted")
+        out.append(o)
+    assert bool((scratch[count:] == 7.5).all()) and torch.equal(scratch[:count], h[order[:count].long() // top])
+    assert torch.equal(out[0], out[1]) and bool((out[0][count:] == 3.25).all())
