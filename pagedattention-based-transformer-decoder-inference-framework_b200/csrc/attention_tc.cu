@@ -60,12 +60,13 @@ __host__ __device__ constexpr int q_bytes(int kb) { return kb * QT * 128; }
 __host__ __device__ constexpr int stage_bytes(int kb, int vb) { return (kb + vb) * KT * 128; }
 __host__ __device__ constexpr int stages_for(int kb, int nq) { return nq == 2 || kb == 3 ? 3 : 2; }
 __host__ __device__ constexpr int threads_for(int nq) { return (5 * nq + 1) * 32; }
-// query buffers: two where they fit, so that the next item's queries come under the current one's products
-__host__ __device__ constexpr int q_bufs(int kb, int nq) { return nq == 2 && kb < 3 ? 2 : 1; }
+// Query buffers: two where they fit, so that the next item's queries come under the current one's products.  A CTA with a table of
+// distance biases has no next item, and the table (up to 40 KB) takes the second one's place.
+__host__ __device__ constexpr int q_bufs(int kb, int nq, bool table) { return nq == 2 && kb < 3 && !table ? 2 : 1; }
 // barriers: kv_full, kv_empty [stage]; per query tile s_full, p_full, o_full [2], q_ready, q_free [2]
 __host__ __device__ constexpr int nbar_for(int kb, int nq) { return 2 * stages_for(kb, nq) + 10 * nq; }
-constexpr size_t smem_for(int kb, int vb, int nq) {
-    return (size_t)nq * q_bufs(kb, nq) * q_bytes(kb) + stages_for(kb, nq) * stage_bytes(kb, vb) + nbar_for(kb, nq) * 8 + 8 + 4 + 4 * 4 + 1024;
+constexpr size_t smem_for(int kb, int vb, int nq, int qb) {
+    return (size_t)nq * qb * q_bytes(kb) + stages_for(kb, nq) * stage_bytes(kb, vb) + nbar_for(kb, nq) * 8 + 8 + 4 + 4 * 4 + 1024;
 }
 
 // 32 bfloat16 numbers: two 32-byte sectors, each by one store where the row's address allows it
@@ -143,13 +144,13 @@ struct Walk {
 };
 
 // KB / VB: blocks of 64 columns of a key / a value; MOD: the score has more than a factor (soft cap or distance bias)
-// QD: columns of a query (the last block may be part of one)
-template <int KB, int VB, int NQ, bool DENSE, bool MOD, int QD>
+// QD: columns of a query (the last block may be part of one); QB: query buffers
+template <int KB, int VB, int NQ, bool DENSE, bool MOD, int QD, int QB>
 __global__ void __launch_bounds__(threads_for(NQ), NQ == 1 && KB < 3 ? 2 : 1)
 attention_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmK2,
                     const __grid_constant__ CUtensorMap tmV, const Args a) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    constexpr int ST = stages_for(KB, NQ), NBAR = nbar_for(KB, NQ), QB = q_bufs(KB, NQ), TMEM_COLS = NQ * 256, D = VB * 64;
+    constexpr int ST = stages_for(KB, NQ), NBAR = nbar_for(KB, NQ), TMEM_COLS = NQ * 256, D = VB * 64;
     constexpr int Q_BYTES = q_bytes(KB), K_BYTES = KB * KT * 128, STAGE = stage_bytes(KB, VB);
     constexpr int W_MMA = 4 * NQ, W_PROD = 5 * NQ;
     constexpr float kLog2e = 1.4426950408889634f;
@@ -599,13 +600,14 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     }
 }
 
-template <int KB, int VB, int NQ, bool DENSE, bool MOD, int QD = KB * 64>
-static int launch(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& k2, const CUtensorMap& v, const Args& a, int ntiles, size_t extra,
-                  cudaStream_t st) {
-    const size_t smem = smem_for(KB, VB, NQ) + extra;
+template <int KB, int VB, int NQ, bool DENSE, bool MOD, int QD, int QB>
+static int launch_bufs(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& k2, const CUtensorMap& v, const Args& a, int ntiles,
+                       size_t extra, cudaStream_t st) {
+    const size_t smem = smem_for(KB, VB, NQ, QB) + extra;
+    if (smem > (size_t)device_info().max_smem_optin) return PA_ERR_UNSUPPORTED;
     const int64_t items = (int64_t)ntiles * a.p.num_kv_heads * a.hchunks;
     if (items > 0x7fffffff) return PA_ERR_INVALID_ARG;
-    auto kern = attention_tc_kernel<KB, VB, NQ, DENSE, MOD, QD>;
+    auto kern = attention_tc_kernel<KB, VB, NQ, DENSE, MOD, QD, QB>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     Args b = a;
@@ -615,6 +617,13 @@ static int launch(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap&
     const int64_t ctas = a.p.bias_kind == 2 || items < most ? items : most;
     kern<<<(unsigned)ctas, threads_for(NQ), smem, st>>>(q, k, k2, v, b);
     PA_RETURN_LAUNCH_STATUS();
+}
+
+template <int KB, int VB, int NQ, bool DENSE, bool MOD, int QD = KB * 64>
+static int launch(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& k2, const CUtensorMap& v, const Args& a, int ntiles, size_t extra,
+                  cudaStream_t st) {
+    if (MOD && a.p.bias_kind == 2) return launch_bufs<KB, VB, NQ, DENSE, MOD, QD, q_bufs(KB, NQ, MOD)>(q, k, k2, v, a, ntiles, extra, st);
+    return launch_bufs<KB, VB, NQ, DENSE, MOD, QD, q_bufs(KB, NQ, false)>(q, k, k2, v, a, ntiles, extra, st);
 }
 
 // Rows of a CTA: tokens per head block and heads.  Four (two) heads of a kv head over 64 tokens where there are that many, so

@@ -30,6 +30,18 @@ def _no_wait_ran_out(lib):
 @pytest.mark.parametrize("mask,size,keep,form", [("causal", 0, 0, "plain"), ("causal", 0, 0, "sink"), ("window", 37, 0, "bucket"),
                                                  ("window", 100, 9, "turned"), ("chunk", 50, 0, "slope")])
 def test_paged_portions(heads, kv_heads, dim, vdim, mask, size, keep, form):
+    _paged_portions(heads, kv_heads, dim, vdim, mask, size, keep, form)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads,kv_heads,bias_len", [(4, 1, 114), (4, 1, 600), (4, 1, 2560), (2, 1, 227), (2, 1, 600), (2, 1, 5120), (1, 1, 454),
+                                                     (1, 1, 10240)])
+def test_long_bias_tables(heads, kv_heads, bias_len):
+    """Tables beside the largest stages: longer than what two buffers of query rows leave, up to the 40 KB that are taken."""
+    _paged_portions(heads, kv_heads, 128, 128, "window", 200, 0, "bucket", bias_len)
+
+
+def _paged_portions(heads, kv_heads, dim, vdim, mask, size, keep, form, bias_len=23):
     from llm_decoder import _cabi
     from llm_decoder.hybrid import MASK_KIND
     from llm_decoder.seq_state import SequenceStateCache
@@ -61,7 +73,7 @@ def test_paged_portions(heads, kv_heads, dim, vdim, mask, size, keep, form):
     cap = 6.0 if form == "bucket" else 0.0
     bias, bias_kind = None, 0
     if form == "bucket":
-        bias, bias_kind = torch.randn(23, heads, generator=g), 2
+        bias, bias_kind = torch.randn(bias_len, heads, generator=g), 2
     elif form == "slope":
         bias, bias_kind = torch.tensor([2.0 ** (-8.0 * (h + 1) / heads) for h in range(heads)]), 1
     rows = batch.rows
@@ -81,7 +93,7 @@ def test_paged_portions(heads, kv_heads, dim, vdim, mask, size, keep, form):
             s = Q[i].double()[:, h * dim:(h + 1) * dim] @ k.T * scale * (float(temp[h]) if temp is not None else 1.0)
             s = cap * torch.tanh(s / cap) if cap else s
             if bias_kind == 2:
-                s = s + bias.double()[dist.clamp(0, 22), h]
+                s = s + bias.double()[dist.clamp(0, bias_len - 1), h]
             elif bias_kind == 1:
                 s = s - float(bias[h]) * dist
             s = s.masked_fill(~vis, -float("inf"))
@@ -103,7 +115,7 @@ def test_paged_portions(heads, kv_heads, dim, vdim, mask, size, keep, form):
         rc = lib.pa_masked_attention_gated(
             proj.data_ptr(), proj.stride(0), 0, kv.key_buffer_.data_ptr(), kv.value_buffer_.data_ptr(), table.data_ptr(), pt.num_beams_,
             pt.num_heads_, pt.num_tiles_, kv.total_pages_, kv.tile_size_, tiles.data_ptr(), ntiles, heads, dim, vdim, scale, cap,
-            MASK_KIND[mask], size, keep, bias_kind, _cabi.ptr(keepalive[0]), 23 if bias_kind == 2 else 0, _cabi.ptr(keepalive[1]),
+            MASK_KIND[mask], size, keep, bias_kind, _cabi.ptr(keepalive[0]), bias_len if bias_kind == 2 else 0, _cabi.ptr(keepalive[1]),
             _cabi.ptr(keepalive[2]), _cabi.ptr(keepalive[3]), None, 0, None, None, 0, 0, out.data_ptr(), 2, kind, _cabi.stream())
         assert rc == 0, rc
         _close(out, want.reshape(rows, -1), max(v.abs().max().item() for v in V) * (1.42 if turn is not None else 1.0))
