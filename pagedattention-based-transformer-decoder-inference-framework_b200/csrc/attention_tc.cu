@@ -298,6 +298,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                     if (QB == 1 && i == 0) load_queries(it);
                     if (QB == 2 && has_next && i == min(ST - 1, it.n_tiles - 1)) load_queries(nxt);
                 }
+                if (QB == 2 && has_next && ok && it.n_tiles == 0) load_queries(nxt);     // an item of no tokens has no keys to wait behind
                 it = nxt;
                 more = has_next;
             }

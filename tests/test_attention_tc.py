@@ -41,31 +41,53 @@ def test_long_bias_tables(heads, kv_heads, bias_len):
     _paged_portions(heads, kv_heads, 128, 128, "window", 200, 0, "bucket", bias_len)
 
 
-def _paged_portions(heads, kv_heads, dim, vdim, mask, size, keep, form, bias_len=23):
+# enough portions that a CTA has several work items in turn (at least 444 with two query tiles, 888 with one), of one key tile and of
+# many, whole and ragged
+MANY_NEW = [[64, 17, 200, 128, 65, 256, 33, 64, 192, 16][i % 10] + (i % 7 == 3) for i in range(90)]
+MANY_CTX = [[0, 70, 0, 300, 1, 0, 512, 0, 63, 0, 190][i % 11] for i in range(90)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form,mask,size", [("plain", "causal", 0), ("slope", "window", 90)])
+def test_work_items_without_tokens(form, mask, size):
+    """Items of no tokens among the others, also first and next to each other: nothing to do, and the walk goes on."""
+    def with_empty(tiles):
+        out = []
+        for i, t in enumerate(tiles):
+            if i % 5 == 0:
+                out += [[t[0], 0, t[2], t[3]]] * (1 + i % 3)
+            out.append(t)
+        return out
+    _paged_portions(10, 2, 128, 128, mask, size, 0, form, ctx=MANY_CTX, new=MANY_NEW, change=with_empty)
+
+
+def _paged_portions(heads, kv_heads, dim, vdim, mask, size, keep, form, bias_len=23, ctx=CTX, new=NEW, change=None):
+    """change: the list of work items (first row, tokens, slot, first position) -> the one that is launched."""
     from llm_decoder import _cabi
     from llm_decoder.hybrid import MASK_KIND
     from llm_decoder.seq_state import SequenceStateCache
     lib, dev = _cabi.lib(), torch.device("cuda")
     g = torch.Generator().manual_seed(heads * 7 + dim + size)
-    per, scale, n = heads // kv_heads, dim ** -0.5 * 2.0, len(NEW)
-    states = SequenceStateCache(n, 4096, 32, dev)
+    per, scale, n = heads // kv_heads, dim ** -0.5 * 2.0, len(new)
+    states = SequenceStateCache(n, 4096 if n == len(NEW) else sum(ctx) + sum(new) + 32 * n, 32, dev)
     kv = states.add_kv_layer(kv_heads, dim, vdim, "bf16")
     kv.key_buffer_.fill_(float("nan"))
     kv.value_buffer_.fill_(float("nan"))
     slots = [states.alloc() for _ in range(n)]
-    for r in range(12):                                     # growth in turns, so that the sequences' pages interleave
-        for i in (2, 0, 3, 1, 6, 5, 4):
-            if CTX[i] > 16 * r:
-                states.extend(slots[i], min(16, CTX[i] - 16 * r))
-    K = [torch.randn(c + m, kv_heads * dim, generator=g).to(BF) for c, m in zip(CTX, NEW)]
-    V = [torch.randn(c + m, kv_heads * vdim, generator=g).to(BF) for c, m in zip(CTX, NEW)]
-    Q = [torch.randn(m, heads * dim, generator=g).to(BF) for m in NEW]
+    turns = [2, 0, 3, 1, 6, 5, 4] + list(range(7, n))
+    for r in range(max(ctx) // 16 + 1):                     # growth in turns, so that the sequences' pages interleave
+        for i in turns:
+            if ctx[i] > 16 * r:
+                states.extend(slots[i], min(16, ctx[i] - 16 * r))
+    K = [torch.randn(c + m, kv_heads * dim, generator=g).to(BF) for c, m in zip(ctx, new)]
+    V = [torch.randn(c + m, kv_heads * vdim, generator=g).to(BF) for c, m in zip(ctx, new)]
+    Q = [torch.randn(m, heads * dim, generator=g).to(BF) for m in new]
     for i in range(n):
-        if CTX[i]:
-            kv.append_rows(torch.cat([K[i][:CTX[i]], V[i][:CTX[i]]], 1).to(dev), 0, kv_heads * dim,
-                           torch.full((CTX[i],), slots[i], dtype=torch.int32, device=dev), torch.arange(CTX[i], dtype=torch.int32, device=dev))
-    batch = states.make_batch([(slots[i], [0] * NEW[i]) for i in range(n)])
-    proj = torch.cat([torch.cat([Q[i], K[i][CTX[i]:], V[i][CTX[i]:]], 1) for i in range(n)], 0).to(dev)
+        if ctx[i]:
+            kv.append_rows(torch.cat([K[i][:ctx[i]], V[i][:ctx[i]]], 1).to(dev), 0, kv_heads * dim,
+                           torch.full((ctx[i],), slots[i], dtype=torch.int32, device=dev), torch.arange(ctx[i], dtype=torch.int32, device=dev))
+    batch = states.make_batch([(slots[i], [0] * new[i]) for i in range(n)])
+    proj = torch.cat([torch.cat([Q[i], K[i][ctx[i]:], V[i][ctx[i]:]], 1) for i in range(n)], 0).to(dev)
     kv.append_rows(proj, heads * dim, heads * dim + kv_heads * dim, batch.row_slot, batch.row_pos)
 
     temp = torch.rand(heads, generator=g) * 2 - 0.5 if form == "sink" else None     # one negative factor among them
@@ -81,7 +103,7 @@ def _paged_portions(heads, kv_heads, dim, vdim, mask, size, keep, form, bias_len
     turn = torch.stack([torch.cos(ang), torch.sin(ang)], -1) if form == "turned" else None
     want, r0 = torch.zeros(rows, heads, vdim, dtype=torch.float64), 0
     for i in range(n):
-        pos, j = torch.arange(CTX[i], CTX[i] + NEW[i])[:, None], torch.arange(CTX[i] + NEW[i])[None]
+        pos, j = torch.arange(ctx[i], ctx[i] + new[i])[:, None], torch.arange(ctx[i] + new[i])[None]
         dist = pos - j
         vis = dist >= 0
         if mask == "window":
@@ -98,9 +120,9 @@ def _paged_portions(heads, kv_heads, dim, vdim, mask, size, keep, form, bias_len
                 s = s - float(bias[h]) * dist
             s = s.masked_fill(~vis, -float("inf"))
             if sink is not None:
-                s = torch.cat([s, sink[h].double().expand(NEW[i], 1)], 1)
-            want[r0:r0 + NEW[i], h] = torch.softmax(s, -1)[:, :k.shape[0]] @ v
-        r0 += NEW[i]
+                s = torch.cat([s, sink[h].double().expand(new[i], 1)], 1)
+            want[r0:r0 + new[i], h] = torch.softmax(s, -1)[:, :k.shape[0]] @ v
+        r0 += new[i]
     if turn is not None:
         u, w = want[..., 0::2].clone(), want[..., 1::2].clone()
         c, s = turn.double()[:, None, :, 0], turn.double()[:, None, :, 1]
@@ -111,6 +133,9 @@ def _paged_portions(heads, kv_heads, dim, vdim, mask, size, keep, form, bias_len
     for q_tiles, kind in ((2, 4), (1, 5)):
         tokens = lib.pa_masked_attention_tc_tile_tokens(heads, kv_heads, dim, vdim, 2, q_tiles)
         tiles, ntiles, _longest = batch.query_tiles(1, tokens, 16)[2]
+        if change:
+            tiles = torch.tensor(change(tiles.tolist()), dtype=torch.int32, device=dev)
+            ntiles = len(tiles)
         out = torch.full((rows, heads * vdim), float("nan"), dtype=BF, device=dev)
         rc = lib.pa_masked_attention_gated(
             proj.data_ptr(), proj.stride(0), 0, kv.key_buffer_.data_ptr(), kv.value_buffer_.data_ptr(), table.data_ptr(), pt.num_beams_,
