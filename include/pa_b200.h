@@ -913,6 +913,11 @@ int pa_moe_tc_errors(int* host_count);
 int pa_moe_grouped_polls(int mode, const void* d_a, int64_t lda, const void* d_w, int K, int n_out, int experts, const int32_t* d_order,
                          const float* d_a_scale, int top, const int32_t* d_meta, int pairs, int act, void* d_out, int polls,
                          pa_stream_t stream);
+/* the same with scratch for the sorted rows (pa_moe_sorted_rows_bytes; NULL: none) and limits of their own for the waits of the epilogue
+ * warps, in the first and in the second CTA of a pair (one CTA a tile: the first).  A row is whole or NaN. */
+int pa_moe_grouped_waits(int mode, const void* d_a, int64_t lda, const void* d_w, int K, int n_out, int experts, const int32_t* d_order,
+                         const float* d_a_scale, int top, const int32_t* d_meta, int pairs, int act, void* d_out, void* d_rows,
+                         size_t rows_bytes, int polls, int first_polls, int second_polls, pa_stream_t stream);
 
 /* ---- decoded tokens with the keys cut into equal shares (masked_decode.cu) ----------------------------------------------
  * pa_masked_decode: pa_masked_attention_gated for tiles of ONE token, bfloat16 softmax attention: the 16-key units of all

@@ -622,7 +622,7 @@ __global__ void __launch_bounds__(kSkWarps * 32) grouped_skinny_kernel(const bf1
 // moe_tc.cu: the tcgen05 form of the grouped products (PA_ERR_UNSUPPORTED: operands that stay on the kernels here)
 int grouped_tc_launch(int mode, const void* A, int64_t lda, const void* W, int K, int n_out, int experts, const int32_t* order,
                       const float* a_scale, int top, const int32_t* offsets, int pairs, int act, void* out, cudaStream_t st,
-                      int polls = 1 << 25, void* rows = nullptr);
+                      void* rows = nullptr, int polls = 1 << 25, int first_polls = 1 << 25, int second_polls = 1 << 25);
 bool grouped_tc_pairs_up(int pairs, int experts);
 
 static bool mma_ok(const void* A, int64_t lda, const void* W, int K) {
@@ -713,7 +713,7 @@ static int moe_gate_up(const void* d_h, int64_t ldh, const void* d_w_gate_up, in
         PA_RETURN_LAUNCH_STATUS();
     }
     if (elem == 2 && mma_ok(d_h, ldh, d_w_gate_up, width)) {
-        const int st = grouped_tc_launch(0, d_h, ldh, d_w_gate_up, width, ff, experts, d_order, d_sel_w, top, d_meta, pairs, act, d_act, as_stream(stream), 1 << 25, d_rows);
+        const int st = grouped_tc_launch(0, d_h, ldh, d_w_gate_up, width, ff, experts, d_order, d_sel_w, top, d_meta, pairs, act, d_act, as_stream(stream), d_rows);
         if (st != PA_ERR_UNSUPPORTED) return st;
         grouped_mma_kernel<0><<<grid, 128, 0, as_stream(stream)>>>(
             static_cast<const bf16_t*>(d_h), ldh, static_cast<const bf16_t*>(d_w_gate_up), width, ff, d_order, d_sel_w, top,
@@ -754,7 +754,7 @@ static int moe_up(const void* d_h, int64_t ldh, const void* d_w_up, int width, i
         PA_RETURN_LAUNCH_STATUS();
     }
     if (elem == 2 && mma_ok(d_h, ldh, d_w_up, width)) {
-        const int st = grouped_tc_launch(2, d_h, ldh, d_w_up, width, ff, experts, d_order, d_sel_w, top, d_meta, pairs, act, d_act, as_stream(stream), 1 << 25, d_rows);
+        const int st = grouped_tc_launch(2, d_h, ldh, d_w_up, width, ff, experts, d_order, d_sel_w, top, d_meta, pairs, act, d_act, as_stream(stream), d_rows);
         if (st != PA_ERR_UNSUPPORTED) return st;
         grouped_mma_kernel<2><<<dim3(nt, (unsigned)((ff + 127) / 128)), 128, 0, as_stream(stream)>>>(
             static_cast<const bf16_t*>(d_h), ldh, static_cast<const bf16_t*>(d_w_up), width, ff, d_order, d_sel_w, top, tiles,

@@ -112,6 +112,7 @@ struct Args {
     bf16_t* out;                // MODE 0, 2: [pairs][n_out], sorted order
     float* out_f32;             // MODE 1: [pairs][n_out], (row, choice) order
     uint32_t polls;             // of a wait
+    uint32_t epilogue_polls[2]; // of a wait of the epilogue warps, by their CTA's place in the pair
 };
 
 __device__ int g_errors;
@@ -298,7 +299,7 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 if (MODE == 1) dst = pair;
                 else sc = __ldg(a.a_scale + pair);
             }
-            tc_wait(tfull(b), (uint32_t)(j >> 1) & 1u, fail_sm, a.polls);
+            tc_wait(tfull(b), (uint32_t)(j >> 1) & 1u, fail_sm, a.epilogue_polls[rank]);
             tc_fence_after();
             const bool lost = tc_failed(fail_sm);       // some wait of the CTA ran out: NaN from here on
             const uint32_t acc = tmem_base + ((uint32_t)(qtr * 32) << 16) + b * BN;
@@ -401,12 +402,13 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             land();
         }
     }
-    if (warp == 1 && tc_failed(fail_sm)) {
-        __nanosleep(1000000);
-        if (lane == 0) atomicAdd(&g_errors, 1);
-    }
     tc_fence_before();
     __syncthreads();
+    if (warp == 1 && tc_failed(fail_sm)) {      // in any of the CTA's roles: products and copies in flight end within microseconds
+        __nanosleep(1000000);
+        if (lane == 0) atomicAdd(&g_errors, 1);
+        __syncwarp();
+    }
     if (PAIR) cluster_sync();   // the other CTA may still read its accumulators or signal this one's barriers
     if (warp == 1) {
         tc_fence_after();
@@ -469,7 +471,8 @@ bool grouped_tc_pairs_up(int pairs, int experts) { return pairs >= mtc::kPairFro
 // mode 0: gate / up pairs, 1: down (rows scattered to (row, choice) order as float), 2: up.  PA_ERR_UNSUPPORTED: the caller's other
 // kernels serve these operands.
 int grouped_tc_launch(int mode, const void* A, int64_t lda, const void* W, int K, int n_out, int experts, const int32_t* order,
-                      const float* a_scale, int top, const int32_t* offsets, int pairs, int act, void* out, cudaStream_t st, int polls, void* rows) {
+                      const float* a_scale, int top, const int32_t* offsets, int pairs, int act, void* out, cudaStream_t st, void* rows, int polls, int first_polls,
+                      int second_polls) {
     using namespace mtc;
     const int64_t w_rows = (int64_t)experts * n_out * (mode == 0 ? 2 : 1);
     if (K % 8 || n_out % 8 || experts > kMostExperts || w_rows >= 0x7fffff00ll || (uintptr_t)out % 16) return PA_ERR_UNSUPPORTED;
@@ -489,7 +492,7 @@ int grouped_tc_launch(int mode, const void* A, int64_t lda, const void* W, int K
     }
     const int strip = mode == 0 ? BN / 2 : BN;
     Args a{static_cast<const bf16_t*>(A), lda, K, n_out, experts, top, act, (n_out + strip - 1) / strip, order, a_scale, offsets,
-           static_cast<bf16_t*>(out), static_cast<float*>(out), (uint32_t)polls};
+           static_cast<bf16_t*>(out), static_cast<float*>(out), (uint32_t)polls, {(uint32_t)first_polls, (uint32_t)second_polls}};
     if (mode == 0) return pair ? launch<0, 2>(tmA, tmW, a, pairs, st) : launch<0, 1>(tmA, tmW, a, pairs, st);
     if (mode == 1) return pair ? launch<1, 2>(tmA, tmW, a, pairs, st) : launch<1, 1>(tmA, tmW, a, pairs, st);
     return pair ? launch<2, 2>(tmA, tmW, a, pairs, st) : launch<2, 1>(tmA, tmW, a, pairs, st);
@@ -499,13 +502,22 @@ int grouped_tc_launch(int mode, const void* A, int64_t lda, const void* W, int K
 
 using namespace pa;
 
+PA_API int pa_moe_grouped_waits(int mode, const void* d_a, int64_t lda, const void* d_w, int K, int n_out, int experts, const int32_t* d_order,
+                                const float* d_a_scale, int top, const int32_t* d_meta, int pairs, int act, void* d_out, void* d_rows,
+                                size_t rows_bytes, int polls, int first_polls, int second_polls, pa_stream_t stream) {
+    PA_CHECK_ARG(mode >= 0 && mode <= 2 && d_a && d_w && d_order && d_meta && d_out && K > 0 && n_out > 0 && experts > 0 && top > 0 && pairs >= 0 &&
+                 act >= 0 && act <= 2 && polls >= 0 && first_polls >= 0 && second_polls >= 0);
+    if (pairs == 0) return PA_OK;
+    if (d_rows && rows_bytes < (size_t)pairs * K * 2) return PA_ERR_WORKSPACE;
+    return grouped_tc_launch(mode, d_a, lda, d_w, K, n_out, experts, d_order, d_a_scale, top, d_meta, pairs, act, d_out, as_stream(stream), d_rows,
+                             polls, first_polls, second_polls);
+}
+
 PA_API int pa_moe_grouped_polls(int mode, const void* d_a, int64_t lda, const void* d_w, int K, int n_out, int experts, const int32_t* d_order,
                                 const float* d_a_scale, int top, const int32_t* d_meta, int pairs, int act, void* d_out, int polls,
                                 pa_stream_t stream) {
-    PA_CHECK_ARG(mode >= 0 && mode <= 2 && d_a && d_w && d_order && d_meta && d_out && K > 0 && n_out > 0 && experts > 0 && top > 0 && pairs >= 0 &&
-                 act >= 0 && act <= 2 && polls >= 0);
-    if (pairs == 0) return PA_OK;
-    return grouped_tc_launch(mode, d_a, lda, d_w, K, n_out, experts, d_order, d_a_scale, top, d_meta, pairs, act, d_out, as_stream(stream), polls, nullptr);
+    return pa_moe_grouped_waits(mode, d_a, lda, d_w, K, n_out, experts, d_order, d_a_scale, top, d_meta, pairs, act, d_out, nullptr, 0, polls, polls,
+                                polls, stream);
 }
 
 PA_API int pa_moe_tc_errors(int* host_count) {

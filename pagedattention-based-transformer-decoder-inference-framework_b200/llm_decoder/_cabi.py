@@ -139,6 +139,7 @@ _SIGS = {
     "pa_latent_gather": ([_vp, _vp, _i32, _i32, _i32, _i32, _i32, _vp, _i32, _i32, _vp, _vp], _i32),
     "pa_attention_tc_errors": ([C.POINTER(_i32)], _i32),
     "pa_moe_tc_errors": ([C.POINTER(_i32)], _i32),
+    "pa_moe_grouped_waits": ([_i32, _vp, _i64, _vp, _i32, _i32, _i32, _vp, _vp, _i32, _vp, _i32, _i32, _vp, _vp, _sz, _i32, _i32, _i32, _vp], _i32),
     "pa_moe_grouped_polls": ([_i32, _vp, _i64, _vp, _i32, _i32, _i32, _vp, _vp, _i32, _vp, _i32, _i32, _vp, _i32, _vp], _i32),
     "pa_router_topk": ([_vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _vp, _vp, _vp, _i32, _vp], _i32),
     "pa_moe_tile_rows": ([], _i32),

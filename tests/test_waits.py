@@ -88,8 +88,32 @@ def grouped():
                 assert torch.isnan(out.float()).all() and ran_out > 0 if polls == 0 else torch.isfinite(out.float()).all() and ran_out == 0
 
 
+def grouped_pairs():
+    """Pairs of CTAs, several tiles for each, with their sorted rows: all waits, or those of one CTA's epilogue alone."""
+    from llm_decoder import _cabi
+    lib, dev, pairs, experts, K, n_out = _cabi.lib(), torch.device("cuda"), 6400, 2, 2048, 3072
+    ids = torch.randint(0, experts, (pairs,), generator=torch.Generator().manual_seed(1)).to(torch.int32).to(dev)
+    order, meta = torch.empty(pairs, dtype=torch.int32, device=dev), torch.empty(lib.pa_moe_meta_ints(pairs, experts), dtype=torch.int32, device=dev)
+    assert lib.pa_moe_sort(ids.data_ptr(), pairs, experts, order.data_ptr(), meta.data_ptr(), _cabi.stream()) == 0
+    a, w = torch.randn(pairs, K, device=dev).to(BF), torch.randn(experts, 2 * n_out, K, device=dev).to(BF)
+    nb = lib.pa_moe_sorted_rows_bytes(pairs, experts, K, 2)
+    rows, most = torch.empty(nb, dtype=torch.uint8, device=dev), 1 << 25
+    for mode in (0, 1, 2):
+        wt = w if mode == 0 else w[:, :n_out].contiguous()
+        for limits in ((most, most, most), (0, 0, 0), (most, 0, most), (most, most, 0), (most, most, most)):
+            out = torch.zeros(pairs, n_out, device=dev, dtype=torch.float32 if mode == 1 else BF)
+            before = _count(lib.pa_moe_tc_errors)
+            assert lib.pa_moe_grouped_waits(mode, a.data_ptr(), K, wt.data_ptr(), K, n_out, experts, order.data_ptr(), None, 1, meta.data_ptr(), pairs,
+                                            0, out.data_ptr(), rows.data_ptr(), nb, *limits, _cabi.stream()) == 0
+            ran_out, lost = _count(lib.pa_moe_tc_errors) - before, torch.isnan(out.float())
+            if min(limits) == most:
+                assert ran_out == 0 and not lost.any()
+            else:
+                assert ran_out > 0 and lost.any() and (limits[0] or lost.all()), (mode, limits)
+
+
 @pytest.mark.gpu
-@pytest.mark.parametrize("case", ["masked_decode", "latent_decode", "grouped"])
+@pytest.mark.parametrize("case", ["masked_decode", "latent_decode", "grouped", "grouped_pairs"])
 def test_rows_of_waits_that_run_out(case):
     r = subprocess.run([sys.executable, os.path.abspath(__file__), case], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.strip().endswith("done"), r.stdout + r.stderr
