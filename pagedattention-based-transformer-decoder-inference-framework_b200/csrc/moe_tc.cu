@@ -20,7 +20,8 @@
 // 134 us (with four epilogue warps 203 us); down 61 us, one CTA 67 us.
 //
 // Every wait is bounded: on a protocol error the CTA raises a flag (pa_moe_tc_errors), lets its copies land, frees its TMEM and
-// writes NaN into the rows of its tiles from there on.
+// writes NaN into the rows of its tiles from there on.  A pair raises it in both CTAs: warps that gave up go through their tiles
+// without waiting, so what they signal no longer says that an accumulator has been read, and no further product may be issued.
 #include "seq_common.cuh"
 #include "tcgen05_utils.cuh"
 
@@ -100,6 +101,11 @@ __device__ __forceinline__ bool wait_pair(uint32_t bar, uint32_t parity, uint32_
         }
     }
     return true;
+}
+
+// a wait that ran out, in the other CTA of the pair too: ahead of whatever this thread signals next
+__device__ __forceinline__ void tell_pair(uint32_t fail_there) {
+    asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], %1;" ::"r"(fail_there), "r"(1u) : "memory");
 }
 
 struct Args {
@@ -225,7 +231,10 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 const int n0 = w.strip * (MODE == 0 ? BN / 2 : BN);
                 const int r1 = w.e * w_rows + n0, r2 = r1 + (MODE == 0 ? a.n_out : BN / 2);
                 for (int kt = 0; kt < nk; ++kt) {
-                    if (!tc_wait(empty(s), ph, fail_sm, a.polls)) break;
+                    if (!tc_wait(empty(s), ph, fail_sm, a.polls)) {
+                        if (PAIR) tell_pair(mapa_shared(fail_sm, rank ^ 1));
+                        break;
+                    }
                     const uint32_t st = base + s * STAGE;
                     constexpr int bytes = PAIR || MODE == 1 ? STAGE : B_BYTES;
                     if (PAIR) {             // this CTA's rows, and its half of the weight rows
@@ -253,13 +262,15 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         int s = 0, j = 0;
         uint32_t ph = 0;
         auto wait = [&](uint32_t bar, uint32_t parity) {
-            return PAIR ? wait_pair(bar, parity, fail_sm, a.polls) : tc_wait(bar, parity, fail_sm, a.polls);
+            const bool ok = PAIR ? wait_pair(bar, parity, fail_sm, a.polls) : tc_wait(bar, parity, fail_sm, a.polls);
+            if (PAIR && !ok) tell_pair(mapa_shared(fail_sm, rank ^ 1));
+            return ok;
         };
         if (rank == 0 && elect_one()) {
             bool ok = true;             // false once a wait ran out, and no further product is issued
             for (; ok && w.next(); ++j) {
                 const int b = j & 1;
-                ok = wait(tempty(b), ((uint32_t)(j >> 1) & 1u) ^ 1u);
+                ok = wait(tempty(b), ((uint32_t)(j >> 1) & 1u) ^ 1u) && !(PAIR && tc_failed(fail_sm));
                 for (int kt = 0; ok && kt < nk; ++kt) {
                     ok = wait(full(s), ph);
                     if (!ok) break;
@@ -299,7 +310,7 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 if (MODE == 1) dst = pair;
                 else sc = __ldg(a.a_scale + pair);
             }
-            tc_wait(tfull(b), (uint32_t)(j >> 1) & 1u, fail_sm, a.epilogue_polls[rank]);
+            if (!tc_wait(tfull(b), (uint32_t)(j >> 1) & 1u, fail_sm, a.epilogue_polls[rank]) && PAIR) tell_pair(mapa_shared(fail_sm, rank ^ 1));
             tc_fence_after();
             const bool lost = tc_failed(fail_sm);       // some wait of the CTA ran out: NaN from here on
             const uint32_t acc = tmem_base + ((uint32_t)(qtr * 32) << 16) + b * BN;

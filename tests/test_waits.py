@@ -99,7 +99,7 @@ def grouped_pairs():
     nb = lib.pa_moe_sorted_rows_bytes(pairs, experts, K, 2)
     rows, most = torch.empty(nb, dtype=torch.uint8, device=dev), 1 << 25
     for mode in (0, 1, 2):
-        wt = w if mode == 0 else w[:, :n_out].contiguous()
+        wt, whole = w if mode == 0 else w[:, :n_out].contiguous(), None
         for limits in ((most, most, most), (0, 0, 0), (most, 0, most), (most, most, 0), (most, most, most)):
             out = torch.zeros(pairs, n_out, device=dev, dtype=torch.float32 if mode == 1 else BF)
             before = _count(lib.pa_moe_tc_errors)
@@ -107,9 +107,11 @@ def grouped_pairs():
                                             0, out.data_ptr(), rows.data_ptr(), nb, *limits, _cabi.stream()) == 0
             ran_out, lost = _count(lib.pa_moe_tc_errors) - before, torch.isnan(out.float())
             if min(limits) == most:
-                assert ran_out == 0 and not lost.any()
-            else:
+                assert ran_out == 0 and not lost.any() and (whole is None or torch.equal(out, whole))
+                whole = out
+            else:                   # what the other CTA writes is what it should be, or NaN too
                 assert ran_out > 0 and lost.any() and (limits[0] or lost.all()), (mode, limits)
+                assert bool((lost | (out == whole)).all()), (mode, limits)
 
 
 @pytest.mark.gpu
