@@ -980,7 +980,10 @@ int pa_latent_decode_polls(const void* d_q_lat, int64_t ql_row_stride, int64_t q
  *   all in float.  Queries go to d_q_out (not d_in), keys and values to the pools (NULL: a layer that reads another
  *   layer's pool; the rows then hold queries only).  d_items [num_items][6] = first row, tokens (at most item_tokens, at
  *   least taps - 1 of which the portion's earlier items hold each), slot, offset within the portion, the portion's length,
- *   first position.  At most 8 taps, heads of at most 512. */
+ *   first position.  At most 8 taps, heads of at most 512.
+ * pa_conv_rope_norm_append_rows: the same with the tokens of all items together, by which the form of the kernel is chosen
+ *   (without: as if every item had item_tokens).  pa_conv_append_in_words: 1 where that is the form for many long items
+ *   (bfloat16 rows of whole 16-byte words, at most 4 taps); units: heads + 2 * kv_heads, columns: of the larger head. */
 int pa_embedding_bigram(const void* d_embed, const void* d_bigram, int elem, const int32_t* d_ids, const int32_t* d_prev_ids,
                         int rows, int width, int vocab, int64_t buckets, int64_t mul_prev, int64_t mul_cur, float scale,
                         float* d_out, float* d_copy, pa_stream_t stream);
@@ -1008,6 +1011,12 @@ int pa_conv_rope_norm_append(const void* d_in, int64_t in_stride, int in_off, in
                              float eps, void* d_q_out, int64_t q_out_stride, void* d_k_pool, void* d_v_pool,
                              const int32_t* d_table, int num_slots, int num_tiles, int total_pages, int tile_size,
                              const int32_t* d_items, int num_items, int item_tokens, int elem, pa_stream_t stream);
+int pa_conv_rope_norm_append_rows(const void* d_in, int64_t in_stride, int in_off, int heads, int kv_heads, int dim, int vdim,
+                                  int taps, const float* d_weight, float* d_state, int rot_dims, const float* d_rope, int norm,
+                                  float eps, void* d_q_out, int64_t q_out_stride, void* d_k_pool, void* d_v_pool,
+                                  const int32_t* d_table, int num_slots, int num_tiles, int total_pages, int tile_size,
+                                  const int32_t* d_items, int num_items, int item_tokens, int64_t rows, int elem, pa_stream_t stream);
+int pa_conv_append_in_words(int units, int columns, int num_items, int64_t rows);
 
 #ifdef __cplusplus
 }

@@ -169,6 +169,7 @@ struct ConvAppendParams {
     int num_slots, num_tiles, total_pages, tile_size;
     const int32_t* items;       // [n][6]: first row, tokens, slot, offset within the portion, portion's length, first position
     int num_items;
+    int64_t rows;               // tokens of all items
     int pairs;                  // every pair of columns starts on a boundary of two elements
     int words;                  // 4 or 8: heads are whole words of that many columns, everything aligned: the vector form
 };
@@ -552,6 +553,7 @@ __device__ __forceinline__ void ca_load_pairs(const float* __restrict__ p, uint6
 }
 
 constexpr int kCaTurns = 16;        // tokens whose turns are staged together
+constexpr int kCaWordTokens = 12;   // tokens an item (on average) from which on this form is taken, see ca_words_pay
 
 template <int LANES, int TAPS>
 __global__ void __launch_bounds__(kCaThreads, 4) conv_rope_norm_append_words_kernel(const ConvAppendParams p) {
@@ -738,15 +740,26 @@ static int ca_launch(const ConvAppendParams& p, cudaStream_t st) {
     PA_RETURN_LAUNCH_STATUS();
 }
 
+// Whether the words form serves many items better than the vector form.  Three conditions, times in us of the vector and the words form
+// on the GPU alone, 16 + 2 x 4 heads, four taps:
+//  - more warps than the vector form holds at once (four a CTA, five CTAs an SM).  Up to there its items all run side by side.  A warp
+//    has one unit of more than 64 columns, two of more than 32: heads of 128, 128 items of 16 tokens 15.7 and 12.2, 1024 items 109 and
+//    83; heads of 64, 128 items (1536 warps) 9.3 and 10.6, 256 items 16.7 and 12.8;
+//  - items long enough for its pairs of tokens and staged turns.  Heads of 128, 512 items of 1 token 11.4 and 13.8, of 4 tokens 16.6 and
+//    18.0, of 8 tokens 26.2 and 24.5, of 12 tokens 43 and 34, of 16 tokens 58 and 42.  Where units leave lanes idle the line is at 12
+//    tokens: heads of 64, 1024 items of 10 tokens 33.7 and 35.2, of 12 tokens 45 and 42; 8 + 2 x 2 heads of 128, 512 items of 8
+//    tokens 15.0 and 16.1, of 12 tokens 20.0 and 20.2, of 16 tokens 25.9 and 24.3;
+//  - heads of more than 32 columns: smaller ones leave half its lanes idle (heads of 32, 1024 items of 16 tokens 25.4 and 42.5).
+static bool ca_words_pay(int units_per_item, int n, int num_items, int64_t rows) {
+    const int64_t warps = (int64_t)num_items * units_per_item / (n > 64 ? 1 : 2);
+    return n > 32 && n <= 128 && rows >= kCaWordTokens * (int64_t)num_items && warps > 20 * device_info().sm_count;
+}
+
 template <typename T>
 static int ca_dispatch(const ConvAppendParams& p, cudaStream_t st) {
     const int n = p.k_pool && p.vdim > p.dim ? p.vdim : p.dim;
     if constexpr (sizeof(T) == 2) {
-        // from as many units on as the form with a warp each does not hold at once (four warps a CTA, five CTAs an SM): up to there
-        // its items all run side by side, and it is the faster one (24 units an item, 64 items 10.8 and 11.4 us, 128 items 18.1 and
-        // 13.2, 512 items 53 and 38)
-        const int64_t units = (int64_t)p.num_items * (p.heads + (p.k_pool ? 2 * p.kv_heads : 0));
-        if (p.words == 8 && (p.w ? p.taps : 1) <= 4 && n <= 128 && units > 20 * device_info().sm_count) {
+        if (p.words == 8 && (p.w ? p.taps : 1) <= 4 && ca_words_pay(p.heads + (p.k_pool ? 2 * p.kv_heads : 0), n, p.num_items, p.rows)) {
             if (n <= 64) return ca_launch_words<8>(p, st);
             return ca_launch_words<16>(p, st);
         }
@@ -1851,11 +1864,12 @@ PA_API int pa_qk_norm_kv_append(void* d_src, int64_t src_stride, int q_off, int 
     PA_RETURN_LAUNCH_STATUS();
 }
 
-PA_API int pa_conv_rope_norm_append(const void* d_in, int64_t in_stride, int in_off, int heads, int kv_heads, int dim, int vdim,
-                                    int taps, const float* d_weight, float* d_state, int rot_dims, const float* d_rope,
-                                    int norm, float eps, void* d_q_out, int64_t q_out_stride, void* d_k_pool, void* d_v_pool,
-                                    const int32_t* d_table, int num_slots, int num_tiles, int total_pages, int tile_size,
-                                    const int32_t* d_items, int num_items, int item_tokens, int elem, pa_stream_t stream) {
+PA_API int pa_conv_rope_norm_append_rows(const void* d_in, int64_t in_stride, int in_off, int heads, int kv_heads, int dim, int vdim,
+                                         int taps, const float* d_weight, float* d_state, int rot_dims, const float* d_rope,
+                                         int norm, float eps, void* d_q_out, int64_t q_out_stride, void* d_k_pool, void* d_v_pool,
+                                         const int32_t* d_table, int num_slots, int num_tiles, int total_pages, int tile_size,
+                                         const int32_t* d_items, int num_items, int item_tokens, int64_t rows, int elem, pa_stream_t stream) {
+    PA_CHECK_ARG(rows >= 0);
     PA_CHECK_ARG(d_in && d_q_out && d_items && num_items >= 0 && heads > 0 && kv_heads > 0 && dim > 0 && vdim > 0 && num_slots > 0);
     PA_CHECK_ARG(rot_dims >= 0 && rot_dims % 2 == 0 && rot_dims <= dim && (rot_dims == 0 || d_rope) && (norm == 0 || norm == 1));
     PA_CHECK_ARG(!d_weight || (taps >= 1 && taps <= kCaMaxTaps && (taps == 1 || d_state) && item_tokens >= taps - 1));
@@ -1868,7 +1882,7 @@ PA_API int pa_conv_rope_norm_append(const void* d_in, int64_t in_stride, int in_
     p.rot_dims = rot_dims; p.taps = taps; p.w = d_weight; p.state = d_state; p.rope = d_rope; p.norm = norm; p.eps = eps;
     p.q_out = d_q_out; p.q_out_stride = q_out_stride; p.k_pool = d_k_pool; p.v_pool = d_v_pool; p.table = d_table;
     p.num_slots = num_slots; p.num_tiles = num_tiles; p.total_pages = total_pages; p.tile_size = tile_size;
-    p.items = d_items; p.num_items = num_items;
+    p.items = d_items; p.num_items = num_items; p.rows = rows;
     const uintptr_t two = 2 * (uintptr_t)(elem == 2 ? 2 : 4);
     p.pairs = dim % 2 == 0 && vdim % 2 == 0 && in_stride % 2 == 0 && in_off % 2 == 0 && q_out_stride % 2 == 0 &&
               ((uintptr_t)d_in | (uintptr_t)d_q_out | (uintptr_t)d_k_pool | (uintptr_t)d_v_pool) % two == 0;
@@ -1884,6 +1898,21 @@ PA_API int pa_conv_rope_norm_append(const void* d_in, int64_t in_stride, int in_
     if (elem == 4) return ca_dispatch<float>(p, as_stream(stream));
     if (elem == 2) return ca_dispatch<bf16_t>(p, as_stream(stream));
     return PA_ERR_UNSUPPORTED;
+}
+
+PA_API int pa_conv_rope_norm_append(const void* d_in, int64_t in_stride, int in_off, int heads, int kv_heads, int dim, int vdim,
+                                    int taps, const float* d_weight, float* d_state, int rot_dims, const float* d_rope,
+                                    int norm, float eps, void* d_q_out, int64_t q_out_stride, void* d_k_pool, void* d_v_pool,
+                                    const int32_t* d_table, int num_slots, int num_tiles, int total_pages, int tile_size,
+                                    const int32_t* d_items, int num_items, int item_tokens, int elem, pa_stream_t stream) {
+    const int64_t rows = num_items > 0 && item_tokens > 0 ? (int64_t)num_items * item_tokens : 0;
+    return pa_conv_rope_norm_append_rows(d_in, in_stride, in_off, heads, kv_heads, dim, vdim, taps, d_weight, d_state, rot_dims, d_rope, norm, eps,
+                                         d_q_out, q_out_stride, d_k_pool, d_v_pool, d_table, num_slots, num_tiles, total_pages, tile_size, d_items,
+                                         num_items, item_tokens, rows, elem, stream);
+}
+
+PA_API int pa_conv_append_in_words(int units, int columns, int num_items, int64_t rows) {
+    return units > 0 && columns > 0 && num_items > 0 && rows >= 0 && ca_words_pay(units, columns, num_items, rows) ? 1 : 0;
 }
 
 PA_API int pa_masked_attention_mma_tile_tokens(int dim, int vdim, int elem) {

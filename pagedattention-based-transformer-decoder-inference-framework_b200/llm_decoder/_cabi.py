@@ -224,6 +224,9 @@ _SIGS = {
                                   _i32, _f32, _vp, _vp, _i64, _i64, _i32, _i32, _i32, _vp, _sz, _vp], _i32),
     "pa_conv_rope_norm_append": ([_vp, _i64, _i32, _i32, _i32, _i32, _i32, _i32, _vp, _vp, _i32, _vp, _i32, _f32, _vp, _i64, _vp,
                                   _vp, _vp, _i32, _i32, _i32, _i32, _vp, _i32, _i32, _i32, _vp], _i32),
+    "pa_conv_rope_norm_append_rows": ([_vp, _i64, _i32, _i32, _i32, _i32, _i32, _i32, _vp, _vp, _i32, _vp, _i32, _f32, _vp, _i64, _vp,
+                                       _vp, _vp, _i32, _i32, _i32, _i32, _vp, _i32, _i32, _i64, _i32, _vp], _i32),
+    "pa_conv_append_in_words": ([_i32, _i32, _i32, _i64], _i32),
     "pa_causal_conv": ([_vp, _i64, _i32, _i32, _i32, _vp, _vp, _i32, _vp, _vp, _i32, _vp, _i64, _i32, _vp], _i32),
 }
 

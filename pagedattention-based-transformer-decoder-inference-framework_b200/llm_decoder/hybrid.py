@@ -734,14 +734,14 @@ class MaskedAttention:
             kv, pt, own = self.kv, self.kv.page_table_, self.own_kv
             items, n = b.portion_items(APPEND_CHUNK)
             q = c.empty(R, self.q_cols)
-            _chk(lib.pa_conv_rope_norm_append(
+            _chk(lib.pa_conv_rope_norm_append_rows(
                 proj.data_ptr(), proj.stride(0), off, self.heads, self.kv_heads, self.dim, self.vdim, self.taps,
                 _cabi.ptr(self.conv_wt) if self.taps else None, _cabi.ptr(self.conv_state), self.rot_dims,
                 _cabi.ptr(c.rope_table(self.rot_dims, self.rot_base, self.rot_scaling)),
                 1 if self.turned_norm else 0, c.model.eps, q.data_ptr(), self.q_cols, kv.key_buffer_.data_ptr() if own else None,
                 kv.value_buffer_.data_ptr() if own else None, pt.device_data().data_ptr(), pt.num_beams_,
-                pt.num_tiles_, kv.total_pages_, kv.tile_size_, items.data_ptr(), n, APPEND_CHUNK, c.elem, s),
-                "pa_conv_rope_norm_append")
+                pt.num_tiles_, kv.total_pages_, kv.tile_size_, items.data_ptr(), n, APPEND_CHUNK, R, c.elem, s),
+                "pa_conv_rope_norm_append_rows")
             return q, 0
         if self.taps:
             chunks, nch, _s0, _sn = b.chunk_items(CONV_CHUNK)

@@ -53,6 +53,19 @@ def test_convolved_rows(heads, kv_heads, dim, vdim, rot_dims, norm, taps, dtype)
         assert torch.equal(out[0][-1], out[1][-1])
 
 
+def test_form_of_many_items():
+    """Where the form for many long items is taken: not for decoded tokens, however many, nor for small heads."""
+    from llm_decoder import _cabi
+    lib, most = _cabi.lib(), 20 * _cabi.device_info()[0]        # warps that the other form holds at once
+    words = lambda units, columns, items, tokens: lib.pa_conv_append_in_words(units, columns, items, int(items * tokens))  # noqa: E731
+    for columns, per in ((128, 1), (72, 1), (64, 2), (40, 2)):
+        items = most * per // 24
+        assert not words(24, columns, items, 16) and words(24, columns, items + per, 16) and words(24, columns, 8 * items, 12)
+        assert not any(words(24, columns, 8 * items, m) for m in (1, 2, 8, 11))
+    for columns in (8, 32, 136):
+        assert not words(24, columns, 100 * most, 16)
+
+
 @pytest.mark.parametrize("kv_rank,rot_dim,rot_dims", [(512, 64, 64), (256, 32, 32), (8, 16, 16), (264, 24, 16), (1024, 8, 0), (40, 0, 0)])
 @pytest.mark.parametrize("pairing", [0, 1])
 @pytest.mark.parametrize("queries", ["turn", "norm", None])
