@@ -126,7 +126,7 @@ __device__ int g_errors;
 __device__ __forceinline__ float act_f32(float v, int act) {
     if (act == 1) return fmaxf(v, 0.f);
     if (act == 2) { const float r = fmaxf(v, 0.f); return r * r; }
-    return __fdividef(v, 1.0f + expf(-v));
+    return silu_f32(v);
 }
 // 32 bytes of an output row; !whole: the row ends after 16 of them (columns come in eights)
 __device__ __forceinline__ void store_words(void* dst, const uint32_t* w, bool whole) {

@@ -122,3 +122,30 @@ def test_pairs_without_an_expert(gated):
         out.append(o)
     assert bool((scratch[count:] == 7.5).all()) and torch.equal(scratch[:count], h[order[:count].long() // top])
     assert torch.equal(out[0], out[1]) and bool((out[0][count:] == 3.25).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [300, 6200])
+def test_silu_of_large_negative_gates(rows):
+    """Gates near -88, whose sigmoid's denominator is above 2^126, with an up value that makes the result an ordinary number.  Bound: gate
+    and up are exact here, expf and the division are off by a few units of 2^-24, and the result is rounded to bfloat16, whose eight bits
+    leave half a unit: up to 2^-8 of the value."""
+    from llm_decoder import _cabi
+    lib, dev, s = _cabi.lib(), torch.device("cuda"), _cabi.stream
+    K, ff = 64, 16
+    gates = torch.tensor([-87.5, -88.0, -88.5, -60.0, -87.0, -20.0, -1.0, 4.0]).repeat(2)
+    w = torch.zeros(1, 2 * ff, K)
+    w[0, :ff, 0], w[0, ff:, 1] = gates, 2.0 ** 100
+    h = torch.zeros(rows, K)
+    h[:, 0], h[:, 1] = 1.0, 2.0
+    hd, wd, ids = h.to(BF).to(dev), w.to(BF).to(dev), torch.zeros(rows, dtype=torch.int32, device=dev)
+    order, out = torch.empty(rows, dtype=torch.int32, device=dev), torch.empty(rows, ff, dtype=BF, device=dev)
+    meta = torch.empty(lib.pa_moe_meta_ints(rows, 1), dtype=torch.int32, device=dev)
+    _cabi.check(lib.pa_moe_sort(ids.data_ptr(), rows, 1, order.data_ptr(), meta.data_ptr(), s()), "sort")
+    nb = lib.pa_moe_sorted_rows_bytes(rows, 1, K, 2)
+    ws = torch.empty(nb, dtype=torch.uint8, device=dev) if nb else None
+    _cabi.check(lib.pa_moe_up_sorted(hd.data_ptr(), K, wd.data_ptr(), 1, K, ff, 1, order.data_ptr(), None, 1, meta.data_ptr(), rows, 0,
+                                     out.data_ptr(), _cabi.ptr(ws), nb, 2, s()), "up")
+    g = gates.double()
+    want = g / (1.0 + torch.exp(-g)) * 2.0 ** 101
+    assert ((out.double().cpu() - want).abs() <= (2.0 ** -8 + 2.0 ** -20) * want.abs()).all()
