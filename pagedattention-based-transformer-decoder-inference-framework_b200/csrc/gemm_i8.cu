@@ -78,14 +78,6 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
         ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
         : "memory");
 }
-__device__ __forceinline__ void tma_load_3d_mc(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2,
-                                               uint32_t bar, uint16_t mask) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.multicast::cluster "
-        "[%0], [%1, {%3, %4, %5}], [%2], %6;"
-        ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "h"(mask)
-        : "memory");
-}
 __device__ __forceinline__ uint32_t cluster_ctarank() {
     uint32_t r;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -115,10 +107,6 @@ __device__ __forceinline__ void umma_i8(uint32_t d_tmem, uint64_t a_desc, uint64
 }
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void umma_commit_mc(uint32_t bar, uint16_t mask) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                 ::"r"(bar), "h"(mask) : "memory");
 }
 // 32 lanes x 32 consecutive 32-bit columns -> 32 registers per thread.
 __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t (&r)[32]) {
@@ -203,13 +191,10 @@ __device__ __forceinline__ void tmem_ld_32x32_nowait(uint32_t taddr, uint32_t (&
 
 // EPI: 0 = integer outputs only (raw s32 and/or split-K reduction), 1/2/3 = s8 output with
 // activation none/relu/gelu (plus optional raw s32).
-// CL: thread-block cluster size along N.  The CL CTAs of a cluster work on adjacent B slabs and
-// need the same A tiles: each loads 1/CL of the A rows and TMA-multicasts them to all CL CTAs,
-// which divides the L2 -> SM traffic for A by CL (the main loop is L2-read bound otherwise).
 constexpr int MAXST = 12;                     // 1-CTA kernel: maximum ring depth
 constexpr int RING_BYTES = 4 * 3 * TILE_BYTES;  // 192 KB of shared memory for the ring in every configuration
 
-template <int EPI, int CL>
+template <int EPI>
 __global__ void __launch_bounds__(NTHREADS, 1)
 gemm_i8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const Args g) {
     extern __shared__ uint8_t smem_raw[];
@@ -244,7 +229,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     if (threadIdx.x == 0) {
         for (int s = 0; s < nst; ++s) {
             mbar_init(full_bar(s), 1);
-            mbar_init(empty_bar(s), CL);  // every CTA of the cluster must have drained slot s
+            mbar_init(empty_bar(s), 1);
         }
         mbar_init(tmem_full_bar, 1);
         mbar_fence_init();
@@ -254,10 +239,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLS);
     tc_fence_before();
     __syncthreads();
-    if (CL > 1) cluster_sync();  // peers' barriers are initialised before any remote arrive lands
     tc_fence_after();
-    const uint32_t crank = (CL > 1) ? cluster_ctarank() : 0u;
-    constexpr uint16_t kMask = (uint16_t)((1u << CL) - 1u);
     uint32_t tmem_base;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
     // programmatic dependent launch: everything above ran under the tail of the kernel in front; its results are read below
@@ -288,20 +270,8 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 const uint32_t a_load = (m_tiles == 2) ? 2u * TILE_BYTES : (a_bytes < (uint32_t)TILE_BYTES ? a_bytes : (uint32_t)TILE_BYTES);
                 mbar_arrive_expect_tx(full_bar(s), a_load + TILE_BYTES);
                 const int k0 = (kb0 + i) * BK;
-                if (CL == 1) {
-                    if (m_tiles == 2) {
-                        tma_load_3d(st, &tmA, k0, m0, batch, full_bar(s));
-                        tma_load_3d(st + TILE_BYTES, &tmA, k0, m0 + BM, batch, full_bar(s));
-                    } else {
-                        tma_load_3d(st, &tmA, k0, m0, batch, full_bar(s));  // box = a_bytes / 128 rows
-                    }
-                } else {
-                    // This CTA's share of the A rows of the stage (tmA's box holds a_rows rows),
-                    // delivered to the same offset in every CTA of the cluster.
-                    const int a_rows = m_tiles * BM / CL;
-                    const int r0 = (int)crank * a_rows;
-                    tma_load_3d_mc(st + r0 * BK, &tmA, k0, m0 + r0, batch, full_bar(s), kMask);
-                }
+                tma_load_3d(st, &tmA, k0, m0, batch, full_bar(s));  // one row tile: box = a_bytes / 128 rows
+                if (m_tiles == 2) tma_load_3d(st + TILE_BYTES, &tmA, k0, m0 + BM, batch, full_bar(s));
                 tma_load_3d(st + a_bytes, &tmB, n0, k0, batch, full_bar(s));
                 if (++s == nst) {
                     s = 0;
@@ -342,9 +312,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         }
                     }
                 }
-                // slot reusable once these MMAs have read it (signalled to every CTA of the cluster)
-                if (CL == 1) umma_commit(empty_bar(s));
-                else umma_commit_mc(empty_bar(s), kMask);
+                umma_commit(empty_bar(s));  // slot reusable once these MMAs have read it
                 if (++s == nst) {
                     s = 0;
                     ph ^= 1u;
@@ -434,7 +402,6 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #endif
     tc_fence_before();
     __syncthreads();
-    if (CL > 1) cluster_sync();  // no CTA exits while peers may still signal its barriers
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem_base, TMEM_COLS);
@@ -495,25 +462,9 @@ __device__ __forceinline__ void umma_commit_2cta(uint32_t bar, uint16_t mask) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                  ::"r"(bar), "h"(mask) : "memory");
 }
-// cta_group::2 load delivered to every CTA of `mask` at the same offset; each copy's bytes complete on the full
-// barrier of the destination's PAIR LEADER (the barrier address names the even CTA of the issuer's pair).
-__device__ __forceinline__ void tma_load_3d_2cta_mc(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2,
-                                                    uint32_t bar_cluster_addr, uint16_t mask) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.multicast::cluster "
-        "[%0], [%1, {%3, %4, %5}], [%2], %6;"
-        ::"r"(dst), "l"(map), "r"(bar_cluster_addr), "r"(c0), "r"(c1), "r"(c2), "h"(mask)
-        : "memory");
-}
-
 // OCC = 2 (used when the grid has more CTA pairs than one wave): two CTAs per SM with a 3-stage ring each (same
 // bytes in flight per SM, 2 x 256 TMEM columns), so the epilogue, set-up and pipeline fill of one tile run under
 // the main loop of the other CTA's tile.
-// CLP = 2: a cluster of FOUR CTAs = two pairs on adjacent column slabs of the same rows.  Both pairs need the
-// same A tile, so every CTA fetches 64 of its 128 A rows and multicasts them to its counterpart in the other
-// pair: A crosses the L2 -> SM fabric once per cluster instead of once per pair (at M = 256 the whole GEMM is
-// bound by that fabric, profiles/r01_gemm_notes.md).  A ring slot is then reusable only when BOTH pairs have
-// consumed it (empty barrier count 2, each leader's commit multicast to all four CTAs).
 // DQ = true: the s8 output is the dynamically quantised row (compute_minmax_scale + batch_quantize,
 // int8_quant.cpp:59-64, 15-28) of act(alpha_row * acc + bias) -- the "fc1 -> int8_quant -> fc2" hand-off of the INT8
 // decoder MLP without the f32 round trip through memory (16 MiB written and re-read per layer at M = 256).  A row's
@@ -522,7 +473,7 @@ __device__ __forceinline__ void tma_load_3d_2cta_mc(uint32_t dst, const CUtensor
 // global memory (atomicMax on the bit patterns), a grid-wide barrier follows (every CTA is resident: the host only
 // uses this instance when the grid fits one wave), pass 2 re-reads TMEM, quantises with the final scale and stores
 // s8.  Values, scale and rounding are bit-identical to the unfused kernels.
-template <int EPI, int OCC, int CLP, bool DQ = false>
+template <int EPI, int OCC, bool DQ = false>
 __global__ void __launch_bounds__(NTHREADS2, OCC)
 gemm_i8_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const Args g) {
     extern __shared__ uint8_t smem_raw[];
@@ -540,12 +491,7 @@ gemm_i8_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     const bool probe_cta = blockIdx.x == 10 && blockIdx.y == 0 && g.probe;
 #endif
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t cluster_rank = cluster_ctarank();
-    const uint32_t crank = cluster_rank & 1u;   // rank inside the CTA pair (0 = leader)
-    const uint32_t cpair = cluster_rank >> 1;   // pair inside the cluster (CLP = 2)
-    const uint32_t lead_rank = cluster_rank & ~1u;
-    const uint16_t pair_mask = (uint16_t)(3u << (2 * cpair));
-    const uint16_t all_mask = (uint16_t)((1u << (2 * CLP)) - 1u);
+    const uint32_t crank = cluster_ctarank();   // rank inside the CTA pair (0 = leader)
     const int n0 = (blockIdx.x >> 1) * BN2;
     const int m_chunk = blockIdx.y / g.ksplit, split = blockIdx.y % g.ksplit;
     const int m0 = m_chunk * 2 * BM;
@@ -558,7 +504,7 @@ gemm_i8_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     if (threadIdx.x == 0) {
         for (int s = 0; s < NST; ++s) {
             mbar_init(full_bar(s), 2);   // one arrive.expect_tx from each CTA's producer (leader's copy is used)
-            mbar_init(empty_bar(s), CLP);  // each pair leader's commit, multicast to every CTA of the cluster
+            mbar_init(empty_bar(s), 1);  // the leader's commit, at both CTAs
         }
         mbar_init(tmem_full_bar, 1);
         mbar_fence_init();
@@ -593,16 +539,11 @@ gemm_i8_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 pw += clock64() - tw0;
 #endif
                 const uint32_t st = base + s * STAGE2_BYTES;
-                const uint32_t lead_full = mapa_shared(full_bar(s), lead_rank);
+                const uint32_t lead_full = mapa_shared(full_bar(s), 0);
                 if (crank == 0) mbar_arrive_expect_tx(full_bar(s), STAGE2_BYTES);
                 else mbar_remote_arrive_expect_tx(lead_full, STAGE2_BYTES);
                 const int k0 = (kb0 + i) * BK;
-                if (CLP == 1) {
-                    tma_load_3d_2cta(st, &tmA, k0, m0 + (int)crank * BM, batch, lead_full);
-                } else {  // tmA's box holds 64 rows: this CTA's share of the A half both pairs need
-                    tma_load_3d_2cta_mc(st + cpair * (TILE_BYTES / 2), &tmA, k0, m0 + (int)crank * BM + (int)cpair * (BM / 2),
-                                        batch, lead_full, (uint16_t)((1u << crank) | (1u << (2 + crank))));
-                }
+                tma_load_3d_2cta(st, &tmA, k0, m0 + (int)crank * BM, batch, lead_full);
                 tma_load_3d_2cta(st + TILE_BYTES, &tmB, n0 + (int)crank * BN, k0, batch, lead_full);
             }
 #ifdef PA_GEMM_PROBE
@@ -628,9 +569,9 @@ gemm_i8_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                     const uint64_t db = make_desc(st + TILE_BYTES + ks * UK * BK, TILE_BYTES, 1024);
                     umma_i8_2cta(tmem_base, da, db, kIdesc2, (i > 0 || ks > 0) ? 1u : 0u);
                 }
-                umma_commit_2cta(empty_bar(s), all_mask);
+                umma_commit_2cta(empty_bar(s), 3);
             }
-            umma_commit_2cta(tmem_full_bar, pair_mask);
+            umma_commit_2cta(tmem_full_bar, 3);
 #ifdef PA_GEMM_PROBE
             if (probe_cta) { g.probe[1] = mw; g.probe[3] = clock64() - t_setup; }
 #endif
@@ -1155,38 +1096,18 @@ static int gemm_i8_launch(const int8_t* d_A, const int8_t* d_B, int8_t* d_C_s8, 
     const bool two_cta = plan.two_cta;
     const int n_slabs = plan.n_slabs, m_chunks = plan.m_chunks;
     const int m_tiles0 = M > BM ? 2 : 1;
-    // Cluster multicast of A needs one M chunk (uniform m_tiles) and n_slabs divisible by CL.
-    int CLs = 1;
-    // Measured (profiles/r01_gemm_notes.md): equal speed for CL = 1/2/4 at the C4 shapes -- the
-    // loop is bound by B bytes in flight, not by L2 reads -- so default to pairs, which cut the
-    // L2 read traffic for A in half and never strand SMs.  PA_GEMM_CLUSTER=1|2|4 overrides.
-    if (m_chunks == 1 && !two_cta) {
-        if (n_slabs % 4 == 0) CLs = 4;
-        else if (n_slabs % 2 == 0) CLs = 2;
-    }
-    const int cl_max = CLs;
-    if (CLs > 2) CLs = 2;
-    const char* cl_env = getenv("PA_GEMM_CLUSTER");
-    if (cl_env && !two_cta) {
-        const int want = atoi(cl_env);
-        if (want == 1 || (want == 2 && cl_max >= 2) || (want == 4 && cl_max == 4)) CLs = want;
-    }
     // 1-CTA kernel ring geometry.  M <= 128: load only ceil(M/8)*8 rows of A per stage and use the
     // saved shared memory for a deeper ring (more weight bytes in flight: small-M GEMMs are pure weight
-    // streaming); no cluster multicast in that case.
+    // streaming).
     int a_rows_box = BM, a_bytes = m_tiles0 * TILE_BYTES, stages = STAGES;
     if (!two_cta && M <= BM) {
-        CLs = 1;
         a_rows_box = ((M + 7) / 8) * 8;
         a_bytes = a_rows_box * BK;
         stages = RING_BYTES / (a_bytes + TILE_BYTES);
         if (stages > MAXST) stages = MAXST;
-    } else if (!two_cta && CLs > 1) {
-        a_rows_box = m_tiles0 * BM / CLs;
     }
     CUtensorMap tmA, tmB;
-    const bool mc_pairs = two_cta && n_slabs % 2 == 0 && !(getenv("PA_GEMM_MC") && atoi(getenv("PA_GEMM_MC")) == 0);
-    if (!make_map(&tmA, d_A, (uint64_t)K, (uint64_t)M, (uint64_t)BATCH, two_cta ? (mc_pairs ? BM / 2 : BM) : a_rows_box))
+    if (!make_map(&tmA, d_A, (uint64_t)K, (uint64_t)M, (uint64_t)BATCH, a_rows_box))
         return PA_ERR_UNSUPPORTED;
     if (!make_map(&tmB, d_B, (uint64_t)N, (uint64_t)K, (uint64_t)BATCH, BK)) return PA_ERR_UNSUPPORTED;
 
@@ -1244,8 +1165,6 @@ static int gemm_i8_launch(const int8_t* d_A, const int8_t* d_B, int8_t* d_C_s8, 
                          !(getenv("PA_GEMM_PERSIST") && atoi(getenv("PA_GEMM_PERSIST")) == 0);
     if (persist) {
         // more tiles than one wave of CTA pairs: persistent pairs with double-buffered TMEM accumulators
-        CUtensorMap tmA2;
-        if (!make_map(&tmA2, d_A, (uint64_t)K, (uint64_t)M, (uint64_t)BATCH, BM)) return PA_ERR_UNSUPPORTED;
         using PKernelFn = void (*)(const CUtensorMap, const CUtensorMap, const Args, int, int, int);
         static const PKernelFn pk[4] = {gemm_i8_persist_kernel<0>, gemm_i8_persist_kernel<1>, gemm_i8_persist_kernel<2>,
                                         gemm_i8_persist_kernel<3>};
@@ -1266,7 +1185,7 @@ static int gemm_i8_launch(const int8_t* d_A, const int8_t* d_B, int8_t* d_C_s8, 
         attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        e = cudaLaunchKernelEx(&cfg, kern, tmA2, tmB, g, n_slabs, m_chunks, (int)tiles2);
+        e = cudaLaunchKernelEx(&cfg, kern, tmA, tmB, g, n_slabs, m_chunks, (int)tiles2);
         if (e != cudaSuccess) return (int)e;
         e = cudaGetLastError();
         return e == cudaSuccess ? PA_OK : (int)e;
@@ -1276,27 +1195,20 @@ static int gemm_i8_launch(const int8_t* d_A, const int8_t* d_B, int8_t* d_C_s8, 
         const int64_t pairs = (int64_t)n_slabs * m_chunks * ksplit * BATCH;
         const int occ2 = (pairs > di.sm_count / 2 && !(getenv("PA_GEMM_OCC2") && atoi(getenv("PA_GEMM_OCC2")) == 0)) ? 1 : 0;
         const size_t smem2 = (size_t)(occ2 ? 3 : STAGES2) * STAGE2_BYTES + 128 + 8 * 128 * sizeof(float) + 1024;  // ring, barriers, bias, align
-        // cluster of two pairs sharing A by multicast when the slabs pair up (PA_GEMM_MC=0 turns it off)
-        const int clp2 = mc_pairs ? 1 : 0;
-        static const KernelFn kernels2[2][2][4] = {
-            {{gemm_i8_2cta_kernel<0, 1, 1>, gemm_i8_2cta_kernel<1, 1, 1>, gemm_i8_2cta_kernel<2, 1, 1>, gemm_i8_2cta_kernel<3, 1, 1>},
-             {gemm_i8_2cta_kernel<0, 2, 1>, gemm_i8_2cta_kernel<1, 2, 1>, gemm_i8_2cta_kernel<2, 2, 1>, gemm_i8_2cta_kernel<3, 2, 1>}},
-            {{gemm_i8_2cta_kernel<0, 1, 2>, gemm_i8_2cta_kernel<1, 1, 2>, gemm_i8_2cta_kernel<2, 1, 2>, gemm_i8_2cta_kernel<3, 1, 2>},
-             {gemm_i8_2cta_kernel<0, 2, 2>, gemm_i8_2cta_kernel<1, 2, 2>, gemm_i8_2cta_kernel<2, 2, 2>, gemm_i8_2cta_kernel<3, 2, 2>}}};
-        KernelFn kern = kernels2[clp2][occ2][epi];
+        static const KernelFn kernels2[2][4] = {
+            {gemm_i8_2cta_kernel<0, 1>, gemm_i8_2cta_kernel<1, 1>, gemm_i8_2cta_kernel<2, 1>, gemm_i8_2cta_kernel<3, 1>},
+            {gemm_i8_2cta_kernel<0, 2>, gemm_i8_2cta_kernel<1, 2>, gemm_i8_2cta_kernel<2, 2>, gemm_i8_2cta_kernel<3, 2>}};
+        KernelFn kern = kernels2[occ2][epi];
         if (dq) {
-            static const KernelFn kernels_dq[2][2] = {
-                {gemm_i8_2cta_kernel<1, 1, 1, true>, gemm_i8_2cta_kernel<2, 1, 1, true>},
-                {gemm_i8_2cta_kernel<1, 1, 2, true>, gemm_i8_2cta_kernel<2, 1, 2, true>}};
-            kern = kernels_dq[clp2][act == PA_ACT_RELU ? 1 : 0];
+            kern = act == PA_ACT_RELU ? gemm_i8_2cta_kernel<2, 1, true> : gemm_i8_2cta_kernel<1, 1, true>;
             e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
             if (e != cudaSuccess) return (int)e;
         }
-        static bool attr_set2[64][2][2][4] = {};
-        if (!dq && !attr_set2[dev & 63][clp2][occ2][epi]) {
+        static bool attr_set2[64][2][4] = {};
+        if (!dq && !attr_set2[dev & 63][occ2][epi]) {
             e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
             if (e != cudaSuccess) return (int)e;
-            attr_set2[dev & 63][clp2][occ2][epi] = true;
+            attr_set2[dev & 63][occ2][epi] = true;
         }
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3((unsigned)(2 * n_slabs), (unsigned)(m_chunks * ksplit), (unsigned)BATCH);
@@ -1305,7 +1217,7 @@ static int gemm_i8_launch(const int8_t* d_A, const int8_t* d_B, int8_t* d_C_s8, 
         cfg.stream = st;
         cudaLaunchAttribute attr[2];
         attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = clp2 ? 4u : 2u;
+        attr[0].val.clusterDim.x = 2;
         attr[0].val.clusterDim.y = 1;
         attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
@@ -1328,34 +1240,25 @@ static int gemm_i8_launch(const int8_t* d_A, const int8_t* d_B, int8_t* d_C_s8, 
         if (e != cudaSuccess) return (int)e;
     } else {
         const size_t smem = (size_t)RING_BYTES + (2 * MAXST + 1) * 8 + 16 + 1024;
-        static const KernelFn kernels[3][4] = {
-            {gemm_i8_kernel<0, 1>, gemm_i8_kernel<1, 1>, gemm_i8_kernel<2, 1>, gemm_i8_kernel<3, 1>},
-            {gemm_i8_kernel<0, 2>, gemm_i8_kernel<1, 2>, gemm_i8_kernel<2, 2>, gemm_i8_kernel<3, 2>},
-            {gemm_i8_kernel<0, 4>, gemm_i8_kernel<1, 4>, gemm_i8_kernel<2, 4>, gemm_i8_kernel<3, 4>}};
-        const int cli = CLs == 4 ? 2 : (CLs == 2 ? 1 : 0);
-        KernelFn kern = kernels[cli][epi];
-        static bool attr_set[64][3][4] = {};
-        if (!attr_set[dev & 63][cli][epi]) {
+        static const KernelFn kernels[4] = {gemm_i8_kernel<0>, gemm_i8_kernel<1>, gemm_i8_kernel<2>, gemm_i8_kernel<3>};
+        KernelFn kern = kernels[epi];
+        static bool attr_set[64][4] = {};
+        if (!attr_set[dev & 63][epi]) {
             e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (e != cudaSuccess) return (int)e;
-            attr_set[dev & 63][cli][epi] = true;
+            attr_set[dev & 63][epi] = true;
         }
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3((unsigned)n_slabs, (unsigned)(m_chunks * ksplit), (unsigned)BATCH);
         cfg.blockDim = dim3(NTHREADS);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = st;
-        cudaLaunchAttribute attr[2];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = (unsigned)CLs;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
+        cudaLaunchAttribute attr[1];
         cfg.attrs = attr;
-        cfg.numAttrs = 1;
         if (!(getenv("PA_GEMM_PDL") && atoi(getenv("PA_GEMM_PDL")) == 0)) {
-            attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            attr[1].val.programmaticStreamSerializationAllowed = 1;
-            cfg.numAttrs = 2;
+            attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[0].val.programmaticStreamSerializationAllowed = 1;
+            cfg.numAttrs = 1;
         }
         e = cudaLaunchKernelEx(&cfg, kern, tmA, tmB, g);
         if (e != cudaSuccess) return (int)e;

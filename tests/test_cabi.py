@@ -32,6 +32,16 @@ def test_header_symbols_exported(cabi):
     assert declared == set(cabi.EXPORTS), declared ^ set(cabi.EXPORTS)
 
 
+def test_no_loads_with_cluster_multicast():
+    """The library also runs on several GPUs, where a TMA or bulk load may not carry cluster multicast (tcgen05.commit may)."""
+    src = os.path.join(ROOT, "pagedattention-based-transformer-decoder-inference-framework_b200", "csrc")
+    named = []
+    for f in sorted(os.listdir(src)):
+        text = re.sub(r'"\s*\n\s*"', "", open(os.path.join(src, f)).read())      # pieces of one instruction
+        named += [(f, m) for m in re.findall(r"cp\.async\.bulk[^\s;]*multicast[^\s;]*", text)]
+    assert not named, named
+
+
 def test_version_and_error_strings(cabi):
     lib = cabi.lib()
     assert lib.pa_version() >= 100
