@@ -53,6 +53,57 @@ def test_convolved_rows(heads, kv_heads, dim, vdim, rot_dims, norm, taps, dtype)
         assert torch.equal(out[0][-1], out[1][-1])
 
 
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,rot_dims,norm", [(16, 4, 128, 128, 128, 1), (12, 2, 64, 128, 32, 1), (16, 4, 64, 64, 64, 0),
+                                                                   (8, 4, 104, 104, 104, 1), (5, 3, 40, 64, 8, 1), (7, 1, 72, 40, 0, 1)])
+@pytest.mark.parametrize("taps", [0, 1, 2, 3, 4])
+def test_convolved_rows_of_many_items(heads, kv_heads, dim, vdim, rot_dims, norm, taps):
+    """The form for many long items: portions of one to 64 tokens (whole, ragged and single-token items), two steps of which the second
+    starts inside pages, pages that are missing, pages out of range, a portion whose slot is none."""
+    from llm_decoder import _cabi
+    from llm_decoder.seq_state import SequenceStateCache
+    lib, dev = _cabi.lib(), torch.device("cuda")
+    units, columns, channels = heads + 2 * kv_heads, max(dim, vdim), heads * dim + kv_heads * (dim + vdim)
+    lens = [48, 16, 31, 15, 32, 17, 64, 2, 16, 29]                     # 19 items of 14.2 tokens on average
+    rounds = -(-(20 * _cabi.device_info()[0] * (1 if columns > 64 else 2) // units + 1) // 19)
+    n, g = 10 * rounds, torch.Generator().manual_seed(dim + taps)
+    wt = (torch.randn(taps, channels, generator=g) * 0.6).to(dev) if taps else None
+    steps = [(lens * rounds)[i:] + (lens * rounds)[:i] for i in (0, 3)]
+    raw = [torch.randn(sum(s), channels, generator=g).to(torch.bfloat16) for s in steps]
+    rope = [torch.randn(sum(s), max(rot_dims, 1), generator=g).to(dev) for s in steps]
+    out = []
+    for off, pad in ((8, 0), (1, 3)):
+        states = SequenceStateCache(n, 144 * n, 16, dev)
+        kv = states.add_kv_layer(kv_heads, dim, vdim, "bf16")
+        kv.key_buffer_.zero_(), kv.value_buffer_.zero_()
+        state = states.add_state((taps - 1) * channels) if taps > 1 else None
+        slots, res = [states.alloc() for _ in range(n)], []
+        for step, x0, turns in zip(steps, raw, rope):
+            batch = states.make_batch([(s, [0] * m) for s, m in zip(slots, step)])
+            x = torch.zeros(batch.rows, off + channels + 8 + pad, dtype=torch.bfloat16, device=dev)
+            x[:, off:off + channels] = x0.to(dev)
+            q = torch.zeros(batch.rows, heads * dim, dtype=torch.bfloat16, device=dev)
+            items, count = batch.portion_items(16)
+            assert lib.pa_conv_append_in_words(units, columns, count, batch.rows) == 1
+            items, lost = items.clone(), batch.portions[4]
+            items[(items[:, 0] >= lost[0]) & (items[:, 0] < lost[0] + lost[1]), 2] = n + 3
+            pt = kv.page_table_
+            table = pt.device_data().clone().reshape(n, kv_heads, -1)
+            table[slots[2], :, 0], table[slots[6], 0, 1], table[slots[0], -1, 2] = -1, kv.total_pages_, -1
+            assert lib.pa_conv_rope_norm_append_rows(
+                x.data_ptr(), x.stride(0), off, heads, kv_heads, dim, vdim, taps, _cabi.ptr(wt), _cabi.ptr(state), rot_dims,
+                turns.data_ptr() if rot_dims else None, norm, 1e-5, q.data_ptr(), heads * dim, kv.key_buffer_.data_ptr(), kv.value_buffer_.data_ptr(),
+                table.data_ptr(), pt.num_beams_, pt.num_tiles_, kv.total_pages_, kv.tile_size_, items.data_ptr(), count, 16, batch.rows, 2,
+                _cabi.stream()) == 0
+            q[lost[0]:lost[0] + lost[1]] = 0            # nobody's rows: what they hold is not said
+            res.append(q)
+        out.append(res + [kv.key_buffer_, kv.value_buffer_] + ([state] if state is not None else []))
+    for got, want in zip(*out):
+        assert bool((want != 0).any())
+        _close(got, want, torch.bfloat16)
+    if taps > 1:
+        assert torch.equal(out[0][-1], out[1][-1])
+
+
 def test_form_of_many_items():
     """Where the form for many long items is taken: not for decoded tokens, however many, nor for small heads."""
     from llm_decoder import _cabi
