@@ -48,6 +48,16 @@ MANY_CTX = [[0, 70, 0, 300, 1, 0, 512, 0, 63, 0, 190][i % 11] for i in range(90)
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(10, 2, 128, 128), (10, 2, 64, 128), (8, 2, 128, 64), (6, 3, 64, 64), (8, 8, 128, 128)])
+@pytest.mark.parametrize("mask,size,keep,form", [("causal", 0, 0, "plain"), ("causal", 0, 0, "sink"), ("window", 70, 9, "gate"), ("chunk", 50, 0, "slope"),
+                                                 ("window", 37, 0, "bucket")])
+def test_several_work_items_per_cta(heads, kv_heads, dim, vdim, mask, size, keep, form):
+    """The walk of a CTA over its items: ring, accumulators and query buffers carried over, queries of whole items (TMA) after ragged ones
+    (their threads) and the other way round, a query tile without rows (ten heads over two: the fifth alone) between others."""
+    _paged_portions(heads, kv_heads, dim, vdim, mask, size, keep, form, ctx=MANY_CTX, new=MANY_NEW, per_cta=3 if kv_heads == 2 and dim == 128 else 2)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("form,mask,size", [("plain", "causal", 0), ("slope", "window", 90)])
 def test_work_items_without_tokens(form, mask, size):
     """Items of no tokens among the others, also first and next to each other: nothing to do, and the walk goes on."""
@@ -61,8 +71,9 @@ def test_work_items_without_tokens(form, mask, size):
     _paged_portions(10, 2, 128, 128, mask, size, 0, form, ctx=MANY_CTX, new=MANY_NEW, change=with_empty)
 
 
-def _paged_portions(heads, kv_heads, dim, vdim, mask, size, keep, form, bias_len=23, ctx=CTX, new=NEW, change=None):
-    """change: the list of work items (first row, tokens, slot, first position) -> the one that is launched."""
+def _paged_portions(heads, kv_heads, dim, vdim, mask, size, keep, form, bias_len=23, ctx=CTX, new=NEW, change=None, per_cta=0):
+    """change: the list of work items (first row, tokens, slot, first position) -> the one that is launched.  per_cta: how many of them
+    some CTA has at least, with two query tiles (one CTA an SM)."""
     from llm_decoder import _cabi
     from llm_decoder.hybrid import MASK_KIND
     from llm_decoder.seq_state import SequenceStateCache
@@ -123,11 +134,14 @@ def _paged_portions(heads, kv_heads, dim, vdim, mask, size, keep, form, bias_len
                 s = torch.cat([s, sink[h].double().expand(new[i], 1)], 1)
             want[r0:r0 + new[i], h] = torch.softmax(s, -1)[:, :k.shape[0]] @ v
         r0 += new[i]
+    gate = torch.randn(rows, heads * vdim + 8, generator=g).to(BF) if form == "gate" else None
+    if gate is not None:
+        want *= torch.sigmoid(gate[:, 8:].double()).reshape(rows, heads, vdim)
     if turn is not None:
         u, w = want[..., 0::2].clone(), want[..., 1::2].clone()
         c, s = turn.double()[:, None, :, 0], turn.double()[:, None, :, 1]
         want[..., 0::2], want[..., 1::2] = u * c + w * s, w * c - u * s
-    keepalive = [t.to(dev).contiguous() if t is not None else None for t in (bias, temp, sink, turn)]
+    keepalive = [t.to(dev).contiguous() if t is not None else None for t in (bias, temp, sink, turn, gate)]
     pt = kv.page_table_
     table = pt.device_data()
     for q_tiles, kind in ((2, 4), (1, 5)):
@@ -136,12 +150,15 @@ def _paged_portions(heads, kv_heads, dim, vdim, mask, size, keep, form, bias_len
         if change:
             tiles = torch.tensor(change(tiles.tolist()), dtype=torch.int32, device=dev)
             ntiles = len(tiles)
+        if q_tiles == 2 and form != "bucket":       # tables of biases: a CTA each
+            assert ntiles * lib.pa_masked_attention_tc_units(heads, kv_heads, 2) > (per_cta - 1) * _cabi.device_info()[0]
         out = torch.full((rows, heads * vdim), float("nan"), dtype=BF, device=dev)
         rc = lib.pa_masked_attention_gated(
             proj.data_ptr(), proj.stride(0), 0, kv.key_buffer_.data_ptr(), kv.value_buffer_.data_ptr(), table.data_ptr(), pt.num_beams_,
             pt.num_heads_, pt.num_tiles_, kv.total_pages_, kv.tile_size_, tiles.data_ptr(), ntiles, heads, dim, vdim, scale, cap,
             MASK_KIND[mask], size, keep, bias_kind, _cabi.ptr(keepalive[0]), bias_len if bias_kind == 2 else 0, _cabi.ptr(keepalive[1]),
-            _cabi.ptr(keepalive[2]), _cabi.ptr(keepalive[3]), None, 0, None, None, 0, 0, out.data_ptr(), 2, kind, _cabi.stream())
+            _cabi.ptr(keepalive[2]), _cabi.ptr(keepalive[3]), None, 0, None, _cabi.ptr(keepalive[4]),
+            heads * vdim + 8 if gate is not None else 0, 8 if gate is not None else 0, out.data_ptr(), 2, kind, _cabi.stream())
         assert rc == 0, rc
         _close(out, want.reshape(rows, -1), max(v.abs().max().item() for v in V) * (1.42 if turn is not None else 1.0))
     _no_wait_ran_out(lib)
@@ -152,18 +169,28 @@ def _paged_portions(heads, kv_heads, dim, vdim, mask, size, keep, form, bias_len
 @pytest.mark.parametrize("sink", [False, True])
 def test_expanded_latent_portions(heads, dim, rot_dim, vdim, kv_rank, sink):
     """Rows of several sequences gathered from a paged latent pool, then attention on keys and values given per head."""
+    _expanded_latent_portions(heads, dim, rot_dim, vdim, kv_rank, sink)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads,dim,rot_dim,vdim,kv_rank", [(7, 128, 64, 128, 64), (7, 64, 32, 64, 96)])
+def test_latent_portions_with_several_work_items_per_cta(heads, dim, rot_dim, vdim, kv_rank):
+    _expanded_latent_portions(heads, dim, rot_dim, vdim, kv_rank, True, MANY_CTX, MANY_NEW)
+
+
+def _expanded_latent_portions(heads, dim, rot_dim, vdim, kv_rank, sink, ctx=CTX, new=NEW):
     from llm_decoder import _cabi
     from llm_decoder.seq_state import SequenceStateCache
     lib, dev = _cabi.lib(), torch.device("cuda")
     g = torch.Generator().manual_seed(heads + dim + rot_dim)
-    kd, n = kv_rank + rot_dim, len(NEW)
-    states = SequenceStateCache(n, 4096, 16, dev)
+    kd, n = kv_rank + rot_dim, len(new)
+    states = SequenceStateCache(n, 4096 if n == len(NEW) else sum(ctx) + sum(new) + 16 * n, 16, dev)
     kv = states.add_kv_layer(1, kd, 0, "bf16")
     slots = [states.alloc() for _ in range(n)]
-    for i in (3, 0, 5, 1, 2, 6, 4):
-        if CTX[i]:
-            states.extend(slots[i], CTX[i])
-    batch = states.make_batch([(s, [0] * m) for s, m in zip(slots, NEW)])
+    for i in [3, 0, 5, 1, 2, 6, 4] + list(range(7, n)):
+        if ctx[i]:
+            states.extend(slots[i], ctx[i])
+    batch = states.make_batch([(s, [0] * m) for s, m in zip(slots, new)])
     kv.key_buffer_.copy_(torch.randn(kv.key_buffer_.shape, generator=g))
     pt = kv.page_table_
     groups = batch.whole_sequences(16, 128)
@@ -174,14 +201,14 @@ def test_expanded_latent_portions(heads, dim, rot_dim, vdim, kv_rank, sink):
                                 kd * 2, items.data_ptr(), nitems, longest, lat.data_ptr(), _cabi.stream()) == 0
     tab, pool = pt.device_data().cpu().reshape(pt.num_beams_, pt.num_tiles_), kv.key_buffer_.cpu()
     first = {int(s): int(r) for s, _t, r in items.cpu()}
-    for s, c, m in zip(slots, CTX, NEW):
+    for s, c, m in zip(slots, ctx, new):
         got = lat[first[s]:first[s] + c + m].cpu()
         assert torch.equal(got, torch.stack([pool[int(tab[s, j // 16]), j % 16] for j in range(c + m)]))
     Kn, V = torch.randn(rows, heads * dim, generator=g).to(BF), torch.randn(rows, heads * vdim, generator=g).to(BF)
     Q = torch.randn(batch.rows, heads * (dim + rot_dim), generator=g).to(BF)
     sk = torch.randn(heads, generator=g) if sink else None
     want, r0, scale = torch.zeros(batch.rows, heads, vdim, dtype=torch.float64), 0, 1.5 * (dim + rot_dim) ** -0.5
-    for s, c, m in zip(slots, CTX, NEW):
+    for s, c, m in zip(slots, ctx, new):
         rr = slice(first[s], first[s] + c + m)
         hidden = torch.arange(c + m)[None] > torch.arange(c, c + m)[:, None]
         for h in range(heads):
@@ -195,6 +222,7 @@ def test_expanded_latent_portions(heads, dim, rot_dim, vdim, kv_rank, sink):
     for q_tiles in (2, 1):
         tokens = lib.pa_masked_attention_tc_tile_tokens(1, 1, dim, vdim, 2, q_tiles)
         tiles, ntiles = batch.whole_sequences(16, tokens)[0][4:]
+        assert n == len(NEW) or ntiles * heads > 3 * _cabi.device_info()[0]
         out = torch.full((batch.rows, heads * vdim), float("nan"), dtype=BF, device=dev)
         assert lib.pa_latent_attention_expanded(Qd.data_ptr(), Qd.stride(0), 0, Kd.data_ptr(), Kd.stride(0), lat.data_ptr(), kd, kv_rank,
                                                 Vd.data_ptr(), Vd.stride(0), rows, tiles.data_ptr(), ntiles, heads, dim, rot_dim, vdim, scale,

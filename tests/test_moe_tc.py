@@ -16,7 +16,9 @@ BF = torch.bfloat16
 @pytest.mark.gpu
 @pytest.mark.parametrize("rows,experts,top,width,ff", [(700, 3, 2, 192, 264), (257, 2, 1, 64, 520), (1300, 20, 2, 136, 128), (129, 1, 1, 72, 8),
                                                         # from 6144 pairs and 256 an expert on also by pairs of CTAs, tiles of 256
-                                                        (6144, 1, 1, 72, 8), (3300, 3, 2, 136, 264), (3205, 24, 2, 320, 136)])
+                                                        (6144, 1, 1, 72, 8), (3300, 3, 2, 136, 264), (3205, 24, 2, 320, 136),
+                                                        # several tiles for each pair: up, down
+                                                        (3200, 2, 2, 136, 3208), (3200, 2, 2, 3080, 136)])
 @pytest.mark.parametrize("act,gated,weighted", [(0, True, False), (1, True, True), (2, False, False)])
 def test_grouped_products(rows, experts, top, width, ff, act, gated, weighted):
     from llm_decoder import _cabi
