@@ -652,6 +652,8 @@ int pa_moe_up(const void* d_h, int64_t ldh, const void* d_w_up, int width, int f
 /* pa_moe_gate_up_act (gated 1) or pa_moe_up (0) with scratch for the rows of the pairs in sorted order, which the products of large
  * batches read faster than scattered ones: pa_moe_sorted_rows_bytes (0: the launch has no use for it; d_rows may be NULL). */
 size_t pa_moe_sorted_rows_bytes(int pairs, int experts, int width, int elem);
+/* The same, and 0 also where the launch takes longer with it. */
+size_t pa_moe_sorted_rows_worth(int pairs, int experts, int width, int ff, int gated, int elem);
 int pa_moe_up_sorted(const void* d_h, int64_t ldh, const void* d_w, int gated, int width, int ff, int experts, const int32_t* d_order,
                      const float* d_sel_w, int top, const int32_t* d_meta, int pairs, int act, void* d_act, void* d_rows,
                      size_t rows_bytes, int elem, pa_stream_t stream);

@@ -622,8 +622,9 @@ __global__ void __launch_bounds__(kSkWarps * 32) grouped_skinny_kernel(const bf1
 // moe_tc.cu: the tcgen05 form of the grouped products (PA_ERR_UNSUPPORTED: operands that stay on the kernels here)
 int grouped_tc_launch(int mode, const void* A, int64_t lda, const void* W, int K, int n_out, int experts, const int32_t* order,
                       const float* a_scale, int top, const int32_t* offsets, int pairs, int act, void* out, cudaStream_t st,
-                      void* rows = nullptr, int polls = 1 << 25, int first_polls = 1 << 25, int second_polls = 1 << 25);
+                      bool pair, void* rows = nullptr, int polls = 1 << 25, int first_polls = 1 << 25, int second_polls = 1 << 25);
 bool grouped_tc_pairs_up(int pairs, int experts);
+bool grouped_tc_pairs_pay(int mode, int pairs, int experts, int K, int n_out);
 
 static bool mma_ok(const void* A, int64_t lda, const void* W, int K) {
     return K % 8 == 0 && lda % 8 == 0 && (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0;
@@ -713,7 +714,8 @@ static int moe_gate_up(const void* d_h, int64_t ldh, const void* d_w_gate_up, in
         PA_RETURN_LAUNCH_STATUS();
     }
     if (elem == 2 && mma_ok(d_h, ldh, d_w_gate_up, width)) {
-        const int st = grouped_tc_launch(0, d_h, ldh, d_w_gate_up, width, ff, experts, d_order, d_sel_w, top, d_meta, pairs, act, d_act, as_stream(stream), d_rows);
+        const int st = grouped_tc_launch(0, d_h, ldh, d_w_gate_up, width, ff, experts, d_order, d_sel_w, top, d_meta, pairs, act, d_act, as_stream(stream),
+                                         grouped_tc_pairs_up(pairs, experts), d_rows);
         if (st != PA_ERR_UNSUPPORTED) return st;
         grouped_mma_kernel<0><<<grid, 128, 0, as_stream(stream)>>>(
             static_cast<const bf16_t*>(d_h), ldh, static_cast<const bf16_t*>(d_w_gate_up), width, ff, d_order, d_sel_w, top,
@@ -754,7 +756,8 @@ static int moe_up(const void* d_h, int64_t ldh, const void* d_w_up, int width, i
         PA_RETURN_LAUNCH_STATUS();
     }
     if (elem == 2 && mma_ok(d_h, ldh, d_w_up, width)) {
-        const int st = grouped_tc_launch(2, d_h, ldh, d_w_up, width, ff, experts, d_order, d_sel_w, top, d_meta, pairs, act, d_act, as_stream(stream), d_rows);
+        const int st = grouped_tc_launch(2, d_h, ldh, d_w_up, width, ff, experts, d_order, d_sel_w, top, d_meta, pairs, act, d_act, as_stream(stream),
+                                         grouped_tc_pairs_up(pairs, experts), d_rows);
         if (st != PA_ERR_UNSUPPORTED) return st;
         grouped_mma_kernel<2><<<dim3(nt, (unsigned)((ff + 127) / 128)), 128, 0, as_stream(stream)>>>(
             static_cast<const bf16_t*>(d_h), ldh, static_cast<const bf16_t*>(d_w_up), width, ff, d_order, d_sel_w, top, tiles,
@@ -776,6 +779,11 @@ PA_API int pa_moe_up(const void* d_h, int64_t ldh, const void* d_w_up, int width
 PA_API size_t pa_moe_sorted_rows_bytes(int pairs, int experts, int width, int elem) {
     return elem == 2 && pairs > 0 && experts > 0 && width > 0 && !skinny_ok(pairs, experts) && grouped_tc_pairs_up(pairs, experts)
                ? (size_t)pairs * width * 2 : 0;
+}
+
+PA_API size_t pa_moe_sorted_rows_worth(int pairs, int experts, int width, int ff, int gated, int elem) {
+    return ff > 0 && experts > 0 && pairs > 0 && grouped_tc_pairs_pay(gated ? 0 : 2, pairs, experts, width, ff)
+               ? pa_moe_sorted_rows_bytes(pairs, experts, width, elem) : 0;
 }
 
 PA_API int pa_moe_up_sorted(const void* d_h, int64_t ldh, const void* d_w, int gated, int width, int ff, int experts, const int32_t* d_order,
@@ -800,7 +808,8 @@ PA_API int pa_moe_down(const void* d_act, const void* d_w_down, int ff, int widt
         PA_RETURN_LAUNCH_STATUS();
     }
     if (elem == 2 && mma_ok(d_act, ff, d_w_down, ff)) {
-        const int st = grouped_tc_launch(1, d_act, ff, d_w_down, ff, width, experts, d_order, nullptr, 1, d_meta, pairs, 0, d_out_pairs, as_stream(stream));
+        const int st = grouped_tc_launch(1, d_act, ff, d_w_down, ff, width, experts, d_order, nullptr, 1, d_meta, pairs, 0, d_out_pairs, as_stream(stream),
+                                         grouped_tc_pairs_pay(1, pairs, experts, ff, width));
         if (st != PA_ERR_UNSUPPORTED) return st;
         dim3 g2((unsigned)pa_moe_max_tiles(pairs, experts), (unsigned)((width + 127) / 128));
         grouped_mma_kernel<1><<<g2, 128, 0, as_stream(stream)>>>(

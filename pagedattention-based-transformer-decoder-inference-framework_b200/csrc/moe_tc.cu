@@ -33,9 +33,7 @@ using namespace tc;
 constexpr int BM = 128, BN = 256, BK = 64;      // rows of a CTA's accumulator, its columns, and columns of a stage
 constexpr int A_BYTES = BM * 128;
 constexpr int kMostExperts = 1024;
-// Pairs of CTAs pay from here on, where their 74 walkers have more than one round of tiles: gate / up with its sorted rows 65 and 73 us,
-// down 35 and 38 us at 8192 pairs of 8 experts, but 50 and 40, 28 and 23 us at 4096 (width 2048, ff 1024).
-constexpr int kPairFrom = 6144;
+constexpr int kPairFrom = 6144;                 // pairs (of row and expert) below which no launch goes by pairs of CTAs
 __host__ __device__ constexpr int b_bytes(int ctas) { return BN / ctas * 128; }
 __host__ __device__ constexpr int stages_for(int ctas) { return ctas == 2 ? 6 : 4; }
 
@@ -476,14 +474,30 @@ __global__ void __launch_bounds__(256) sorted_rows_kernel(const uint4* __restric
 
 }  // namespace mtc
 
-// Whether a launch of this many pairs goes by pairs of CTAs: enough tiles for them, and rows enough for tiles of 256.
+// Whether a launch of this many pairs can go by pairs of CTAs: enough of them, and rows enough for tiles of 256.
 bool grouped_tc_pairs_up(int pairs, int experts) { return pairs >= mtc::kPairFrom && (int64_t)pairs >= 256ll * experts; }
 
-// mode 0: gate / up pairs, 1: down (rows scattered to (row, choice) order as float), 2: up.  PA_ERR_UNSUPPORTED: the caller's other
-// kernels serve these operands.
+// Whether it should.  A tile of a pair takes 0.8 of the time of the two tiles of one CTA each, against which stand (us of one CTA a tile and
+// of pairs, with the sorted rows where they are needed, 8 experts):
+//  - a last tile of 256 that is half empty, for every expert: 1024 rows each are asked for (16 experts, down with ff 1024, width 2048:
+//    8192 pairs 43.6 and 44.8, 16384 pairs 74.6 and 67.1);
+//  - walkers with one round of tiles and little more: two are asked for (down, ff 1024, width 1024: 8192 pairs = 128 tiles 21.8 and 22.2,
+//    12288 pairs 32.6 and 30.6);
+//  - a tile's start and end, which few columns do not hide, and the activations: down asks for 1024 columns (8192 pairs, width 2048, ff 512:
+//    27.9 and 30.2, ff 1024: 41.9 and 38.0), gate / up for 2048 (16384 pairs, ff 2048, width 1024: 146 and 169, width 2048: 243 and 220);
+//  - for gate / up the copy of the rows, which the tiles of a row share: twelve strips (16384 pairs, width 2048, ff 512: 75 and 86, ff 1024: 134
+//    and 131, ff 1536: 184 and 179; width 4096, ff 1024: 240 and 239, ff 2048: 456 and 420).
+bool grouped_tc_pairs_pay(int mode, int pairs, int experts, int K, int n_out) {
+    const int strip = mode == 0 ? mtc::BN / 2 : mtc::BN, strips = (n_out + strip - 1) / strip;
+    return grouped_tc_pairs_up(pairs, experts) && (int64_t)pairs >= 1024ll * experts && (int64_t)(pairs / 256) * strips >= device_info().sm_count &&
+           (mode == 1 ? K >= 1024 : K >= 2048 && strips >= 12);
+}
+
+// mode 0: gate / up pairs, 1: down (rows scattered to (row, choice) order as float), 2: up.  pair: by pairs of CTAs, which modes 0 and 2
+// do where they are given scratch for the sorted rows.  PA_ERR_UNSUPPORTED: the caller's other kernels serve these operands.
 int grouped_tc_launch(int mode, const void* A, int64_t lda, const void* W, int K, int n_out, int experts, const int32_t* order,
-                      const float* a_scale, int top, const int32_t* offsets, int pairs, int act, void* out, cudaStream_t st, void* rows, int polls, int first_polls,
-                      int second_polls) {
+                      const float* a_scale, int top, const int32_t* offsets, int pairs, int act, void* out, cudaStream_t st, bool pair, void* rows, int polls,
+                      int first_polls, int second_polls) {
     using namespace mtc;
     const int64_t w_rows = (int64_t)experts * n_out * (mode == 0 ? 2 : 1);
     if (K % 8 || n_out % 8 || experts > kMostExperts || w_rows >= 0x7fffff00ll || (uintptr_t)out % 16) return PA_ERR_UNSUPPORTED;
@@ -491,7 +505,7 @@ int grouped_tc_launch(int mode, const void* A, int64_t lda, const void* W, int K
     CUtensorMap tmA, tmW;
     if (!make_bf16_map(&tmW, W, w_rows, K, K, BN / 2)) return PA_ERR_UNSUPPORTED;
     tmA = tmW;
-    const bool pair = grouped_tc_pairs_up(pairs, experts) && (mode == 1 || (rows && (uintptr_t)rows % 16 == 0));
+    if (mode != 1 && (!rows || (uintptr_t)rows % 16)) pair = false;
     if (mode == 1 && !make_bf16_map(&tmA, A, pairs, K, lda, BM)) return PA_ERR_UNSUPPORTED;
     if (mode != 1 && pair) {
         if (!make_bf16_map(&tmA, rows, pairs, K, K, BM)) return PA_ERR_UNSUPPORTED;
@@ -520,8 +534,8 @@ PA_API int pa_moe_grouped_waits(int mode, const void* d_a, int64_t lda, const vo
                  act >= 0 && act <= 2 && polls >= 0 && first_polls >= 0 && second_polls >= 0);
     if (pairs == 0) return PA_OK;
     if (d_rows && rows_bytes < (size_t)pairs * K * 2) return PA_ERR_WORKSPACE;
-    return grouped_tc_launch(mode, d_a, lda, d_w, K, n_out, experts, d_order, d_a_scale, top, d_meta, pairs, act, d_out, as_stream(stream), d_rows,
-                             polls, first_polls, second_polls);
+    return grouped_tc_launch(mode, d_a, lda, d_w, K, n_out, experts, d_order, d_a_scale, top, d_meta, pairs, act, d_out, as_stream(stream),
+                             grouped_tc_pairs_up(pairs, experts), d_rows, polls, first_polls, second_polls);
 }
 
 PA_API int pa_moe_grouped_polls(int mode, const void* d_a, int64_t lda, const void* d_w, int K, int n_out, int experts, const int32_t* d_order,

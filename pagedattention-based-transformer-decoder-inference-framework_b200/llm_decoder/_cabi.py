@@ -150,6 +150,7 @@ _SIGS = {
     "pa_moe_down": ([_vp, _vp, _i32, _i32, _i32, _vp, _vp, _i32, _vp, _i32, _vp], _i32),
     "pa_moe_gate_up_act": ([_vp, _i64, _vp, _i32, _i32, _i32, _vp, _vp, _i32, _vp, _i32, _i32, _vp, _i32, _vp], _i32),
     "pa_moe_sorted_rows_bytes": ([_i32, _i32, _i32, _i32], _sz),
+    "pa_moe_sorted_rows_worth": ([_i32, _i32, _i32, _i32, _i32, _i32], _sz),
     "pa_moe_up_sorted": ([_vp, _i64, _vp, _i32, _i32, _i32, _i32, _vp, _vp, _i32, _vp, _i32, _i32, _vp, _vp, _sz, _i32, _vp], _i32),
     "pa_moe_up": ([_vp, _i64, _vp, _i32, _i32, _i32, _vp, _vp, _i32, _vp, _i32, _i32, _vp, _i32, _vp], _i32),
     "pa_embedding_rows_scaled": ([_vp, _i32, _vp, _i32, _i32, _i32, _f32, _vp, _vp], _i32),

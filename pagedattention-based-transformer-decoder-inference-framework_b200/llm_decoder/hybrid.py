@@ -1171,7 +1171,7 @@ class MoEFF:
         _chk(lib.pa_moe_sort(sel_id.data_ptr(), pairs, self.experts, order.data_ptr(), meta.data_ptr(), s), "pa_moe_sort")
         act = c.empty(pairs, self.ff)
         in_w = sel_w.data_ptr() if self.weight_on == "input" else None
-        nb = lib.pa_moe_sorted_rows_bytes(pairs, self.experts, wdt, c.elem)
+        nb = lib.pa_moe_sorted_rows_worth(pairs, self.experts, wdt, self.ff, 1 if self.gated else 0, c.elem)
         rows = c.empty(nb, dtype=torch.uint8) if nb else None
         _chk(lib.pa_moe_up_sorted(h.data_ptr(), h.stride(0), self.w_gate_up.data_ptr(), 1 if self.gated else 0, wdt, self.ff,
                                   self.experts, order.data_ptr(), in_w, self.top, meta.data_ptr(), pairs, self.act, act.data_ptr(),

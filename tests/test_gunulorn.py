@@ -789,19 +789,19 @@ def test_large_step_with_identity_outputs():
     of large steps read rows in the sorted order, which ends before these pairs.  Bound: an activation carries three roundings to
     bfloat16, doubled in the product of gate and up (4 * 2^-9 of the largest), the second product is float; asked is twice that."""
     from llm_decoder import hybrid
-    experts, rows, width, ff = 8, 4096, 128, 64
+    experts, rows, width, ff = 4, 4096, 2048, 1536
     config = R.make_config([R.conv_layer(mlp=R.moe_mlp(experts=experts, identity=2, top=2, ff=ff))], width=width)
     W = R.random_weights(config)
     model = _model(config, W, "bfloat16", max_tokens=rows)
     batch = model.states.make_batch([(model.states.alloc(), [0] * rows)])
     h = torch.randn(rows, width, generator=torch.Generator().manual_seed(2)).to(torch.bfloat16)
     out = model.layers[0].ff.forward(hybrid._Ctx(model, batch), h.cuda())
-    ids, routed = out["sel_id"].cpu(), out["routed"].double().cpu()
-    assert int((ids >= experts).sum()) > 0 and model._lib.pa_moe_sorted_rows_bytes(2 * rows, experts, width, 2) > 0
-    x = h.double().repeat_interleave(2, 0)
+    ids, routed = out["sel_id"], out["routed"].double()
+    assert int((ids >= experts).sum()) > 0 and model._lib.pa_moe_sorted_rows_worth(2 * rows, experts, width, ff, 1, 2) > 0
+    x = h.cuda().double().repeat_interleave(2, 0)
     for e in range(experts):
         r = ids == e
-        gate, up, down = (W["l0.mlp.e%d.%s" % (e, n)].to(torch.bfloat16).double() for n in ("gate", "up", "down"))
+        gate, up, down = (W["l0.mlp.e%d.%s" % (e, n)].cuda().double() for n in ("gate", "up", "down"))
         z = x[r] @ gate.T
         mid = z * torch.sigmoid(z) * (x[r] @ up.T)
         assert ((routed[r] - mid @ down.T).abs() <= 8 * 2.0 ** -9 * mid.abs().max() * down.abs().sum(1)).all()

@@ -54,6 +54,11 @@ def test_grouped_products(rows, experts, top, width, ff, act, gated, weighted):
         assert torch.equal(mid, mid2)
     _cabi.check(lib.pa_moe_down(mid.data_ptr(), wdd.data_ptr(), ff, width, experts, order.data_ptr(), meta.data_ptr(), pairs, out.data_ptr(), 2,
                                 s()), "down")
+    if nb:                      # by pairs of CTAs whether or not they pay at this size
+        out2 = torch.full_like(out, float("nan"))
+        _cabi.check(lib.pa_moe_grouped_polls(1, mid.data_ptr(), ff, wdd.data_ptr(), ff, width, experts, order.data_ptr(), None, 1, meta.data_ptr(),
+                                             pairs, 0, out2.data_ptr(), 1 << 25, s()), "down by pairs")
+        assert torch.equal(out, out2)
     o = order.long().cpu()
     assert sorted(o.tolist()) == list(range(pairs)) and bool((ids[o][1:] >= ids[o][:-1]).all())
     a = h[o // top].double() * (sel_w[o].double()[:, None] if weighted else 1.0)
@@ -151,3 +156,16 @@ def test_silu_of_large_negative_gates(rows):
     g = gates.double()
     want = g / (1.0 + torch.exp(-g)) * 2.0 ** 101
     assert ((out.double().cpu() - want).abs() <= (2.0 ** -8 + 2.0 ** -20) * want.abs()).all()
+
+
+@pytest.mark.gpu
+def test_where_pairs_of_ctas_pay():
+    """The rule asks for full tiles, two rounds of them, and enough columns; what it names is what the scratch is for."""
+    from llm_decoder import _cabi
+    lib = _cabi.lib()
+    worth = lambda *a: lib.pa_moe_sorted_rows_worth(*a, 2)  # noqa: E731
+    assert worth(16384, 8, 2048, 2048, 1) == 16384 * 2048 * 2 == worth(16384, 8, 2048, 3072, 0)
+    assert worth(16384, 16, 2048, 2048, 1) > 0 and worth(8192, 8, 4096, 1536, 1) > 0
+    for few in ((16384, 8, 2048, 1024, 1), (16384, 8, 2048, 2048, 0), (16384, 8, 1024, 4096, 1), (8192, 16, 2048, 2048, 1), (4096, 4, 2048, 4096, 1)):
+        assert worth(*few) == 0
+    assert lib.pa_moe_sorted_rows_worth(16384, 8, 2048, 2048, 1, 4) == 0
