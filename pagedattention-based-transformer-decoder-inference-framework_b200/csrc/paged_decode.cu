@@ -22,6 +22,7 @@
 //     handed out through a global atomic counter (dynamic balance; a static
 //     equal split lost ~4% to SM-to-SM rate differences, profiles/), each chunk
 //     emits an (m, l, O) partial that a small combine kernel merges per row.
+#include <atomic>
 #include <cstdlib>
 
 #include "mma_utils.cuh"
@@ -1626,7 +1627,15 @@ static int launch_decode(DecodeArgs& a, bool overlap, void* ws, size_t ws_bytes,
     const bool no_memset = xch_tail && static_chunks;
     if (no_memset) a.row_done = a.xch_epochs + rows;
     auto kern = fused_merge ? paged_decode_overlap_kernel<D, KV, NWk, S, true> : paged_decode_overlap_kernel<D, KV, NWk, S, false>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // Asked for once per kernel and device: the runtime's look-up of a kernel costs 0.1 to 0.2 us (by how many the library has), of a call
+    // of 8.  Always the device's most, so that calls of other sizes and threads find it enough.
+    static std::atomic<bool> allowed[64][2];
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess && !allowed[dev & 63][fused_merge].load(std::memory_order_acquire)) {
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, di.max_smem_optin);
+        if (e == cudaSuccess) allowed[dev & 63][fused_merge].store(true, std::memory_order_release);
+    }
     if (e != cudaSuccess) return (int)e;
     if (!no_memset) e = cudaMemsetAsync(ws, 0, fused_merge ? ws_header_bytes(rows) : sizeof(unsigned int), st);
     if (e != cudaSuccess) return (int)e;
