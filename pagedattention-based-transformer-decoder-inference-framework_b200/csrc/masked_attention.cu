@@ -530,13 +530,7 @@ __global__ void __launch_bounds__(kCaThreads, EPL == 4 && TAPS <= 4 ? 5 : 1) con
     }
 }
 
-// The same for many items of bfloat16 rows of whole 16-byte words, heads of at most 128: a unit is LANES lanes with eight columns
-// each, a CTA has one item and kCaThreads / LANES of its units.  Tokens go two at a time: their sums of squares are reduced
-// together, so that one chain of shuffles serves two rows, and the raw rows of the four after them are on their way meanwhile.
-// The turns of sixteen tokens are staged in shared memory, where all units of the CTA read them.
-// What bounds it: instructions and occupancy (128 registers); 4 x 2048 tokens, 16 + 2 x 4 heads of 128, four taps (100 MB): 37 us
-// = 2.7 TB/s, the form above 52 us.  64 decoded tokens: 6.5 and 3.9 us, so that few items stay with the form above (ca_dispatch).
-// the same as pairs
+// a word's columns, and as many floats, as pairs
 template <typename T, int EPL>
 __device__ __forceinline__ void ca_word_pairs(const CaWord<T, EPL>& r, uint64_t (&f)[EPL / 2]) {
     float x[EPL];
@@ -552,6 +546,12 @@ __device__ __forceinline__ void ca_load_pairs(const float* __restrict__ p, uint6
     for (int i = 0; i < EPL / 2; ++i) f[i] = f32x2::pack2(x[2 * i], x[2 * i + 1]);
 }
 
+// The same for many items of bfloat16 rows of whole 16-byte words, heads of at most 128: a unit is LANES lanes with eight columns
+// each, a CTA has one item and kCaThreads / LANES of its units.  Tokens go two at a time: their sums of squares are reduced
+// together, so that one chain of shuffles serves two rows, and the raw rows of the four after them are on their way meanwhile.
+// The turns of sixteen tokens are staged in shared memory, where all units of the CTA read them.
+// What bounds it: instructions and occupancy (128 registers); 4 x 2048 tokens, 16 + 2 x 4 heads of 128, four taps (100 MB): 37 us
+// = 2.7 TB/s, the form above 52 us.  Which of the two serves: ca_words_pay.
 constexpr int kCaTurns = 16;        // tokens whose turns are staged together
 constexpr int kCaWordTokens = 12;   // tokens an item (on average) from which on this form is taken, see ca_words_pay
 

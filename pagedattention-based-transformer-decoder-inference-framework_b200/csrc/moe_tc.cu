@@ -4,7 +4,7 @@
 //
 // Persistent: one CTA per SM walks tiles of 128 sorted pairs x 256 weight rows (MODE 0: 128 gate rows and the matching 128 up
 // rows) of one expert, the row tiles of a strip of weight rows next to each other so that the strip stays in L2.  Large batches go
-// by pairs of CTAs (cta_group::2): 256 sorted pairs x 256 weight rows, each CTA with its 128 rows and a half of the weight rows, so
+// by pairs of CTAs (cta_group::2) where that pays (grouped_tc_pairs_pay): 256 sorted pairs x 256 weight rows, each CTA with its 128 rows and a half of the weight rows, so
 // that a stage is 32 KB instead of 48.
 //   warp 0        TMA: weight boxes of 128 rows x 64 columns, and the rows of A where they are sorted (MODE 1: the activations; pairs
 //                 of CTAs: the token rows, copied into sorted order beforehand, which at 2048 columns takes 1.2 ns a row)
@@ -16,8 +16,8 @@
 // A routing weight on the expert's input is applied to the accumulated product, which is linear in it.
 //
 // What bounds it: the products' issue (a stage's 512 cycles of tensor pipe come every 740 in the pair) and, for down, the float
-// rows (134 MB).  Measured, 16384 pairs of 8 experts, width 2048, ff 1024: gate / up 97 us and 20 us for the sorted rows, one CTA
-// 134 us (with four epilogue warps 203 us); down 61 us, one CTA 67 us.
+// rows (134 MB).  Measured, 16384 pairs of 8 experts, width 2048: ff 1024 gate / up 134 us (with four epilogue warps 164; by pairs of CTAs
+// with the copy of the rows 131), down 65 us (one CTA 71); ff 2048 gate / up 220 us (one CTA 243), down 108 us (119).
 //
 // Every wait is bounded: on a protocol error the CTA raises a flag (pa_moe_tc_errors), lets its copies land, frees its TMEM and
 // writes NaN into the rows of its tiles from there on.  A pair raises it in both CTAs: warps that gave up go through their tiles
