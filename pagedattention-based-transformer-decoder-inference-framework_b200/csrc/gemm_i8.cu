@@ -26,6 +26,7 @@
 #include <cstdlib>
 #include <mutex>
 
+#include "cta_pair.cuh"
 #include "pa_common.cuh"
 
 namespace pa {
@@ -77,15 +78,6 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
         "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
         ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
         : "memory");
-}
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tmem_alloc(uint32_t smem_dst, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols));
@@ -425,15 +417,6 @@ constexpr int NTHREADS2 = 320;
 constexpr uint32_t kIdesc2 = (2u << 4) | (1u << 7) | (1u << 10) | (0u << 15) | (1u << 16) |
                              ((uint32_t)(BN2 >> 3) << 17) | ((uint32_t)((2 * BM) >> 4) << 24);
 
-__device__ __forceinline__ uint32_t mapa_shared(uint32_t addr, uint32_t cta_rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(cta_rank));
-    return r;
-}
-__device__ __forceinline__ void mbar_remote_arrive_expect_tx(uint32_t cluster_addr, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cluster.b64 _, [%0], %1;" ::"r"(cluster_addr), "r"(bytes)
-                 : "memory");
-}
 __device__ __forceinline__ void tma_load_3d_2cta(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2,
                                                  uint32_t bar_cluster_addr) {
     asm volatile(
@@ -441,13 +424,6 @@ __device__ __forceinline__ void tma_load_3d_2cta(uint32_t dst, const CUtensorMap
         "[%0], [%1, {%3, %4, %5}], [%2];"
         ::"r"(dst), "l"(map), "r"(bar_cluster_addr), "r"(c0), "r"(c1), "r"(c2)
         : "memory");
-}
-__device__ __forceinline__ void tmem_alloc2(uint32_t smem_dst, uint32_t ncols) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
-}
-__device__ __forceinline__ void tmem_dealloc2(uint32_t taddr, uint32_t ncols) {
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols));
 }
 __device__ __forceinline__ void umma_i8_2cta(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                              uint32_t accumulate) {
@@ -457,10 +433,6 @@ __device__ __forceinline__ void umma_i8_2cta(uint32_t d_tmem, uint64_t a_desc, u
         "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
-}
-__device__ __forceinline__ void umma_commit_2cta(uint32_t bar, uint16_t mask) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                 ::"r"(bar), "h"(mask) : "memory");
 }
 // OCC = 2 (used when the grid has more CTA pairs than one wave): two CTAs per SM with a 3-stage ring each (same
 // bytes in flight per SM, 2 x 256 TMEM columns), so the epilogue, set-up and pipeline fill of one tile run under
@@ -511,7 +483,7 @@ gemm_i8_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tmA));
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tmB));
     }
-    if (warp == 1) tmem_alloc2(tmem_slot, BN2);
+    if (warp == 1) tmem_alloc_pair(tmem_slot, BN2);
     tc_fence_before();
     __syncthreads();
     cluster_sync();  // both CTAs' barriers initialised and TMEM allocated before any cross-CTA signal
@@ -569,9 +541,9 @@ gemm_i8_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                     const uint64_t db = make_desc(st + TILE_BYTES + ks * UK * BK, TILE_BYTES, 1024);
                     umma_i8_2cta(tmem_base, da, db, kIdesc2, (i > 0 || ks > 0) ? 1u : 0u);
                 }
-                umma_commit_2cta(empty_bar(s), 3);
+                umma_commit_pair(empty_bar(s));
             }
-            umma_commit_2cta(tmem_full_bar, 3);
+            umma_commit_pair(tmem_full_bar);
 #ifdef PA_GEMM_PROBE
             if (probe_cta) { g.probe[1] = mw; g.probe[3] = clock64() - t_setup; }
 #endif
@@ -780,7 +752,7 @@ gemm_i8_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     cluster_sync();  // the peer may still be reading its accumulators / signalling this CTA's barriers
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc2(tmem_base, BN2);
+        tmem_dealloc_pair(tmem_base, BN2);
     }
 }
 
@@ -799,9 +771,6 @@ __device__ __forceinline__ void mbar_wait_trap(uint32_t bar, uint32_t parity) {
     while (!mbar_try_wait(bar, parity)) {
         if (++n > (1u << 27)) __trap();
     }
-}
-__device__ __forceinline__ void mbar_remote_arrive(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 
 template <int EPI>
@@ -836,7 +805,7 @@ gemm_i8_persist_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tmA));
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tmB));
     }
-    if (warp == 1) tmem_alloc2(tmem_slot, 2 * BN2);
+    if (warp == 1) tmem_alloc_pair(tmem_slot, 2 * BN2);
     tc_fence_before();
     __syncthreads();
     cluster_sync();
@@ -889,9 +858,9 @@ gemm_i8_persist_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
                         const uint64_t db = make_desc(st + TILE_BYTES + ks * UK * BK, TILE_BYTES, 1024);
                         umma_i8_2cta(tmem_base + buf * BN2, da, db, kIdesc2, (i > 0 || ks > 0) ? 1u : 0u);
                     }
-                    umma_commit_2cta(empty_bar(s), 3);
+                    umma_commit_pair(empty_bar(s));
                 }
-                umma_commit_2cta(tfull_bar(buf), 3);
+                umma_commit_pair(tfull_bar(buf));
             }
         }
     } else {
@@ -980,7 +949,7 @@ gemm_i8_persist_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     cluster_sync();
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc2(tmem_base, 2 * BN2);
+        tmem_dealloc_pair(tmem_base, 2 * BN2);
     }
 }
 

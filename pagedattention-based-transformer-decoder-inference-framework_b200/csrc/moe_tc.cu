@@ -22,6 +22,7 @@
 // Every wait is bounded: on a protocol error the CTA raises a flag (pa_moe_tc_errors), lets its copies land, frees its TMEM and
 // writes NaN into the rows of its tiles from there on.  A pair raises it in both CTAs: warps that gave up go through their tiles
 // without waiting, so what they signal no longer says that an accumulator has been read, and no further product may be issued.
+#include "cta_pair.cuh"
 #include "seq_common.cuh"
 #include "tcgen05_utils.cuh"
 
@@ -37,38 +38,11 @@ constexpr int kPairFrom = 6144;                 // pairs (of row and expert) bel
 __host__ __device__ constexpr int b_bytes(int ctas) { return BN / ctas * 128; }
 __host__ __device__ constexpr int stages_for(int ctas) { return ctas == 2 ? 6 : 4; }
 
-// ---- the pair: tcgen05 with cta_group::2, barriers of the other CTA
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t mapa_shared(uint32_t addr, uint32_t cta_rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(cta_rank));
-    return r;
-}
-__device__ __forceinline__ void remote_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void remote_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cluster.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
+// ---- the pair (cta_pair.cuh)
 // a box into this CTA's shared memory, its bytes counted by a barrier of the pair's first CTA
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
                  "l"(map), "r"(bar), "r"(c0), "r"(c1) : "memory");
-}
-__device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_dst, uint32_t ncols) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
-}
-__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols));
 }
 __device__ __forceinline__ void umma_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
@@ -77,9 +51,6 @@ __device__ __forceinline__ void umma_f16_pair(uint32_t d_tmem, uint64_t a_desc, 
         "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
-}
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {        // at both CTAs
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
 }
 // tc_wait for arrivals of the other CTA
 __device__ __forceinline__ bool try_pair(uint32_t bar, uint32_t parity) {
@@ -238,7 +209,7 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                     if (PAIR) {             // this CTA's rows, and its half of the weight rows
                         const uint32_t bar = mapa_shared(full(s), 0);
                         if (rank == 0) mbar_arrive_expect_tx(full(s), bytes);
-                        else remote_expect_tx(bar, bytes);
+                        else mbar_remote_arrive_expect_tx(bar, bytes);
                         tma_load_2d_pair(st + A_BYTES, &tmW, kt * BK, rank == 0 ? r1 : r2, bar);
                         tma_load_2d_pair(st, &tmA, kt * BK, w.m0 + rank * BM, bar);
                     } else {
@@ -358,7 +329,7 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             tc_fence_before();
             if (PAIR) {
                 __syncwarp();
-                if (lane == 0) remote_arrive(mapa_shared(tempty(b), 0));
+                if (lane == 0) mbar_remote_arrive(mapa_shared(tempty(b), 0));
             } else {
                 mbar_arrive_cnt(tempty(b));
             }
